@@ -81,6 +81,41 @@ def test_ntt_arbitrary_generator_exact_network(zk, curve):
             assert np.array_equal(dropin(zk, curve, inv, m, gen, x), Z.oracle_ntt(curve, m, gen, x, inv)), (m, inv)
 
 
+@pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("m", (14, 17, 18, 19, 21))
+def test_ntt_matrix_form_digit_splits(zk, curve, m):
+    """the matrix form's group and digit splits (4 4|3 3 3, 4 3 3, 4 4 3, one and two outputs groups a
+    CTA), for a generator that is no root of unity, elements at both ends of the range among them"""
+    x = Z.rand_fr(curve, 1 << m, 14100 + m)
+    x[::7] = Z.to_limbs(Z.R[curve] - 1, 4)
+    x[3::11] = 0
+    gen = Z.rand_fr(curve, 1, 14200 + m)[0]
+    zk.lib().zkg_set_ntt_kmax(0)   # no explicit pass size: the matrix form
+    for inv in (False, True):
+        assert np.array_equal(dropin(zk, curve, inv, m, gen, x), Z.oracle_ntt(curve, m, gen, x, inv)), inv
+
+
+@pytest.mark.parametrize("curve", Z.CURVES)
+def test_ntt_matrix_form_three_groups_match_tile_form(zk, curve):
+    """2^25 elements: two twiddle boundaries; the register-tile form (an explicit largest pass) computes
+    the same network"""
+    import torch
+    m = 25
+    x = torch.randint(0, 256, (32 << m,), dtype=torch.uint8, device="cuda").view(torch.int64).view(1 << m, 4)
+    x[:, 3] &= (1 << 61) - 1
+    gen = Z.rand_fr(curve, 1, 14300)[0]
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    zk.lib().zkg_set_ntt_kmax(0)
+    for inv in (False, True):
+        zk.ntt_device(curve, m, x, y, inverse=inv, gen=gen)
+        zk.lib().zkg_set_ntt_kmax(8)
+        try:
+            zk.ntt_device(curve, m, x, z, inverse=inv, gen=gen)
+        finally:
+            zk.lib().zkg_set_ntt_kmax(0)
+        assert torch.equal(y, z), inv
+
+
 def test_ntt_bn254_2pow20_vs_oracle(zk):
     m = 20
     x = Z.rand_fr(Z.BN254, 1 << m, 14000)

@@ -1722,7 +1722,8 @@ struct zkg_batch {
   std::vector<Ntt> ntts;
   bool built = false;
   zkb::MultiPlan mp;
-  std::vector<zkb::NttPlan*> plans;
+  std::vector<zkb::NttPlan*> plans;       // per NTT; transforms of one size, generator and direction share one
+  std::vector<zkb::NttPlan*> own_plans;   // each plan once
   void* ws = nullptr;           // device workspace (MSM pipeline + NTT scratch)
   size_t conv_off = 0;          // bases in the FP64 pipeline's radix (inside ws), 0 = integer pipeline
   uint32_t conv_n = 0;          // bases converted per run (largest request)
@@ -1747,7 +1748,7 @@ struct zkg_batch {
   ~zkg_batch() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    for (auto p : plans) delete p;
+    for (auto p : own_plans) delete p;
     if (ws) cudaFree(ws);
     if (pin) cudaFreeHost(pin);
     for (auto s : s_ntt) cudaStreamDestroy(s);
@@ -1760,6 +1761,22 @@ struct zkg_batch {
 
 namespace zkb {
 
+// The plan of NTT i of the batch: an earlier transform's, when size, generator and direction agree.
+static zkg_status batch_plan(zkg_batch* b, size_t i, bool tiles) {
+  const auto& t = b->ntts[i];
+  NttPlan* pl = nullptr;
+  for (size_t j = 0; j < i && !pl; j++) {
+    const auto& o = b->ntts[j];
+    if (o.m == t.m && o.inverse == t.inverse && std::memcmp(o.gen, t.gen, 32) == 0) pl = b->plans[j];
+  }
+  if (!pl) {
+    ZKB_TRY(ntt_plan_new(b->curve, t.m, t.gen, t.inverse, 0, b->s_main, &pl, tiles));
+    b->own_plans.push_back(pl);
+  }
+  b->plans.push_back(pl);
+  return ZKG_OK;
+}
+
 // Persistent-kernel form of a batch (FP64 pipelines): one graph of the MSM sort launches, one
 // k_batch_work launch (accumulation + all NTT passes), then the MSM merge / fold / reduction.
 template <class C, int NL>
@@ -1771,10 +1788,8 @@ static zkg_status batch_build_persistent(zkg_batch* b, const host::Field<NL>& F)
   ZKB_TRY(make_multi_plan<CD>(ns, sc, b->mp));
   ZKB_CUDA(cudaStreamCreateWithFlags(&b->s_main, cudaStreamNonBlocking));
   for (size_t i = 0; i < b->ntts.size(); i++) {
-    NttPlan* pl = nullptr;
-    ZKB_TRY(ntt_plan_new(b->curve, b->ntts[i].m, b->ntts[i].gen, b->ntts[i].inverse, 0, b->s_main, &pl));
-    b->plans.push_back(pl);
-    if (!pl->dpf) return set_status(ZKG_ERR_UNSUPPORTED, "batch", "persistent mode needs FP64 NTT plans");
+    ZKB_TRY(batch_plan(b, i, true));
+    if (!b->plans[i]->dpf) return set_status(ZKG_ERR_UNSUPPORTED, "batch", "persistent mode needs FP64 NTT plans");
   }
   auto rup = [](size_t x) { return (x + 255) & ~size_t(255); };
   size_t total = rup(b->mp.bytes);
@@ -1969,9 +1984,7 @@ static zkg_status batch_build(zkg_batch* b, const host::Field<NL>& F) {
   }
   std::vector<size_t> maxN(nstreams, 0);
   for (size_t i = 0; i < b->ntts.size(); i++) {
-    NttPlan* pl = nullptr;
-    ZKB_TRY(ntt_plan_new(b->curve, b->ntts[i].m, b->ntts[i].gen, b->ntts[i].inverse, 0, b->s_main, &pl));
-    b->plans.push_back(pl);
+    ZKB_TRY(batch_plan(b, i, false));
     maxN[i % nstreams] = std::max(maxN[i % nstreams], (size_t)1 << b->ntts[i].m);
   }
   size_t total = (b->mp.bytes + 255) & ~size_t(255);
@@ -2067,6 +2080,7 @@ static zkg_status batch_run(zkg_batch* b, const host::Field<NL>& F) {
     std::memcpy(&err, static_cast<const char*>(b->pin) + b->err_pin_off, 4);
     if (err) return set_status(ZKG_ERR_TIMEOUT, "zkg_batch_run", "an NTT pass waited too long for its input");
   }
+  for (NttPlan* pl : b->own_plans) ZKB_TRY(ntt_plan_fault(*pl));
   std::vector<uint64_t*> outs;
   std::vector<int> kinds;
   for (auto& m : b->msms) { outs.push_back(m.out); kinds.push_back(m.kind); }
@@ -2244,9 +2258,10 @@ static void srv_loop(Srv* S, const host::Field<NL>* F) {
       if (!sl.busy || sl.finishing) continue;
       const cudaError_t q = cudaEventQuery(sl.done);
       if (q == cudaErrorNotReady) continue;
-      if (q != cudaSuccess) {   // the device reported an error for this request's work
+      const zkg_status nf = q == cudaSuccess ? ntt_plan_fault(*S->plans[sl.req.k]) : ZKG_OK;
+      if (q != cudaSuccess || nf != ZKG_OK) {   // the device reported an error for this request's work
         (void)cudaGetLastError();
-        if (S->error == ZKG_OK) S->error = set_status(ZKG_ERR_CUDA, "server", cudaGetErrorString(q));
+        if (S->error == ZKG_OK) S->error = nf != ZKG_OK ? nf : set_status(ZKG_ERR_CUDA, "server", cudaGetErrorString(q));
         S->results[sl.req.ticket] = {true, -1.0};
         srv_free(*S, sl.off, sl.bytes);
         sl.busy = false;

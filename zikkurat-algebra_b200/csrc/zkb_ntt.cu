@@ -23,6 +23,7 @@
 // 32-byte elements. The tile lives in shared memory; each thread runs 3 butterfly stages at a
 // time on 8 elements held in registers.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <cstdlib>
 #include <vector>
@@ -92,16 +93,176 @@ static zkg_status upload(uint32_t** dst, const std::vector<host::El<4>>& v) {
   return ZKG_OK;
 }
 
+// Passes as matrix products (zkb_ntt_mat.cuh); ZKB_NTT_MAT=0 keeps the register form
+static int g_ntt_mat = [] {
+  const char* v = std::getenv("ZKB_NTT_MAT");
+  return v ? std::atoi(v) : 1;
+}();
+// The matrix form needs 128 columns that share a matrix, so two groups of at least 7 bits. An
+// explicit largest pass (zkg_set_ntt_kmax) and the integer products (ZKB_NTT_DPF=0) name the
+// register form.
+static constexpr int NTT_MAT_MMIN = 14;
+static bool ntt_use_mat(int m) { return g_ntt_mat && g_ntt_dpf && !g_ntt_kmax_set && m >= NTT_MAT_MMIN; }
+
+// Bits of the groups (7 to 12 each, two up to 2^24, three above): the fewest passes, then the
+// smallest matrices. A group of G bits runs ceil(G / 4) passes of 4 and 3 bits, the 4s first.
+static std::vector<int> ntt_mat_digits(int G) {
+  const int np = (G + 3) / 4;
+  std::vector<int> d(np, 3);
+  for (int i = 0; i < G - 3 * np; i++) d[i] = 4;
+  return d;
+}
+static std::vector<int> ntt_mat_groups(int m) {
+  auto cost = [](int G) {
+    double bytes = 0;
+    int u = 0;
+    for (int k : ntt_mat_digits(G)) { bytes += std::ldexp(1024.0, 2 * k + u); u += k; }
+    return (double)((G + 3) / 4) * 1e12 + bytes;
+  };
+  std::vector<int> best;
+  double bc = 1e300;
+  for (int a = 7; a <= 12; a++)
+    for (int b = 7; b <= 12; b++) {
+      const int c = m - a - b;
+      if (m <= 24 ? c != 0 : (c < 7 || c > 12)) continue;
+      const double t = cost(a) + cost(b) + (c ? cost(c) : 0.0);
+      if (t < bc) {
+        bc = t;
+        best = {a, b};
+        if (c) best.push_back(c);
+      }
+    }
+  return best;
+}
+
+// y[k1] = sum_t F[k1][t] x[t]: the 2^k-point decimation-in-time network with twiddles w^j
+static std::vector<host::El<4>> net_apply(const host::Field<4>& F, std::vector<host::El<4>> x, host::El<4> w) {
+  const size_t n = x.size();
+  if (n == 1) return x;
+  std::vector<host::El<4>> e(n / 2), o(n / 2), y(n);
+  for (size_t i = 0; i < n / 2; i++) { e[i] = x[2 * i]; o[i] = x[2 * i + 1]; }
+  e = net_apply(F, e, host::mul(F, w, w));
+  o = net_apply(F, o, host::mul(F, w, w));
+  host::El<4> p = host::one(F);
+  for (size_t j = 0; j < n / 2; j++) {
+    const host::El<4> t = host::mul(F, o[j], p);
+    y[j] = host::add(F, e[j], t);
+    y[j + n / 2] = host::sub(F, e[j], t);
+    p = host::mul(F, p, w);
+  }
+  return y;
+}
+
+static host::El<4> pow_2k(const host::Field<4>& F, host::El<4> x, int k) {
+  for (int i = 0; i < k; i++) x = host::mul(F, x, x);
+  return x;
+}
+
+// Matrices and group twiddles of a matrix-form plan; h is the network's generator, scale the
+// inverse's (1/2)^m, folded into the first pass's matrix. One device block holds everything, filled
+// from one upload of network matrices and powers (a batch builds a plan per transform: separate
+// allocations made its first run a third longer).
+template <class P>
+static zkg_status build_mat(const host::Field<4>& F, NttPlan* pl, const host::El<4>& h, const host::El<4>& scale,
+                            const host::El<4>& rp, cudaStream_t st) {
+  const int m = pl->m;
+  const std::vector<int> groups = ntt_mat_groups(m);
+  const int sms = device_sm_count();
+  pl->mat = true;
+  ZKB_CUDA(cudaHostAlloc(&pl->h_fault, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+  *pl->h_fault = 0;
+  std::vector<host::El<4>> hv;   // what the build kernels read
+  auto powers = [&](size_t n, const host::El<4>& x0, const host::El<4>& g) {
+    const size_t at = hv.size();
+    host::El<4> x = x0;
+    for (size_t i = 0; i < n; i++) { hv.push_back(x); x = host::mul(F, x, g); }
+    return at;
+  };
+  size_t bytes = 0;
+  auto take = [&](size_t n) { const size_t o = bytes; bytes += (n + 1023) & ~size_t(1023); return o; };
+  struct Src { size_t net, pw, dst; };
+  std::vector<Src> src;               // per pass, forward order
+  std::vector<NttMatPass> fwd;
+  size_t gtw[2] = {0, 0};
+  int s = 0;
+  for (size_t gi = 0; gi < groups.size(); gi++) {
+    const int S = s;
+    const std::vector<int> digits = ntt_mat_digits(groups[gi]);
+    for (size_t di = 0; di < digits.size(); di++) {
+      NttMatPass q = {};
+      q.k = digits[di];
+      q.s = s;
+      q.Mp = m - s - q.k;
+      q.S = S;
+      q.u = s - S;
+      const int R = 1 << q.k;
+      // half the outputs per CTA when a whole set of them leaves SMs idle
+      q.nout = (1 << (m - q.k - 7)) * (R / 8) < sms ? 4 : 8;
+      q.tw = -1;
+      const size_t b = pl->inverse ? gi - 1 : gi;   // the boundary this pass's outputs cross, if any
+      if (pl->inverse ? (di == 0 && gi > 0) : (di + 1 == digits.size() && gi + 1 < groups.size())) {
+        q.tw = (int)b;
+        q.tw_S = 0;
+        for (size_t j = 0; j < b; j++) q.tw_S += groups[j];
+      }
+      Src f;
+      f.net = hv.size();
+      hv.resize(f.net + (size_t)R * R);
+      const host::El<4> w = pow_2k(F, h, m - q.k);
+      for (int t = 0; t < R; t++) {
+        std::vector<host::El<4>> x(R, host::zero<4>());
+        x[t] = s == 0 && pl->inverse ? scale : host::one(F);
+        x = net_apply(F, x, w);
+        for (int k1 = 0; k1 < R; k1++) hv[f.net + (size_t)k1 * R + t] = x[k1];
+      }
+      f.pw = powers((size_t)1 << (q.k + q.u), host::one(F), pow_2k(F, h, S + q.Mp));
+      f.dst = take((size_t)1024 << (2 * q.k + q.u));
+      src.push_back(f);
+      fwd.push_back(q);
+      pl->passes.push_back({q.k, q.s, q.Mp});
+      s += q.k;
+    }
+    if (gi + 1 < groups.size()) gtw[gi] = take((size_t)32 << (m - S));
+  }
+  // powers for the twiddles: h^e = A[e mod 2^a] B[e >> a], both in FP64 radix (x R -> x R')
+  const int a = (m + 1) / 2;
+  const size_t A = powers((size_t)1 << a, rp, h), B = powers((size_t)1 << (m - a), rp, pow_2k(F, h, a));
+  const size_t o_hv = take(hv.size() * 32);
+  if (cudaMalloc(&pl->d_mblk, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    pl->d_mblk = nullptr;
+    return set_status(ZKG_ERR_NOMEM, "ntt plan", "matrices");
+  }
+  pl->bytes = bytes;
+  char* base = static_cast<char*>(pl->d_mblk);
+  const uint32_t* dh = reinterpret_cast<const uint32_t*>(base + o_hv);
+  ZKB_CUDA(cudaMemcpyAsync(base + o_hv, hv.data(), hv.size() * 32, cudaMemcpyHostToDevice, st));
+  for (size_t i = 0; i < fwd.size(); i++) {
+    NttMatPass& q = fwd[i];
+    q.d_mat = reinterpret_cast<uint8_t*>(base + src[i].dst);
+    ZKB_TRY(ntt_mat_build<P>(dh + src[i].net * 8, dh + src[i].pw * 8, q.k, q.u, pl->inverse, q.nout, q.d_mat, st));
+  }
+  s = 0;
+  for (size_t gi = 0; gi + 1 < groups.size(); gi++) {   // after group gi: h^((r kappa) << S)
+    pl->d_gtw[gi] = reinterpret_cast<uint32_t*>(base + gtw[gi]);
+    ZKB_TRY(ntt_mat_twiddles<P>(pl->d_gtw[gi], dh + A * 8, dh + B * 8, a, m - s - groups[gi], s, 1u << (m - s), st));
+    s += groups[gi];
+  }
+  if (pl->inverse) std::reverse(fwd.begin(), fwd.end());
+  pl->mpasses = fwd;
+  ZKB_CUDA(cudaStreamSynchronize(st));
+  return ZKG_OK;
+}
+
 template <class P>
 static zkg_status build_plan_uncached(const host::Field<4>& F, int curve, int m, const uint64_t* gen, int inverse,
-                                      int kmax, cudaStream_t stream, NttPlan** out) {
+                                      int kmax, bool mat, cudaStream_t stream, NttPlan** out) {
   NttPlan* pl = new NttPlan();
   pl->curve = curve;
   pl->m = m;
   pl->inverse = inverse;
   pl->kmax = kmax;
   std::memcpy(pl->gen, gen, 32);
-  pl->passes = ntt_schedule(m, kmax);
   pl->dpf = g_ntt_dpf != 0;
   // tables in radix R' when the passes multiply on the FP64 pipe: x R -> x R R' / R
   using PD = typename DpfOf<P>::type;
@@ -113,6 +274,20 @@ static zkg_status build_plan_uncached(const host::Field<4>& F, int curve, int m,
   };
   host::El<4> g = el_from_u64<4>(gen);
   host::El<4> h = inverse ? host::inv(F, g) : g;   // network generator
+  // (1/2)^m, the inverse's final scale (bn128_poly_mont.c:565-622 halves at every level)
+  host::El<4> scale = host::one(F);
+  if (inverse) {
+    host::El<4> two = host::zero<4>();
+    two.v[0] = 2;
+    scale = host::pow_u64(F, host::inv(F, host::from_std(F, two)), (uint64_t)m);
+  }
+  if (mat) {
+    const zkg_status st = build_mat<P>(F, pl, h, scale, rp, stream);
+    if (st != ZKG_OK) { delete pl; return st; }
+    *out = pl;
+    return ZKG_OK;
+  }
+  pl->passes = ntt_schedule(m, kmax);
   // small-network tables: w_k = h^(2^(m-k)), powers 0 .. 2^(k-1)-1
   for (const NttPass& q : pl->passes) {
     if (pl->d_om[q.k]) continue;
@@ -124,13 +299,6 @@ static zkg_status build_plan_uncached(const host::Field<4>& F, int curve, int m,
     conv(tab);
     zkg_status st = upload(&pl->d_om[q.k], tab);
     if (st != ZKG_OK) { delete pl; return st; }
-  }
-  // (1/2)^m, the inverse's final scale (bn128_poly_mont.c:565-622 halves at every level)
-  host::El<4> scale = host::one(F);
-  if (inverse) {
-    host::El<4> two = host::zero<4>();
-    two.v[0] = 2;
-    scale = host::pow_u64(F, host::inv(F, host::from_std(F, two)), (uint64_t)m);
   }
   if (pl->passes.size() >= 2) {
     const uint32_t N = 1u << m;
@@ -186,12 +354,12 @@ static zkg_status build_plan(Context& cx, const host::Field<4>& F, int curve, in
                              NttPlan** out) {
   for (NttPlan* p : cx.ntt_plans)
     if (p->curve == curve && p->m == m && p->inverse == inverse && p->kmax == effective_kmax(curve, m) &&
-        p->dpf == (g_ntt_dpf != 0) && std::memcmp(p->gen, gen, 32) == 0) {
+        p->dpf == (g_ntt_dpf != 0) && p->mat == ntt_use_mat(m) && std::memcmp(p->gen, gen, 32) == 0) {
       *out = p;
       return ZKG_OK;
     }
   NttPlan* pl = nullptr;
-  ZKB_TRY(build_plan_uncached<P>(F, curve, m, gen, inverse, effective_kmax(curve, m), cx.stream, &pl));
+  ZKB_TRY(build_plan_uncached<P>(F, curve, m, gen, inverse, effective_kmax(curve, m), ntt_use_mat(m), cx.stream, &pl));
   // bounded cache: drop the oldest plans beyond 64 plans or 4 GiB of tables (a 2^24 forward and
   // inverse pair holds 1.5 GiB)
   cx.ntt_plans.push_back(pl);
@@ -223,7 +391,8 @@ static zkg_status ntt_run(Context& cx, const NttPlan& pl, const uint32_t* d_src,
     // the i-th executed pass writes tgt when (np-1-i) is even, scratch otherwise
     uint32_t* out = ((np - 1 - i) % 2 == 0) ? d_tgt : scratch;
     const NttPass& q = pl.inverse ? pl.passes[np - 1 - i] : pl.passes[i];
-    if (pl.dpf) ZKB_TRY(ntt_launch_pass<typename DpfOf<P>::type>(pl, q, in, out, pl.inverse && i == np - 1, st));
+    if (pl.mat) ZKB_TRY(ntt_mat_launch_pass<P>(pl, i, in, out, cx.sm_count, st));
+    else if (pl.dpf) ZKB_TRY(ntt_launch_pass<typename DpfOf<P>::type>(pl, q, in, out, pl.inverse && i == np - 1, st));
     else ZKB_TRY(ntt_launch_pass<P>(pl, q, in, out, pl.inverse && i == np - 1, st));
     in = out;
   }
@@ -270,6 +439,7 @@ static zkg_status ntt_entry(const host::Field<4>& F, int curve, int m, const uin
     ZKB_TRY(copy_d2h(cx, tgt, d_tgt, bytes, st));
   }
   ZKB_CUDA(cudaEventElapsedTime(&cx.last_kernel_ms, cx.ev_a, cx.ev_b));
+  ZKB_TRY(ntt_plan_fault(*pl));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
 
@@ -351,6 +521,7 @@ static zkg_status ntt_shifted_entry(const host::Field<4>& F, int curve, const ui
   ZKB_CUDA(cudaEventRecord(cx.ev_b, st));
   ZKB_TRY(copy_d2h(cx, tgt, d_c, bytes, st));
   ZKB_CUDA(cudaEventElapsedTime(&cx.last_kernel_ms, cx.ev_a, cx.ev_b));
+  ZKB_TRY(ntt_plan_fault(*pl));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
 
@@ -403,16 +574,25 @@ static zkg_status ntt_asym_entry(const host::Field<4>& F, int curve, int m_src, 
   ZKB_CUDA(cudaEventRecord(cx.ev_b, st));
   ZKB_TRY(copy_d2h(cx, tgt, d_tgt, bt, st));
   ZKB_CUDA(cudaEventElapsedTime(&cx.last_kernel_ms, cx.ev_a, cx.ev_b));
+  ZKB_TRY(ntt_plan_fault(*pl));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
 
 zkg_status ntt_plan_new(int curve, int m, const uint64_t* gen, int inverse, int kmax, cudaStream_t st,
-                        NttPlan** out) {
+                        NttPlan** out, bool tiles) {
   if (m < 0 || m > NTT_MMAX) return set_status(ZKG_ERR_ARG, "ntt", "m out of range [0, 30]");
+  const bool mat = !tiles && kmax <= 0 && ntt_use_mat(m);
   if (kmax <= 0) kmax = effective_kmax(curve, m);
-  if (curve == ZKG_BN254) return build_plan_uncached<BnFr>(host::BN_FR, curve, m, gen, inverse, kmax, st, out);
-  if (curve == ZKG_BLS12_381) return build_plan_uncached<BlsFr>(host::BLS_FR, curve, m, gen, inverse, kmax, st, out);
+  if (curve == ZKG_BN254) return build_plan_uncached<BnFr>(host::BN_FR, curve, m, gen, inverse, kmax, mat, st, out);
+  if (curve == ZKG_BLS12_381) return build_plan_uncached<BlsFr>(host::BLS_FR, curve, m, gen, inverse, kmax, mat, st, out);
   return set_status(ZKG_ERR_ARG, "ntt", "unknown curve");
+}
+
+zkg_status ntt_plan_fault(const NttPlan& pl) {
+  volatile uint32_t* w = pl.h_fault;
+  if (!w || !*w) return ZKG_OK;
+  *w = 0;
+  return set_status(ZKG_ERR_TIMEOUT, "ntt", "a bounded wait inside a pass ran out");
 }
 
 zkg_status ntt_plan_execute(const NttPlan& pl, const uint32_t* d_src, uint32_t* d_tgt, uint32_t* scratch,

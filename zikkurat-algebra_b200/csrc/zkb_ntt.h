@@ -21,6 +21,15 @@ struct NttPass {
   int k, s, Mp;   // bits in this pass, bits before it, bits after it (forward order)
 };
 
+// One pass of the matrix form (zkb_ntt_mat.cuh), in execution order.
+struct NttMatPass {
+  int k, s, Mp;            // as NttPass
+  int S, u;                // bits before the pass's group, bits of the group before the pass
+  int nout;                // outputs per CTA
+  uint8_t* d_mat;          // 2^u matrices
+  int tw, tw_S;            // group twiddles applied to the outputs (-1: none); bits before that group
+};
+
 struct NttPlan {
   int curve = -1, m = -1, inverse = 0, kmax = 0;
   bool dpf = false;                  // tables in radix R' = 2^260: passes multiply on the FP64 pipe
@@ -30,8 +39,15 @@ struct NttPlan {
   uint32_t* d_tw_last = nullptr;     // inverse with >= 2 passes: d_tw times (1/2)^m, for the last pass
   uint32_t* d_om[NTT_KMAX + 1] = {nullptr};
   uint32_t* d_scale = nullptr;       // (1/2)^m for the inverse
+  bool mat = false;                  // matrix form: mpasses and d_gtw instead of d_tw and d_om
+  std::vector<NttMatPass> mpasses;
+  uint32_t* d_gtw[2] = {nullptr};    // twiddles between the groups, in position order
+  void* d_mblk = nullptr;            // the device block both lie in
+  uint32_t* h_fault = nullptr;       // host-mapped word, set by a pass whose bounded wait ran out
   size_t bytes = 0;
   ~NttPlan() {
+    if (d_mblk) cudaFree(d_mblk);
+    if (h_fault) cudaFreeHost(h_fault);
     if (d_tw) cudaFree(d_tw);
     if (d_tw_last) cudaFree(d_tw_last);
     for (auto p : d_om) if (p) cudaFree(p);
@@ -47,10 +63,26 @@ zkg_status ntt_launch_pass(const NttPlan& pl, const NttPass& q, const uint32_t* 
 template <class P>
 zkg_status ntt_launch_table(uint32_t* T, const uint32_t* A, const uint32_t* Bt, int a, uint32_t N, cudaStream_t st);
 
+// The matrix form (defined per field): pass `exec` of the plan's mpasses; one pass's matrices from
+// its network matrix and the powers of its fold base; a group boundary's twiddles in FP64 radix.
+template <class P>
+zkg_status ntt_mat_launch_pass(const NttPlan& pl, int exec, const uint32_t* in, uint32_t* out, int sms,
+                               cudaStream_t st);
+template <class P>
+zkg_status ntt_mat_build(const uint32_t* net, const uint32_t* pw, int k, int u, int inverse, int nout, uint8_t* dst,
+                         cudaStream_t st);
+template <class P>
+zkg_status ntt_mat_twiddles(uint32_t* T, const uint32_t* A, const uint32_t* B, int a, int lo, int S, uint32_t n,
+                            cudaStream_t st);
+
 // A plan owned by the caller (not entered in the context's cache): for batches and servers that
-// keep plans alive across graph replays. Built synchronously on stream st.
+// keep plans alive across graph replays. Built synchronously on stream st. tiles: the register form
+// whatever the size (the batch's persistent kernel runs its tiles).
 zkg_status ntt_plan_new(int curve, int m, const uint64_t* gen, int inverse, int kmax, cudaStream_t st,
-                        NttPlan** out);
+                        NttPlan** out, bool tiles = false);
+// ZKG_ERR_TIMEOUT (and the plan's word cleared) when a bounded wait inside one of its passes ran
+// out; to be called once the plan's work has finished.
+zkg_status ntt_plan_fault(const NttPlan& pl);
 // Runs a plan d_src -> d_tgt on stream st; scratch (2^m elements) is needed with >= 2 passes.
 zkg_status ntt_plan_execute(const NttPlan& pl, const uint32_t* d_src, uint32_t* d_tgt, uint32_t* scratch,
                             cudaStream_t st);
