@@ -224,6 +224,23 @@ def test_msm_skewed_digit_distribution(zk, curve):
 
 
 @pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("n", [33, 1023, 1024, 1025, 9000])
+def test_msm_small_sizes_any_distribution(zk, curve, n):
+    """the small sort and the quad accumulation at the edges of their ranges, with segments from empty to
+    all points long (long ones are summed in pieces), null entries and bases at infinity"""
+    rng = np.random.default_rng(n)
+    ks = Z.rand_fr(curve, n, 7100 + n)
+    few = ks[rng.integers(0, 3, n)]
+    sparse = ks * (rng.integers(0, 50, n) == 0)[:, None].astype(np.uint64)
+    bases = Z.gen_bases_cpu(curve, Z.rand_fr(curve, n, 7200 + n)).reshape(n, -1)
+    bases[5::17] = 0
+    for name, sc in (("random", ks), ("equal", np.tile(ks[0], (n, 1))), ("few", few), ("sparse", sparse)):
+        for coeff, mont in (("mont", True), ("std", False)):
+            got = call(zk, curve, "proj", coeff, "affine", sc, 4, bases)
+            assert np.array_equal(got, Z.oracle_msm_affine(curve, sc, 4, mont, bases)), (name, coeff)
+
+
+@pytest.mark.parametrize("curve", Z.CURVES)
 def test_msm_deterministic_and_consistent_outputs(zk, curve):
     n = 20000
     ks = Z.rand_fr(curve, n, 24000)

@@ -20,16 +20,13 @@
 //                    memory by cp.async) into an XYZZ accumulator, products on the FP64 pipe
 //                    (zkb_dpf.cuh). Complete segments go straight to the bucket array;
 //                    segments cut by a chunk boundary leave partial sums in slots.
-//   6. merge, fold   a segment cut across at most 9 chunks is summed from its slots by one
-//                    thread (nearly every cut segment at large n spans two); longer ones are
-//                    folded by levels, again in equal chunks, so any digit distribution is
-//                    load balanced.
+//   6. merge         a segment cut by chunk boundaries is summed from its slots (zkb_msm_tail.cuh);
+//                    a long one (any digit distribution) in pieces, a block a piece. MSMs of few
+//                    entries skip chunks altogether: four lanes sum one segment
 //   7. bucket reduce (the point-range parts of a host-buffer MSM summed first, in one parallel
 //                    pass) per (window, group of K buckets) running sums (T_g, R_g), then per
-//                    window the plain sums U_R = sum R_g and U_k = sum_{g: bit k of g} T_g,
-//                    so that sum_b b*S_b = U_R + K * sum_k 2^k U_k needs no doublings on
-//                    the GPU
-//   8. host tail     Horner over windows and bits, normalisation, output encoding.
+//                    window sum_b b*S_b = sum R_g + K * sum_k 2^k sum_{g: bit k of g} T_g
+//   8. host tail     Horner over windows, normalisation, output encoding.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -48,18 +45,13 @@
 #include "zkb_ntt.h"
 #include "zkb_batch_work.h"
 #include "zkb_msm_accum.cuh"
+#include "zkb_msm_tail.cuh"
 #include "zkb_msm_tree.cuh"
 #include "zkb_runtime.h"
 
 namespace zkb {
 
-static constexpr int MAX_LEVELS = 12;
 static constexpr int MAX_TREE = 8;   // affine tree levels (zkb_msm_tree.cuh)
-
-struct LevelHist {
-  int n;
-  uint32_t L[MAX_LEVELS];
-};
 
 // ------------------------------------------------------------------------ scalar handling
 
@@ -82,15 +74,16 @@ __device__ __forceinline__ uint32_t scalar_bits(const uint32_t* __restrict__ w, 
   return (uint32_t)(((lo | (hi << 32)) >> sh) & ((1ull << c) - 1));
 }
 
-// signed digit for window `win` given the running carry; returns bucket (0 = none)
-__device__ __forceinline__ uint32_t next_digit(const uint32_t* w, int nw, int win, int c,
+// signed digit of the next window (`width` bits from bit `bit` on) given the running carry; returns
+// its bucket (0 = none)
+__device__ __forceinline__ uint32_t next_digit(const uint32_t* w, int nw, int bit, int width,
                                                uint32_t& carry, uint32_t& neg) {
-  const uint32_t raw = scalar_bits(w, nw, win * c, c) + carry;
-  const uint32_t half = 1u << (c - 1);
+  const uint32_t raw = scalar_bits(w, nw, bit, width) + carry;
+  const uint32_t half = 1u << (width - 1);
   if (raw > half) {
     carry = 1;
     neg = 1;
-    return (1u << c) - raw;
+    return (1u << width) - raw;
   }
   carry = 0;
   neg = 0;
@@ -101,30 +94,52 @@ __device__ __forceinline__ uint32_t next_digit(const uint32_t* w, int nw, int wi
 // entry), for k_msm_scatter_d
 // rank (with dig): the entry's position within its (window, bucket) segment, the value its count
 // increment returned, so the scatter needs no atomics
-__global__ void k_msm_hist(int n, const uint32_t* __restrict__ scal, int nw, int c, int nwin,
-                           uint32_t B, uint32_t* __restrict__ cnt, uint32_t* chk = nullptr,
+// Windows go HB at a time: their digits first, then their count increments, then the ranks these
+// returned, so a thread has HB increments in flight instead of waiting for each (1000 points: 20 -> 7 us).
+static constexpr int HB = 8;
+template <class Digit>
+__device__ __forceinline__ void hist_windows(int n, int i, int nwin, WinShape ws, uint32_t* __restrict__ cnt,
+                                             uint32_t* chk, uint32_t* __restrict__ dig, uint32_t* __restrict__ rank,
+                                             Digit digit) {
+  for (int w0 = 0; w0 < nwin; w0 += HB) {
+    uint32_t b[HB], r[HB];
+#pragma unroll
+    for (int j = 0; j < HB; j++) {
+      b[j] = 0;
+      if (w0 + j < nwin) {
+        uint32_t neg;
+        b[j] = digit(w0 + j, neg);
+        if (chk && b[j] > ws.buckets(w0 + j)) { atomicOr(chk, CHK_BUCKET); b[j] = 0; }
+        if (dig) dig[(size_t)(w0 + j) * n + i] = b[j] | (b[j] ? neg << 31 : 0u);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < HB; j++)
+      if (b[j]) r[j] = atomicAdd(cnt + ws.seg(w0 + j) + (b[j] - 1), 1u);
+    if (dig) {
+#pragma unroll
+      for (int j = 0; j < HB; j++)
+        if (b[j]) rank[(size_t)(w0 + j) * n + i] = r[j];
+    }
+  }
+}
+
+__global__ void k_msm_hist(int n, const uint32_t* __restrict__ scal, int nw, WinShape ws, int nwin,
+                           uint32_t* __restrict__ cnt, uint32_t* chk = nullptr,
                            uint32_t* __restrict__ dig = nullptr, uint32_t* __restrict__ rank = nullptr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t* w = scal + (size_t)nw * i;
-  uint32_t carry = 0, neg;
-  for (int win = 0; win < nwin; win++) {
-    uint32_t b = next_digit(w, nw, win, c, carry, neg);
-    if (chk && b > B) { atomicOr(chk, 1u); b = 0; }
-    if (dig) {
-      dig[(size_t)win * n + i] = b | (b ? neg << 31 : 0u);
-      if (b) rank[(size_t)win * n + i] = atomicAdd(cnt + (size_t)win * B + (b - 1), 1u);
-    } else if (b) {
-      atomicAdd(cnt + (size_t)win * B + (b - 1), 1u);
-    }
-  }
+  uint32_t carry = 0;
+  hist_windows(n, i, nwin, ws, cnt, chk, dig, rank,
+               [&](int win, uint32_t& neg) { return next_digit(w, nw, ws.start(win), ws.width(win), carry, neg); });
 }
 
 // The histogram for Montgomery Fr scalars with stored digits: each thread converts its scalar to
 // standard form in registers (the reference's to_std, bn128_G1_proj.c:638-642), so no standard
 // copy of the scalars is written or read back.
 template <class C>
-__global__ void k_msm_hist_mont(int n, const uint64_t* __restrict__ in, int c, int nwin, uint32_t B,
+__global__ void k_msm_hist_mont(int n, const uint64_t* __restrict__ in, WinShape ws, int nwin,
                                 uint32_t* __restrict__ cnt, uint32_t* chk, uint32_t* __restrict__ dig,
                                 uint32_t* __restrict__ rank) {
   using Fr = typename C::Fr;
@@ -132,29 +147,25 @@ __global__ void k_msm_hist_mont(int n, const uint64_t* __restrict__ in, int c, i
   if (i >= n) return;
   const Fe<Fr> sv = fe_from_mont(fe_load_nc<Fr>(reinterpret_cast<const uint32_t*>(in) + 8 * (size_t)i));
   uint32_t carry = 0;
-  const uint32_t half = 1u << (c - 1);
-  for (int win = 0; win < nwin; win++) {
-    const int bit = win * c, wi = bit >> 5, sh = bit & 31;
+  hist_windows(n, i, nwin, ws, cnt, chk, dig, rank, [&](int win, uint32_t& neg) {
+    const int bit = ws.start(win), width = ws.width(win), wi = bit >> 5, sh = bit & 31;
     uint64_t pair = 0;   // words wi, wi + 1 of the scalar (past the end: 0)
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       if (k == wi) pair |= sv.v[k];
       if (k == wi + 1) pair |= (uint64_t)sv.v[k] << 32;
     }
-    const uint32_t raw = (uint32_t)((pair >> sh) & ((1ull << c) - 1)) + carry;
-    const uint32_t neg = raw > half ? 1u : 0u;
+    const uint32_t raw = (uint32_t)((pair >> sh) & ((1ull << width) - 1)) + carry;
+    neg = raw > (1u << (width - 1)) ? 1u : 0u;
     carry = neg;
-    uint32_t b = neg ? (1u << c) - raw : raw;
-    if (chk && b > B) { atomicOr(chk, 1u); b = 0; }
-    dig[(size_t)win * n + i] = b | (b ? neg << 31 : 0u);
-    if (b) rank[(size_t)win * n + i] = atomicAdd(cnt + (size_t)win * B + (b - 1), 1u);
-  }
+    return neg ? (1u << width) - raw : raw;
+  });
 }
 
 // Window-major scatter from the stored digits and ranks (grid y = window): coalesced 4-byte reads
 // per (window, point), the entry's position = its segment's offset + its rank, no atomics
 __global__ void k_msm_scatter_d(int n, const uint32_t* __restrict__ dig, const uint32_t* __restrict__ rank,
-                                uint32_t B, const uint32_t* __restrict__ off, uint32_t* __restrict__ entries,
+                                WinShape ws, const uint32_t* __restrict__ off, uint32_t* __restrict__ entries,
                                 uint32_t* chk, uint32_t total) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int win = blockIdx.y;
@@ -162,31 +173,32 @@ __global__ void k_msm_scatter_d(int n, const uint32_t* __restrict__ dig, const u
   const uint32_t v = __ldg(dig + (size_t)win * n + i);
   const uint32_t b = v & 0x7fffffffu;
   if (b) {
-    const uint32_t pos = __ldg(off + (size_t)win * B + (b - 1)) + __ldg(rank + (size_t)win * n + i);
+    const uint32_t pos = __ldg(off + ws.seg(win) + (b - 1)) + __ldg(rank + (size_t)win * n + i);
     if (chk && pos >= total) { atomicOr(chk, CHK_ENTRY); return; }
     entries[pos] = (uint32_t)i | (v & 0x80000000u);
   }
 }
 
-__global__ void k_msm_scatter(int n, const uint32_t* __restrict__ scal, int nw, int c, int nwin,
-                              uint32_t B, uint32_t* __restrict__ cursor, uint32_t* __restrict__ entries) {
+__global__ void k_msm_scatter(int n, const uint32_t* __restrict__ scal, int nw, WinShape ws, int nwin,
+                              uint32_t* __restrict__ cursor, uint32_t* __restrict__ entries) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t* w = scal + (size_t)nw * i;
   uint32_t carry = 0, neg;
   for (int win = 0; win < nwin; win++) {
-    const uint32_t b = next_digit(w, nw, win, c, carry, neg);
+    const uint32_t b = next_digit(w, nw, ws.start(win), ws.width(win), carry, neg);
     if (b) {
-      const uint32_t pos = atomicAdd(cursor + (size_t)win * B + (b - 1), 1u);
+      const uint32_t pos = atomicAdd(cursor + ws.seg(win) + (b - 1), 1u);
       entries[pos] = (uint32_t)i | (neg << 31);
     }
   }
 }
 
 // Window-major digits. The carry into window w of the signed recoding above is a function of the
-// scalar's low w*c bits alone: with digits in (-2^(c-1), 2^(c-1)], the digits of windows below
-// w represent exactly the values in (-H_w + S_w - 2^(wc), H_w] with H_w = sum_{j<w} 2^(jc + c - 1)
-// and S_w = sum_{j<w} 2^(jc), so carry_w = [ (s mod 2^(wc)) > H_w ]. Each (window, point) digit is
+// scalar's low bits alone (those below the window's first, b_w): with digits in (-2^(c-1), 2^(c-1)] for
+// a window of c bits, the digits of windows below w represent exactly the values in
+// (-H_w + S_w - 2^(b_w), H_w] with H_w = sum_{j<w} 2^(b_j + c_j - 1) and S_w = sum_{j<w} 2^(b_j), so
+// carry_w = [ (s mod 2^(b_w)) > H_w ]. Each (window, point) digit is
 // then computed on its own, and the histogram and scatter run one window after another (grid y =
 // window): a window's 4-byte entries (n * 4 bytes) stay in L2 until their sectors are complete,
 // instead of all windows' entries being written at random over the whole array.
@@ -195,9 +207,8 @@ struct CarryTable {
   uint32_t h[HT_WORDS];   // word k of H_w at [w * nw + k]
 };
 
-__device__ __forceinline__ uint32_t carry_into(const uint32_t* __restrict__ w, int nw, int win, int c,
+__device__ __forceinline__ uint32_t carry_into(const uint32_t* __restrict__ w, int nw, int bits,
                                                const uint32_t* __restrict__ H) {
-  const int bits = win * c;
   if (bits == 0) return 0;
   const int top = min((bits - 1) >> 5, nw - 1);
   for (int k = top; k >= 0; k--) {
@@ -209,49 +220,50 @@ __device__ __forceinline__ uint32_t carry_into(const uint32_t* __restrict__ w, i
   return 0;
 }
 
-__device__ __forceinline__ uint32_t digit_at(const uint32_t* __restrict__ w, int nw, int win, int c,
+__device__ __forceinline__ uint32_t digit_at(const uint32_t* __restrict__ w, int nw, int win, WinShape ws,
                                              const CarryTable& T, uint32_t& neg) {
-  const uint32_t raw = scalar_bits(w, nw, win * c, c) + carry_into(w, nw, win, c, T.h + win * nw);
-  const uint32_t half = 1u << (c - 1);
+  const int width = ws.width(win);
+  const uint32_t raw = scalar_bits(w, nw, ws.start(win), width) + carry_into(w, nw, ws.start(win), T.h + win * nw);
+  const uint32_t half = 1u << (width - 1);
   neg = raw > half ? 1u : 0u;
-  return neg ? (1u << c) - raw : raw;
+  return neg ? (1u << width) - raw : raw;
 }
 
 // chk (device bounds checks, null = off): bucket b in [1, B], scatter position below `total`
-__global__ void k_msm_hist_w(int n, const uint32_t* __restrict__ scal, int nw, int c, uint32_t B, const CarryTable T,
+__global__ void k_msm_hist_w(int n, const uint32_t* __restrict__ scal, int nw, WinShape ws, const CarryTable T,
                              uint32_t* __restrict__ cnt, uint32_t* chk) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int win = blockIdx.y;
   if (i >= n) return;
   uint32_t neg;
-  const uint32_t b = digit_at(scal + (size_t)nw * i, nw, win, c, T, neg);
-  if (chk && b > B) { atomicOr(chk, CHK_BUCKET); return; }
-  if (b) atomicAdd(cnt + (size_t)win * B + (b - 1), 1u);
+  const uint32_t b = digit_at(scal + (size_t)nw * i, nw, win, ws, T, neg);
+  if (chk && b > ws.buckets(win)) { atomicOr(chk, CHK_BUCKET); return; }
+  if (b) atomicAdd(cnt + ws.seg(win) + (b - 1), 1u);
 }
 
-__global__ void k_msm_scatter_w(int n, const uint32_t* __restrict__ scal, int nw, int c, uint32_t B, const CarryTable T,
+__global__ void k_msm_scatter_w(int n, const uint32_t* __restrict__ scal, int nw, WinShape ws, const CarryTable T,
                                 uint32_t* __restrict__ cursor, uint32_t* __restrict__ entries, uint32_t* chk,
                                 uint32_t total) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int win = blockIdx.y;
   if (i >= n) return;
   uint32_t neg;
-  const uint32_t b = digit_at(scal + (size_t)nw * i, nw, win, c, T, neg);
-  if (chk && b > B) { atomicOr(chk, CHK_BUCKET); return; }
+  const uint32_t b = digit_at(scal + (size_t)nw * i, nw, win, ws, T, neg);
+  if (chk && b > ws.buckets(win)) { atomicOr(chk, CHK_BUCKET); return; }
   if (b) {
-    const uint32_t pos = atomicAdd(cursor + (size_t)win * B + (b - 1), 1u);
+    const uint32_t pos = atomicAdd(cursor + ws.seg(win) + (b - 1), 1u);
     if (chk && pos >= total) { atomicOr(chk, CHK_ENTRY); return; }
     entries[pos] = (uint32_t)i | (neg << 31);
   }
 }
 
 // H_w for every window (host side); false when the table does not fit CarryTable
-static bool make_carry_table(int nwin, int nw, int c, CarryTable& T) {
+static bool make_carry_table(int nwin, int nw, WinShape ws, CarryTable& T) {
   if ((size_t)nwin * nw > (size_t)HT_WORDS) return false;
   std::memset(T.h, 0, sizeof(T.h));
   for (int w = 0; w < nwin; w++)
     for (int j = 0; j < w; j++) {
-      const int bit = j * c + c - 1;
+      const int bit = ws.start(j) + ws.width(j) - 1;
       if ((bit >> 5) < nw) T.h[w * nw + (bit >> 5)] |= 1u << (bit & 31);
     }
   return true;
@@ -337,6 +349,115 @@ __global__ void k_scan_add(uint32_t* __restrict__ out, uint32_t* __restrict__ cu
   if (i == 0) out[n] = bsums[nb];
 }
 
+// The whole scan in one block (three launches took 11 us for 7 K counts). Loops kept rolled: a kernel
+// this short runs its instructions from a cold cache, and 32 unrolled loads took 12 us.
+static constexpr uint32_t SCAN_ONE = SCAN_T * 32;
+__global__ void __launch_bounds__(SCAN_T) k_scan_one(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                     uint32_t* __restrict__ cursor, uint32_t n) {
+  __shared__ uint32_t smw[32];
+  const uint32_t e = (n + SCAN_T - 1) / SCAN_T, lo = min(n, threadIdx.x * e), hi = min(n, lo + e);
+  uint32_t s = 0, total;
+#pragma unroll 4
+  for (uint32_t k = lo; k < hi; k++) s += in[k];
+  uint32_t pre = block_excl_scan(s, smw, total);
+#pragma unroll 4
+  for (uint32_t k = lo; k < hi; k++) {
+    const uint32_t v = in[k];
+    out[k] = pre;
+    cursor[k] = pre;
+    pre += v;
+  }
+  if (threadIdx.x == 0) out[n] = total;
+}
+
+// Exclusive prefix sum of n counts into out (and cursor); out[n] = the total. bs: block sums.
+static zkg_status scan_counts(const uint32_t* cnt, uint32_t* out, uint32_t* cursor, uint32_t* bs, uint32_t n,
+                              cudaStream_t st) {
+  if (n <= SCAN_ONE)
+    return launch("scan_one", k_scan_one, dim3(1), dim3(SCAN_T), 0, st, cnt, out, cursor, n);
+  const uint32_t nb = (n + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
+  ZKB_TRY(launch("scan_blocks", k_scan_blocks, dim3(nb), dim3(SCAN_T), 0, st, cnt, out, bs, n));
+  ZKB_TRY(launch("scan_top", k_scan_top, dim3(1), dim3(SCAN_T), 0, st, bs, nb));
+  return launch("scan_add", k_scan_add, dim3((n + 255) / 256), dim3(256), 0, st, out, cursor, (const uint32_t*)bs, n, nb);
+}
+
+// The sort of a small MSM, one block a window: digits (with bias = sum over windows of
+// (2^(width - 1) - 1) 2^start, the signed digit of any one window is its field of scalar + bias, less
+// 2^(width - 1) - 1; a standard-form scalar is recoded from its lowest window up to the block's), counts, their scan and the entries, all in shared memory, in place of a clear, the
+// histogram, the scan and the scatter (31 us and their launch gaps at 1000 points). Window w's entries
+// are [wn, (w + 1)n); points with digit 0 come last, as null entries of its last bucket.
+static constexpr int SMALL_N = 1024, SMALL_B = 4096, SMALL_W = 64, SMALL_T = 1024;
+static bool sort_small_fits(int n, int nwin, uint32_t B) {
+  return n <= SMALL_N && nwin <= SMALL_W && B <= (uint32_t)SMALL_B;
+}
+struct Bias { uint32_t v[8]; };
+static Bias digit_bias(const WinShape& ws, int nwin) {
+  uint32_t w[9] = {0};
+  for (int j = 0; j < nwin; j++)
+    for (int b = ws.start(j); b < ws.start(j) + ws.width(j) - 1; b++)
+      if (b < 256) w[b >> 5] |= 1u << (b & 31);
+  Bias r;
+  std::memcpy(r.v, w, sizeof(r.v));
+  return r;
+}
+template <class C, bool MONT>
+__global__ void __launch_bounds__(SMALL_T) k_sort_small(int n, const uint32_t* __restrict__ scal, int nw, WinShape ws,
+                                                        const Bias bias, uint32_t nseg, uint32_t* __restrict__ off,
+                                                        uint32_t* __restrict__ entries, uint32_t* __restrict__ nonzero) {
+  using Fr = typename C::Fr;
+  static_assert(SMALL_N == SMALL_T, "one point a thread");
+  __shared__ uint32_t cnt[SMALL_B + 1], smw[32];
+  const int win = blockIdx.x, i = threadIdx.x;
+  const uint32_t B = ws.buckets(win);
+  for (uint32_t b = threadIdx.x; b <= B; b += SMALL_T) cnt[b] = 0;
+  __syncthreads();
+  uint32_t b = B, neg = 0, rank = 0;   // bucket; B (after the last): digit 0
+  if (i < n) {
+    uint32_t d = 0;
+    if constexpr (MONT) {
+      Fe<Fr> sv = fe_from_mont(fe_load_nc<Fr>(scal + 8 * (size_t)i));
+      sv.v[0] = add_cc(sv.v[0], bias.v[0]);
+#pragma unroll
+      for (int k = 1; k < 7; k++) sv.v[k] = addc_cc(sv.v[k], bias.v[k]);
+      sv.v[7] = addc(sv.v[7], bias.v[7]);
+      const int bit = ws.start(win), width = ws.width(win), wi = bit >> 5;
+      uint64_t pair = 0;   // words wi, wi + 1 (past the end: 0)
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        if (k == wi) pair |= sv.v[k];
+        if (k == wi + 1) pair |= (uint64_t)sv.v[k] << 32;
+      }
+      const int v = (int)((pair >> (bit & 31)) & ((1ull << width) - 1)) - (int)((1u << (width - 1)) - 1);
+      neg = v < 0;
+      d = (uint32_t)(v < 0 ? -v : v);
+    } else {
+      uint32_t carry = 0;
+      for (int w = 0; w <= win; w++) d = next_digit(scal + (size_t)nw * i, nw, ws.start(w), ws.width(w), carry, neg);
+    }
+    if (d) b = d - 1;
+    rank = atomicAdd(cnt + b, 1u);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) atomicAdd(nonzero, (uint32_t)n - cnt[B]);
+  const uint32_t e = (B + SMALL_T - 1) / SMALL_T, lo = min(B, threadIdx.x * e), hi = min(B, lo + e);
+  uint32_t s = 0, total;
+  for (uint32_t k = lo; k < hi; k++) s += cnt[k];
+  uint32_t pre = block_excl_scan(s, smw, total);
+  for (uint32_t k = lo; k < hi; k++) {
+    const uint32_t c = cnt[k];
+    cnt[k] = pre;
+    off[ws.seg(win) + k] = (uint32_t)(win * n) + pre;
+    pre += c;
+  }
+  __syncthreads();   // thread 0 read cnt[B] above
+  if (threadIdx.x == 0) {
+    cnt[B] = total;
+    if (win == (int)gridDim.x - 1) off[nseg] = gridDim.x * (uint32_t)n;
+  }
+  __syncthreads();
+  if (i < n) entries[(size_t)win * n + cnt[b] + rank] = b == B ? NULL_ENTRY : (uint32_t)i | (neg << 31);
+}
+
 // ------------------------------------------------------------------ bucket accumulation
 // (accum_block and its helpers: zkb_msm_accum.cuh)
 
@@ -362,37 +483,6 @@ __global__ void __launch_bounds__(NT, 1) k_msm_accum_w(const uint32_t* __restric
                                                        uint32_t* __restrict__ spt, uint32_t* chk, uint32_t npts) {
   extern __shared__ uint4 pf_dyn[];
   accum_block<C, PF, NT>(blockIdx.x, entries, off, nseg, nchunks, L, bases, bsum, skey, spt, pf_dyn, chk, npts);
-}
-
-// Cut segments that span at most RUN_MAX + 1 level-1 chunks (with ~64-entry segments and
-// ~128-entry chunks, nearly every cut segment spans two) are summed here into the bucket array,
-// one thread per segment start, and their slots are cleared, so the fold levels only carry
-// longer segments. A cut segment s starting in chunk t leaves its B partial in slot 2t + 1 and
-// the A partial of every later chunk it reaches in slot 2t' (a chunk inside s routes its whole
-// sum as A); it ends in chunk (off[s + 1] - 1) / L.
-static constexpr uint32_t RUN_MAX = 8;
-template <class C>
-__global__ void __launch_bounds__(256, 2) k_msm_pair_merge(const uint32_t* __restrict__ off, uint32_t nchunks,
-                                                           uint32_t L, uint32_t* __restrict__ skey,
-                                                           const uint32_t* __restrict__ spt,
-                                                           uint32_t* __restrict__ bsum, uint32_t* chk,
-                                                           uint32_t nseg) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t + 1 >= nchunks) return;
-  const uint32_t s = skey[2 * t + 1];
-  if (s == INVALID) return;
-  if (chk && s >= nseg) { atomicOr(chk, CHK_SEGMENT); return; }
-  const uint32_t last = (__ldg(off + s + 1) - 1) / L;   // chunk holding the segment's last entry
-  if (last - t > RUN_MAX) return;                       // left to the fold levels
-  Xyzz<F> acc = xyzz_load<F>(spt + (size_t)(2 * t + 1) * XW);
-  for (uint32_t u = t + 1; u <= last; u++) {
-    xyzz_add_paired(acc, xyzz_load<F>(spt + (size_t)(2 * u) * XW));
-    skey[2 * u] = INVALID;   // A slots of chunks t+1..last: no other thread reads or writes them
-  }
-  xyzz_store<F>(bsum + (size_t)s * XW, acc);
-  skey[2 * t + 1] = INVALID;
 }
 
 // ---------------------------------------------------------- the FP64-product pipeline
@@ -425,49 +515,6 @@ __global__ void k_msm_xyzz_from_dpf(uint32_t n, uint32_t* __restrict__ pts, cons
 
 
 
-// Fold partial sums left by the previous level. Slots carry their segment id (INVALID for an
-// unused slot); the range of segment s at this level follows from its range one level down:
-// chunks cs..ce of length L_prev hold its pieces at slots 2cs+1 .. 2ce.
-template <class C>
-__global__ void __launch_bounds__(256) k_msm_seg_level(const uint32_t* __restrict__ ikey,
-                                                       const uint32_t* __restrict__ ipt, uint32_t Y, uint32_t L,
-                                                       uint32_t nchunks, LevelHist hist,
-                                                       const uint32_t* __restrict__ off,
-                                                       uint32_t* __restrict__ bsum, uint32_t* __restrict__ okey,
-                                                       uint32_t* __restrict__ opt) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nchunks) return;
-  const uint64_t start = (uint64_t)t * L;
-  const uint64_t end = min(start + L, (uint64_t)Y);
-  uint32_t keyA = INVALID, keyB = INVALID;
-  uint32_t cur = INVALID;
-  Xyzz<F> acc = xyzz_inf<F>();
-  auto flush = [&](uint32_t s) {
-    uint64_t lo = __ldg(off + s), hi = __ldg(off + s + 1);
-    for (int j = 0; j < hist.n; j++) {
-      const uint64_t cs = lo / hist.L[j], ce = (hi - 1) / hist.L[j];
-      lo = 2 * cs + 1;
-      hi = 2 * ce + 1;
-    }
-    route_run<F>(s, acc, lo, hi, start, L, t, bsum, opt, keyA, keyB);
-  };
-  for (uint64_t y = start; y < end; y++) {
-    const uint32_t k = __ldg(ikey + y);
-    if (k == INVALID) continue;
-    if (k != cur) {
-      if (cur != INVALID) flush(cur);
-      cur = k;
-      acc = xyzz_inf<F>();
-    }
-    xyzz_add_paired(acc, xyzz_load<F>(ipt + y * XW));
-  }
-  if (cur != INVALID) flush(cur);
-  okey[2 * (size_t)t] = keyA;
-  okey[2 * (size_t)t + 1] = keyB;
-}
-
 // ------------------------------------------------------------------------- bucket reduce
 
 // Bucket arrays of up to four point-range parts of one MSM (same window layout); a bucket's sum
@@ -491,60 +538,6 @@ __global__ void k_msm_merge_parts(PartSet parts, uint32_t nseg, uint32_t* __rest
   for (int q = 0; q < parts.n; q++)
     if (__ldg(parts.off[q] + s) != __ldg(parts.off[q] + s + 1)) xyzz_add_paired(acc, xyzz_load<F>(parts.bsum[q] + (size_t)s * XW));
   xyzz_store<F>(out + (size_t)s * XW, acc);
-}
-
-// thread (w, g): buckets j = g*K .. g*K+K-1 of window w (bucket number j+1):
-// T = sum S_j, R = sum (j - g*K + 1) S_j (running sum from the top)
-template <class C>
-__global__ void __launch_bounds__(128) k_msm_bucket_rs(PartSet parts, uint32_t B, uint32_t nwin, uint32_t K,
-                                                       uint32_t G, uint32_t* __restrict__ Tout,
-                                                       uint32_t* __restrict__ Rout) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nwin * G) return;
-  const uint32_t w = t / G, g = t % G;
-  Xyzz<F> T = xyzz_inf<F>(), R = xyzz_inf<F>();
-  for (int l = (int)K - 1; l >= 0; l--) {
-    const size_t s = (size_t)w * B + (size_t)g * K + l;
-    for (int q = 0; q < parts.n; q++)
-      if (!parts.off[q] || __ldg(parts.off[q] + s) != __ldg(parts.off[q] + s + 1))
-        xyzz_add_paired(T, xyzz_load<F>(parts.bsum[q] + s * XW));
-    xyzz_add_paired(R, T);
-  }
-  xyzz_store<F>(Tout + (size_t)t * XW, T);
-  xyzz_store<F>(Rout + (size_t)t * XW, R);
-}
-
-// block (w, k): k < gbits -> U_k = sum over g with bit k set of T_g; k == gbits -> sum of R_g
-template <class C>
-__global__ void __launch_bounds__(256, 2) k_msm_bucket_bits(const uint32_t* __restrict__ Tin,
-                                                         const uint32_t* __restrict__ Rin, uint32_t G,
-                                                         int gbits, uint32_t* __restrict__ U) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  extern __shared__ uint4 smem_u4[];
-  uint32_t* sm = reinterpret_cast<uint32_t*>(smem_u4);
-  const uint32_t w = blockIdx.x, k = blockIdx.y;
-  Xyzz<F> acc = xyzz_inf<F>();
-  for (uint32_t g = threadIdx.x; g < G; g += blockDim.x) {
-    if ((int)k < gbits) {
-      if ((g >> k) & 1u) xyzz_add_paired(acc, xyzz_load<F>(Tin + ((size_t)w * G + g) * XW));
-    } else {
-      xyzz_add_paired(acc, xyzz_load<F>(Rin + ((size_t)w * G + g) * XW));
-    }
-  }
-  xyzz_store<F>(sm + threadIdx.x * XW, acc);
-  __syncthreads();
-  for (uint32_t half = blockDim.x >> 1; half > 0; half >>= 1) {
-    if (threadIdx.x < half) {
-      Xyzz<F> a = xyzz_load<F>(sm + threadIdx.x * XW);
-      xyzz_add_paired(a, xyzz_load<F>(sm + (threadIdx.x + half) * XW));
-      xyzz_store<F>(sm + threadIdx.x * XW, a);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) xyzz_store<F>(U + ((size_t)w * (gbits + 1) + k) * XW, xyzz_canon(xyzz_load<F>(sm)));
 }
 
 // ---------------------------------------------------------------------------- planning
@@ -599,15 +592,14 @@ static MsmTune& msm_tune(int curve, int lg) {
   return g_tune[curve][lg < 0 ? 0 : (lg > 31 ? 31 : lg)];
 }
 
-// Buckets per running-sum group of the bucket reduction. Each group is one thread's sequential
-// chain of 2 K1 additions: long groups keep the bucket_bits tail small (2^22 points: 32 measured
-// best), but for small MSMs (few windows x buckets) they leave the GPU idle, so K1 shrinks until
-// nwin * B / K1 reaches 16 K threads.
+// Buckets per running-sum group of the bucket reduction. A group is a chain of K1 + 1 additions of two
+// quads; long groups keep the window sums small, short ones the chain, so K1 shrinks from 32 until
+// nwin * B / K1 reaches 4 K groups (32 K threads, a quarter of the GPU's).
 static uint32_t pick_k1(uint32_t nwin, uint32_t B, int tuned = 0) {
   if (g_tune_K1 > 0) return std::min<uint32_t>(B, (uint32_t)g_tune_K1);
   if (tuned > 0) return std::min<uint32_t>(B, (uint32_t)tuned);
   uint32_t k = 32;
-  while (k > 2 && (uint64_t)nwin * B / k < 16384) k >>= 1;
+  while (k > 2 && (uint64_t)nwin * B / k < 4096) k >>= 1;
   return std::min<uint32_t>(B, k);
 }
 
@@ -777,15 +769,24 @@ static uint32_t chunk_len(uint64_t total, uint64_t wave, int tuned = 0) {
   return (uint32_t)((total + k * wave - 1) / (k * wave));
 }
 
+// The quad accumulation's chunk length: about two warps a scheduler, at least 4 entries (a shorter
+// chunk costs more in merges than its chain saves).
+static uint32_t quad_chunk_len(uint64_t total) {
+  if (g_tune_L1 > 0) return (uint32_t)g_tune_L1;
+  const uint64_t quads = 64ull * (uint64_t)std::max(1, device_sm_count());
+  return (uint32_t)std::max<uint64_t>(4, (total + quads - 1) / quads);
+}
+
 struct MsmPlan {
   int n = 0, c = 0, nwin = 0, nw = 0;
   uint32_t B = 0, nseg = 0;
   uint64_t total_max = 0;   // nwin * n
   int L1 = 64;
-  int nlev = 0;             // levels after the first
-  uint32_t Llev[MAX_LEVELS];
-  uint64_t Ylev[MAX_LEVELS];   // slot positions read by level k (k >= 2)
-  uint32_t nch[MAX_LEVELS + 1]; // chunks per level (index 0 = level 1)
+  uint32_t nch = 0;         // chunks of the accumulation
+  bool quad = false;        // accumulation with a quad a chunk (few entries)
+  bool small = false;       // sorted by k_sort_small (few points)
+  WinShape win = {0, 0};
+  uint32_t pcap = 0;        // pieces of long segments, at most
   uint32_t K1 = 0, G = 0;
   int gbits = 0;
   int pf = 2;               // prefetch stages of the accumulation
@@ -797,7 +798,8 @@ struct MsmPlan {
   uint32_t tthr[MAX_TREE];
   uint64_t acc_total = 0;   // entries of the chunk accumulation (a bound when tree > 0)
   // byte offsets into one arena block
-  size_t o_std, o_cnt, o_off, o_cur, o_bs, o_ent, o_keyA, o_ptA, o_keyB, o_ptB, o_bsum, o_T, o_R, o_U, bytes;
+  size_t o_std, o_cnt, o_off, o_cur, o_bs, o_ent, o_keyA, o_ptA, o_bsum, o_T, o_R, o_U, o_V, bytes;
+  size_t o_prec, o_pdone, o_ppt;   // pieces of long segments (their count follows the histogram's counts)
   bool use_dig = false;   // digits and ranks stored at o_dig, o_rank (nwin x n words each)
   size_t o_dig = 0, o_rank = 0;
   size_t o_toff[2], o_tpts[2], o_tpre, o_ttt, o_tscr;
@@ -813,8 +815,9 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   if (P.c < 2 || P.c > 24) return set_status(ZKG_ERR_ARG, "msm", "window width out of range [2, 24]");
   P.nwin = (scalar_bits + 1 + P.c - 1) / P.c;
   P.nw = mont ? 8 : 2 * nlimbs;
-  P.B = 1u << (P.c - 1);
-  P.nseg = (uint32_t)P.nwin * P.B;
+  P.win = win_shape(scalar_bits + 1, P.nwin);
+  P.B = 1u << (P.win.width(0) - 1);
+  P.nseg = P.win.seg(P.nwin);
   P.total_max = (uint64_t)P.nwin * (uint64_t)n;
   if (P.total_max >= (1ull << 31)) return set_status(ZKG_ERR_ARG, "msm", "too many (window, point) entries for one launch");
   const MsmTune& T = msm_tune(C::ID, round_log2((uint64_t)n));
@@ -830,23 +833,11 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   }
   P.L1 = (int)chunk_len(P.acc_total, accum_wave<C>(), T.L1);
   P.pf = g_msm_pf_env || T.pf < 0 ? g_msm_pf : T.pf;
-  P.nch[0] = (uint32_t)((P.acc_total + P.L1 - 1) / P.L1);
-  if (P.nch[0] == 0) P.nch[0] = 1;
-  // later levels: slot arrays of 2 * previous chunks, folded in chunks of 16
-  P.nlev = 0;
-  uint64_t Y = 2ull * P.nch[0];
-  uint32_t prev_chunks = P.nch[0];
-  while (prev_chunks > 1) {
-    if (P.nlev >= MAX_LEVELS - 1) return set_status(ZKG_ERR_ARG, "msm", "level overflow");
-    const uint32_t L = 16;
-    P.Llev[P.nlev] = L;
-    P.Ylev[P.nlev] = Y;
-    const uint32_t ch = (uint32_t)((Y + L - 1) / L);
-    P.nch[P.nlev + 1] = ch;
-    P.nlev++;
-    Y = 2ull * ch;
-    prev_chunks = ch;
-  }
+  P.quad = P.tree == 0 && P.total_max <= QUAD_TOTAL;
+  if (P.quad) P.L1 = (int)quad_chunk_len(P.total_max);
+  P.small = P.quad && sort_small_fits(n, P.nwin, P.B);
+  P.nch = std::max<uint32_t>(1, (uint32_t)((P.acc_total + P.L1 - 1) / P.L1));
+  P.pcap = P.nch / 8 + 2;   // a long segment has more than RUN_MAX + 1 partial sums
   P.K1 = pick_k1((uint32_t)P.nwin, P.B, T.K1);
   P.G = P.B / P.K1;
   P.gbits = ilog2_floor(P.G);
@@ -855,7 +846,7 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   auto take = [&](size_t bytes) { size_t r = o; o = (o + bytes + 255) & ~size_t(255); return r; };
   const bool dig_path = g_msm_digits && g_msm_wmajor;   // P.use_dig below
   P.o_std = take(mont && !dig_path ? (size_t)n * 32 : 0);
-  P.o_cnt = take((size_t)P.nseg * 4 + 4);
+  P.o_cnt = take((size_t)(P.nseg + 2 + P.nwin) * 4);   // then: pieces; non-zero digits (k_sort_small); finished blocks a window
   P.o_off = take((size_t)P.nseg * 4 + 4);
   P.o_cur = take((size_t)P.nseg * 4 + 4);
   const uint32_t nb = (P.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
@@ -865,19 +856,16 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   P.use_dig = dig_path;
   P.o_dig = take(P.use_dig ? (size_t)P.total_max * 4 + 4 : 0);
   P.o_rank = take(P.use_dig ? (size_t)P.total_max * 4 + 4 : 0);
-  uint64_t slotsA = 2ull * P.nch[0], slotsB = 0;
-  for (int k = 1; k <= P.nlev; k++) {
-    if (k % 2 == 1) slotsB = std::max<uint64_t>(slotsB, 2ull * P.nch[k]);
-    else slotsA = std::max<uint64_t>(slotsA, 2ull * P.nch[k]);
-  }
-  P.o_keyA = take(slotsA * 4);
-  P.o_ptA = take(slotsA * XB);
-  P.o_keyB = take(slotsB * 4 + 4);
-  P.o_ptB = take(slotsB * XB + 4);
+  P.o_keyA = take((size_t)P.nch * 8);
+  P.o_ptA = take((size_t)P.nch * 2 * XB);
+  P.o_prec = take((size_t)P.pcap * sizeof(Piece));
+  P.o_pdone = take((size_t)P.pcap * 4);
+  P.o_ppt = take((size_t)P.pcap * XB);
   P.o_bsum = take((size_t)P.nseg * XB);
   P.o_T = take((size_t)P.nwin * P.G * XB);
   P.o_R = take((size_t)P.nwin * P.G * XB);
   P.o_U = take((size_t)P.nwin * (P.gbits + 1) * XB);
+  P.o_V = take((size_t)P.nwin * XB);
   P.o_toff[0] = P.o_toff[1] = P.o_tpts[0] = P.o_tpts[1] = P.o_tpre = P.o_ttt = P.o_tscr = 0;
   if (P.tree > 0) {
     constexpr size_t AB = 8 * F::N, FB = 4 * F::N;   // bytes of an affine point, of a field element
@@ -893,15 +881,15 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   return ZKG_OK;
 }
 
-// per-window sums U of a finished FP64-product pipeline back to radix R (before the host tail)
+// window values V of a finished FP64-product pipeline back to radix R (before the host tail)
 template <class CP>
 static zkg_status msm_u_to_radix(const MsmPlan& P, char* ws, cudaStream_t st) {
   if constexpr (radix_conv_v<typename CP::Fp>) {
     Fe<typename CP::Fp> kin, kout;
     dpf_consts_for<CP>(kin, kout);
-    const uint32_t npts = (uint32_t)P.nwin * (P.gbits + 1);
+    const uint32_t npts = (uint32_t)P.nwin;
     ZKB_TRY(launch("msm_xyzz_from_dpf", k_msm_xyzz_from_dpf<CP>, dim3((4 * npts + 255) / 256), dim3(256), 0, st,
-                   npts, reinterpret_cast<uint32_t*>(ws + P.o_U), kout));
+                   npts, reinterpret_cast<uint32_t*>(ws + P.o_V), kout));
   }
   return ZKG_OK;
 }
@@ -959,7 +947,6 @@ template <class C>
 static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, const uint32_t* ent, const uint32_t* off,
                                   const uint32_t* bases, cudaStream_t st, uint32_t* chk) {
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
-  const uint32_t nb = (P.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
   const uint32_t* in_off = off;
   const uint32_t* in_pts = bases;
   for (int l = 0; l < P.tree; l++) {
@@ -967,11 +954,7 @@ static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, const uint32_t* en
     uint32_t* out_pts = U32(P.o_tpts[l & 1]);
     ZKB_TRY(launch("msm_tree_counts", k_tree_counts, dim3((P.nseg + 255) / 256), dim3(256), 0, st, in_off, P.nseg,
                    U32(P.o_cnt)));
-    ZKB_TRY(launch("scan_blocks", k_scan_blocks, dim3(nb), dim3(SCAN_T), 0, st, (const uint32_t*)U32(P.o_cnt),
-                   out_off, U32(P.o_bs), P.nseg));
-    ZKB_TRY(launch("scan_top", k_scan_top, dim3(1), dim3(SCAN_T), 0, st, U32(P.o_bs), nb));
-    ZKB_TRY(launch("scan_add", k_scan_add, dim3((P.nseg + 255) / 256), dim3(256), 0, st, out_off, U32(P.o_cur),
-                   (const uint32_t*)U32(P.o_bs), P.nseg, nb));
+    ZKB_TRY(scan_counts(U32(P.o_cnt), out_off, U32(P.o_cur), U32(P.o_bs), P.nseg, st));
     const uint32_t npts = l == 0 ? (uint32_t)P.n : (uint32_t)P.tQ[l - 1];
     if (l == 0)
       ZKB_TRY((launch_tree_level<C, true>(P, P.tthr[l], st, ent, in_pts, in_off, out_off, U32(P.o_tpre), U32(P.o_ttt),
@@ -983,6 +966,27 @@ static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, const uint32_t* en
     in_pts = out_pts;
   }
   return ZKG_OK;
+}
+
+// The segments that chunk boundaries cut: short ones, then long ones.
+template <class C>
+static zkg_status msm_launch_merge(const PieceList& pl, const uint32_t* off, uint32_t* chk, uint32_t nch, uint32_t L1,
+                                   const uint32_t* key, const uint32_t* pt, uint32_t* bsum, uint32_t nseg,
+                                   cudaStream_t st) {
+  ZKB_TRY(launch("msm_cut_merge", k_cut_merge<C>, dim3((nch + 31) / 32), dim3(128), 0, st, off, nch, L1, key, pt, bsum,
+                 chk, nseg, pl));
+  const dim3 gp(std::min<uint32_t>(pl.cap, 4 * (uint32_t)std::max(1, device_sm_count())));
+  return launch("msm_pieces", k_pieces<C>, gp, dim3(128), 0, st, pl, pt, bsum);
+}
+
+// Bucket sums to window values: T, R, U, done, V are the caller's buffers, G the largest number of groups.
+template <class C>
+static zkg_status msm_launch_windows(const MReqs& q, uint32_t ngroups, uint32_t nblk, uint32_t G,
+                                     const uint32_t* bsum, const uint32_t* off, uint32_t* T, uint32_t* R, uint32_t* U,
+                                     uint32_t* done, uint32_t* V, cudaStream_t st) {
+  ZKB_TRY(launch("msm_bucket_rs", k_bucket_rs<C>, dim3((ngroups + 15) / 16), dim3(128), 0, st, q, ngroups, bsum, off, T, R));
+  return launch("msm_window_bits", k_window_bits<C>, dim3(nblk), dim3(window_bits_threads(G)), 0, st, q,
+                (const uint32_t*)T, (const uint32_t*)R, U, done, V);
 }
 
 // Sort the scalars of one point range into (window, bucket) segments and accumulate its bucket
@@ -999,44 +1003,46 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
   if (first) ZKB_CUDA(cudaEventRecord(cx.ev_phase[0], st));
   const uint32_t* scal = reinterpret_cast<const uint32_t*>(d_scal);
   const bool hist_mont = mont && P.use_dig;   // conversion inside the histogram
+  if (P.small) {
+    ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt) + P.nseg, 0, (size_t)(2 + P.nwin) * 4, st));
+    auto small = mont ? k_sort_small<C, true> : k_sort_small<C, false>;
+    ZKB_TRY(launch("msm_sort_small", small, dim3(P.nwin), dim3(SMALL_T), 0, st, n, scal, P.nw, P.win,
+                   digit_bias(P.win, P.nwin), P.nseg, U32(P.o_off), U32(P.o_ent), U32(P.o_cnt) + P.nseg + 1));
+  } else {
   if (mont && !hist_mont) {
     ZKB_TRY(launch("msm_scalar_from_mont", k_msm_scalar_from_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st,
                    n, d_scal, U32(P.o_std)));
     scal = U32(P.o_std);
   }
-  ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)P.nseg * 4, st));
+  ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)(P.nseg + 2 + P.nwin) * 4, st));
   CarryTable ct;
-  const bool wmajor = g_msm_wmajor && make_carry_table(P.nwin, P.nw, P.c, ct);
+  const bool wmajor = g_msm_wmajor && make_carry_table(P.nwin, P.nw, P.win, ct);
   // the histogram reads each scalar once and loops over its windows (the window-major histogram
   // re-reads the scalars per window and measured slower); the scatter is window-major, from the
   // digits the histogram stores (P.o_dig) or, without them, re-deriving each digit from its scalar
   uint32_t* dig = P.use_dig ? U32(P.o_dig) : nullptr;
   uint32_t* rank = P.use_dig ? U32(P.o_rank) : nullptr;
   if (hist_mont)
-    ZKB_TRY(launch("msm_hist_mont", k_msm_hist_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st, n, d_scal, P.c,
-                   P.nwin, P.B, U32(P.o_cnt), chk, dig, rank));
+    ZKB_TRY(launch("msm_hist_mont", k_msm_hist_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st, n, d_scal, P.win,
+                   P.nwin, U32(P.o_cnt), chk, dig, rank));
   else if (wmajor && g_msm_hist_wmajor && !dig)
-    ZKB_TRY(launch("msm_hist_w", k_msm_hist_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw, P.c,
-                   P.B, ct, U32(P.o_cnt), chk));
+    ZKB_TRY(launch("msm_hist_w", k_msm_hist_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw, P.win,
+                   ct, U32(P.o_cnt), chk));
   else
-    ZKB_TRY(launch("msm_hist", k_msm_hist, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.c, P.nwin,
-                   P.B, U32(P.o_cnt), chk, dig, rank));
-  const uint32_t nb = (P.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
-  ZKB_TRY(launch("scan_blocks", k_scan_blocks, dim3(nb), dim3(SCAN_T), 0, st, (const uint32_t*)U32(P.o_cnt),
-                 U32(P.o_off), U32(P.o_bs), P.nseg));
-  ZKB_TRY(launch("scan_top", k_scan_top, dim3(1), dim3(SCAN_T), 0, st, U32(P.o_bs), nb));
-  ZKB_TRY(launch("scan_add", k_scan_add, dim3((P.nseg + 255) / 256), dim3(256), 0, st, U32(P.o_off),
-                 U32(P.o_cur), (const uint32_t*)U32(P.o_bs), P.nseg, nb));
+    ZKB_TRY(launch("msm_hist", k_msm_hist, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win, P.nwin,
+                   U32(P.o_cnt), chk, dig, rank));
+  ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st));
   if (dig)
     ZKB_TRY(launch("msm_scatter_d", k_msm_scatter_d, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n,
-                   (const uint32_t*)dig, (const uint32_t*)rank, P.B, (const uint32_t*)U32(P.o_off), U32(P.o_ent),
+                   (const uint32_t*)dig, (const uint32_t*)rank, P.win, (const uint32_t*)U32(P.o_off), U32(P.o_ent),
                    chk, (uint32_t)P.total_max));
   else if (wmajor)
     ZKB_TRY(launch("msm_scatter_w", k_msm_scatter_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw,
-                   P.c, P.B, ct, U32(P.o_cur), U32(P.o_ent), chk, (uint32_t)P.total_max));
+                   P.win, ct, U32(P.o_cur), U32(P.o_ent), chk, (uint32_t)P.total_max));
   else
-    ZKB_TRY(launch("msm_scatter", k_msm_scatter, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.c,
-                   P.nwin, P.B, U32(P.o_cur), U32(P.o_ent)));
+    ZKB_TRY(launch("msm_scatter", k_msm_scatter, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win,
+                   P.nwin, U32(P.o_cur), U32(P.o_ent)));
+  }
   const uint32_t* bases = reinterpret_cast<const uint32_t*>(d_bases);
   if (first) ZKB_CUDA(cudaEventRecord(cx.ev_phase[1], st));
   if (bases_ready) ZKB_CUDA(cudaStreamWaitEvent(st, bases_ready, 0));
@@ -1064,46 +1070,35 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
       acc_npts = (uint32_t)P.tQ[P.tree - 1];
     }
   }
-  ZKB_TRY(launch_accum<C>(P.nch[0], st, ent, off, P.nseg, (uint32_t)P.L1, bases, U32(P.o_bsum), U32(P.o_keyA),
-                          U32(P.o_ptA), P.pf, chk, acc_npts));
+  const PieceList pl = {U32(P.o_cnt) + P.nseg, P.pcap, reinterpret_cast<Piece*>(ws + P.o_prec), U32(P.o_pdone),
+                        U32(P.o_ppt)};
+  if (P.quad)
+    ZKB_TRY(launch("msm_quad_accum", k_quad_accum<C>, dim3((P.nch + 31) / 32), dim3(128), 0, st, ent, off, P.nseg, P.nch,
+                   (uint32_t)P.L1, bases, U32(P.o_bsum), U32(P.o_keyA), U32(P.o_ptA), chk, acc_npts));
+  else
+    ZKB_TRY(launch_accum<C>(P.nch, st, ent, off, P.nseg, (uint32_t)P.L1, bases, U32(P.o_bsum), U32(P.o_keyA),
+                            U32(P.o_ptA), P.pf, chk, acc_npts));
   if (last) ZKB_CUDA(cudaEventRecord(cx.ev_phase[2], st));
-  // fold_part >= 0: the fold levels run on the side stream (they are latency-bound and use few
-  // SMs, so the next part's sort and accumulation fill the rest); ev_fold[fold_part] marks them done
+  // fold_part >= 0: the merge of cut segments runs on the side stream (it is latency-bound, so the
+  // next part's sort and accumulation fill the rest); ev_fold[fold_part] marks it done
   const cudaStream_t fst = fold_part >= 0 ? cx.side_stream : st;
   if (fold_part >= 0) {
     ZKB_CUDA(cudaEventRecord(cx.ev_acc[fold_part], st));
     ZKB_CUDA(cudaStreamWaitEvent(fst, cx.ev_acc[fold_part], 0));
   }
-  ZKB_TRY(launch("msm_pair_merge", k_msm_pair_merge<C>, dim3((P.nch[0] + 255) / 256), dim3(256), 0, fst, off, P.nch[0], (uint32_t)P.L1,
-                 U32(P.o_keyA), (const uint32_t*)U32(P.o_ptA), U32(P.o_bsum), chk, P.nseg));
-  LevelHist hist;
-  hist.n = 1;
-  hist.L[0] = (uint32_t)P.L1;
-  for (int k = 0; k < P.nlev; k++) {
-    const bool fromA = (k % 2 == 0);
-    const uint32_t* ik = U32(fromA ? P.o_keyA : P.o_keyB);
-    const uint32_t* ip = U32(fromA ? P.o_ptA : P.o_ptB);
-    uint32_t* ok = U32(fromA ? P.o_keyB : P.o_keyA);
-    uint32_t* op = U32(fromA ? P.o_ptB : P.o_ptA);
-    const uint32_t ch = P.nch[k + 1];
-    ZKB_TRY(launch("msm_seg_level", k_msm_seg_level<C>, dim3((ch + 255) / 256), dim3(256), 0, fst, ik, ip,
-                   (uint32_t)P.Ylev[k], P.Llev[k], ch, hist, off, U32(P.o_bsum), ok, op));
-    hist.L[hist.n++] = P.Llev[k];
-  }
+  ZKB_TRY(msm_launch_merge<C>(pl, off, chk, P.nch, (uint32_t)P.L1, U32(P.o_keyA), U32(P.o_ptA), U32(P.o_bsum), P.nseg,
+                              fst));
   if (last) ZKB_CUDA(cudaEventRecord(cx.ev_phase[3], fst));
   if (fold_part >= 0) ZKB_CUDA(cudaEventRecord(cx.ev_fold[fold_part], fst));
   return ZKG_OK;
 }
 
-// Bucket reduction over the parts' bucket arrays (phase 7) into U of workspace ws0 / plan P0.
+// Bucket reduction over the parts' bucket arrays (phase 7) into V of workspace ws0 / plan P0.
 template <class C>
 static zkg_status msm_launch_reduce(Context& cx, const MsmPlan& P0, char* ws0, const PartSet& parts,
                                     cudaStream_t st, bool record_phase = true) {
   NvtxRange nvtx("zkb.msm.bucket_reduce");
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws0 + o); };
-  const uint32_t nthr = (uint32_t)P0.nwin * P0.G;
   PartSet rs = parts;
   if (parts.n > 1) {   // one parallel merge into part 0's bucket array, then running sums over it
     uint32_t* merged = U32(P0.o_bsum);
@@ -1113,57 +1108,50 @@ static zkg_status msm_launch_reduce(Context& cx, const MsmPlan& P0, char* ws0, c
     rs.bsum[0] = merged;
     rs.off[0] = nullptr;   // merged sums are present for every segment (the identity where all parts were empty)
   }
-  ZKB_TRY(launch("msm_bucket_rs", k_msm_bucket_rs<C>, dim3((nthr + 127) / 128), dim3(128), 0, st, rs, P0.B,
-                 (uint32_t)P0.nwin, P0.K1, P0.G, U32(P0.o_T), U32(P0.o_R)));
-  const size_t smem = 256 * XW * 4;
-  ZKB_TRY(launch("msm_bucket_bits", k_msm_bucket_bits<C>, dim3(P0.nwin, P0.gbits + 1), dim3(256), smem, st,
-                 (const uint32_t*)U32(P0.o_T), (const uint32_t*)U32(P0.o_R), P0.G, P0.gbits, U32(P0.o_U)));
+  MReqs q = {};
+  q.one.n = (uint32_t)P0.n;
+  q.one.nwin = (uint32_t)P0.nwin;
+  q.one.win = P0.win;
+  q.one.K1 = P0.K1;
+  q.one.G = P0.G;
+  q.one.gbits = (uint32_t)P0.gbits;
+  ZKB_TRY(msm_launch_windows<C>(q, (uint32_t)P0.nwin * P0.G, (uint32_t)(P0.nwin * (P0.gbits + 1)), P0.G, rs.bsum[0],
+                                rs.off[0], U32(P0.o_T), U32(P0.o_R), U32(P0.o_U), U32(P0.o_cnt) + P0.nseg + 2,
+                                U32(P0.o_V), st));
   if (record_phase) ZKB_CUDA(cudaEventRecord(cx.ev_phase[4], st));
   return ZKG_OK;
 }
 
-// Host tail: Horner over bits and windows on the per-window sums.
+// Host tail: Horner over the window values.
 template <int NL>
-static host::Xyzz<NL> msm_host_combine(const host::Field<NL>& F, const MsmPlan& P, const uint64_t* U) {
-  auto ld = [&](int w, int k) {
-    host::Xyzz<NL> r;
-    const uint64_t* p = U + ((size_t)w * (P.gbits + 1) + k) * 4 * NL;
-    std::memcpy(r.X.v, p, 8 * NL);
-    std::memcpy(r.Y.v, p + NL, 8 * NL);
-    std::memcpy(r.ZZ.v, p + 2 * NL, 8 * NL);
-    std::memcpy(r.ZZZ.v, p + 3 * NL, 8 * NL);
-    return r;
-  };
-  int k1bits = 0;
-  while ((1u << k1bits) < P.K1) k1bits++;
+static host::Xyzz<NL> msm_host_combine(const host::Field<NL>& F, const WinShape& win, int nwin, const uint64_t* V) {
   host::Xyzz<NL> res = host::xyzz_inf<NL>();
-  for (int w = P.nwin - 1; w >= 0; w--) {
-    if (w != P.nwin - 1)
-      for (int i = 0; i < P.c; i++) res = host::xyzz_dbl(F, res);
-    host::Xyzz<NL> V = host::xyzz_inf<NL>();
-    for (int k = P.gbits - 1; k >= 0; k--) {
-      V = host::xyzz_dbl(F, V);
-      V = host::xyzz_add(F, V, ld(w, k));
-    }
-    for (int i = 0; i < k1bits; i++) V = host::xyzz_dbl(F, V);
-    V = host::xyzz_add(F, V, ld(w, P.gbits));
-    res = host::xyzz_add(F, res, V);
+  for (int w = nwin - 1; w >= 0; w--) {
+    for (int i = 0; i < win.width(w); i++) res = host::xyzz_dbl(F, res);
+    host::Xyzz<NL> v;
+    const uint64_t* p = V + (size_t)w * 4 * NL;
+    std::memcpy(v.X.v, p, 8 * NL);
+    std::memcpy(v.Y.v, p + NL, 8 * NL);
+    std::memcpy(v.ZZ.v, p + 2 * NL, 8 * NL);
+    std::memcpy(v.ZZZ.v, p + 3 * NL, 8 * NL);
+    res = host::xyzz_add(F, res, v);
   }
   return res;
 }
 
-// Reads back U and the addition counts, runs the host tail and writes the output encoding.
+// Reads back V and the addition counts, runs the host tail and writes the output encoding.
 template <class C, int NL>
 static zkg_status msm_finish(Context& cx, const host::Field<NL>& F, const MsmPlan& P0, char* ws0,
                              char* const* ws, const MsmPlan* P, int nparts, int kind, uint64_t* tgt,
                              cudaStream_t st) {
-  const size_t ubytes = (size_t)P0.nwin * (P0.gbits + 1) * 4 * NL * 8;
+  const size_t ubytes = (size_t)P0.nwin * 4 * NL * 8;
   ZKB_TRY(pinned_reserve(cx, ubytes + 64));
   char* pin = static_cast<char*>(cx.pinned);
-  ZKB_CUDA(cudaMemcpyAsync(pin, ws0 + P0.o_U, ubytes, cudaMemcpyDeviceToHost, st));
+  ZKB_CUDA(cudaMemcpyAsync(pin, ws0 + P0.o_V, ubytes, cudaMemcpyDeviceToHost, st));
   // number of (window, point) entries with a non-zero digit = mixed additions performed
   for (int q = 0; q < nparts; q++)
-    ZKB_CUDA(cudaMemcpyAsync(pin + ubytes + 4 * q, ws[q] + P[q].o_off + (size_t)P[q].nseg * 4, 4,
+    ZKB_CUDA(cudaMemcpyAsync(pin + ubytes + 4 * q,
+                             ws[q] + (P[q].small ? P[q].o_cnt + 4 : P[q].o_off) + (size_t)P[q].nseg * 4, 4,
                              cudaMemcpyDeviceToHost, st));
   ZKB_CUDA(cudaStreamSynchronize(st));
   cx.last_msm_entries = 0;
@@ -1177,7 +1165,7 @@ static zkg_status msm_finish(Context& cx, const host::Field<NL>& F, const MsmPla
   ZKB_CUDA(cudaEventElapsedTime(&cx.last_kernel_ms, cx.ev_phase[0], cx.ev_phase[4]));
   cx.nphase = 4;
   for (int i = 0; i < 4; i++) ZKB_CUDA(cudaEventElapsedTime(&cx.last_phase_ms[i], cx.ev_phase[i], cx.ev_phase[i + 1]));
-  const host::Xyzz<NL> r = msm_host_combine<NL>(F, P0, reinterpret_cast<const uint64_t*>(pin));
+  const host::Xyzz<NL> r = msm_host_combine<NL>(F, P0.win, P0.nwin, reinterpret_cast<const uint64_t*>(pin));
   host::xyzz_write<NL>(F, r, kind, tgt);
   return ZKG_OK;
 }
@@ -1388,32 +1376,6 @@ static zkg_status msm_dev_entry(const host::Field<NL>& F, int n, const uint64_t*
 // the scan, the chunked accumulation and the folding levels run unchanged over all requests'
 // segments at once, so small requests share the GPU instead of each under-filling it.
 
-struct MReq {
-  const uint64_t* scal_in;   // the request's Montgomery scalars (device), 4 limbs each
-  uint32_t pt_off;           // first point in the batch's concatenated standard scalars
-  uint32_t n, c, nwin, B;    // points, window width, windows, buckets per window
-  uint32_t seg_base;         // first segment
-  uint32_t K1, G, gbits;     // running-sum group size, groups per window, log2 G
-  uint32_t thr_off;          // first running-sum thread (= first T/R entry)
-  uint32_t blk_off;          // first (window, k) reduction block (= first U entry)
-  uint32_t rank_base;        // first rank word (window-major per request: base + win n + point)
-};
-
-template <int FIELD>
-__device__ __forceinline__ uint32_t mreq_key(const MReq& r) {
-  return FIELD == 0 ? r.pt_off : (FIELD == 1 ? r.thr_off : r.blk_off);
-}
-// largest r with key(r) <= x (keys ascending, key(0) = 0)
-template <int FIELD>
-__device__ __forceinline__ int mreq_find(const MReq* __restrict__ reqs, int nreq, uint32_t x) {
-  int lo = 0, hi = nreq;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (mreq_key<FIELD>(reqs[mid]) <= x) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
 template <class C>
 __global__ void k_mmsm_from_mont(const MReq* __restrict__ reqs, int nreq, uint32_t npts, uint32_t* __restrict__ out) {
   using Fr = typename C::Fr;
@@ -1432,12 +1394,13 @@ __global__ void k_mmsm_hist(const MReq* __restrict__ reqs, int nreq, uint32_t np
   if (i >= npts) return;
   const MReq q = reqs[mreq_find<0>(reqs, nreq, i)];
   const uint32_t* w = scal + 8 * (size_t)i;
+  const WinShape ws = q.win;
   uint32_t carry = 0, neg;
   for (int win = 0; win < (int)q.nwin; win++) {
-    const uint32_t b = next_digit(w, 8, win, (int)q.c, carry, neg);
+    const uint32_t b = next_digit(w, 8, ws.start(win), ws.width(win), carry, neg);
     if (b)
       rank[q.rank_base + (size_t)win * q.n + (i - q.pt_off)] =
-          atomicAdd(cnt + q.seg_base + (size_t)win * q.B + (b - 1), 1u);
+          atomicAdd(cnt + q.seg_base + ws.seg(win) + (b - 1), 1u);
   }
 }
 
@@ -1448,69 +1411,16 @@ __global__ void k_mmsm_scatter(const MReq* __restrict__ reqs, int nreq, uint32_t
   if (i >= npts) return;
   const MReq q = reqs[mreq_find<0>(reqs, nreq, i)];
   const uint32_t* w = scal + 8 * (size_t)i;
+  const WinShape ws = q.win;
   uint32_t carry = 0, neg;
   for (int win = 0; win < (int)q.nwin; win++) {
-    const uint32_t b = next_digit(w, 8, win, (int)q.c, carry, neg);
+    const uint32_t b = next_digit(w, 8, ws.start(win), ws.width(win), carry, neg);
     if (b) {
-      const uint32_t pos = __ldg(off + q.seg_base + (size_t)win * q.B + (b - 1)) +
+      const uint32_t pos = __ldg(off + q.seg_base + ws.seg(win) + (b - 1)) +
                            __ldg(rank + q.rank_base + (size_t)win * q.n + (i - q.pt_off));
       entries[pos] = (i - q.pt_off) | (neg << 31);
     }
   }
-}
-
-template <class C>
-__global__ void __launch_bounds__(128) k_mmsm_bucket_rs(const MReq* __restrict__ reqs, int nreq, uint32_t nthr,
-                                                        const uint32_t* __restrict__ bsum,
-                                                        const uint32_t* __restrict__ off,
-                                                        uint32_t* __restrict__ Tout, uint32_t* __restrict__ Rout) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nthr) return;
-  const MReq q = reqs[mreq_find<1>(reqs, nreq, t)];
-  const uint32_t tl = t - q.thr_off, w = tl / q.G, g = tl % q.G;
-  Xyzz<F> T = xyzz_inf<F>(), R = xyzz_inf<F>();
-  for (int l = (int)q.K1 - 1; l >= 0; l--) {
-    const size_t s = q.seg_base + (size_t)w * q.B + (size_t)g * q.K1 + l;
-    if (__ldg(off + s) != __ldg(off + s + 1)) xyzz_add_paired(T, xyzz_load<F>(bsum + s * XW));
-    xyzz_add_paired(R, T);
-  }
-  xyzz_store<F>(Tout + (size_t)t * XW, T);
-  xyzz_store<F>(Rout + (size_t)t * XW, R);
-}
-
-template <class C>
-__global__ void __launch_bounds__(256) k_mmsm_bucket_bits(const MReq* __restrict__ reqs, int nreq,
-                                                          const uint32_t* __restrict__ Tin,
-                                                          const uint32_t* __restrict__ Rin, uint32_t* __restrict__ U) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  extern __shared__ uint4 smem_u4[];
-  uint32_t* sm = reinterpret_cast<uint32_t*>(smem_u4);
-  const uint32_t b = blockIdx.x;
-  const MReq q = reqs[mreq_find<2>(reqs, nreq, b)];
-  const uint32_t bl = b - q.blk_off, w = bl / (q.gbits + 1), k = bl % (q.gbits + 1);
-  Xyzz<F> acc = xyzz_inf<F>();
-  for (uint32_t g = threadIdx.x; g < q.G; g += blockDim.x) {
-    const size_t idx = (size_t)q.thr_off + (size_t)w * q.G + g;
-    if (k < q.gbits) {
-      if ((g >> k) & 1u) xyzz_add_paired(acc, xyzz_load<F>(Tin + idx * XW));
-    } else {
-      xyzz_add_paired(acc, xyzz_load<F>(Rin + idx * XW));
-    }
-  }
-  xyzz_store<F>(sm + threadIdx.x * XW, acc);
-  __syncthreads();
-  for (uint32_t half = blockDim.x >> 1; half > 0; half >>= 1) {
-    if (threadIdx.x < half) {
-      Xyzz<F> a = xyzz_load<F>(sm + threadIdx.x * XW);
-      xyzz_add_paired(a, xyzz_load<F>(sm + (threadIdx.x + half) * XW));
-      xyzz_store<F>(sm + threadIdx.x * XW, a);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) xyzz_store<F>(U + (size_t)b * XW, xyzz_canon(xyzz_load<F>(sm)));
 }
 
 // ------------------------------------------------------------------------- batch plan
@@ -1518,13 +1428,14 @@ __global__ void __launch_bounds__(256) k_mmsm_bucket_bits(const MReq* __restrict
 struct MultiPlan {
   std::vector<MReq> reqs;     // descriptors of the non-empty requests
   std::vector<int> owner;     // batch MSM index of each descriptor
-  uint32_t npts = 0, nseg = 0, nthr = 0, nblk = 0;
+  uint32_t npts = 0, nseg = 0, nthr = 0, nblk = 0, nwins = 0;
   uint64_t total_max = 0;
-  int L1 = 128, nlev = 0;
-  uint32_t Llev[MAX_LEVELS];
-  uint64_t Ylev[MAX_LEVELS];
-  uint32_t nch[MAX_LEVELS + 1];
-  size_t o_std, o_cnt, o_off, o_cur, o_bs, o_ent, o_keyA, o_ptA, o_keyB, o_ptB, o_bsum, o_T, o_R, o_U, o_reqs, bytes;
+  int L1 = 128;
+  uint32_t nch = 0;           // chunks of the accumulation
+  uint32_t gmax = 0;          // running-sum groups of the widest window
+  uint32_t pcap = 0;          // pieces of long segments, at most
+  size_t o_std, o_cnt, o_off, o_cur, o_bs, o_ent, o_keyA, o_ptA, o_bsum, o_T, o_R, o_U, o_V, o_reqs, bytes;
+  size_t o_prec, o_pdone, o_ppt;
   size_t o_rank = 0;          // entry ranks (total_max words)
 };
 
@@ -1538,24 +1449,28 @@ static zkg_status make_multi_plan(const std::vector<int>& ns, const std::vector<
     MReq q;
     q.scal_in = scal[i];
     q.n = (uint32_t)ns[i];
-    q.c = (uint32_t)pick_window(C::ID, ns[i], C::SCALAR_BITS);
-    q.nwin = (C::SCALAR_BITS + 1 + q.c - 1) / q.c;
-    q.B = 1u << (q.c - 1);
+    const int c = pick_window(C::ID, ns[i], C::SCALAR_BITS);
+    q.nwin = (uint32_t)((C::SCALAR_BITS + 1 + c - 1) / c);
+    q.win = win_shape(C::SCALAR_BITS + 1, (int)q.nwin);
+    const uint32_t B = q.win.buckets(0);
     // the batch as a whole fills the GPU: work-efficient groups of 32 for every request
-    q.K1 = std::min<uint32_t>(q.B, g_tune_K1 > 0 ? (uint32_t)g_tune_K1 : 32u);
-    q.G = q.B / q.K1;
+    q.K1 = std::min<uint32_t>(B, g_tune_K1 > 0 ? (uint32_t)g_tune_K1 : 32u);
+    q.G = B / q.K1;
+    M.gmax = std::max(M.gmax, q.G);
     q.gbits = (uint32_t)ilog2_floor(q.G);
     q.pt_off = M.npts;
     q.seg_base = M.nseg;
     q.thr_off = M.nthr;
     q.blk_off = M.nblk;
+    q.win_off = M.nwins;
     q.rank_base = (uint32_t)M.total_max;   // < 2^31, checked below for the running total
-    const uint64_t np = (uint64_t)M.npts + q.n, ns_ = (uint64_t)M.nseg + (uint64_t)q.nwin * q.B;
+    const uint64_t np = (uint64_t)M.npts + q.n, ns_ = (uint64_t)M.nseg + q.win.seg((int)q.nwin);
     if (np >= (1ull << 31) || ns_ >= (1ull << 30)) return set_status(ZKG_ERR_ARG, "batch", "batch too large");
     M.npts = (uint32_t)np;
     M.nseg = (uint32_t)ns_;
     M.nthr += q.nwin * q.G;
     M.nblk += q.nwin * (q.gbits + 1);
+    M.nwins += q.nwin;
     M.total_max += (uint64_t)q.nwin * q.n;
     M.reqs.push_back(q);
     M.owner.push_back((int)i);
@@ -1563,22 +1478,12 @@ static zkg_status make_multi_plan(const std::vector<int>& ns, const std::vector<
   if (M.reqs.empty()) return ZKG_OK;
   if (M.total_max >= (1ull << 31)) return set_status(ZKG_ERR_ARG, "batch", "too many (window, point) entries");
   M.L1 = (int)chunk_len(M.total_max, accum_wave<C>());
-  M.nch[0] = (uint32_t)std::max<uint64_t>(1, (M.total_max + M.L1 - 1) / M.L1);
-  uint64_t Y = 2ull * M.nch[0];
-  uint32_t prev = M.nch[0];
-  while (prev > 1) {
-    if (M.nlev >= MAX_LEVELS - 1) return set_status(ZKG_ERR_ARG, "batch", "level overflow");
-    M.Llev[M.nlev] = 16;
-    M.Ylev[M.nlev] = Y;
-    const uint32_t ch = (uint32_t)((Y + 15) / 16);
-    M.nch[++M.nlev] = ch;
-    Y = 2ull * ch;
-    prev = ch;
-  }
+  M.nch = (uint32_t)std::max<uint64_t>(1, (M.total_max + M.L1 - 1) / M.L1);
+  M.pcap = M.nch / 8 + 2;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t r = o; o = (o + bytes + 255) & ~size_t(255); return r; };
   M.o_std = take((size_t)M.npts * 32);
-  M.o_cnt = take((size_t)M.nseg * 4 + 4);
+  M.o_cnt = take((size_t)M.nseg * 4 + 4 + (size_t)M.nwins * 4);   // then: pieces; finished blocks a window
   M.o_off = take((size_t)M.nseg * 4 + 4);
   M.o_cur = take((size_t)M.nseg * 4 + 4);
   const uint32_t nb = (M.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
@@ -1586,19 +1491,16 @@ static zkg_status make_multi_plan(const std::vector<int>& ns, const std::vector<
   M.o_bs = take((size_t)nb * 4 + 4);
   M.o_ent = take((size_t)M.total_max * 4 + 4);
   M.o_rank = take((size_t)M.total_max * 4 + 4);
-  uint64_t slotsA = 2ull * M.nch[0], slotsB = 0;
-  for (int k = 1; k <= M.nlev; k++) {
-    if (k % 2 == 1) slotsB = std::max<uint64_t>(slotsB, 2ull * M.nch[k]);
-    else slotsA = std::max<uint64_t>(slotsA, 2ull * M.nch[k]);
-  }
-  M.o_keyA = take(slotsA * 4);
-  M.o_ptA = take(slotsA * XB);
-  M.o_keyB = take(slotsB * 4 + 4);
-  M.o_ptB = take(slotsB * XB + 4);
+  M.o_keyA = take((size_t)M.nch * 8);
+  M.o_ptA = take((size_t)M.nch * 2 * XB);
+  M.o_prec = take((size_t)M.pcap * sizeof(Piece));
+  M.o_pdone = take((size_t)M.pcap * 4);
+  M.o_ppt = take((size_t)M.pcap * XB);
   M.o_bsum = take((size_t)M.nseg * XB);
   M.o_T = take((size_t)M.nthr * XB);
   M.o_R = take((size_t)M.nthr * XB);
   M.o_U = take((size_t)M.nblk * XB);
+  M.o_V = take((size_t)M.nwins * XB);
   M.o_reqs = take(M.reqs.size() * sizeof(MReq));
   M.bytes = o;
   return ZKG_OK;
@@ -1610,8 +1512,6 @@ static zkg_status make_multi_plan(const std::vector<int>& ns, const std::vector<
 template <class C>
 static zkg_status multi_msm_launch(const MultiPlan& M, char* ws, const uint64_t* d_bases, cudaStream_t st,
                                    int phase = 0) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
   const MReq* reqs = reinterpret_cast<const MReq*>(ws + M.o_reqs);
   const int nreq = (int)M.reqs.size();
@@ -1621,44 +1521,30 @@ static zkg_status multi_msm_launch(const MultiPlan& M, char* ws, const uint64_t*
   const uint32_t* off = U32(M.o_off);
   if (phase != 2) {
   ZKB_TRY(launch("mmsm_from_mont", k_mmsm_from_mont<C>, gp, dim3(256), 0, st, reqs, nreq, M.npts, U32(M.o_std)));
-  ZKB_CUDA(cudaMemsetAsync(U32(M.o_cnt), 0, (size_t)M.nseg * 4, st));
+  ZKB_CUDA(cudaMemsetAsync(U32(M.o_cnt), 0, (size_t)(M.nseg + 1 + M.nwins) * 4, st));
   ZKB_TRY(launch("mmsm_hist", k_mmsm_hist, gp, dim3(256), 0, st, reqs, nreq, M.npts, (const uint32_t*)U32(M.o_std),
                  U32(M.o_cnt), U32(M.o_rank)));
-  const uint32_t nb = (M.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
-  ZKB_TRY(launch("scan_blocks", k_scan_blocks, dim3(nb), dim3(SCAN_T), 0, st, (const uint32_t*)U32(M.o_cnt),
-                 U32(M.o_off), U32(M.o_bs), M.nseg));
-  ZKB_TRY(launch("scan_top", k_scan_top, dim3(1), dim3(SCAN_T), 0, st, U32(M.o_bs), nb));
-  ZKB_TRY(launch("scan_add", k_scan_add, dim3((M.nseg + 255) / 256), dim3(256), 0, st, U32(M.o_off),
-                 U32(M.o_cur), (const uint32_t*)U32(M.o_bs), M.nseg, nb));
+  ZKB_TRY(scan_counts(U32(M.o_cnt), U32(M.o_off), U32(M.o_cur), U32(M.o_bs), M.nseg, st));
   ZKB_TRY(launch("mmsm_scatter", k_mmsm_scatter, gp, dim3(256), 0, st, reqs, nreq, M.npts,
                  (const uint32_t*)U32(M.o_std), (const uint32_t*)U32(M.o_off), (const uint32_t*)U32(M.o_rank),
                  U32(M.o_ent)));
   if (phase == 1) return ZKG_OK;
-  ZKB_TRY(launch_accum<C>(M.nch[0], st, ent, off, M.nseg, (uint32_t)M.L1, bases, U32(M.o_bsum), U32(M.o_keyA),
+  ZKB_TRY(launch_accum<C>(M.nch, st, ent, off, M.nseg, (uint32_t)M.L1, bases, U32(M.o_bsum), U32(M.o_keyA),
                           U32(M.o_ptA)));
   }
-  ZKB_TRY(launch("mmsm_pair_merge", k_msm_pair_merge<C>, dim3((M.nch[0] + 255) / 256), dim3(256), 0, st, off, M.nch[0], (uint32_t)M.L1,
-                 U32(M.o_keyA), (const uint32_t*)U32(M.o_ptA), U32(M.o_bsum), (uint32_t*)nullptr, M.nseg));
-  LevelHist hist;
-  hist.n = 1;
-  hist.L[0] = (uint32_t)M.L1;
-  for (int k = 0; k < M.nlev; k++) {
-    const bool fromA = (k % 2 == 0);
-    const uint32_t ch = M.nch[k + 1];
-    ZKB_TRY(launch("mmsm_seg_level", k_msm_seg_level<C>, dim3((ch + 255) / 256), dim3(256), 0, st,
-                   (const uint32_t*)U32(fromA ? M.o_keyA : M.o_keyB), (const uint32_t*)U32(fromA ? M.o_ptA : M.o_ptB),
-                   (uint32_t)M.Ylev[k], M.Llev[k], ch, hist, off, U32(M.o_bsum), U32(fromA ? M.o_keyB : M.o_keyA),
-                   U32(fromA ? M.o_ptB : M.o_ptA)));
-    hist.L[hist.n++] = M.Llev[k];
-  }
-  ZKB_TRY(launch("mmsm_bucket_rs", k_mmsm_bucket_rs<C>, dim3((M.nthr + 127) / 128), dim3(128), 0, st, reqs, nreq,
-                 M.nthr, (const uint32_t*)U32(M.o_bsum), off, U32(M.o_T), U32(M.o_R)));
-  ZKB_TRY(launch("mmsm_bucket_bits", k_mmsm_bucket_bits<C>, dim3(M.nblk), dim3(256), (size_t)256 * XW * 4, st, reqs,
-                 nreq, (const uint32_t*)U32(M.o_T), (const uint32_t*)U32(M.o_R), U32(M.o_U)));
+  const PieceList pl = {U32(M.o_cnt) + M.nseg, M.pcap, reinterpret_cast<Piece*>(ws + M.o_prec), U32(M.o_pdone),
+                        U32(M.o_ppt)};
+  ZKB_TRY(msm_launch_merge<C>(pl, off, nullptr, M.nch, (uint32_t)M.L1, U32(M.o_keyA), U32(M.o_ptA), U32(M.o_bsum),
+                              M.nseg, st));
+  MReqs q = {};
+  q.tab = reqs;
+  q.n = nreq;
+  ZKB_TRY(msm_launch_windows<C>(q, M.nthr, M.nblk, M.gmax, U32(M.o_bsum), off, U32(M.o_T), U32(M.o_R), U32(M.o_U),
+                                U32(M.o_cnt) + M.nseg + 1, U32(M.o_V), st));
   return ZKG_OK;
 }
 
-// Host tails of a finished batch (U copied to host), spread over CPU threads.
+// Host tails of a finished batch (V copied to host), spread over CPU threads.
 template <int NL>
 static void multi_msm_tails(const host::Field<NL>& F, const MultiPlan& M, const uint64_t* U,
                             const std::vector<uint64_t*>& outs, const std::vector<int>& kinds) {
@@ -1666,12 +1552,7 @@ static void multi_msm_tails(const host::Field<NL>& F, const MultiPlan& M, const 
   auto work = [&](int lo, int hi) {
     for (int r = lo; r < hi; r++) {
       const MReq& q = M.reqs[r];
-      MsmPlan P;
-      P.c = (int)q.c;
-      P.nwin = (int)q.nwin;
-      P.gbits = (int)q.gbits;
-      P.K1 = q.K1;
-      const host::Xyzz<NL> res = msm_host_combine<NL>(F, P, U + (size_t)q.blk_off * 4 * NL);
+      const host::Xyzz<NL> res = msm_host_combine<NL>(F, q.win, (int)q.nwin, U + (size_t)q.win_off * 4 * NL);
       host::xyzz_write<NL>(F, res, kinds[M.owner[r]], outs[M.owner[r]]);
     }
   };
@@ -1844,7 +1725,7 @@ static zkg_status batch_build_persistent(zkg_batch* b, const host::Field<NL>& F)
       if (d.dep >= 0) { d.dep_count += 1; break; }
   }
   const uint32_t bt = (uint32_t)batch_work_threads(b->curve);   // chunks per accumulation task
-  const uint32_t nacc = b->mp.reqs.empty() ? 0u : (b->mp.nch[0] + bt - 1) / bt;
+  const uint32_t nacc = b->mp.reqs.empty() ? 0u : (b->mp.nch + bt - 1) / bt;
   // queue: the tiles of pass step e, then a share of the accumulation blocks, for every step; the
   // accumulation between two steps covers the time the earlier step's tiles take to finish, so a
   // later step's tiles rarely wait, and the queue ends with accumulation work that fills every SM
@@ -1889,7 +1770,7 @@ static zkg_status batch_build_persistent(zkg_batch* b, const host::Field<NL>& F)
     ZKB_CUDA(cudaMemcpy(ws + o_descs, descs.data(), descs.size() * sizeof(NttPassDesc), cudaMemcpyHostToDevice));
   if (!b->mp.reqs.empty())
     ZKB_CUDA(cudaMemcpy(ws + b->mp.o_reqs, b->mp.reqs.data(), b->mp.reqs.size() * sizeof(MReq), cudaMemcpyHostToDevice));
-  b->ubytes = (size_t)b->mp.nblk * 4 * NL * 8;
+  b->ubytes = (size_t)b->mp.nwins * 4 * NL * 8;
   b->err_pin_off = rup(b->ubytes);
   ZKB_CUDA(cudaMallocHost(&b->pin, b->err_pin_off + 64));
   ZKB_CUDA(cudaEventCreate(&b->ev0));
@@ -1912,7 +1793,7 @@ static zkg_status batch_build_persistent(zkg_batch* b, const host::Field<NL>& F)
     W.ent = reinterpret_cast<const uint32_t*>(ws + b->mp.o_ent);
     W.off = reinterpret_cast<const uint32_t*>(ws + b->mp.o_off);
     W.nseg = b->mp.nseg;
-    W.nch = b->mp.nch[0];
+    W.nch = b->mp.nch;
     W.L = (uint32_t)b->mp.L1;
     if (b->conv_off) msm_bases = reinterpret_cast<const uint64_t*>(ws + b->conv_off);
     W.bases = reinterpret_cast<const uint32_t*>(msm_bases);
@@ -1945,9 +1826,9 @@ static zkg_status batch_build_persistent(zkg_batch* b, const host::Field<NL>& F)
     if (!b->mp.reqs.empty()) {
       ZKB_TRY(multi_msm_launch<CD>(b->mp, ws, msm_bases, st, 2));
       if constexpr (radix_conv_v<typename CD::Fp>)
-        ZKB_TRY(launch("msm_xyzz_from_dpf", k_msm_xyzz_from_dpf<CD>, dim3((4 * b->mp.nblk + 255) / 256), dim3(256),
-                       0, st, (uint32_t)b->mp.nblk, reinterpret_cast<uint32_t*>(ws + b->mp.o_U), dpf_kout<CD>()));
-      ZKB_CUDA(cudaMemcpyAsync(b->pin, ws + b->mp.o_U, b->ubytes, cudaMemcpyDeviceToHost, st));
+        ZKB_TRY(launch("msm_xyzz_from_dpf", k_msm_xyzz_from_dpf<CD>, dim3((4 * b->mp.nwins + 255) / 256), dim3(256),
+                       0, st, (uint32_t)b->mp.nwins, reinterpret_cast<uint32_t*>(ws + b->mp.o_V), dpf_kout<CD>()));
+      ZKB_CUDA(cudaMemcpyAsync(b->pin, ws + b->mp.o_V, b->ubytes, cudaMemcpyDeviceToHost, st));
     }
     ZKB_CUDA(cudaMemcpyAsync(static_cast<char*>(b->pin) + b->err_pin_off, W.error, 4, cudaMemcpyDeviceToHost, st));
     return ZKG_OK;
@@ -2004,7 +1885,7 @@ static zkg_status batch_build(zkg_batch* b, const host::Field<NL>& F) {
   char* ws = static_cast<char*>(b->ws);
   if (!b->mp.reqs.empty())
     ZKB_CUDA(cudaMemcpy(ws + b->mp.o_reqs, b->mp.reqs.data(), b->mp.reqs.size() * sizeof(MReq), cudaMemcpyHostToDevice));
-  b->ubytes = (size_t)b->mp.nblk * 4 * NL * 8;
+  b->ubytes = (size_t)b->mp.nwins * 4 * NL * 8;
   ZKB_CUDA(cudaMallocHost(&b->pin, std::max<size_t>(b->ubytes, 64)));
   ZKB_CUDA(cudaEventCreate(&b->ev0));
   ZKB_CUDA(cudaEventCreate(&b->ev1));
@@ -2031,18 +1912,18 @@ static zkg_status batch_build(zkg_batch* b, const host::Field<NL>& F) {
         ZKB_TRY(launch("msm_bases_to_dpf", k_msm_bases_to_dpf<CD>, dim3((b->conv_n + 255) / 256), dim3(256), 0,
                        b->s_main, b->conv_n, reinterpret_cast<const uint32_t*>(b->d_bases), kin, conv));
         ZKB_TRY(multi_msm_launch<CD>(b->mp, ws, reinterpret_cast<const uint64_t*>(conv), b->s_main));
-        ZKB_TRY(launch("msm_xyzz_from_dpf", k_msm_xyzz_from_dpf<CD>, dim3((4 * b->mp.nblk + 255) / 256), dim3(256), 0,
-                       b->s_main, (uint32_t)b->mp.nblk, reinterpret_cast<uint32_t*>(ws + b->mp.o_U), kout));
+        ZKB_TRY(launch("msm_xyzz_from_dpf", k_msm_xyzz_from_dpf<CD>, dim3((4 * b->mp.nwins + 255) / 256), dim3(256), 0,
+                       b->s_main, (uint32_t)b->mp.nwins, reinterpret_cast<uint32_t*>(ws + b->mp.o_V), kout));
       } else if (g_msm_dpf) {   // bases already in the pipeline's form
         ZKB_TRY(multi_msm_launch<CD>(b->mp, ws, b->d_bases, b->s_main));
         if constexpr (radix_conv_v<typename CD::Fp>)
-          ZKB_TRY(launch("msm_xyzz_from_dpf", k_msm_xyzz_from_dpf<CD>, dim3((4 * b->mp.nblk + 255) / 256), dim3(256),
-                         0, b->s_main, (uint32_t)b->mp.nblk, reinterpret_cast<uint32_t*>(ws + b->mp.o_U),
+          ZKB_TRY(launch("msm_xyzz_from_dpf", k_msm_xyzz_from_dpf<CD>, dim3((4 * b->mp.nwins + 255) / 256), dim3(256),
+                         0, b->s_main, (uint32_t)b->mp.nwins, reinterpret_cast<uint32_t*>(ws + b->mp.o_V),
                          dpf_kout<CD>()));
       } else {
         ZKB_TRY(multi_msm_launch<C>(b->mp, ws, b->d_bases, b->s_main));
       }
-      ZKB_CUDA(cudaMemcpyAsync(b->pin, ws + b->mp.o_U, b->ubytes, cudaMemcpyDeviceToHost, b->s_main));
+      ZKB_CUDA(cudaMemcpyAsync(b->pin, ws + b->mp.o_V, b->ubytes, cudaMemcpyDeviceToHost, b->s_main));
     }
     for (int i = 0; i < nstreams; i++) {
       ZKB_CUDA(cudaEventRecord(b->ev_fork[i], b->s_ntt[i]));
@@ -2230,9 +2111,9 @@ static zkg_status srv_launch(Srv& S, SrvSlot& sl) {
                                nullptr, false, false));
     ZKB_TRY(msm_launch_reduce<C>(*cx, sl.P, ws, parts, sl.st, false));
   }
-  const size_t ubytes = (size_t)sl.P.nwin * (sl.P.gbits + 1) * 4 * NL * 8;
+  const size_t ubytes = (size_t)sl.P.nwin * 4 * NL * 8;
   if (sl.pin_cap < ubytes) return set_status(ZKG_ERR_ARG, "server", "slot staging smaller than a request's sums");
-  ZKB_CUDA(cudaMemcpyAsync(sl.pin, ws + sl.P.o_U, ubytes, cudaMemcpyDeviceToHost, sl.st));
+  ZKB_CUDA(cudaMemcpyAsync(sl.pin, ws + sl.P.o_V, ubytes, cudaMemcpyDeviceToHost, sl.st));
   ZKB_CUDA(cudaEventRecord(sl.done, sl.st));
   return ZKG_OK;
 }
@@ -2275,7 +2156,7 @@ static void srv_loop(Srv* S, const host::Field<NL>* F) {
     if (!done.empty()) {
       lk.unlock();
       for (SrvSlot* sl : done) {
-        const host::Xyzz<NL> r = msm_host_combine<NL>(*F, sl->P, static_cast<const uint64_t*>(sl->pin));
+        const host::Xyzz<NL> r = msm_host_combine<NL>(*F, sl->P.win, sl->P.nwin, static_cast<const uint64_t*>(sl->pin));
         host::xyzz_write<NL>(*F, r, ZKG_OUT_AFFINE, sl->req.out);
       }
       lk.lock();
@@ -2388,7 +2269,7 @@ static zkg_status srv_start(Srv* S, const host::Field<NL>* F, const host::Field<
       return set_status(ZKG_ERR_ARG, "zkg_server_create", "HBM budget smaller than one request of the largest size");
     S->req_bytes[k] = b;
     S->req_plan[k] = P;
-    ubytes_max = std::max(ubytes_max, (size_t)P.nwin * (P.gbits + 1) * 4 * NL * 8);
+    ubytes_max = std::max(ubytes_max, (size_t)P.nwin * 4 * NL * 8);
   }
   ZKB_CUDA(cudaMalloc(&S->pool, S->budget));
   S->free_list[0] = S->budget;
