@@ -342,91 +342,137 @@ __device__ __forceinline__ Fe<P> fe_pow(const Fe<P>& a, const uint32_t (&e)[EW])
   return acc;
 }
 
-// a^-1 = a^(p-2) (Fermat); 0 maps to 0, as the reference's inversion does
-// (bn128_Fr_std.c:298-301)
+// Inverse of the integer a (0 < a < 2p, prime to p) modulo p, in words, for one thread that others wait
+// for: Bernstein and Yang's division steps ("Fast constant-time gcd computation and modular inversion",
+// 2019) in variable time, 30 at a time. The steps of one batch see only the low words of f and g and
+// give a matrix (u v; q r) with entries up to 2^30; then
+//     f, g <- (u f + v g) / 2^30, (q f + r g) / 2^30            exactly, two's complement
+//     d, e <- (u d + v e) / 2^30, (q d + r e) / 2^30   mod p    in [0, p), by a Montgomery step
+// keep d a = f and e a = g (mod p) from f = p, g = a, d = 0, e = 1 until g = 0, f = +-1. At most
+// (49 * bits + 57) / 17 steps. About 18 batches of ~1500 cycles for 254 bits; halving and subtracting
+// whole numbers bit by bit took ~500 rounds of word chains, a^(p-2) ~380 products one after the other.
 template <class P>
-__device__ __forceinline__ Fe<P> fe_inv_fermat(const Fe<P>& a) {
-  uint32_t e[P::N];   // p - 2 (BLS12-381 r has low word 1, so the borrow can propagate)
-  uint32_t borrow = 2;
+__device__ __noinline__ Fe<P> inv_words(const Fe<P> a) {
+  constexpr int N = P::N;
+  constexpr uint32_t M30 = (1u << 30) - 1;
+  uint32_t f[N + 1], g[N + 1], d[N], e[N];
 #pragma unroll
-  for (int i = 0; i < P::N; i++) {
-    const uint32_t w = P::mod(i);
-    e[i] = w - borrow;
-    borrow = w < borrow ? 1u : 0u;
+  for (int k = 0; k < N; k++) { f[k] = P::mod(k); g[k] = a.v[k]; d[k] = 0; e[k] = 0; }
+  f[N] = g[N] = 0;
+  e[0] = 1;
+  int eta = -1;   // -delta
+#pragma unroll 1
+  for (int batch = 0; batch < (49 * (32 * N + 1) + 57) / 17 / 30 + 1; batch++) {
+    uint32_t any = 0;
+#pragma unroll
+    for (int k = 0; k <= N; k++) any |= g[k];
+    if (!any) break;
+    int u = 1, v = 0, q = 0, r = 1, left = 30;
+    uint32_t x = f[0], y = g[0];
+    while (true) {
+      const int z = __ffs((int)(y | (1u << left))) - 1;   // even g: delta + 1, g / 2 (u, v scale instead)
+      y >>= z;
+      u = (int)((uint32_t)u << z);
+      v = (int)((uint32_t)v << z);
+      eta -= z;
+      left -= z;
+      if (left == 0) break;
+      if (eta < 0) {   // delta > 0, g odd: (f, g) <- (g, -f), then g gets a multiple of f below
+        eta = -eta;
+        uint32_t t = x; x = y; y = 0u - t;
+        int w = u; u = q; q = -w;
+        w = v; v = r; r = -w;
+      }
+      // g + m f has its low bits zero for m = -g / f modulo a power of two (f is its own inverse mod 8);
+      // delta stays <= 0 for eta + 1 steps, so that many bits may go at once
+      const int bits = min(min(eta + 1, left), 6);
+      const uint32_t fi = x * (2u - x * x);
+      const int m = (int)((0u - y * fi) & ((1u << bits) - 1));
+      y += (uint32_t)m * x;
+      q += m * u;
+      r += m * v;
+    }
+    auto fg = [&](int s, int t, uint32_t (&o)[N + 1]) {   // (s f + t g) >> 30
+      long long c = 0;
+      uint32_t w[N + 1];
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        c += (long long)s * f[k] + (long long)t * g[k];
+        w[k] = (uint32_t)c;
+        c >>= 32;
+      }
+      c += (long long)s * (int)f[N] + (long long)t * (int)g[N];
+      w[N] = (uint32_t)c;
+#pragma unroll
+      for (int k = 0; k < N; k++) o[k] = (w[k] >> 30) | (w[k + 1] << 2);
+      o[N] = (uint32_t)((int)w[N] >> 30);
+    };
+    auto de = [&](int s, int t, uint32_t (&o)[N]) {   // (s d + t e + 2^30 p + k p) / 2^30 < 3p, reduced
+      long long c = 0;   // |s| + |t| <= 2^30, so a column stays below 2^63
+      uint32_t w[N + 1];
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        c += (long long)s * d[k] + (long long)t * e[k] + ((long long)P::mod(k) << 30);
+        w[k] = (uint32_t)c;
+        c >>= 32;
+      }
+      w[N] = (uint32_t)c;
+      const uint32_t km = (w[0] * P::n0) & M30;   // k = -(s d + t e) / p mod 2^30
+      unsigned long long h = 0;
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        h += (unsigned long long)km * P::mod(k) + w[k];
+        w[k] = (uint32_t)h;
+        h >>= 32;
+      }
+      w[N] += (uint32_t)h;
+#pragma unroll
+      for (int k = 0; k < N; k++) o[k] = (w[k] >> 30) | (w[k + 1] << 2);
+      uint32_t hi = w[N] >> 30;   // 3p may need one bit more than N words
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        uint32_t t2[N];
+        t2[0] = sub_cc(o[0], P::mod(0));
+#pragma unroll
+        for (int k = 1; k < N; k++) t2[k] = subc_cc(o[k], P::mod(k));
+        const uint32_t th = subc(hi, 0);
+        const bool less = (int)th < 0;
+#pragma unroll
+        for (int k = 0; k < N; k++) o[k] = less ? o[k] : t2[k];
+        hi = less ? hi : th;
+      }
+    };
+    uint32_t nf[N + 1], ng[N + 1], nd[N], ne[N];
+    fg(u, v, nf);
+    fg(q, r, ng);
+    de(u, v, nd);
+    de(q, r, ne);
+#pragma unroll
+    for (int k = 0; k <= N; k++) { f[k] = nf[k]; g[k] = ng[k]; }
+#pragma unroll
+    for (int k = 0; k < N; k++) { d[k] = nd[k]; e[k] = ne[k]; }
   }
-  return fe_pow<P, P::N>(a, e);
+  Fe<P> o;   // f = 1: d, f = -1: p - d (d is not 0)
+  uint32_t b = 0;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const unsigned long long t = (unsigned long long)P::mod(k) - d[k] - b;
+    o.v[k] = (int)f[N] < 0 ? (uint32_t)t : d[k];
+    b = (uint32_t)(t >> 63);
+  }
+  return o;
 }
 
-// a^-1 for a Montgomery element a = x R (result x^-1 R; 0 maps to 0), by the binary extended
-// Euclidean algorithm on the integer a and p (each step halves u or v, or subtracts the smaller
-// from the larger, so at most 2 (bits(a) + bits(p)) steps; capped at 32 N * 8). The integer
-// inverse a^-1 = x^-1 R^-1 is brought back to Montgomery form by one product with R^3 =
-// mont(R^2, R^2). Its dependency chain is a few thousand word operations, against ~380
-// sequential products for a^(p-2): the inversion one thread runs for a whole block.
+// a^-1 for a Montgomery element a = x R (result x^-1 R; 0 maps to 0, as the reference's inversion does,
+// bn128_Fr_std.c:298-301): the integer inverse x^-1 R^-1, brought back by one product with R^3 =
+// mont(R^2, R^2).
 template <class P>
-__device__ Fe<P> fe_inv_binary(const Fe<P>& a) {
-  constexpr int N = P::N;
-  if (fe_is_zero(a)) return fe_zero<P>();
-  uint32_t u[N], v[N], x1[N], x2[N];
-  for (int k = 0; k < N; k++) { u[k] = a.v[k]; v[k] = P::mod(k); x1[k] = 0; x2[k] = 0; }
-  x1[0] = 1;
-  auto is_one = [](const uint32_t* w) {
-    uint32_t o = w[0] ^ 1u;
-    for (int k = 1; k < N; k++) o |= w[k];
-    return o == 0;
-  };
-  auto halve = [](uint32_t* w) {
-    for (int k = 0; k < N - 1; k++) w[k] = (w[k] >> 1) | (w[k + 1] << 31);
-    w[N - 1] >>= 1;
-  };
-  auto halve_mod = [&](uint32_t* x) {   // x / 2 mod p (x + p < 2^(32 N): p has a spare top bit)
-    if (x[0] & 1u) {
-      uint64_t c = 0;
-      for (int k = 0; k < N; k++) {
-        c += (uint64_t)x[k] + P::mod(k);
-        x[k] = (uint32_t)c;
-        c >>= 32;
-      }
-    }
-    halve(x);
-  };
-  auto geq = [](const uint32_t* x, const uint32_t* y) {
-    for (int k = N - 1; k >= 0; k--)
-      if (x[k] != y[k]) return x[k] > y[k];
-    return true;
-  };
-  auto sub = [](uint32_t* x, const uint32_t* y) {   // x -= y; returns the borrow
-    uint32_t b = 0;
-    for (int k = 0; k < N; k++) {
-      const uint64_t d = (uint64_t)x[k] - y[k] - b;
-      x[k] = (uint32_t)d;
-      b = (uint32_t)(d >> 63);
-    }
-    return b;
-  };
-  auto sub_mod = [&](uint32_t* x, const uint32_t* y) {   // x = x - y mod p
-    if (sub(x, y)) {
-      uint64_t c = 0;
-      for (int k = 0; k < N; k++) {
-        c += (uint64_t)x[k] + P::mod(k);
-        x[k] = (uint32_t)c;
-        c >>= 32;
-      }
-    }
-  };
-  for (int it = 0; it < 32 * N * 8; it++) {
-    if (is_one(u) || is_one(v)) break;
-    if (!(u[0] & 1u)) { halve(u); halve_mod(x1); }
-    else if (!(v[0] & 1u)) { halve(v); halve_mod(x2); }
-    else if (geq(u, v)) { sub(u, v); sub_mod(x1, x2); }
-    else { sub(v, u); sub_mod(x2, x1); }
-  }
-  Fe<P> r;
-  const bool one_u = is_one(u);
-  for (int k = 0; k < N; k++) r.v[k] = one_u ? x1[k] : x2[k];
+__device__ __forceinline__ Fe<P> fe_inv(const Fe<P>& a) {
+  if (fe_is_zero_mod(a)) return fe_zero<P>();
   Fe<P> r2;
-  for (int k = 0; k < N; k++) r2.v[k] = P::r2(k);
-  return fe_mul(r, fe_mul(r2, r2));
+#pragma unroll
+  for (int k = 0; k < P::N; k++) r2.v[k] = P::r2(k);
+  return fe_mul(inv_words(a), fe_mul(r2, r2));
 }
 
 // x -> x * R^-1 (Montgomery -> standard), the reference's to_std (bn128_Fr_mont.c:330)

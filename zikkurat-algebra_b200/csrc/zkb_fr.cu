@@ -10,8 +10,8 @@
 //   - mul_by_powers: the reference loop starts at i = 1 with x = A, so tgt[0] is left unwritten
 //     and tgt[i] = src[i] * A * B^(i-1) for i >= 1 (bn128_arr_mont.c:203-211); kept as is;
 //   - batch inversion: Montgomery's trick over the strided subset i = t, t + T, ... of each
-//     thread, the thread products combined across the block by two scans, one inversion (binary
-//     extended Euclid) per block. The reference multiplies all n elements into one
+//     thread, the thread products combined across the block by two scans, one inversion (division
+//     steps) per block. The reference multiplies all n elements into one
 //     product and inverts it, so one zero element makes every output zero; a device flag
 //     reproduces that;
 //   - dot product: block partial sums, then one block sums the partials (modular sums are exact
@@ -163,16 +163,13 @@ __global__ void k_fr_powers(int n, int shift, const uint32_t* src, const uint32_
 }
 
 // Batch inversion with one inversion per block: each thread multiplies its strided subset
-// (prefix products kept in scratch), the block combines the thread products by two scans, thread 0
-// inverts the block's total, and each thread derives the inverse of its own product as
-// inv(total) * (product of the threads before it) * (product of the threads after it), then
-// runs its backward pass. A zero element makes the total zero and every output zero, as in the
-// reference; *zero_flag records it for the operations that need it.
+// (prefix products kept in scratch), the block inverts the thread products by one inversion
+// (block_inverse), and each thread runs its backward pass. A zero element makes the total zero and
+// every output zero, as in the reference; *zero_flag records it for the operations that need it.
 template <class P>
-__global__ void __launch_bounds__(256) k_fr_batch_inv_blk(int n, const uint32_t* a, uint32_t* __restrict__ scratch,
+__global__ void __launch_bounds__(256, 3) k_fr_batch_inv_blk(int n, const uint32_t* a, uint32_t* __restrict__ scratch,
                                                           uint32_t* out, int* __restrict__ zero_flag) {
-  __shared__ Fe<P> sw[9];
-  __shared__ Fe<P> s_inv;
+  __shared__ Fe<P> sw[16];
   const size_t T = (size_t)gridDim.x * blockDim.x;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   Fe<P> acc = fe_one<P>();
@@ -184,13 +181,8 @@ __global__ void __launch_bounds__(256) k_fr_batch_inv_blk(int n, const uint32_t*
     st<P>(scratch, i, acc);
     last = i;
   }
-  Fe<P> total, total2;
-  const Fe<P> before = block_mul_excl_scan<P, false>(acc, sw, total);
-  const Fe<P> after = block_mul_excl_scan<P, true>(acc, sw, total2);
-  if (threadIdx.x == 0) s_inv = fe_inv_binary(total);
-  __syncthreads();
+  Fe<P> inv = block_inverse<P, 8>(acc, sw);
   if (t >= (size_t)n) return;
-  Fe<P> inv = fe_mul(fe_mul(s_inv, before), after);   // inverse of this thread's product
   for (size_t i = last;; i -= T) {
     const Fe<P> x = ld<P>(a, i);      // read before out[i] is written (a may alias out)
     st<P>(out, i, i >= t + T ? fe_mul(inv, ld<P>(scratch, i - T)) : inv);
@@ -333,7 +325,7 @@ static zkg_status fr_launch_map(Context& cx, int op, int n, const uint32_t* a, c
     }
     case FR_INV:
     case FR_DIV: {
-      // about 32 elements per thread's chain, one inversion (binary extended Euclid) per block of
+      // about 8 elements per thread's chain, one inversion (division steps) per block of
       // 256 threads, and at most one wave of resident blocks (a second wave would wait for the
       // first one's serial inversions before starting its own)
       static int inv_per_sm[64];   // resident blocks per SM, per device (the context lock is held)
@@ -345,7 +337,7 @@ static zkg_status fr_launch_map(Context& cx, int op, int n, const uint32_t* a, c
       }
       const size_t wave = (size_t)cx.sm_count * bps * 256;
       const size_t T = std::min<size_t>(std::min<size_t>(((size_t)n + 255) & ~size_t(255), wave),
-                                        std::max<size_t>(2048, (size_t)n / 32));
+                                        std::max<size_t>(2048, (size_t)n / 8));
       const unsigned g = (unsigned)((T + 255) / 256);
       ZKB_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
       uint32_t* inv_out = op == FR_INV ? out : scratch2;

@@ -76,7 +76,7 @@ __device__ void xyzz_write_out(const Xyzz<F>& p, int kind, uint32_t* __restrict_
     fe_store<F>(out + 2 * F::N, fe_zero<F>());
     return;
   }
-  const Fe<F> d = fe_inv_fermat(fe_mul(p.ZZ, p.ZZZ));
+  const Fe<F> d = fe_inv(fe_mul(p.ZZ, p.ZZZ));
   Fe<F> x = fe_mul(p.X, fe_mul(d, p.ZZZ)), y = fe_mul(p.Y, fe_mul(d, p.ZZ));
   if (CONV) {
     x = fe_mul(x, kout);

@@ -930,8 +930,8 @@ static zkg_status launch_tree_level(const MsmPlan& P, uint32_t nthr, cudaStream_
   ZKB_TRY((tree_smem_limit<true, C, L0, NTF, PFF>(k_tree_fwd<C, L0, NTF, PFF>, smf)));
   ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, L0, NTF, PFF>, dim3((nthr + NTF - 1) / NTF), dim3(NTF), smf, st, ent,
                  in_pts, in_off, out_off, P.nseg, P.tB, nthr, pre, tt, chk, npts));
-  // simultaneous inversion of the thread products: about 16 per thread
-  const size_t T = std::min<size_t>(((size_t)nthr + 255) & ~size_t(255), std::max<size_t>(2048, (size_t)nthr / 16));
+  // simultaneous inversion of the thread products: about 4 per thread
+  const size_t T = std::min<size_t>(((size_t)nthr + 255) & ~size_t(255), std::max<size_t>(2048, (size_t)nthr / 4));
   ZKB_TRY(launch("msm_tree_inv", k_tree_inv<F>, dim3((unsigned)((T + 255) / 256)), dim3(256), 0, st, nthr, tt, scr));
   // backward pass: one block per SM, as the accumulation (BN254: 384 threads, 166 registers)
   constexpr int NTB = F::N == 8 ? 384 : 256;

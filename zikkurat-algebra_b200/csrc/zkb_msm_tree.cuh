@@ -9,7 +9,7 @@
 //   1. output offsets: exclusive scan of ceil(m_s / 2) over the segments (the sort's scan kernels);
 //   2. k_tree_fwd: each thread takes B consecutive output slots, forms their denominators and
 //      stores the running product before each one; the thread's whole product goes to tt;
-//   3. k_tree_inv: tt is inverted in place (simultaneous inversion again, one binary-Euclid
+//   3. k_tree_inv: tt is inverted in place (simultaneous inversion again, one
 //      inversion per block);
 //   4. k_tree_bwd: each thread walks its slots backwards, peeling one denominator inverse per slot
 //      off the inverse of its product, and writes each slot's sum as canonical affine coordinates.
@@ -227,8 +227,7 @@ __global__ void __launch_bounds__(NT) k_tree_fwd(const uint32_t* __restrict__ en
 template <class F>
 __global__ void __launch_bounds__(256) k_tree_inv(uint32_t n, uint32_t* __restrict__ tt, uint32_t* __restrict__ scr) {
   constexpr int FW = F::N;
-  __shared__ Fe<F> sw[9];
-  __shared__ Fe<F> s_inv;
+  __shared__ Fe<F> sw[16];
   const size_t T = (size_t)gridDim.x * blockDim.x;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   Fe<F> acc = fe_one<F>();
@@ -238,13 +237,8 @@ __global__ void __launch_bounds__(256) k_tree_inv(uint32_t n, uint32_t* __restri
     fe_store<F>(scr + i * FW, acc);
     last = i;
   }
-  Fe<F> total, total2;
-  const Fe<F> before = block_mul_excl_scan<F, false>(acc, sw, total);
-  const Fe<F> after = block_mul_excl_scan<F, true>(acc, sw, total2);
-  if (threadIdx.x == 0) s_inv = fe_inv_binary(fe_canon(total));
-  __syncthreads();
+  Fe<F> inv = block_inverse<F, 8>(acc, sw);
   if (t >= (size_t)n) return;
-  Fe<F> inv = fe_mul(fe_mul(s_inv, before), after);   // inverse of this thread's product
   for (size_t i = last;; i -= T) {
     const Fe<F> x = fe_load<F>(tt + i * FW);
     fe_store<F>(tt + i * FW, i >= t + T ? fe_mul(inv, fe_load<F>(scr + (i - T) * FW)) : inv);

@@ -5,7 +5,7 @@
 //
 // Fixed-base comb: T[j][v] = v * 16^j * G for j < 64, v < 16 is built once on the host in
 // XYZZ coordinates; each thread adds one table entry per 4-bit digit of its scalar and converts
-// the sum to affine with a Fermat inversion.
+// the sum to affine with one inversion.
 #include <cstring>
 #include <vector>
 
@@ -34,7 +34,7 @@ __global__ void k_g1_gen_mul(int n, const uint64_t* __restrict__ ks, const uint3
     fe_store<F>(o + F::N, fe_zero<F>());
     return;
   }
-  const Fe<F> d = fe_inv_fermat(fe_mul(acc.ZZ, acc.ZZZ));
+  const Fe<F> d = fe_inv(fe_mul(acc.ZZ, acc.ZZZ));
   fe_store<F>(o, fe_mul(acc.X, fe_mul(d, acc.ZZZ)));
   fe_store<F>(o + F::N, fe_mul(acc.Y, fe_mul(d, acc.ZZ)));
 }
