@@ -43,6 +43,7 @@
 #include "zkb_curve.cuh"
 #include "zkb_dpf.cuh"
 #include "zkb_host_ec.h"
+#include "zkb_quad.cuh"
 #include "zkb_runtime.h"
 
 namespace zkb {
@@ -235,6 +236,149 @@ __global__ void k_g1fft_stage(int m, int s, const uint32_t* __restrict__ tw, con
   }
   xyzz_store<F>(a + (size_t)i0 * XW, o0);
   xyzz_store<F>(a + (size_t)i1 * XW, o1);
+}
+
+// The same stage by quads (zkb_quad.cuh), for transforms with too few butterflies to fill the GPU: a
+// scalar multiplication is a chain of ~210 point operations, and at 2^14 points a thread a butterfly
+// left one warp a scheduler (1.10 ms a stage; this 0.46). A butterfly has HALVES quads: with 2, each
+// multiplies by one half of the split scalar (quad 1 the image under phi) and the two results are
+// added: the shortest chain, at 1.5 times the work; with 1, the quad takes both halves in one scan.
+// The top stage of an inverse transform has two scalars and always two quads, one a scalar.
+// Tables 1P..8P lie in shared memory, a column a thread (sm), with the images' X in one more (smb).
+static constexpr int QUAD_T = 128;
+template <class F>
+__device__ __forceinline__ Fe<F> tab_ld(const uint32_t* sm, int e) {
+  Fe<F> r;
+#pragma unroll
+  for (int i = 0; i < F::N; i++) r.v[i] = sm[(e * F::N + i) * QUAD_T + threadIdx.x];
+  return r;
+}
+template <class F>
+__device__ __forceinline__ void tab_st(uint32_t* sm, int e, const Fe<F>& a) {
+#pragma unroll
+  for (int i = 0; i < F::N; i++) sm[(e * F::N + i) * QUAD_T + threadIdx.x] = a.v[i];
+}
+// [k]P with the digits of `both` halves (dg, dg2), or of one half (dg); all lanes call it
+template <class F>
+__device__ __noinline__ Fe<F> quad_mul_glv(const Fe<F> P, const uint32_t (&k)[GLV_WORDS], bool both, int half,
+                                           const Fe<F> beta, uint32_t* sm, uint32_t* smb) {
+  const int L = quad_lane();
+  uint32_t d1[5], d2[5];
+  glv_digits(half ? k + 5 : k, d1);
+  glv_digits(k + 5, d2);
+  const uint32_t s1 = (k[10] >> half) & 1u, s2 = (k[10] >> 1) & 1u;
+  Fe<F> t = P;
+  tab_st(sm, 0, t);
+#pragma unroll 1
+  for (int e = 2; e <= 8; e++) {   // 2P by doubling, then + P
+    t = e == 2 ? quad_dbl(t) : quad_add(t, P);
+    tab_st(sm, e - 1, t);
+  }
+  if (__any_sync(FULL, both)) {
+#pragma unroll 1
+    for (int e = 0; e < 8; e++) {
+      const Fe<F> b = fe_mul(tab_ld<F>(sm, e), beta);
+      if (L == 0)
+#pragma unroll
+        for (int i = 0; i < F::N; i++) smb[(e * F::N + i) * (QUAD_T / 4) + (threadIdx.x >> 2)] = b.v[i];
+    }
+  }
+  auto digit = [](const uint32_t (&dg)[5], int w) {
+    uint32_t v = 0;
+#pragma unroll
+    for (int i = 0; i < 5; i++)
+      if (i == (w >> 3)) v = dg[i];
+    return (int)((v >> (4 * (w & 7))) & 15u) - 7;
+  };
+  Fe<F> acc = fe_zero<F>();
+#pragma unroll 1
+  for (int w = 34; w >= 0; w--) {
+    if (w != 34)
+#pragma unroll 1
+      for (int i = 0; i < 4; i++) acc = quad_dbl(acc);
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      if (h == 1 && !__any_sync(FULL, both)) break;
+      const int d = h == 0 ? digit(d1, w) : both ? digit(d2, w) : 0;
+      const int e = (d < 0 ? -d : d) - 1;
+      Fe<F> q = fe_zero<F>();
+      if (d != 0) {
+        q = tab_ld<F>(sm, e);
+        if (h == 1 && L == 0)
+#pragma unroll
+          for (int i = 0; i < F::N; i++) q.v[i] = smb[(e * F::N + i) * (QUAD_T / 4) + (threadIdx.x >> 2)];
+        if (L == 1 && (d < 0) != ((h ? s2 : s1) != 0)) q = fe_neg(q);
+      }
+      acc = quad_add(acc, q);
+    }
+  }
+  return acc;
+}
+
+template <class C, bool INV, int HALVES>
+__global__ void __launch_bounds__(QUAD_T) k_g1fft_stage_quad(int m, int s, const uint32_t* __restrict__ tw,
+                                                             const uint32_t* __restrict__ top,
+                                                             const Fe<typename C::Fp> beta, uint32_t* __restrict__ a) {
+  using F = typename C::Fp;
+  constexpr int XW = 4 * F::N;
+  extern __shared__ uint4 smem_u4[];
+  uint32_t* sm = reinterpret_cast<uint32_t*>(smem_u4);
+  uint32_t* smb = sm + 8 * F::N * QUAD_T;
+  const uint32_t nbf = 1u << (m - 1);
+  const uint32_t quad = (blockIdx.x * QUAD_T + threadIdx.x) >> 2;
+  const uint32_t t = quad / HALVES, sub = quad % HALVES;
+  const bool live = t < nbf;
+  const int L = quad_lane();
+  const uint32_t h = 1u << (s - 1), j = live ? t & (h - 1) : 0;
+  const uint32_t i0 = ((t >> (s - 1)) << s) + j, i1 = i0 + h;
+  Fe<F> u = fe_zero<F>(), v = fe_zero<F>();
+  if (live) {
+    u = quad_load<F>(a + (size_t)i0 * XW);
+    v = quad_load<F>(a + (size_t)i1 * XW);
+  }
+  const bool two = INV && top != nullptr;   // two scalars: quad `sub` has its own
+  uint32_t k[GLV_WORDS];
+  load_glv(two ? top + (size_t)GLV_WORDS * (sub ? j : 0) : tw + (size_t)GLV_WORDS * (j << (m - s)), k);
+  auto neg = [&](const Fe<F>& x) { return L == 1 ? fe_neg(x) : x; };
+  // [k]x in every quad of the butterfly (its own scalar with `two`)
+  auto mul = [&](const Fe<F>& x) {
+    const bool mine = two || j != 0;
+    if (!__any_sync(FULL, mine)) return x;
+    if (HALVES == 1 || two) return fe_sel(mine, quad_mul_glv(x, k, true, 0, beta, sm, smb), x);
+    const Fe<F> bx = fe_mul(x, beta);
+    Fe<F> r = quad_mul_glv(fe_sel(sub == 1 && L == 0, bx, x), k, false, (int)sub, beta, sm, smb);
+    r = quad_add(r, fe_shfl_xor(r, 4));
+    return fe_sel(mine, r, x);
+  };
+  if (!INV) {
+    const Fe<F> r = mul(v);
+    if (HALVES == 2) {
+      const Fe<F> o = quad_add(u, sub ? neg(r) : r);
+      if (live) quad_store(a + (size_t)(sub ? i1 : i0) * XW, o);
+    } else {
+      const Fe<F> o0 = quad_add(u, r), o1 = quad_add(u, neg(r));
+      if (live) {
+        quad_store(a + (size_t)i0 * XW, o0);
+        quad_store(a + (size_t)i1 * XW, o1);
+      }
+    }
+  } else if (HALVES == 2) {
+    Fe<F> o = quad_add(u, sub ? neg(v) : v);
+    if (two) {
+      o = mul(o);
+    } else {
+      const Fe<F> d = fe_shfl(o, (threadIdx.x & 31) | 4);   // u - v, for both quads
+      const Fe<F> r = mul(d);
+      if (sub) o = r;
+    }
+    if (live) quad_store(a + (size_t)(sub ? i1 : i0) * XW, o);
+  } else {
+    const Fe<F> o0 = quad_add(u, v), o1 = mul(quad_add(u, neg(v)));
+    if (live) {
+      quad_store(a + (size_t)i0 * XW, o0);
+      quad_store(a + (size_t)i1 * XW, o1);
+    }
+  }
 }
 
 // out[i] = normalised a[bitrev(i)] (or a[i])
@@ -460,6 +604,19 @@ static bool glv_split(const GlvConst& G, const uint64_t k[4], uint32_t out[12]) 
   return true;
 }
 
+// Largest transforms by quads, and with two quads a butterfly.
+static constexpr int QUAD_MMAX = 14, QUAD_MHALVES = 13;
+template <class CP, int HALVES>
+static zkg_status launch_stage_quad(int inverse, int m, int s, const uint32_t* tw, const uint32_t* top,
+                                    const Fe<typename CP::Fp>& beta, uint32_t* a, cudaStream_t st) {
+  constexpr size_t smem = 8 * CP::Fp::N * (QUAD_T + QUAD_T / 4) * 4;
+  const size_t quads = ((size_t)1 << (m - 1)) * HALVES;
+  auto k = inverse ? k_g1fft_stage_quad<CP, true, HALVES> : k_g1fft_stage_quad<CP, false, HALVES>;
+  ZKB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  return launch("g1fft_stage", k, dim3((unsigned)((quads * 4 + QUAD_T - 1) / QUAD_T)), dim3(QUAD_T), smem, st, m, s, tw,
+                top, beta, a);
+}
+
 // CP: the curve type the point arithmetic runs on (C, or its FP64-product twin, zkb_dpf.cuh)
 template <class CP, class C, int NL>
 static zkg_status g1_fft_run(Context& cx, int jac, int m, const uint64_t* gen, const uint32_t* d_src,
@@ -525,14 +682,24 @@ static zkg_status g1_fft_run(Context& cx, int jac, int m, const uint64_t* gen, c
   const dim3 grid_n((unsigned)((n + 127) / 128));
   ZKB_TRY(launch("g1fft_load", k_g1fft_load<CP>, grid_n, blk, 0, st, m, jac, inverse ? 0 : 1, d_src, kin, a));
   const dim3 grid_h((unsigned)((half + 127) / 128));
-  if (!inverse) {
+  const uint32_t* d_top = d_tw + (size_t)GLV_WORDS * ntw;
+  if (m >= 1 && m <= QUAD_MMAX) {
+    for (int k = 0; k < m; k++) {
+      const int s = inverse ? m - k : k + 1;
+      const bool two = inverse && k == 0;
+      if (m <= QUAD_MHALVES || two)
+        ZKB_TRY((launch_stage_quad<CP, 2>(inverse, m, s, d_tw, two ? d_top : nullptr, beta, a, st)));
+      else
+        ZKB_TRY((launch_stage_quad<CP, 1>(inverse, m, s, d_tw, nullptr, beta, a, st)));
+    }
+  } else if (!inverse) {
     for (int s = 1; s <= m; s++)
       ZKB_TRY(launch("g1fft_stage", k_g1fft_stage<CP, false>, grid_h, blk, 0, st, m, s, (const uint32_t*)d_tw,
                      (const uint32_t*)nullptr, beta, a));
   } else {
     for (int s = m; s >= 1; s--)
       ZKB_TRY(launch("g1fft_stage", k_g1fft_stage<CP, true>, grid_h, blk, 0, st, m, s, (const uint32_t*)d_tw,
-                     s == m ? (const uint32_t*)(d_tw + (size_t)GLV_WORDS * ntw) : (const uint32_t*)nullptr, beta, a));
+                     s == m ? d_top : (const uint32_t*)nullptr, beta, a));
   }
   ZKB_TRY(launch("g1fft_store", k_g1fft_store<CP>, grid_n, blk, 0, st, m, inverse ? 1 : 0, (const uint32_t*)a, kout,
                  d_out));
