@@ -555,7 +555,7 @@ zkg_status zkg_server_destroy(zkg_server *s);
  * search, each setting timed on the device). chosen[L - log_min] receives the window width (may
  * be NULL); zkg_msm_tuned_config reports all four settings of a size (0 / -1 = default rule;
  * returns 1 when the size is tuned, 0 when not, -1 on bad arguments).
- * zkg_autotune_ntt times the NTT's largest pass size (6..11) per m in the tile form (below 2^14
+ * zkg_autotune_ntt times the NTT's largest pass size (6..11) per m in the tile form (below 2^9
  * elements, and in a batch's persistent kernel); larger transforms run as matrix products.
  * Tuned settings apply to every later call of the process on that curve and size, the drop-in
  * entry points included. With the environment variable ZKG_TUNE_CACHE naming a file they are
@@ -581,7 +581,7 @@ int zkg_set_msm_tree(int levels, int slots_per_thread);
 int zkg_msm_window_for(zkg_curve curve, int npoints);
 /* Largest NTT pass (log2 of the per-pass network size, 1..11; default 8; 0 = back to the
  * default and the autotuner's per-size choices). An explicit size selects the tile form for every
- * transform; the default runs 2^14 elements and more as matrix products. Returns the previous
+ * transform; the default runs 2^9 elements and more as matrix products. Returns the previous
  * value. Results do not depend on it. */
 int zkg_set_ntt_kmax(int k);
 

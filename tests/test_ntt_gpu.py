@@ -82,7 +82,7 @@ def test_ntt_arbitrary_generator_exact_network(zk, curve):
 
 
 @pytest.mark.parametrize("curve", Z.CURVES)
-@pytest.mark.parametrize("m", (14, 17, 18, 19, 21))
+@pytest.mark.parametrize("m", (9, 10, 11, 12, 13, 14, 17, 18, 19, 21))
 def test_ntt_matrix_form_digit_splits(zk, curve, m):
     """the matrix form's group and digit splits (4 4|3 3 3, 4 3 3, 4 4 3, one and two outputs groups a
     CTA), for a generator that is no root of unity, elements at both ends of the range among them"""

@@ -98,14 +98,16 @@ static int g_ntt_mat = [] {
   const char* v = std::getenv("ZKB_NTT_MAT");
   return v ? std::atoi(v) : 1;
 }();
-// The matrix form needs 128 columns that share a matrix, so two groups of at least 7 bits. An
-// explicit largest pass (zkg_set_ntt_kmax) and the integer products (ZKB_NTT_DPF=0) name the
-// register form.
-static constexpr int NTT_MAT_MMIN = 14;
+// Sizes of the matrix form: from 2^9 on (2^9 20 -> 18 us, 2^8 equal, 2^7 13 -> 16). An explicit largest pass (zkg_set_ntt_kmax) and the
+// integer products (ZKB_NTT_DPF=0) name the register form.
+static constexpr int NTT_MAT_MMIN = 9;
 static bool ntt_use_mat(int m) { return g_ntt_mat && g_ntt_dpf && !g_ntt_kmax_set && m >= NTT_MAT_MMIN; }
 
-// Bits of the groups (7 to 12 each, two up to 2^24, three above): the fewest passes, then the
-// smallest matrices. A group of G bits runs ceil(G / 4) passes of 4 and 3 bits, the 4s first.
+// Bits of the groups: from 2^14 elements on 7 to 12 each (128 columns share a matrix), two up to 2^24,
+// three above: the fewest passes, then the smallest matrices. A group of G bits runs ceil(G / 4) passes
+// of 4 and 3 bits, the 4s first. Below 2^14 every pass is a group, with a twiddle product between any
+// two: a transform that small is all latency, and a pass takes ~6 us (2^12: 67 -> 22 us with three
+// passes of 4 bits, the register form has two of 6).
 static std::vector<int> ntt_mat_digits(int G) {
   const int np = (G + 3) / 4;
   std::vector<int> d(np, 3);
@@ -120,6 +122,7 @@ static std::vector<int> ntt_mat_groups(int m) {
     return (double)((G + 3) / 4) * 1e12 + bytes;
   };
   std::vector<int> best;
+  if (m < 14) return ntt_mat_digits(m);
   double bc = 1e300;
   for (int a = 7; a <= 12; a++)
     for (int b = 7; b <= 12; b++) {
@@ -183,7 +186,7 @@ static zkg_status build_mat(const host::Field<4>& F, NttPlan* pl, const host::El
   struct Src { size_t net, pw, dst; };
   std::vector<Src> src;               // per pass, forward order
   std::vector<NttMatPass> fwd;
-  size_t gtw[2] = {0, 0};
+  size_t gtw[4] = {0, 0, 0, 0};
   int s = 0;
   for (size_t gi = 0; gi < groups.size(); gi++) {
     const int S = s;
@@ -197,7 +200,7 @@ static zkg_status build_mat(const host::Field<4>& F, NttPlan* pl, const host::El
       q.u = s - S;
       const int R = 1 << q.k;
       // half the outputs per CTA when a whole set of them leaves SMs idle
-      q.nout = (1 << (m - q.k - 7)) * (R / 8) < sms ? 4 : 8;
+      q.nout = (1 << std::max(0, m - q.k - 7)) * (R / 8) < sms ? 4 : 8;
       q.tw = -1;
       const size_t b = pl->inverse ? gi - 1 : gi;   // the boundary this pass's outputs cross, if any
       if (pl->inverse ? (di == 0 && gi > 0) : (di + 1 == digits.size() && gi + 1 < groups.size())) {

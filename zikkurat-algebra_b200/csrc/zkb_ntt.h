@@ -41,7 +41,7 @@ struct NttPlan {
   uint32_t* d_scale = nullptr;       // (1/2)^m for the inverse
   bool mat = false;                  // matrix form: mpasses and d_gtw instead of d_tw and d_om
   std::vector<NttMatPass> mpasses;
-  uint32_t* d_gtw[2] = {nullptr};    // twiddles between the groups, in position order
+  uint32_t* d_gtw[4] = {nullptr};    // twiddles between the groups, in position order
   void* d_mblk = nullptr;            // the device block both lie in
   uint32_t* h_fault = nullptr;       // host-mapped word, set by a pass whose bounded wait ran out
   size_t bytes = 0;

@@ -19,20 +19,23 @@
 // by a table in the order of the elements' positions (read as a stream). A 2^24 transform has one
 // such product an element instead of 14; every exponent is the literal one of the reference's
 // network, so the result is the same for any generator. 128 consecutive columns (one tile) share
-// their kappa when S + M' >= 7, which holds from 2^14 elements on.
+// their kappa when S + M' >= 7, which holds from 2^14 elements on; below that every pass is its own group.
 //
-// One CTA per SM: warp 0 feeds A (128 columns x one element, 4 KB contiguous) into a ring and B (plain bulk copies) when the tile's matrix changes; warp 1 issues the MMAs (M = 128,
-// K = 32: one transform element, N = 32 NOUT); 16 warps read the finished sums back from tensor
+// One CTA per SM: warp 0 feeds A (128 columns x one element, 4 KB contiguous) into a ring and B (plain
+// bulk copies) when the tile's matrix changes; warp 1 issues the MMAs (M = 128,
+// K = 32: one transform element, N = 32 NOUT); 16 or 24 warps read the finished sums back from tensor
 // memory while the next tile's MMAs fill the other half of it. Passes write what the next one reads
 // as 4 KB runs, the 16-byte halves of every element already in the order of the 32-byte swizzle (only
 // the first pass, on the caller's data, needs TMA boxes for that). For k = 4 a CTA holds B for 8 of
 // the 16 outputs (128 KB) and another CTA has the other half, which reads the same A from L2.
 //
-// Measured (B200, BN254, kernel time, against the tile form's product-bound passes): 2^14 75 -> 24 us,
-// 2^18 105 -> 50 us, 2^20 341 -> 145 us, 2^22 1.21 -> 0.49 ms, 2^24 5.03 -> 2.44 ms forward, 5.07 ->
-// 2.10 ms inverse. What bounds a pass now: the epilogue (2^22: 72 us a pass without twiddles, 47 us
-// with the fold and the stores taken out; the one with the twiddle product 170 us); the tensor pipe
-// is half busy. Ring slots of four elements (16 KB): one barrier an element took 0.69 ms at 2^22.
+// Measured (B200, BN254, kernel time, against the tile form's product-bound passes): 2^12 67 -> 21 us,
+// 2^14 75 -> 23 us, 2^18 105 -> 50 us, 2^20 341 -> 141 us, 2^22 1.21 -> 0.48 ms, 2^24 5.03 -> 2.03 ms
+// forward, 5.07 -> 2.06 ms inverse. At 2^24 a pass without twiddles takes 275 us: 1.6 GB through L2 (A is
+// read by two CTAs) at 5.8 TB/s, the tensor pipe half busy, HBM's floor 164 us; the pass with the twiddle
+// product 650 us, bound by its ~620 instructions an element at 96 registers and 16 warps. Ring slots of
+// four elements (16 KB): one barrier an element took 0.69 ms at 2^22. Forward stores: keeping kappa in
+// the low bits for M' < 7 instead scattered one pass's 32-byte stores over 2 MB strides (697 us).
 #pragma once
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -111,8 +114,7 @@ struct NttMatArgs {
   int m, k, s, Mp, S, u;
   int inverse;             // load and store sides exchanged
   int first, last;         // first / last pass: plain order of an element's 16-byte halves
-  int kappa_low;           // forward, columns as (r << s) | kappa instead of (kappa << Mp) | r
-  int t_sh, r_bits, k_sh, r_sh;   // forward stores: (r >> r_bits) << t_sh | kappa' << k_sh | (r mod 2^r_bits) << r_sh
+  int t_sh, r_bits;        // forward stores: (r >> r_bits) << t_sh | kappa' << r_bits | (r mod 2^r_bits)
   int tw_S;                // group twiddles: index ((kappa' >> tw_S) << bits left) | remaining position
   uint32_t ntiles, items;  // items = ntiles * (outputs / NOUT), output group outermost
 };
@@ -212,10 +214,12 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
   const uint32_t first = blockIdx.x * per + min(blockIdx.x, rest);
   const uint32_t last = first + per + (blockIdx.x < rest ? 1u : 0u);
   const uint32_t mM = (1u << g.Mp) - 1;
+  const uint32_t ncols = 1u << (g.m - K);   // fewer than 128 (one tile, partly empty) below 2^(7 + K) elements
+  const uint32_t rows = min(128u, ncols) * 32u;
   // the matrix of an item: output group and kappa of its tile
   auto key_of = [&](uint32_t item) -> uint32_t {
     const uint32_t c0 = (item % g.ntiles) * 128u, og = item / g.ntiles;
-    return ((g.kappa_low ? c0 & ((1u << g.s) - 1) : c0 >> g.Mp) >> g.S) * Sh::GROUPS + og;
+    return ((c0 >> g.Mp) >> g.S) * Sh::GROUPS + og;
   };
 
   if (warp == 0 && lane == 0) {   // ---- producer
@@ -244,7 +248,7 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
         const uint32_t slot = it % NS, round = it / NS;
         ok = mbar_wait(empty + 8 * slot, (round & 1) ^ 1, &s_stop);
         if (!ok) break;
-        mbar_expect(full + 8 * slot, NM_SLOT);
+        mbar_expect(full + 8 * slot, NM_TS * (g.first ? NM_ROWS : rows));
 #pragma unroll
         for (int j = 0; j < NM_TS; j++) {
           const uint32_t dst = sA + slot * NM_SLOT + j * NM_ROWS;
@@ -255,7 +259,7 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
                 : "memory");
           else
             asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                         "l"(g.in + (((size_t)(t + j) << (g.m - K)) + c0) * 32), "r"(NM_ROWS), "r"(full + 8 * slot)
+                         "l"(g.in + (((size_t)(t + j) << (g.m - K)) + c0) * 32), "r"(rows), "r"(full + 8 * slot)
                          : "memory");
         }
       }
@@ -314,17 +318,17 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
 #pragma unroll 1
     for (uint32_t job = (warp - 4) >> 2; job < jobs; job += STEP) {
       const uint32_t n = job / NOUT, j = job % NOUT, item = first + n, buf = n & 1;
-      const uint32_t c = (item % g.ntiles) * 128u + quarter * 32u + lane;
+      uint32_t c = (item % g.ntiles) * 128u + quarter * 32u + lane;
+      const bool valid = c < ncols;
+      c = valid ? c : 0;
       const uint32_t o = (item / g.ntiles) * NOUT + j;
-      const uint32_t r = g.kappa_low ? c >> g.s : c & mM;
-      uint32_t kap = g.kappa_low ? c & ((1u << g.s) - 1) : c >> g.Mp;   // kappa' and what is left below it
-      uint32_t rem = r, dst;
+      uint32_t kap = c >> g.Mp, rem = c & mM, dst;   // kappa', and what is left below it
       if (g.inverse) {
         rem |= o << g.Mp;
         dst = (kap << (g.Mp + K)) | rem;
       } else {
         kap |= o << g.s;
-        dst = ((r >> g.r_bits) << g.t_sh) | (kap << g.k_sh) | ((r & ((1u << g.r_bits) - 1)) << g.r_sh);
+        dst = ((rem >> g.r_bits) << g.t_sh) | (kap << g.r_bits) | (rem & ((1u << g.r_bits) - 1));
       }
       Fe<PL> w;
       if (TW) w = fe_load_nc<PL>(g.tw + (size_t)(((kap >> g.tw_S) << (g.inverse ? g.Mp + K : g.Mp)) | rem) * 8);
@@ -346,6 +350,7 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
 #pragma unroll
         for (int i = 0; i < 8; i++) v.v[i] = a.v[i];
       }
+      if (!valid) continue;
       uint32_t* p = g.out + (size_t)dst * 8;
       const uint32_t x = g.last ? 0u : dst & 4u;   // the swizzle of the next pass's rows: bit 2 of the index
       *reinterpret_cast<uint4*>(p + x) = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
@@ -470,18 +475,14 @@ zkg_status ntt_mat_launch_pass(const NttPlan& pl, int exec, const uint32_t* in, 
   g.first = exec == 0;
   g.last = exec == (int)pl.mpasses.size() - 1;
   g.tw_S = q.tw_S;
-  // forward layouts: the digit a pass transforms on top, below it (kappa << M') | r while M' >= 7,
-  // (r << s) | kappa after that, so that every pass reads 4 KB runs
-  g.kappa_low = !pl.inverse && q.Mp < 7;
-  g.t_sh = g.r_bits = g.k_sh = g.r_sh = 0;
+  // forward layouts: the digit a pass transforms on top, below it (kappa << M') | r, so that every pass
+  // reads 4 KB runs and a quarter of a tile writes runs of at least 2^M' elements
+  g.t_sh = g.r_bits = 0;
   if (!pl.inverse && !g.last) {
-    const NttMatPass& nx = pl.mpasses[exec + 1];
-    g.t_sh = pl.m - nx.k;
-    g.r_bits = nx.Mp;
-    g.k_sh = nx.Mp < 7 ? 0 : nx.Mp;
-    g.r_sh = nx.Mp < 7 ? nx.s : 0;
+    g.t_sh = pl.m - pl.mpasses[exec + 1].k;
+    g.r_bits = pl.mpasses[exec + 1].Mp;
   }
-  g.ntiles = 1u << (pl.m - q.k - 7);
+  g.ntiles = 1u << std::max(0, pl.m - q.k - 7);
   g.items = g.ntiles * ((1u << q.k) / q.nout);
   if (g.tw) return nm_dispatch<P, true>(map, g, q.nout, sms, st);
   return nm_dispatch<P, false>(map, g, q.nout, sms, st);
