@@ -218,6 +218,23 @@ def test_binary_msm_random_vs_oracle(zk, curve, nrows, npts):
         assert np.array_equal(bin_call(zk, curve, "proj", "affine", co, bases, False), want)
 
 
+@pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("nrows,npts", [(1, 1), (2, 33), (13, 3000), (14, 257), (15, 3000), (29, 1025)])
+def test_binary_msm_row_groups(zk, curve, nrows, npts):
+    """row groups of one width and of two, rows of all ones, all zeros and one bit, bases at infinity"""
+    rng = np.random.default_rng(nrows * 1000 + npts)
+    co = rng.integers(0, 2, (nrows, npts)).astype(np.uint8) * 255
+    co[nrows // 2] = 1
+    if nrows > 2:
+        co[0] = 0
+        co[nrows - 1] = 0
+        co[nrows - 1, npts - 1] = 7
+    bases = Z.gen_bases_cpu(curve, Z.rand_fr(curve, npts, 9700 + npts)).reshape(npts, -1)
+    bases[3::19] = 0
+    want = affine_rows(curve, "proj", Z.oracle_msm_binary(curve, co, bases))
+    assert np.array_equal(zk.binary_multi_msm(curve, co, bases, affine=True), want)
+
+
 def _binary_large(zk, curve, nrows, npts, seed, sample_rows):
     """large binary MSMs (several column chunks): sampled rows against the oracle, and
     row + complement = sum of all bases for every row"""

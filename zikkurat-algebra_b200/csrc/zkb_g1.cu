@@ -23,18 +23,12 @@
 // Binary MSMs: *_MSM_binary_coeff_* (bn128_G1_proj.c:684-698) sums the bases whose byte
 // coefficient is non-zero; *_multi_MSM_binary_coeff_* (bn128_G1_proj.c:718-782) does that for
 // each row of an nrows x npoints byte matrix, with the bases split into windows of c columns and
-// all 2^c subset sums of a window precomputed, so a row adds one table entry per window. Both
-// run here as one pipeline:
-//   - "direct" (few rows): thread (row, g) madds the selected affine bases of columns
-//     g, g + G, ...;
-//   - "windowed" (many rows): per window of c columns the subset-sum table T[k][0..2^c) is built
-//     in c level launches (T[k][2^l + i] = T[k][i] + P[kc + l]); thread (row, g) then adds
-//     T[k][idx] for windows k = g, g + G, ...;
-//   - columns are processed in chunks (host coefficient rows and bases are gathered into pinned
-//     staging and copied while the previous chunk computes); per-(row, g) partial sums carry
-//     across chunks and are reduced per row at the end.
-// The choice between direct and windowed, c and G only changes the order of additions; every
-// result is the same group element, written in the drop-in's output encoding.
+// all 2^c subset sums of a window precomputed, so a row adds one table entry per window. Here the
+// rows are grouped instead and the columns go to buckets by their bits in a group (zkb_msm_bits.h):
+// 64 rows of 2^18 columns are 17 M field products against 60 M by subset sums. Columns are processed
+// in chunks (host coefficient rows and bases are gathered into pinned staging and copied while the
+// previous chunk computes); every chunk leaves one partial sum a row, added up at the end. The order
+// of additions differs; every result is the same group element, written in the drop-in's encoding.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -43,6 +37,7 @@
 #include "zkb_curve.cuh"
 #include "zkb_dpf.cuh"
 #include "zkb_host_ec.h"
+#include "zkb_msm_bits.h"
 #include "zkb_quad.cuh"
 #include "zkb_runtime.h"
 
@@ -394,79 +389,6 @@ __global__ void k_g1fft_store(int m, int bitrev, const uint32_t* __restrict__ a,
 }
 
 // ------------------------------------------------------------------------ binary MSM kernels
-// Direct: thread (row, g) madds bases of the chunk's columns g, g + G, ... whose coefficient
-// byte is non-zero. Affine (0, 0) bases are the identity and are skipped.
-template <class C>
-__global__ void k_bin_direct(int nrows, int cw, const uint8_t* __restrict__ coeffs, size_t ld,
-                             const uint32_t* __restrict__ bases, int G, uint32_t* __restrict__ partial, int first) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= (size_t)nrows * G) return;
-  const int row = (int)(tid / G), g = (int)(tid % G);
-  Xyzz<F> acc = first ? xyzz_inf<F>() : xyzz_load<F>(partial + tid * XW);
-  const uint8_t* r = coeffs + (size_t)row * ld;
-  for (int col = g; col < cw; col += G) {
-    if (!r[col]) continue;
-    const Affine<F> b = affine_load<F>(bases + (size_t)col * 2 * F::N);
-    if (fe_is_zero(b.x) && fe_is_zero(b.y)) continue;
-    xyzz_madd(acc, b);
-  }
-  xyzz_store<F>(partial + tid * XW, acc);
-}
-
-// Subset-sum tables, level l: T[k][2^l + i] = T[k][i] + P[kc + l] for i < 2^l (level 0 writes
-// T[k][0] = identity and T[k][1] = P[kc]). Columns past the chunk width are the identity.
-template <class C>
-__global__ void k_bin_table(int nwin, int c, int l, int cw, const uint32_t* __restrict__ bases,
-                            uint32_t* __restrict__ table) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t per = (size_t)1 << l;
-  if (tid >= (size_t)nwin * per) return;
-  const size_t k = tid >> l, i = tid & (per - 1);
-  uint32_t* T = table + (k << c) * XW;
-  const int col = (int)k * c + l;
-  bool has = col < cw;
-  Affine<F> b;
-  if (has) {
-    b = affine_load<F>(bases + (size_t)col * 2 * F::N);
-    has = !(fe_is_zero(b.x) && fe_is_zero(b.y));
-  }
-  if (l == 0) {
-    xyzz_store<F>(T, xyzz_inf<F>());
-    xyzz_store<F>(T + XW, has ? xyzz_from_affine(b) : xyzz_inf<F>());
-    return;
-  }
-  Xyzz<F> e = xyzz_load<F>(T + i * XW);
-  if (has) xyzz_madd(e, b);
-  xyzz_store<F>(T + (per + i) * XW, e);
-}
-
-// Windowed: thread (row, g) adds T[k][idx(row, k)] for windows k = g, g + G, ...
-template <class C>
-__global__ void k_bin_rows(int nrows, int nwin, int c, int cw, const uint8_t* __restrict__ coeffs, size_t ld,
-                           const uint32_t* __restrict__ table, int G, uint32_t* __restrict__ partial, int first) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= (size_t)nrows * G) return;
-  const int row = (int)(tid / G), g = (int)(tid % G);
-  Xyzz<F> acc = first ? xyzz_inf<F>() : xyzz_load<F>(partial + tid * XW);
-  const uint8_t* r = coeffs + (size_t)row * ld;
-  for (int k = g; k < nwin; k += G) {
-    uint32_t idx = 0;
-    const int c0 = k * c;
-    for (int j = 0; j < c; j++) {
-      const int col = c0 + j;
-      if (col < cw && r[col]) idx |= 1u << j;
-    }
-    if (idx) acc = xyzz_sum(acc, xyzz_load<F>(table + (((size_t)k << c) + idx) * XW));
-  }
-  xyzz_store<F>(partial + tid * XW, acc);
-}
-
 // Sums of segments: block (seg b of row r) reduces in[r][b*256 .. min(L, b*256+256)) into
 // out[r][b]; 128 threads, shared-memory tree.
 template <class C>
@@ -766,37 +688,28 @@ static zkg_status g1_fft_dev(int jac, int m, const uint64_t* gen, const uint64_t
 
 // ------------------------------------------------------------------------ binary MSM host side
 struct BinPlan {
-  int windowed = 0;   // 0: direct madds; 1: subset-sum tables of c columns
-  int c = 1;
-  int G = 1;          // partial sums per row
-  int cw = 0;         // columns per chunk (a multiple of c)
+  int rho = 1;            // rows a group
+  int batch = 0;          // rows a launch
+  int cw = 0;             // columns a chunk
+  int G = 1;              // chunks = partial sums a row
+  size_t bits_bytes = 0;  // workspace of one launch
 };
+static constexpr int BIN_ROWS = 32768;   // rows a launch (grid dimensions) and a reduction, at most
 
-// Cost per column in field products: direct = rows * (1/2) * 10 (one madd per selected base at
-// density 1/2); windowed = ((2^c - 1 - c) * 10 + rows * (1 - 2^-c) * 14) / c (table madds plus
-// one full addition per row and window).
-static BinPlan bin_plan(int nrows, int npoints, int nl, int sm_count) {
-  BinPlan P;
-  double best = 5.0 * nrows;
-  for (int c = 2; c <= 12; c++) {
-    const double cost = ((double)((1 << c) - 1 - c) * 10.0 + nrows * (1.0 - std::ldexp(1.0, -c)) * 14.0) / c;
-    if (cost < best * 0.95) { best = cost; P.windowed = 1; P.c = c; }
+// Chunks of up to 64 M entries (a column has one a group of rows); from host buffers also 32 MiB of
+// coefficients and of bases.
+static zkg_status bin_plan(int nrows, int npoints, int nl, bool host, BinPlan& P) {
+  P.batch = std::min(nrows, BIN_ROWS);
+  P.rho = msm_bits_group(P.batch, npoints);
+  const int ngroups = (P.batch + P.rho - 1) / P.rho;
+  size_t cw = std::min<size_t>((size_t)npoints, ((size_t)1 << 26) / ngroups);
+  if (host) {
+    cw = std::min<size_t>(cw, ((size_t)32 << 20) / std::max(1, nrows));
+    cw = std::min<size_t>(cw, ((size_t)32 << 20) / (2 * (size_t)nl * 8));
   }
-  const size_t xb = 4 * (size_t)nl * 8;
-  // chunk: coefficients <= 32 MiB, bases <= 32 MiB, tables <= 256 MiB
-  size_t cw = std::min<size_t>((size_t)npoints, ((size_t)32 << 20) / std::max(1, nrows));
-  cw = std::min<size_t>(cw, ((size_t)32 << 20) / (2 * (size_t)nl * 8));
-  if (P.windowed) cw = std::min<size_t>(cw, (((size_t)256 << 20) / (xb << P.c)) * P.c);
-  cw = std::max<size_t>(cw, (size_t)P.c);
-  cw = (cw + P.c - 1) / P.c * P.c;
-  P.cw = (int)cw;
-  const long units = P.windowed ? (long)(cw / P.c) : (long)cw;   // per-row work items in a chunk
-  const long target = (long)sm_count * 512;                      // threads to keep the SMs busy
-  long G = (target + nrows - 1) / nrows;
-  G = std::max(1L, std::min(G, units));
-  G = std::min(G, 65536L);
-  P.G = (int)G;
-  return P;
+  P.cw = (int)std::max<size_t>(cw, 1);
+  P.G = (npoints + P.cw - 1) / P.cw;
+  return msm_bits_bytes(nl == 4 ? ZKG_BN254 : ZKG_BLS12_381, P.batch, P.cw, P.rho, &P.bits_bytes);
 }
 
 // Runs the chunk loop. get_chunk(q, col0, cw, &coeffs, &ld, &bases) makes chunk q's coefficient
@@ -804,61 +717,43 @@ static BinPlan bin_plan(int nrows, int npoints, int nl, int sm_count) {
 template <class C, int NL, class Get>
 static zkg_status bin_run(Context& cx, const BinPlan& P, int nrows, int npoints, char* ws, cudaStream_t st,
                           Get get_chunk, int kind, uint32_t* d_out) {
-  using F = typename C::Fp;
-  const size_t xb = 4 * NL * 8;
+  constexpr size_t XW = 4 * C::Fp::N;
   uint32_t* partial = reinterpret_cast<uint32_t*>(ws);
-  ws += rup256((size_t)nrows * P.G * xb);
-  uint32_t* table = reinterpret_cast<uint32_t*>(ws);
+  char* work = ws + rup256((size_t)nrows * P.G * XW * 4);
   const dim3 blk(128);
-  const size_t nthr = (size_t)nrows * P.G;
-  const int nchunks = (npoints + P.cw - 1) / P.cw;
-  for (int q = 0; q < nchunks; q++) {
+  for (int q = 0; q < P.G; q++) {
     const int col0 = q * P.cw;
     const int cw = std::min(P.cw, npoints - col0);
     const uint8_t* coeffs = nullptr;
     size_t ld = 0;
     const uint32_t* bases = nullptr;
     ZKB_TRY(get_chunk(q, col0, cw, &coeffs, &ld, &bases));
-    if (!P.windowed) {
-      ZKB_TRY(launch("bin_direct", k_bin_direct<C>, dim3((unsigned)((nthr + 127) / 128)), blk, 0, st, nrows, cw,
-                     coeffs, ld, bases, P.G, partial, q == 0 ? 1 : 0));
-    } else {
-      const int nwin = (cw + P.c - 1) / P.c;
-      for (int l = 0; l < P.c; l++) {
-        const size_t nt = (size_t)nwin << l;
-        ZKB_TRY(launch("bin_table", k_bin_table<C>, dim3((unsigned)((nt + 127) / 128)), blk, 0, st, nwin, P.c, l, cw,
-                       bases, table));
-      }
-      ZKB_TRY(launch("bin_rows", k_bin_rows<C>, dim3((unsigned)((nthr + 127) / 128)), blk, 0, st, nrows, nwin, P.c,
-                     cw, coeffs, ld, (const uint32_t*)table, P.G, partial, q == 0 ? 1 : 0));
-    }
+    for (int r = 0; r < nrows; r += P.batch)
+      ZKB_TRY(msm_bits_launch(cx, C::ID == 0 ? ZKG_BN254 : ZKG_BLS12_381, std::min(P.batch, nrows - r), cw, P.rho,
+                              coeffs + (size_t)r * ld, ld, bases, work, partial + ((size_t)r * P.G + q) * XW,
+                              (size_t)P.G * XW, st));
     ZKB_TRY(get_chunk(-1 - q, 0, 0, nullptr, nullptr, nullptr));   // chunk q's inputs are consumed
   }
   // reduce G partials per row: 256 per block per pass
   int L = P.G;
   uint32_t* in = partial;
-  uint32_t* tmp = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(table));   // reuse the table region
+  uint32_t* tmp = reinterpret_cast<uint32_t*>(work);   // the launches' workspace is free again
   while (L > 1) {
     const int B = (L + 255) / 256;
-    ZKB_TRY(launch("xyzz_reduce", k_xyzz_reduce<C>, dim3((unsigned)B, (unsigned)nrows), blk, 0, st, L, B,
-                   (const uint32_t*)in, tmp));
+    for (int r = 0; r < nrows; r += BIN_ROWS)
+      ZKB_TRY(launch("xyzz_reduce", k_xyzz_reduce<C>, dim3((unsigned)B, (unsigned)std::min(BIN_ROWS, nrows - r)), blk, 0,
+                     st, L, B, (const uint32_t*)in + (size_t)r * L * XW, tmp + (size_t)r * B * XW));
     std::swap(in, tmp);
     L = B;
   }
-  ZKB_TRY(launch("xyzz_write", k_xyzz_write<C>, dim3((unsigned)((nrows + 127) / 128)), blk, 0, st, nrows, kind,
-                 (const uint32_t*)in, d_out));
-  (void)sizeof(F);
-  return ZKG_OK;
+  return launch("xyzz_write", k_xyzz_write<C>, dim3((unsigned)((nrows + 31) / 32)), dim3(32), 0, st, nrows, kind,
+                (const uint32_t*)in, d_out);
 }
 
 template <int NL>
 static size_t bin_ws_bytes(const BinPlan& P, int nrows) {
-  const size_t xb = 4 * NL * 8;
-  const size_t part = rup256((size_t)nrows * P.G * xb);
-  const size_t nwin = (size_t)(P.cw + P.c - 1) / P.c;
-  size_t tab = P.windowed ? rup256((nwin << P.c) * xb) : 0;
-  tab = std::max(tab, part);   // the reduction's ping-pong buffer reuses the table region
-  return part + tab;
+  const size_t part = rup256((size_t)nrows * P.G * 4 * NL * 8);
+  return part + std::max(rup256(P.bits_bytes), P.G > 1 ? part : 0);   // the reduction's second buffer
 }
 
 static zkg_status bin_check(zkg_curve curve, int kind, int nrows, int npoints, const void* rows, const void* bases,
@@ -886,7 +781,8 @@ static zkg_status bin_host(const host::Field<NL>& Fp, int kind, int nrows, int n
   ZKB_TRY(get_context(&cxp));
   Context& cx = *cxp;
   std::lock_guard<std::mutex> lk(cx.mu);
-  const BinPlan P = bin_plan(nrows, npoints, NL, cx.sm_count);
+  BinPlan P;
+  ZKB_TRY(bin_plan(nrows, npoints, NL, true, P));
   const size_t bb = 2 * NL * 8;
   const size_t coef_chunk = rup256((size_t)nrows * P.cw), base_chunk = rup256((size_t)P.cw * bb);
   const size_t out_bytes = rup256((size_t)nrows * ow * 8);
@@ -980,7 +876,8 @@ static zkg_status bin_dev(int kind, int nrows, int npoints, const uint8_t* d_coe
     ZKB_CUDA(cudaStreamSynchronize(st));
     return set_status(ZKG_OK, nullptr, nullptr);
   }
-  const BinPlan P = bin_plan(nrows, npoints, NL, cx.sm_count);
+  BinPlan P;
+  ZKB_TRY(bin_plan(nrows, npoints, NL, false, P));
   const size_t bytes = bin_ws_bytes<NL>(P, nrows);
   ZKB_TRY(cx.arena.reserve(bytes));
   cx.arena.reset();

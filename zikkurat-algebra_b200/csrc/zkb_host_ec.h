@@ -110,7 +110,8 @@ inline bool has_mulx_adx() {
           : [a] "r"(A), "d"(B), "m"(*(const uint64_t(*)[4])(A)) \
           : "cc")
 inline void mul_adx(const Field<4>& F, const uint64_t* a, const uint64_t* b, uint64_t* r) {
-  uint64_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, lo, hi, z;
+  uint64_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0;
+  [[maybe_unused]] uint64_t lo, hi, z;
   ZKB_MUL_ROW4(t0, t1, t2, t3, t4, a, b[0]);
   ZKB_MUL_ROW4(t0, t1, t2, t3, t4, F.p, t0 * F.n0);
   ZKB_MUL_ROW4(t1, t2, t3, t4, t0, a, b[1]);
@@ -135,7 +136,8 @@ inline void mul_adx(const Field<4>& F, const uint64_t* a, const uint64_t* b, uin
           : [a] "r"(A), "d"(B), "m"(*(const uint64_t(*)[6])(A)) \
           : "cc")
 inline void mul_adx(const Field<6>& F, const uint64_t* a, const uint64_t* b, uint64_t* r) {
-  uint64_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, lo, hi, z;
+  uint64_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0;
+  [[maybe_unused]] uint64_t lo, hi, z;
   ZKB_MUL_ROW6(t0, t1, t2, t3, t4, t5, t6, a, b[0]);
   ZKB_MUL_ROW6(t0, t1, t2, t3, t4, t5, t6, F.p, t0 * F.n0);
   ZKB_MUL_ROW6(t1, t2, t3, t4, t5, t6, t0, a, b[1]);

@@ -45,6 +45,7 @@
 #include "zkb_ntt.h"
 #include "zkb_batch_work.h"
 #include "zkb_msm_accum.cuh"
+#include "zkb_msm_bits.h"
 #include "zkb_msm_tail.cuh"
 #include "zkb_msm_tree.cuh"
 #include "zkb_runtime.h"
@@ -1366,6 +1367,167 @@ static zkg_status msm_dev_entry(const host::Field<NL>& F, int n, const uint64_t*
   return msm_dev_run<C, C, NL>(F, n, d_expos, nlimbs, mont, d_grps, kind, tgt);
 }
 
+
+// ======================================================================= 0/1 row sums
+//
+// (zkb_msm_bits.h) Group w holds width(w) rows; its buckets are all 2^width patterns, so the shape is
+// that of windows one bit wider (2^(width + 1 - 1) buckets), pattern 0 staying empty.
+static WinShape bits_shape(int nrows, int ngroups) {
+  WinShape s = win_shape(nrows, ngroups);
+  s.base++;
+  return s;
+}
+static int bits_groups(int nrows, int rho) { return (nrows + rho - 1) / rho; }
+
+int msm_bits_group(int nrows, double ncols) {
+  double best = 1e300;
+  int br = 1;
+  for (int rho = 1; rho <= std::min(nrows, 14); rho++) {
+    const double cost = bits_groups(nrows, rho) * 10.0 * (1.0 - std::ldexp(1.0, -rho)) * ncols +
+                        (double)nrows * std::ldexp(16.0, rho - 1);
+    if (cost < best) { best = cost; br = rho; }
+  }
+  return br;
+}
+
+// dig, rank as in hist_windows; thread i takes column i (neighbouring threads read neighbouring bytes).
+// Few rows, or rows that are mostly ones, send many columns to one bucket, so the lanes of a warp with
+// the same pattern count it once.
+__global__ void k_bits_hist(int n, const uint8_t* __restrict__ coeffs, size_t ld, WinShape ws, int ngroups,
+                            uint32_t* __restrict__ cnt, uint32_t* __restrict__ dig, uint32_t* __restrict__ rank) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  for (int w = 0; w < ngroups; w++) {
+    const int rows = ws.width(w) - 1, r0 = ws.start(w) - w;   // the shape's windows are one bit wider
+    uint32_t v = 0;
+    if (i < n)
+      for (int j = 0; j < rows; j++) v |= (__ldg(coeffs + (size_t)(r0 + j) * ld + i) ? 1u : 0u) << j;
+    const uint32_t same = __match_any_sync(0xffffffffu, v);
+    const int leader = __ffs((int)same) - 1;
+    uint32_t at = 0;
+    if (v && lane == leader) at = atomicAdd(cnt + ws.seg(w) + v, (uint32_t)__popc(same));
+    at = __shfl_sync(0xffffffffu, at, leader) + (uint32_t)__popc(same & ((1u << lane) - 1));
+    if (i < n) {
+      dig[(size_t)w * n + i] = v ? v + 1 : 0u;   // bucket numbers are positions + 1
+      if (v) rank[(size_t)w * n + i] = at;
+    }
+  }
+}
+
+// Block r: the sum of its group's buckets with row r's bit set, canonical.
+template <class C>
+__global__ void __launch_bounds__(256) k_bits_rows(WinShape ws, const uint32_t* __restrict__ off,
+                                                   const uint32_t* __restrict__ bsum, uint32_t* __restrict__ out,
+                                                   size_t stride) {
+  using F = typename C::Fp;
+  constexpr int XW = 4 * F::N;
+  __shared__ __align__(16) uint32_t sm[8 * XW];
+  const uint32_t r = blockIdx.x;
+  const uint32_t few = (uint32_t)ws.base - 1, wide = (uint32_t)ws.extra * (few + 1);   // rows of a narrow group, of the wide ones
+  const int w = (int)(r < wide ? r / (few + 1) : ws.extra + (r - wide) / few);
+  const uint32_t k = r - (uint32_t)(ws.start(w) - w), cnt = ws.buckets(w) >> 1, quad = threadIdx.x >> 2;
+  const uint32_t s0 = ws.seg(w);
+  auto item = [&](uint32_t j) {
+    const uint32_t s = s0 + (((j >> k) << (k + 1)) | (1u << k) | (j & ((1u << k) - 1)));
+    return j < cnt && __ldg(off + s) != __ldg(off + s + 1) ? quad_load<F>(bsum + (size_t)s * XW) : fe_zero<F>();
+  };
+  Fe<F> a = fe_zero<F>(), nx = item(quad);
+#pragma unroll 1
+  for (uint32_t j0 = 0; j0 < cnt; j0 += 64) {
+    const Fe<F> x = nx;
+    nx = item(j0 + 64 + quad);
+    a = quad_add(a, x);
+  }
+  a = quad_warp_sum(a);
+  if ((threadIdx.x & 31) < 4) quad_store(sm + (threadIdx.x >> 5) * XW, a);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  a = quad_warp_sum(quad_load<F>(sm + quad * XW));
+  if (threadIdx.x < 4) quad_store(out + (size_t)r * stride, fe_canon(a));
+}
+
+struct BitsPlan {
+  WinShape win;
+  int ngroups;
+  uint32_t nseg, L1, nch, pcap;
+  uint64_t total;
+  bool quad;
+  size_t o_cnt, o_off, o_cur, o_bs, o_dig, o_rank, o_ent, o_key, o_pt, o_prec, o_pdone, o_ppt, o_bsum, bytes;
+};
+template <class C>
+static zkg_status bits_plan(int nrows, int ncols, int rho, BitsPlan& P) {
+  constexpr size_t XB = 16 * C::Fp::N;
+  P.ngroups = bits_groups(nrows, rho);
+  P.win = bits_shape(nrows, P.ngroups);
+  P.nseg = P.win.seg(P.ngroups);
+  P.total = (uint64_t)P.ngroups * (uint64_t)ncols;
+  if (P.total >= (1ull << 31)) return set_status(ZKG_ERR_ARG, "msm_binary", "too many entries for one launch");
+  P.quad = P.total <= QUAD_TOTAL;
+  P.L1 = P.quad ? quad_chunk_len(P.total) : chunk_len(P.total, accum_wave<C>());
+  P.nch = std::max<uint32_t>(1, (uint32_t)((P.total + P.L1 - 1) / P.L1));
+  P.pcap = P.nch / 8 + 2;
+  const uint32_t nb = (P.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
+  if (nb > (uint32_t)SCAN_T * SCAN_E) return set_status(ZKG_ERR_ARG, "msm_binary", "too many buckets");
+  size_t o = 0;
+  auto take = [&](size_t bytes) { const size_t r = o; o = (o + bytes + 255) & ~size_t(255); return r; };
+  P.o_cnt = take((size_t)P.nseg * 4 + 4);   // then: pieces
+  P.o_off = take((size_t)P.nseg * 4 + 4);
+  P.o_cur = take((size_t)P.nseg * 4 + 4);
+  P.o_bs = take((size_t)nb * 4 + 4);
+  P.o_dig = take(P.total * 4);
+  P.o_rank = take(P.total * 4);
+  P.o_ent = take(P.total * 4);
+  P.o_key = take((size_t)P.nch * 8);
+  P.o_pt = take((size_t)P.nch * 2 * XB);
+  P.o_prec = take((size_t)P.pcap * sizeof(Piece));
+  P.o_pdone = take((size_t)P.pcap * 4);
+  P.o_ppt = take((size_t)P.pcap * XB);
+  P.o_bsum = take((size_t)P.nseg * XB);
+  P.bytes = o;
+  return ZKG_OK;
+}
+
+template <class C>
+static zkg_status bits_launch(int nrows, int ncols, int rho, const uint8_t* coeffs, size_t ld, const uint32_t* bases,
+                              char* ws, uint32_t* out, size_t stride, uint32_t* chk, cudaStream_t st) {
+  BitsPlan P;
+  ZKB_TRY(bits_plan<C>(nrows, ncols, rho, P));
+  auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
+  ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)P.nseg * 4 + 4, st));
+  const dim3 gc((ncols + 255) / 256);
+  ZKB_TRY(launch("bits_hist", k_bits_hist, gc, dim3(256), 0, st, ncols, coeffs, ld, P.win, P.ngroups, U32(P.o_cnt),
+                 U32(P.o_dig), U32(P.o_rank)));
+  ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st));
+  ZKB_TRY(launch("msm_scatter_d", k_msm_scatter_d, dim3(gc.x, P.ngroups), dim3(256), 0, st, ncols,
+                 (const uint32_t*)U32(P.o_dig), (const uint32_t*)U32(P.o_rank), P.win, (const uint32_t*)U32(P.o_off),
+                 U32(P.o_ent), chk, (uint32_t)P.total));
+  const uint32_t *off = U32(P.o_off), *ent = U32(P.o_ent);
+  if (P.quad)
+    ZKB_TRY(launch("msm_quad_accum", k_quad_accum<C>, dim3((P.nch + 31) / 32), dim3(128), 0, st, ent, off, P.nseg, P.nch,
+                   P.L1, bases, U32(P.o_bsum), U32(P.o_key), U32(P.o_pt), chk, (uint32_t)ncols));
+  else
+    ZKB_TRY(launch_accum<C>(P.nch, st, ent, off, P.nseg, P.L1, bases, U32(P.o_bsum), U32(P.o_key), U32(P.o_pt), -1, chk,
+                            (uint32_t)ncols));
+  const PieceList pl = {U32(P.o_cnt) + P.nseg, P.pcap, reinterpret_cast<Piece*>(ws + P.o_prec), U32(P.o_pdone),
+                        U32(P.o_ppt)};
+  ZKB_TRY(msm_launch_merge<C>(pl, off, chk, P.nch, P.L1, U32(P.o_key), U32(P.o_pt), U32(P.o_bsum), P.nseg, st));
+  return launch("bits_rows", k_bits_rows<C>, dim3(nrows), dim3(256), 0, st, P.win, off,
+                (const uint32_t*)U32(P.o_bsum), out, stride);
+}
+
+zkg_status msm_bits_bytes(int curve, int nrows, int ncols, int rho, size_t* bytes) {
+  BitsPlan P;
+  ZKB_TRY(curve == ZKG_BN254 ? bits_plan<BN254E>(nrows, ncols, rho, P) : bits_plan<BLS12_381E>(nrows, ncols, rho, P));
+  *bytes = P.bytes;
+  return ZKG_OK;
+}
+
+zkg_status msm_bits_launch(Context& cx, int curve, int nrows, int ncols, int rho, const uint8_t* coeffs, size_t ld,
+                           const uint32_t* bases, char* ws, uint32_t* out, size_t stride, cudaStream_t st) {
+  uint32_t* chk = dev_check_word(cx);
+  if (curve == ZKG_BN254)
+    return bits_launch<BN254E>(nrows, ncols, rho, coeffs, ld, bases, ws, out, stride, chk, st);
+  return bits_launch<BLS12_381E>(nrows, ncols, rho, coeffs, ld, bases, ws, out, stride, chk, st);
+}
 
 // =================================================================== batched MSMs (many sizes)
 //

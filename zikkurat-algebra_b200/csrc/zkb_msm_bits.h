@@ -1,0 +1,21 @@
+// Row sums of a 0/1 matrix over one base set by the MSM's bucket pipeline (zkb_msm.cu): the rows are
+// taken `rho` at a time, a column's bits in such a group are a bucket number, every column is one mixed
+// addition per group, and a row's sum is the sum of its group's buckets with its bit set.
+#pragma once
+#include <cstdint>
+
+#include "zkb_runtime.h"
+
+namespace zkb {
+
+// Rows a group for `ncols` columns of `nrows` rows, by field products: a mixed addition (10) for every
+// column and group that is not all zeros, 2^(rho - 1) additions (16 lane products) for every row.
+int msm_bits_group(int nrows, double ncols);
+// Workspace bytes for up to `ncols` columns.
+zkg_status msm_bits_bytes(int curve, int nrows, int ncols, int rho, size_t* bytes);
+// Enqueues the row sums of ncols columns (coeffs: row r at coeffs + r ld, non-zero bytes select) on st:
+// row r's XYZZ point, canonical, goes to out + r stride (words).
+zkg_status msm_bits_launch(Context& cx, int curve, int nrows, int ncols, int rho, const uint8_t* coeffs, size_t ld,
+                           const uint32_t* bases, char* ws, uint32_t* out, size_t stride, cudaStream_t st);
+
+}  // namespace zkb
