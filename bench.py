@@ -62,8 +62,8 @@ FMA_SLOTS_PER_MADD = 10 * (128 + 2 * 128 + 8)
 # DRAM bytes (read + write) of one bucket-accumulation launch (k_msm_accum_w<BN254E, 384, 2>) by
 # log2 n, from `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
 # -k regex:k_msm_accum -c 1` on `python bench.py --steps 2 --warmup 3 --no-extra --no-cpu --no-ntt
-# --no-tune`; re-captured whenever the kernel changes
-ACCUM_DRAM_BYTES = {22: 6.828788480e9}
+# --no-tune` with ZKB_MSM_TREE=0; re-captured whenever the kernel changes
+ACCUM_DRAM_BYTES = {22: 7.148766208e9}
 
 
 def hbm_peak():
@@ -406,8 +406,16 @@ def run_msm(args, zk, L, torch, stream, rank, world, dist, imad_peak, fp64_peak)
                          "through the reference's bn128_G1_proj_MSM_mont_coeff_proj_out, partials added with "
                          "bn128_G1_proj_add; result equal to the GPU's" % args.log_n}
 
-    # roofline of the bucket-accumulation kernel
-    accum_ms = phases[1] / args.steps
+    # roofline of the bucket-accumulation kernel: the same MSM without the affine tree levels, which
+    # otherwise leave it the last few additions of each bucket only
+    prev = L.zkg_set_msm_tree(0, 0)
+    step()
+    accum_ms = 0.0
+    for _ in range(3):
+        assert np.array_equal(step(), ref_out), "MSM result without tree levels differs"
+        L.zkg_last_phase_ms(ph, 4)
+        accum_ms += ph[1] / 3
+    L.zkg_set_msm_tree(prev, 0)
     accum_imad = float(adds.value) * IMAD_PER_MADD
     accum_fp64 = float(adds.value) * FP64_PER_MADD
     achieved = accum_fp64 / (accum_ms * 1e-3)
@@ -428,7 +436,8 @@ def run_msm(args, zk, L, torch, stream, rank, world, dist, imad_peak, fp64_peak)
                 "h2d_bytes_per_step": n * 32 + n * 64, "d2h_bytes_per_step": 64,
                 "wall_ms_per_step": 1e3 * wall_e2e, "device_ms_per_step": e2e_ms,
                 "pageable_host_buffers_wall_ms_per_step": 1e3 * wall_pageable},
-        "roofline": {"kernel": "k_msm_accum_w<BN254E, 384, 2> (bucket mixed additions, exact-radix FP64-pipe field products)",
+        "roofline": {"kernel": "k_msm_accum_w<BN254E, 384, 2> (bucket mixed additions, exact-radix FP64-pipe field "
+                               "products); all of the MSM's additions in it, run without the affine tree levels",
                      "bound": "fp64",
                      "achieved": achieved / 1e12, "peak": fp64_peak / 1e12, "unit": "T FP64 ops/s",
                      "frac": achieved / fp64_peak if fp64_peak > 0 else None,
@@ -450,7 +459,7 @@ def run_msm(args, zk, L, torch, stream, rank, world, dist, imad_peak, fp64_peak)
                                          "frac": accum_imad / (accum_ms * 1e-3) / imad_peak if imad_peak > 0 else None,
                                          "convention": "the same additions counted as 264 IMAD per product "
                                                        "(8x32-bit CIOS, 4w^2+w), against the measured mad.lo.u32 rate"}},
-        "phases_ms": {"sort": phases[0] / args.steps, "accumulate": accum_ms,
+        "phases_ms": {"sort": phases[0] / args.steps, "accumulate": phases[1] / args.steps,
                       "fold_levels": phases[2] / args.steps, "bucket_reduce": phases[3] / args.steps},
         "clocks": clocks, "gpu_launches": int(launches),
     }

@@ -149,6 +149,32 @@ def test_msm_affine_tree_levels_match_oracle(zk, curve):
         L.zkg_set_msm_tree(prev, -1)
 
 
+@pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("n", [1 << 17, 90001])
+def test_msm_affine_tree_waves(zk, curve, n):
+    """levels of one and of several waves of threads, the last one ragged, equal sum (s_i k_i) G; a
+    quarter of the scalars share one value, so segments from empty to n / 4 entries are padded"""
+    torch = pytest.importorskip("torch")
+    L = zk.lib()
+    ks = Z.rand_fr(curve, n, 29200 + n)
+    sc = Z.rand_fr(curve, n, 29300 + n)
+    sc[: n // 4] = sc[0]
+    d_k = torch.from_numpy(ks.view(np.int64)).cuda()
+    d_s = torch.from_numpy(sc.view(np.int64)).cuda()
+    d_b = torch.empty((n, 2 * Z.NLP[curve]), dtype=torch.int64, device="cuda")
+    zk.g1_gen_mul_device(curve, n, d_k, d_b)
+    torch.cuda.synchronize()
+    want = Z.msm_identity_affine(curve, ks, sc)
+    prev = L.zkg_set_msm_tree(-1, 0)
+    try:
+        for levels, slots in ((0, 64), (1, 4), (2, 5), (3, 64), (3, 9)):
+            L.zkg_set_msm_tree(levels, slots)
+            got = zk.msm_device(curve, n, d_s, d_b, mont=True, kind=zk.OUT_AFFINE)
+            assert np.array_equal(got, want), (n, levels, slots)
+    finally:
+        L.zkg_set_msm_tree(prev, -1)
+
+
 def _degenerate_checks(zk, curve):
     nl = Z.NLP[curve]
     n = 300

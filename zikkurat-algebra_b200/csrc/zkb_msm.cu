@@ -13,8 +13,8 @@
 //   2. scan          exclusive prefix sum of the counts -> one segment per (window, bucket)
 //   3. scatter       point indices (+ sign bit) placed at segment offset + rank, window after
 //                    window, no atomics
-//   4. affine tree   (BLS12-381, long segments) the first levels as affine pair sums with one
-//                    simultaneous inversion per level (zkb_msm_tree.cuh)
+//   4. affine tree   (long segments) the first levels as affine pair sums with one simultaneous
+//                    inversion per level (zkb_msm_tree.cuh)
 //   5. accumulate    equal-length chunks of the segmented array, one chunk per thread:
 //                    mixed additions of affine bases (the next one prefetched into shared
 //                    memory by cp.async) into an XYZZ accumulator, products on the FP64 pipe
@@ -300,13 +300,13 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* sm_war
 }
 
 __global__ void __launch_bounds__(SCAN_T) k_scan_blocks(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                        uint32_t* __restrict__ bsums, uint32_t n) {
+                                                        uint32_t* __restrict__ bsums, uint32_t n, uint32_t pad) {
   __shared__ uint32_t smw[32];
   const size_t base = (size_t)blockIdx.x * SCAN_T * SCAN_E + (size_t)threadIdx.x * SCAN_E;
   uint32_t v[SCAN_E], s = 0;
 #pragma unroll
   for (int e = 0; e < SCAN_E; e++) {
-    v[e] = (base + e < n) ? in[base + e] : 0u;
+    v[e] = (base + e < n) ? (in[base + e] + pad) & ~pad : 0u;
     s += v[e];
   }
   uint32_t total;
@@ -354,16 +354,16 @@ __global__ void k_scan_add(uint32_t* __restrict__ out, uint32_t* __restrict__ cu
 // this short runs its instructions from a cold cache, and 32 unrolled loads took 12 us.
 static constexpr uint32_t SCAN_ONE = SCAN_T * 32;
 __global__ void __launch_bounds__(SCAN_T) k_scan_one(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                     uint32_t* __restrict__ cursor, uint32_t n) {
+                                                     uint32_t* __restrict__ cursor, uint32_t n, uint32_t pad) {
   __shared__ uint32_t smw[32];
   const uint32_t e = (n + SCAN_T - 1) / SCAN_T, lo = min(n, threadIdx.x * e), hi = min(n, lo + e);
   uint32_t s = 0, total;
 #pragma unroll 4
-  for (uint32_t k = lo; k < hi; k++) s += in[k];
+  for (uint32_t k = lo; k < hi; k++) s += (in[k] + pad) & ~pad;
   uint32_t pre = block_excl_scan(s, smw, total);
 #pragma unroll 4
   for (uint32_t k = lo; k < hi; k++) {
-    const uint32_t v = in[k];
+    const uint32_t v = (in[k] + pad) & ~pad;
     out[k] = pre;
     cursor[k] = pre;
     pre += v;
@@ -371,13 +371,14 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_one(const uint32_t* __restrict_
   if (threadIdx.x == 0) out[n] = total;
 }
 
-// Exclusive prefix sum of n counts into out (and cursor); out[n] = the total. bs: block sums.
+// Exclusive prefix sum of n counts, each rounded up to a multiple of pad + 1 (a power of two), into out
+// (and cursor); out[n] = the total. bs: block sums.
 static zkg_status scan_counts(const uint32_t* cnt, uint32_t* out, uint32_t* cursor, uint32_t* bs, uint32_t n,
-                              cudaStream_t st) {
+                              cudaStream_t st, uint32_t pad = 0) {
   if (n <= SCAN_ONE)
-    return launch("scan_one", k_scan_one, dim3(1), dim3(SCAN_T), 0, st, cnt, out, cursor, n);
+    return launch("scan_one", k_scan_one, dim3(1), dim3(SCAN_T), 0, st, cnt, out, cursor, n, pad);
   const uint32_t nb = (n + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
-  ZKB_TRY(launch("scan_blocks", k_scan_blocks, dim3(nb), dim3(SCAN_T), 0, st, cnt, out, bs, n));
+  ZKB_TRY(launch("scan_blocks", k_scan_blocks, dim3(nb), dim3(SCAN_T), 0, st, cnt, out, bs, n, pad));
   ZKB_TRY(launch("scan_top", k_scan_top, dim3(1), dim3(SCAN_T), 0, st, bs, nb));
   return launch("scan_add", k_scan_add, dim3((n + 255) / 256), dim3(256), 0, st, out, cursor, (const uint32_t*)bs, n, nb);
 }
@@ -610,17 +611,26 @@ static int ilog2_floor(uint64_t x) {
   return r;
 }
 
-// Cost model: nwin * (n madds + 2^(c-1) buckets * w madd-equivalents) + per-window tail. w = 2.8
-// for BN254; 3.5 for BLS12-381, whose affine tree levels make an entry cheaper against a bucket's
-// running-sum additions (measured at 2^22: c = 16 29.5 ms, the 2.8 rule's c = 18 33.8 ms).
-static double bucket_weight(int curve) { return curve == ZKG_BLS12_381 ? 3.5 : 2.8; }
+// Cost model in mixed additions: nwin * (n + a per-window tail) + w per bucket. A bucket's two
+// running-sum additions weigh more where the bucket kernels are latency-bound (n from 2^17 on) and
+// more again once the affine tree makes an entry cheaper (from 2^19 on). Best measured c / picked,
+// BN254: 2^16 12 or 13 / 13, 2^17 13 / 13, 2^18 13 / 13, 2^19 14 / 14, 2^20 15 / 15, 2^21 15 / 15,
+// 2^22 15 or 16 / 16; BLS12-381: 2^17 13 / 13, 2^18 13 / 13, 2^19 15 / 15, 1000003 14 / 14, 2^21
+// 15 / 15, 2^22 16 / 16 (2^22 with the weight of small n: c = 18, 31.6 ms against 27.0).
+static double bucket_weight(int curve, int n) {
+  const bool bls = curve == ZKG_BLS12_381;
+  if (n < (1 << 17)) return bls ? 3.5 : 2.8;
+  if (n < (1 << 18)) return 5.0;
+  if (n < (bls ? 800000 : 1 << 21)) return 8.0;
+  return bls ? 16.0 : 12.0;
+}
 static int auto_window(int n, int scalar_bits, double w) {
   if (n <= 1) return 2;
   double best = 1e300;
   int bestc = 2;
   for (int c = 2; c <= 20; c++) {
     const int nwin = (scalar_bits + 1 + c - 1) / c;
-    const double cost = (double)nwin * ((double)n + w * (double)(1u << (c - 1)) + 4000.0);
+    const double cost = (double)nwin * ((double)n + 4000.0) + w * (double)win_shape(scalar_bits + 1, nwin).seg(nwin);
     if (cost < best) { best = cost; bestc = c; }
   }
   return bestc;
@@ -636,17 +646,19 @@ static int pick_window(int curve, int n, int scalar_bits) {
     const MsmTune& T = msm_tune(curve, round_log2((uint64_t)n));
     if (T.c > 0) return T.c;
   }
-  return auto_window(n, scalar_bits, bucket_weight(curve));
+  return auto_window(n, scalar_bits, bucket_weight(curve, n));
 }
 
 // Affine tree levels before the chunk accumulation (zkb_msm_tree.cuh). ZKB_MSM_TREE = the number
-// of levels (0 = none). By default BLS12-381 runs trees by the entries per bucket segment e:
-// none below 64, then log2(e) - 4 levels up to three (measured at c = 16: 2^18 and 2^20 points,
-// e = 32: the tree costs 0-40%; 2^21, e = 64: 2 levels 15.9 ms against 17.1; 2^22, e = 128:
-// 3 levels 28.5 ms against 33.1). BN254 runs none (its mixed addition is cheap enough that the
-// levels' extra passes over memory cancel their fewer products: 14.3-14.4 ms at 2^22 either way).
-// ZKB_MSM_TREE_B: output slots per tree thread (its simultaneous-inversion batch); by default 64
-// from e = 128 (2^22: 28.5 ms against 29.0 with 32), 32 below.
+// of levels (0 = none). By default by the entries per bucket segment e, from 8 M entries on (a level's
+// three launches and its inversions cost 60 us for BN254, 120 us for BLS12-381). Measured with 32 or 64
+// slots a thread, BN254: 2^19 c = 14 (e = 90) 0 / 1 / 2 levels 2461 / 2398 / 2523 us, 2^20 c = 15 (64)
+// 4213 / 3910 / 4136, 2^21 c = 15 (128) 7904 / 7171 / 7030, 2^22 c = 16 (132) 14548 / 13659 / 13108 and
+// three 13104; BLS12-381: 2^19 c = 15 (52) 5309 / 4845 / 4943, 1000003 c = 14 (166) 9484 / 8253 / 7718
+// and three 7882.
+// ZKB_MSM_TREE_B: output slots per tree thread (its simultaneous-inversion batch), about: 128 where the
+// levels keep several waves of threads (2^22: BN254 12.67 ms against 12.86 with 64, BLS12-381 26.66
+// against 26.96), 64 below (2^20 3.88 ms against 3.94 with 128; 2^19 2.34 with either).
 static int g_tree_env = env_int("ZKB_MSM_TREE", -1);
 static uint32_t g_tree_B = (uint32_t)std::max(0, env_int("ZKB_MSM_TREE_B", 0));   // 0: by e
 
@@ -658,15 +670,19 @@ static int pick_tree(uint64_t total, uint32_t nseg, int tuned) {
     int k = g_tree_env >= 0 ? g_tree_env : tuned - 1;
     if (k < 0) {
       const uint64_t e = total / std::max<uint32_t>(1, nseg);
-      if (C::Fp::N == 8 || e < 64) return 0;
-      k = std::min(3, ilog2_floor(e) - 4);
+      if (total < 8000000) return 0;
+      if (C::Fp::N == 8) k = e < 40 ? 0 : e < 92 ? 1 : e < 200 ? 2 : 3;
+      else k = e < 28 ? 0 : e < 60 ? 1 : e < 200 ? 2 : 3;
     }
-    return std::max(0, std::min(k, MAX_TREE));
+    // padding stays below the entries themselves, or small
+    k = std::max(0, std::min(k, MAX_TREE));
+    while (k > 0 && (uint64_t)nseg * ((1u << k) - 1) > std::max<uint64_t>(total, 1u << 22)) k--;
+    return k;
   }
 }
-static uint32_t pick_tree_slots(uint64_t total, uint32_t nseg) {
+static uint32_t pick_tree_slots(uint64_t total) {
   if (g_tree_B) return std::max<uint32_t>(4, g_tree_B);
-  return total / std::max<uint32_t>(1, nseg) >= 128 ? 64u : 32u;
+  return total >= 1u << 25 ? 128u : 64u;
 }
 
 // Launch shape of the accumulation (ZKB_MSM_ACCUM_SHAPE): 0 = 256-thread blocks, two per SM for
@@ -791,20 +807,27 @@ struct MsmPlan {
   uint32_t K1 = 0, G = 0;
   int gbits = 0;
   int pf = 2;               // prefetch stages of the accumulation
-  // affine tree levels before the chunk accumulation (zkb_msm_tree.cuh): level l's output count
-  // is at most tQ[l]; tthr[l] threads of tB output slots each
-  int tree = 0;
-  uint32_t tB = 32;
-  uint64_t tQ[MAX_TREE];
-  uint32_t tthr[MAX_TREE];
+  int tree = 0;             // affine tree levels before the chunk accumulation (zkb_msm_tree.cuh)
+  uint32_t tB = 32;         // slots per tree thread
+  uint64_t total_pad = 0;   // entries with the padding the tree needs, at most
   uint64_t acc_total = 0;   // entries of the chunk accumulation (a bound when tree > 0)
   // byte offsets into one arena block
   size_t o_std, o_cnt, o_off, o_cur, o_bs, o_ent, o_keyA, o_ptA, o_bsum, o_T, o_R, o_U, o_V, bytes;
   size_t o_prec, o_pdone, o_ppt;   // pieces of long segments (their count follows the histogram's counts)
   bool use_dig = false;   // digits and ranks stored at o_dig, o_rank (nwin x n words each)
   size_t o_dig = 0, o_rank = 0;
-  size_t o_toff[2], o_tpts[2], o_tpre, o_ttt, o_tscr;
+  size_t o_toff, o_tpts[2], o_tpre, o_ttt, o_tscr;
 };
+
+// Threads of a tree level: blocks of tree_nt threads, one resident per SM.
+template <class C> constexpr int tree_nt() { return C::Fp::N == 8 ? 384 : 256; }
+template <class C>
+static uint32_t tree_wave() { return (uint32_t)std::max(1, device_sm_count()) * tree_nt<C>(); }
+template <class C>
+static uint32_t tree_threads(const MsmPlan& P, int level) {
+  const uint32_t wave = tree_wave<C>();
+  return wave * tree_waves(P.total_pad >> (level + 1), wave, P.tB);
+}
 
 template <class C>
 static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force = 0) {
@@ -824,13 +847,12 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   const MsmTune& T = msm_tune(C::ID, round_log2((uint64_t)n));
   P.tree = pick_tree<C>(P.total_max, P.nseg, T.tree);
   P.acc_total = P.total_max;
-  if (P.tree > 0) {
-    P.tB = pick_tree_slots(P.total_max, P.nseg);
-    for (int l = 0; l < P.tree; l++) {   // sum_s ceil(m_s / 2^(l+1)) <= total / 2^(l+1) + nseg
-      P.tQ[l] = std::min<uint64_t>(P.acc_total, (P.total_max >> (l + 1)) + P.nseg);
-      P.tthr[l] = (uint32_t)((P.tQ[l] + P.tB - 1) / P.tB);
-      P.acc_total = P.tQ[l];
-    }
+  if (P.tree > 0) {   // segments padded to multiples of 2^tree
+    P.tB = pick_tree_slots(P.total_max);
+    P.total_pad = P.total_max + (uint64_t)P.nseg * ((1u << P.tree) - 1);
+    P.acc_total = P.total_pad >> P.tree;
+  } else {
+    P.total_pad = P.total_max;
   }
   P.L1 = (int)chunk_len(P.acc_total, accum_wave<C>(), T.L1);
   P.pf = g_msm_pf_env || T.pf < 0 ? g_msm_pf : T.pf;
@@ -847,13 +869,13 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   auto take = [&](size_t bytes) { size_t r = o; o = (o + bytes + 255) & ~size_t(255); return r; };
   const bool dig_path = g_msm_digits && g_msm_wmajor;   // P.use_dig below
   P.o_std = take(mont && !dig_path ? (size_t)n * 32 : 0);
-  P.o_cnt = take((size_t)(P.nseg + 2 + P.nwin) * 4);   // then: pieces; non-zero digits (k_sort_small); finished blocks a window
+  P.o_cnt = take((size_t)(P.nseg + 2 + P.nwin) * 4);   // then: pieces; non-zero digits (k_sort_small, tree); finished blocks a window
   P.o_off = take((size_t)P.nseg * 4 + 4);
   P.o_cur = take((size_t)P.nseg * 4 + 4);
   const uint32_t nb = (P.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
   if (nb > (uint32_t)SCAN_T * SCAN_E) return set_status(ZKG_ERR_ARG, "msm", "too many buckets");
   P.o_bs = take((size_t)nb * 4 + 4);
-  P.o_ent = take((size_t)P.total_max * 4 + 4);
+  P.o_ent = take((size_t)P.total_pad * 4 + 8);
   P.use_dig = dig_path;
   P.o_dig = take(P.use_dig ? (size_t)P.total_max * 4 + 4 : 0);
   P.o_rank = take(P.use_dig ? (size_t)P.total_max * 4 + 4 : 0);
@@ -867,16 +889,16 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   P.o_R = take((size_t)P.nwin * P.G * XB);
   P.o_U = take((size_t)P.nwin * (P.gbits + 1) * XB);
   P.o_V = take((size_t)P.nwin * XB);
-  P.o_toff[0] = P.o_toff[1] = P.o_tpts[0] = P.o_tpts[1] = P.o_tpre = P.o_ttt = P.o_tscr = 0;
+  P.o_toff = P.o_tpts[0] = P.o_tpts[1] = P.o_tpre = P.o_ttt = P.o_tscr = 0;
   if (P.tree > 0) {
     constexpr size_t AB = 8 * F::N, FB = 4 * F::N;   // bytes of an affine point, of a field element
-    P.o_toff[0] = take((size_t)P.nseg * 4 + 4);
-    P.o_toff[1] = take((size_t)P.nseg * 4 + 4);
-    P.o_tpts[0] = take(P.tQ[0] * AB);
-    P.o_tpts[1] = take(P.tree > 1 ? P.tQ[1] * AB : 0);
-    P.o_tpre = take(P.tQ[0] * FB);
-    P.o_ttt = take((size_t)P.tthr[0] * FB);
-    P.o_tscr = take((size_t)P.tthr[0] * FB);
+    const uint64_t q0 = P.total_pad / 2 + 1, thr = tree_threads<C>(P, 0);
+    P.o_toff = take((size_t)P.nseg * 4 + 4);
+    P.o_tpts[0] = take(q0 * AB);
+    P.o_tpts[1] = take(P.tree > 1 ? (q0 / 2 + 1) * AB : 0);
+    P.o_tpre = take(q0 * FB);
+    P.o_ttt = take(thr * FB);
+    P.o_tscr = take(thr * FB);
   }
   P.bytes = o;
   return ZKG_OK;
@@ -909,63 +931,51 @@ static zkg_status tree_smem_limit(K kernel, size_t bytes) {
 // prefetch stages of the tree's backward pass (ZKB_MSM_TREE_PF = 2 or 3); the forward pass has 3
 static int g_tree_pf = env_int("ZKB_MSM_TREE_PF", 2);
 
-template <class C, bool L0, int NT, int PF>
-static zkg_status launch_tree_bwd(const MsmPlan& P, uint32_t nthr, cudaStream_t st, const uint32_t* ent,
-                                  const uint32_t* in_pts, const uint32_t* in_off, const uint32_t* out_off,
-                                  const uint32_t* pre, const uint32_t* tinv, uint32_t* out_pts, uint32_t* chk,
-                                  uint32_t npts) {
+template <class C, bool L0, int PF>
+static zkg_status launch_tree_bwd(const MsmPlan& P, int level, uint32_t nthr, cudaStream_t st, const uint32_t* ent,
+                                  const uint32_t* in_pts, const uint32_t* total, const uint32_t* pre,
+                                  const uint32_t* tinv, uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
+  constexpr int NT = tree_nt<C>();
   const size_t smem = (size_t)PF * tree_bwd_pieces<typename C::Fp>() * NT * 16;
   ZKB_TRY((tree_smem_limit<false, C, L0, NT, PF>(k_tree_bwd<C, L0, NT, PF>, smem)));
-  return launch("msm_tree_bwd", k_tree_bwd<C, L0, NT, PF>, dim3((nthr + NT - 1) / NT), dim3(NT), smem, st, ent,
-                in_pts, in_off, out_off, P.nseg, P.tB, nthr, pre, tinv, out_pts, chk, npts);
+  return launch("msm_tree_bwd", k_tree_bwd<C, L0, NT, PF>, dim3(nthr / NT), dim3(NT), smem, st, ent, in_pts, total,
+                level, tree_wave<C>(), P.tB, pre, tinv, out_pts, level == P.tree - 1 ? 1 : 0, chk, npts);
 }
 
 template <class C, bool L0>
-static zkg_status launch_tree_level(const MsmPlan& P, uint32_t nthr, cudaStream_t st, const uint32_t* ent,
-                                    const uint32_t* in_pts, const uint32_t* in_off, const uint32_t* out_off,
-                                    uint32_t* pre, uint32_t* tt, uint32_t* scr, uint32_t* out_pts, uint32_t* chk,
-                                    uint32_t npts) {
+static zkg_status launch_tree_level(const MsmPlan& P, int level, cudaStream_t st, const uint32_t* ent,
+                                    const uint32_t* in_pts, const uint32_t* total, uint32_t* pre, uint32_t* tt,
+                                    uint32_t* scr, uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
   using F = typename C::Fp;
-  constexpr int NTF = 256, PFF = 3;
-  const size_t smf = (size_t)PFF * tree_fwd_pieces<F>() * NTF * 16;
-  ZKB_TRY((tree_smem_limit<true, C, L0, NTF, PFF>(k_tree_fwd<C, L0, NTF, PFF>, smf)));
-  ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, L0, NTF, PFF>, dim3((nthr + NTF - 1) / NTF), dim3(NTF), smf, st, ent,
-                 in_pts, in_off, out_off, P.nseg, P.tB, nthr, pre, tt, chk, npts));
+  constexpr int NT = tree_nt<C>(), PFF = 3;
+  const uint32_t nthr = tree_threads<C>(P, level);
+  const size_t smf = (size_t)PFF * tree_fwd_pieces<F>() * NT * 16;
+  ZKB_TRY((tree_smem_limit<true, C, L0, NT, PFF>(k_tree_fwd<C, L0, NT, PFF>, smf)));
+  ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, L0, NT, PFF>, dim3(nthr / NT), dim3(NT), smf, st, ent, in_pts, total,
+                 level, tree_wave<C>(), P.tB, pre, tt, chk, npts));
   // simultaneous inversion of the thread products: about 4 per thread
   const size_t T = std::min<size_t>(((size_t)nthr + 255) & ~size_t(255), std::max<size_t>(2048, (size_t)nthr / 4));
   ZKB_TRY(launch("msm_tree_inv", k_tree_inv<F>, dim3((unsigned)((T + 255) / 256)), dim3(256), 0, st, nthr, tt, scr));
-  // backward pass: one block per SM, as the accumulation (BN254: 384 threads, 166 registers)
-  constexpr int NTB = F::N == 8 ? 384 : 256;
   if (g_tree_pf >= 3)
-    return launch_tree_bwd<C, L0, NTB, 3>(P, nthr, st, ent, in_pts, in_off, out_off, pre, tt, out_pts, chk, npts);
-  return launch_tree_bwd<C, L0, NTB, 2>(P, nthr, st, ent, in_pts, in_off, out_off, pre, tt, out_pts, chk, npts);
+    return launch_tree_bwd<C, L0, 3>(P, level, nthr, st, ent, in_pts, total, pre, tt, out_pts, chk, npts);
+  return launch_tree_bwd<C, L0, 2>(P, level, nthr, st, ent, in_pts, total, pre, tt, out_pts, chk, npts);
 }
 
-// The affine tree levels of one point range (zkb_msm_tree.cuh): level l reads the sorted entries
-// and bases (l = 0) or level l - 1's list, and writes its offsets to o_toff[l & 1] and its points
-// to o_tpts[l & 1]. The sort's count, cursor and scan buffers are free by now and are reused.
+// The affine tree levels of one point range (zkb_msm_tree.cuh), after the sort has placed the entries of
+// the padded segments: level l reads the entries and bases (l = 0) or level l - 1's list and writes its
+// points to o_tpts[l & 1]; the last list's offsets go to o_toff.
 template <class C>
-static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, const uint32_t* ent, const uint32_t* off,
+static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, uint32_t* ent, const uint32_t* off,
                                   const uint32_t* bases, cudaStream_t st, uint32_t* chk) {
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
-  const uint32_t* in_off = off;
-  const uint32_t* in_pts = bases;
-  for (int l = 0; l < P.tree; l++) {
-    uint32_t* out_off = U32(P.o_toff[l & 1]);
-    uint32_t* out_pts = U32(P.o_tpts[l & 1]);
-    ZKB_TRY(launch("msm_tree_counts", k_tree_counts, dim3((P.nseg + 255) / 256), dim3(256), 0, st, in_off, P.nseg,
-                   U32(P.o_cnt)));
-    ZKB_TRY(scan_counts(U32(P.o_cnt), out_off, U32(P.o_cur), U32(P.o_bs), P.nseg, st));
-    const uint32_t npts = l == 0 ? (uint32_t)P.n : (uint32_t)P.tQ[l - 1];
-    if (l == 0)
-      ZKB_TRY((launch_tree_level<C, true>(P, P.tthr[l], st, ent, in_pts, in_off, out_off, U32(P.o_tpre), U32(P.o_ttt),
-                                          U32(P.o_tscr), out_pts, chk, npts)));
-    else
-      ZKB_TRY((launch_tree_level<C, false>(P, P.tthr[l], st, ent, in_pts, in_off, out_off, U32(P.o_tpre),
-                                           U32(P.o_ttt), U32(P.o_tscr), out_pts, chk, npts)));
-    in_off = out_off;
-    in_pts = out_pts;
-  }
+  ZKB_TRY(launch("msm_tree_pad", k_tree_pad, dim3(P.nseg / 256 + 1), dim3(256), 0, st, (const uint32_t*)U32(P.o_cnt), off,
+                 P.nseg, P.tree, ent, U32(P.o_toff), U32(P.o_cnt) + P.nseg + 1));
+  const uint32_t* total = off + P.nseg;
+  ZKB_TRY((launch_tree_level<C, true>(P, 0, st, ent, bases, total, U32(P.o_tpre), U32(P.o_ttt), U32(P.o_tscr),
+                                      U32(P.o_tpts[0]), chk, (uint32_t)P.n)));
+  for (int l = 1; l < P.tree; l++)
+    ZKB_TRY((launch_tree_level<C, false>(P, l, st, nullptr, U32(P.o_tpts[(l - 1) & 1]), total, U32(P.o_tpre),
+                                         U32(P.o_ttt), U32(P.o_tscr), U32(P.o_tpts[l & 1]), nullptr, 0)));
   return ZKG_OK;
 }
 
@@ -1032,14 +1042,15 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
   else
     ZKB_TRY(launch("msm_hist", k_msm_hist, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win, P.nwin,
                    U32(P.o_cnt), chk, dig, rank));
-  ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st));
+  ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st,
+                      P.tree > 0 ? (1u << P.tree) - 1 : 0u));
   if (dig)
     ZKB_TRY(launch("msm_scatter_d", k_msm_scatter_d, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n,
                    (const uint32_t*)dig, (const uint32_t*)rank, P.win, (const uint32_t*)U32(P.o_off), U32(P.o_ent),
-                   chk, (uint32_t)P.total_max));
+                   chk, (uint32_t)P.total_pad));
   else if (wmajor)
     ZKB_TRY(launch("msm_scatter_w", k_msm_scatter_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw,
-                   P.win, ct, U32(P.o_cur), U32(P.o_ent), chk, (uint32_t)P.total_max));
+                   P.win, ct, U32(P.o_cur), U32(P.o_ent), chk, (uint32_t)P.total_pad));
   else
     ZKB_TRY(launch("msm_scatter", k_msm_scatter, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win,
                    P.nwin, U32(P.o_cur), U32(P.o_ent)));
@@ -1063,12 +1074,12 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
   if constexpr (!radix_conv_v<typename C::Fp>) {
     if (P.tree > 0) {   // affine tree levels; the chunk accumulation takes the last level's list
       NvtxRange nvtx_tree("zkb.msm.affine_tree");
-      ZKB_TRY(msm_tree_launch<C>(P, ws, ent, off, bases, st, chk));
+      ZKB_TRY(msm_tree_launch<C>(P, ws, U32(P.o_ent), off, bases, st, chk));
       const int lt = (P.tree - 1) & 1;
       ent = nullptr;
-      off = U32(P.o_toff[lt]);
+      off = U32(P.o_toff);
       bases = U32(P.o_tpts[lt]);
-      acc_npts = (uint32_t)P.tQ[P.tree - 1];
+      acc_npts = (uint32_t)P.acc_total;
     }
   }
   const PieceList pl = {U32(P.o_cnt) + P.nseg, P.pcap, reinterpret_cast<Piece*>(ws + P.o_prec), U32(P.o_pdone),
@@ -1152,7 +1163,7 @@ static zkg_status msm_finish(Context& cx, const host::Field<NL>& F, const MsmPla
   // number of (window, point) entries with a non-zero digit = mixed additions performed
   for (int q = 0; q < nparts; q++)
     ZKB_CUDA(cudaMemcpyAsync(pin + ubytes + 4 * q,
-                             ws[q] + (P[q].small ? P[q].o_cnt + 4 : P[q].o_off) + (size_t)P[q].nseg * 4, 4,
+                             ws[q] + (P[q].small || P[q].tree > 0 ? P[q].o_cnt + 4 : P[q].o_off) + (size_t)P[q].nseg * 4, 4,
                              cudaMemcpyDeviceToHost, st));
   ZKB_CUDA(cudaStreamSynchronize(st));
   cx.last_msm_entries = 0;
@@ -2501,7 +2512,7 @@ static zkg_status autotune_msm(const host::Field<NL>& F, const uint64_t* d_bases
       return t;
     };
     T = MsmTune();
-    const int c0 = auto_window(n, C::SCALAR_BITS, bucket_weight(C::ID));
+    const int c0 = auto_window(n, C::SCALAR_BITS, bucket_weight(C::ID, n));
     float best = 1e30f;
     MsmTune bestT;
     for (int c = std::max(2, c0 - 2); c <= std::min(20, c0 + 2) && st == ZKG_OK; c++) {
@@ -2938,7 +2949,7 @@ int zkg_set_msm_window(int c) {
 int zkg_msm_window_for(zkg_curve curve, int npoints) {
   if (zkb::g_window_override > 0) return zkb::g_window_override;
   return zkb::auto_window(npoints, curve == ZKG_BLS12_381 ? zkb::BLS12_381::SCALAR_BITS : zkb::BN254::SCALAR_BITS,
-                          zkb::bucket_weight(curve));
+                          zkb::bucket_weight(curve, npoints));
 }
 
 }  // extern "C"
