@@ -78,6 +78,22 @@ def test_g1_fft_random_vs_oracle(zk, curve, m):
                 assert np.array_equal(got, want), (fam, tag, fn)
 
 
+@pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("g", [1, 2, 7, 16, -1])
+def test_g1_fft_short_scalars(zk, curve, g):
+    """scalars whose windows are mostly empty, identity points, and butterflies whose sum or difference
+    is the identity"""
+    m = 4
+    gen = Z.to_limbs((g % zk.R_MOD[curve]) * (1 << 256) % zk.R_MOD[curve], 4)
+    src = rand_points(curve, 1 << m, 9600, False)
+    src[8] = src[0]
+    src[5], src[13] = np.zeros_like(src[5]), np.zeros_like(src[13])
+    src[5, Z.NLP[curve]] = src[13, Z.NLP[curve]] = 1
+    for inv, fn in ((0, "forward"), (1, "inverse")):
+        got = fft_call(zk, curve, "proj", fn, m, gen, src)
+        assert np.array_equal(got, Z.oracle_g1_fft(curve, False, m, gen, src, inv)), fn
+
+
 def _discrete_log_check(zk, curve, m, seed):
     """x_i = k_i G: forward FFT must give [NTT(k)_j] G, and the inverse must return x"""
     import torch

@@ -235,7 +235,7 @@ __global__ void k_g1fft_stage(int m, int s, const uint32_t* __restrict__ tw, con
 
 // The same stage by quads (zkb_quad.cuh), for transforms with too few butterflies to fill the GPU: a
 // scalar multiplication is a chain of ~210 point operations, and at 2^14 points a thread a butterfly
-// left one warp a scheduler (1.10 ms a stage; this 0.46). A butterfly has HALVES quads: with 2, each
+// left one warp a scheduler (BN254 16.4 ms; this 11.8). A butterfly has HALVES quads: with 2, each
 // multiplies by one half of the split scalar (quad 1 the image under phi) and the two results are
 // added: the shortest chain, at 1.5 times the work; with 1, the quad takes both halves in one scan.
 // The top stage of an inverse transform has two scalars and always two quads, one a scalar.
@@ -288,9 +288,6 @@ __device__ __noinline__ Fe<F> quad_mul_glv(const Fe<F> P, const uint32_t (&k)[GL
   Fe<F> acc = fe_zero<F>();
 #pragma unroll 1
   for (int w = 34; w >= 0; w--) {
-    if (w != 34)
-#pragma unroll 1
-      for (int i = 0; i < 4; i++) acc = quad_dbl(acc);
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
       if (h == 1 && !__any_sync(FULL, both)) break;
@@ -304,7 +301,14 @@ __device__ __noinline__ Fe<F> quad_mul_glv(const Fe<F> P, const uint32_t (&k)[GL
           for (int i = 0; i < F::N; i++) q.v[i] = smb[(e * F::N + i) * (QUAD_T / 4) + (threadIdx.x >> 2)];
         if (L == 1 && (d < 0) != ((h ? s2 : s1) != 0)) q = fe_neg(q);
       }
-      acc = quad_add(acc, q);
+      if constexpr (F::DPF) {
+        acc = h == 0 ? quad_window(acc, q) : quad_add(acc, q);   // the first window finds the identity
+      } else {
+        if (h == 0 && w != 34)
+#pragma unroll 1
+          for (int i = 0; i < 4; i++) acc = quad_dbl(acc);
+        acc = quad_add(acc, q);
+      }
     }
   }
   return acc;
