@@ -1020,40 +1020,40 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
     ZKB_TRY(launch("msm_sort_small", small, dim3(P.nwin), dim3(SMALL_T), 0, st, n, scal, P.nw, P.win,
                    digit_bias(P.win, P.nwin), P.nseg, U32(P.o_off), U32(P.o_ent), U32(P.o_cnt) + P.nseg + 1));
   } else {
-  if (mont && !hist_mont) {
-    ZKB_TRY(launch("msm_scalar_from_mont", k_msm_scalar_from_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st,
-                   n, d_scal, U32(P.o_std)));
-    scal = U32(P.o_std);
-  }
-  ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)(P.nseg + 2 + P.nwin) * 4, st));
-  CarryTable ct;
-  const bool wmajor = g_msm_wmajor && make_carry_table(P.nwin, P.nw, P.win, ct);
-  // the histogram reads each scalar once and loops over its windows (the window-major histogram
-  // re-reads the scalars per window and measured slower); the scatter is window-major, from the
-  // digits the histogram stores (P.o_dig) or, without them, re-deriving each digit from its scalar
-  uint32_t* dig = P.use_dig ? U32(P.o_dig) : nullptr;
-  uint32_t* rank = P.use_dig ? U32(P.o_rank) : nullptr;
-  if (hist_mont)
-    ZKB_TRY(launch("msm_hist_mont", k_msm_hist_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st, n, d_scal, P.win,
-                   P.nwin, U32(P.o_cnt), chk, dig, rank));
-  else if (wmajor && g_msm_hist_wmajor && !dig)
-    ZKB_TRY(launch("msm_hist_w", k_msm_hist_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw, P.win,
-                   ct, U32(P.o_cnt), chk));
-  else
-    ZKB_TRY(launch("msm_hist", k_msm_hist, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win, P.nwin,
-                   U32(P.o_cnt), chk, dig, rank));
-  ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st,
-                      P.tree > 0 ? (1u << P.tree) - 1 : 0u));
-  if (dig)
-    ZKB_TRY(launch("msm_scatter_d", k_msm_scatter_d, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n,
-                   (const uint32_t*)dig, (const uint32_t*)rank, P.win, (const uint32_t*)U32(P.o_off), U32(P.o_ent),
-                   chk, (uint32_t)P.total_pad));
-  else if (wmajor)
-    ZKB_TRY(launch("msm_scatter_w", k_msm_scatter_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw,
-                   P.win, ct, U32(P.o_cur), U32(P.o_ent), chk, (uint32_t)P.total_pad));
-  else
-    ZKB_TRY(launch("msm_scatter", k_msm_scatter, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win,
-                   P.nwin, U32(P.o_cur), U32(P.o_ent)));
+    if (mont && !hist_mont) {
+      ZKB_TRY(launch("msm_scalar_from_mont", k_msm_scalar_from_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st,
+                     n, d_scal, U32(P.o_std)));
+      scal = U32(P.o_std);
+    }
+    ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)(P.nseg + 2 + P.nwin) * 4, st));
+    CarryTable ct;
+    const bool wmajor = g_msm_wmajor && make_carry_table(P.nwin, P.nw, P.win, ct);
+    // the histogram reads each scalar once and loops over its windows (the window-major histogram
+    // re-reads the scalars per window and measured slower); the scatter is window-major, from the
+    // digits the histogram stores (P.o_dig) or, without them, re-deriving each digit from its scalar
+    uint32_t* dig = P.use_dig ? U32(P.o_dig) : nullptr;
+    uint32_t* rank = P.use_dig ? U32(P.o_rank) : nullptr;
+    if (hist_mont)
+      ZKB_TRY(launch("msm_hist_mont", k_msm_hist_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st, n, d_scal, P.win,
+                     P.nwin, U32(P.o_cnt), chk, dig, rank));
+    else if (wmajor && g_msm_hist_wmajor && !dig)
+      ZKB_TRY(launch("msm_hist_w", k_msm_hist_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw, P.win,
+                     ct, U32(P.o_cnt), chk));
+    else
+      ZKB_TRY(launch("msm_hist", k_msm_hist, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win, P.nwin,
+                     U32(P.o_cnt), chk, dig, rank));
+    ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st,
+                        P.tree > 0 ? (1u << P.tree) - 1 : 0u));
+    if (dig)
+      ZKB_TRY(launch("msm_scatter_d", k_msm_scatter_d, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n,
+                     (const uint32_t*)dig, (const uint32_t*)rank, P.win, (const uint32_t*)U32(P.o_off), U32(P.o_ent),
+                     chk, (uint32_t)P.total_pad));
+    else if (wmajor)
+      ZKB_TRY(launch("msm_scatter_w", k_msm_scatter_w, dim3((n + 255) / 256, P.nwin), dim3(256), 0, st, n, scal, P.nw,
+                     P.win, ct, U32(P.o_cur), U32(P.o_ent), chk, (uint32_t)P.total_pad));
+    else
+      ZKB_TRY(launch("msm_scatter", k_msm_scatter, dim3((n + 255) / 256), dim3(256), 0, st, n, scal, P.nw, P.win,
+                     P.nwin, U32(P.o_cur), U32(P.o_ent)));
   }
   const uint32_t* bases = reinterpret_cast<const uint32_t*>(d_bases);
   if (first) ZKB_CUDA(cudaEventRecord(cx.ev_phase[1], st));
