@@ -424,6 +424,9 @@ zkg_status zkg_msm_binary(zkg_curve curve, zkg_out_kind out_kind, int nrows, int
                           const uint8_t *const *rows, const uint64_t *bases, uint64_t *out);
 zkg_status zkg_msm_binary_device(zkg_curve curve, zkg_out_kind out_kind, int nrows, int npoints,
                                  const uint8_t *d_coeffs, size_t ld, const uint64_t *d_bases, uint64_t *d_out);
+/* Device memory of a binary MSM, planned on the host (no GPU needed): info[0] bytes a launch is given,
+ * info[1] the most any of its launches uses, info[2] the call's workspace in all. */
+zkg_status zkg_msm_binary_plan(zkg_curve curve, int from_host, int nrows, int npoints, size_t info[3]);
 
 /* ------------------------------------------------------------------- Fr vector operations
  * zkg_fr_map computes out[i] = op(a[i], b[i], c[i]; A, B) on host buffers of n Montgomery Fr

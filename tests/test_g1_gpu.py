@@ -289,6 +289,13 @@ def test_binary_msm_bls12_381_single_row_chunked(zk):
     _binary_large(zk, Z.BLS12_381, 1, (1 << 19) + 12345, 9900, [0])
 
 
+@pytest.mark.parametrize("curve,nrows,npts", [(Z.BN254, 1, 1035752), (Z.BN254, 14, 1035752), (Z.BN254, 64, 1035752),
+                                              (Z.BLS12_381, 1, 690502), (Z.BLS12_381, 14, 690502)])
+def test_binary_msm_ragged_last_chunk(zk, curve, nrows, npts):
+    """last column chunks a little shorter than the others: shorter accumulation chunks, and more of them"""
+    _binary_large(zk, curve, nrows, npts, 9950 + nrows, [0])
+
+
 def test_binary_msm_rejects_bad_arguments(zk):
     L = zk.lib()
     b = np.zeros(16, np.uint64)

@@ -696,7 +696,7 @@ struct BinPlan {
   int batch = 0;          // rows a launch
   int cw = 0;             // columns a chunk
   int G = 1;              // chunks = partial sums a row
-  size_t bits_bytes = 0;  // workspace of one launch
+  size_t bits_bytes = 0;  // workspace of the launches: the largest any of them needs
 };
 static constexpr int BIN_ROWS = 32768;   // rows a launch (grid dimensions) and a reduction, at most
 
@@ -713,7 +713,16 @@ static zkg_status bin_plan(int nrows, int npoints, int nl, bool host, BinPlan& P
   }
   P.cw = (int)std::max<size_t>(cw, 1);
   P.G = (npoints + P.cw - 1) / P.cw;
-  return msm_bits_bytes(nl == 4 ? ZKG_BN254 : ZKG_BLS12_381, P.batch, P.cw, P.rho, &P.bits_bytes);
+  // A launch's workspace does not grow steadily with its size (a little fewer entries can make shorter and
+  // so more chunks), so the last rows and the last columns are asked for as well.
+  P.bits_bytes = 0;
+  for (const int rows : {P.batch, nrows % P.batch})
+    for (const int cols : {P.cw, npoints % P.cw}) {
+      size_t b = 0;
+      if (rows && cols) ZKB_TRY(msm_bits_bytes(nl == 4 ? ZKG_BN254 : ZKG_BLS12_381, rows, cols, P.rho, &b));
+      P.bits_bytes = std::max(P.bits_bytes, b);
+    }
+  return ZKG_OK;
 }
 
 // Runs the chunk loop. get_chunk(q, col0, cw, &coeffs, &ld, &bases) makes chunk q's coefficient
@@ -734,7 +743,7 @@ static zkg_status bin_run(Context& cx, const BinPlan& P, int nrows, int npoints,
     ZKB_TRY(get_chunk(q, col0, cw, &coeffs, &ld, &bases));
     for (int r = 0; r < nrows; r += P.batch)
       ZKB_TRY(msm_bits_launch(cx, C::ID == 0 ? ZKG_BN254 : ZKG_BLS12_381, std::min(P.batch, nrows - r), cw, P.rho,
-                              coeffs + (size_t)r * ld, ld, bases, work, partial + ((size_t)r * P.G + q) * XW,
+                              coeffs + (size_t)r * ld, ld, bases, work, P.bits_bytes, partial + ((size_t)r * P.G + q) * XW,
                               (size_t)P.G * XW, st));
     ZKB_TRY(get_chunk(-1 - q, 0, 0, nullptr, nullptr, nullptr));   // chunk q's inputs are consumed
   }
@@ -917,6 +926,24 @@ extern "C" zkg_status zkg_g1_fft_device(zkg_curve curve, int jac, int m, const u
   ZKB_TRY(g1_fft_check(curve, m, gen, d_src, d_tgt));
   if (curve == ZKG_BN254) return g1_fft_dev<BN254, 4>(jac ? 1 : 0, m, gen, d_src, d_tgt, inverse ? 1 : 0);
   return g1_fft_dev<BLS12_381, 6>(jac ? 1 : 0, m, gen, d_src, d_tgt, inverse ? 1 : 0);
+}
+
+extern "C" zkg_status zkg_msm_binary_plan(zkg_curve curve, int from_host, int nrows, int npoints, size_t info[3]) {
+  if ((curve != ZKG_BN254 && curve != ZKG_BLS12_381) || nrows < 1 || npoints < 1 || !info)
+    return set_status(ZKG_ERR_ARG, "msm_binary_plan", "bad argument");
+  const int nl = curve == ZKG_BN254 ? 4 : 6;
+  BinPlan P;
+  ZKB_TRY(bin_plan(nrows, npoints, nl, from_host != 0, P));
+  info[0] = P.bits_bytes;
+  info[1] = 0;
+  for (int r = 0; r < nrows; r += P.batch)   // the launches of bin_run
+    for (int q = 0; q < P.G; q++) {
+      size_t b = 0;
+      ZKB_TRY(msm_bits_bytes(curve, std::min(P.batch, nrows - r), std::min(P.cw, npoints - q * P.cw), P.rho, &b));
+      info[1] = std::max(info[1], b);
+    }
+  info[2] = nl == 4 ? bin_ws_bytes<4>(P, nrows) : bin_ws_bytes<6>(P, nrows);
+  return set_status(ZKG_OK, nullptr, nullptr);
 }
 
 extern "C" zkg_status zkg_msm_binary(zkg_curve curve, int out_kind, int nrows, int npoints,

@@ -1499,9 +1499,11 @@ static zkg_status bits_plan(int nrows, int ncols, int rho, BitsPlan& P) {
 
 template <class C>
 static zkg_status bits_launch(int nrows, int ncols, int rho, const uint8_t* coeffs, size_t ld, const uint32_t* bases,
-                              char* ws, uint32_t* out, size_t stride, uint32_t* chk, cudaStream_t st) {
+                              char* ws, size_t ws_bytes, uint32_t* out, size_t stride, uint32_t* chk,
+                              cudaStream_t st) {
   BitsPlan P;
   ZKB_TRY(bits_plan<C>(nrows, ncols, rho, P));
+  if (P.bytes > ws_bytes) return set_status(ZKG_ERR_NOMEM, "msm_binary", "workspace smaller than the launch needs");
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
   ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)P.nseg * 4 + 4, st));
   const dim3 gc((ncols + 255) / 256);
@@ -1533,11 +1535,12 @@ zkg_status msm_bits_bytes(int curve, int nrows, int ncols, int rho, size_t* byte
 }
 
 zkg_status msm_bits_launch(Context& cx, int curve, int nrows, int ncols, int rho, const uint8_t* coeffs, size_t ld,
-                           const uint32_t* bases, char* ws, uint32_t* out, size_t stride, cudaStream_t st) {
+                           const uint32_t* bases, char* ws, size_t ws_bytes, uint32_t* out, size_t stride,
+                           cudaStream_t st) {
   uint32_t* chk = dev_check_word(cx);
   if (curve == ZKG_BN254)
-    return bits_launch<BN254E>(nrows, ncols, rho, coeffs, ld, bases, ws, out, stride, chk, st);
-  return bits_launch<BLS12_381E>(nrows, ncols, rho, coeffs, ld, bases, ws, out, stride, chk, st);
+    return bits_launch<BN254E>(nrows, ncols, rho, coeffs, ld, bases, ws, ws_bytes, out, stride, chk, st);
+  return bits_launch<BLS12_381E>(nrows, ncols, rho, coeffs, ld, bases, ws, ws_bytes, out, stride, chk, st);
 }
 
 // =================================================================== batched MSMs (many sizes)
