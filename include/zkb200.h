@@ -506,7 +506,8 @@ zkg_status zkg_msm_resident_host(zkg_bases *h, int npoints, const uint64_t *expo
  * 32-bit-product pipelines always use graph branches.
  * zkg_batch_set_wait_limit (before the first run): polls a pass waits for the one before it
  * (default 2^24, about 2 s) before the run fails with ZKG_ERR_TIMEOUT; inject_stall != 0 makes
- * one pass wait for a tile that never comes (tests of that path). zkg_batch_persistent reports
+ * one pass wait for a tile that never comes (tests of that path; in the graph form, whose passes wait
+ * on their own copies and tensor-core work, the first NTT's passes give up at their first wait). zkg_batch_persistent reports
  * whether the batch runs the persistent kernel (1), its grid and its number of tasks. */
 typedef struct zkg_batch zkg_batch;
 zkg_status zkg_batch_create(zkg_curve curve, const uint64_t *d_bases, int n_bases, zkg_batch **out);

@@ -104,6 +104,35 @@ def test_batch_runs_one_persistent_kernel_with_bounded_waits(zk):
 
 
 @pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("m", [9, 14, 18])
+def test_matrix_pass_that_gives_up_ends_with_a_status(zk, curve, m):
+    """a matrix-form NTT pass whose bounded wait runs out leaves with its copies and MMAs finished: the
+    run returns ZKG_ERR_TIMEOUT, and the next transforms and batches on the device are right"""
+    import torch
+    x = torch.from_numpy(Z.rand_fr(curve, 1 << m, 46000 + m).view(np.int64)).cuda()
+    want, got = torch.empty_like(x), torch.empty_like(x)
+    zk.ntt_device(curve, m, x, want)
+    d_b = _bases(zk, curve, 16, 46001)
+    for stall in (True, False):
+        b = zk.Batch(curve, d_b, 16)
+        if stall:
+            b.set_wait_limit(1 << 24, inject_stall=True)
+        b.add_ntt(m, x, got)
+        if stall:
+            with pytest.raises(zk.ZkgError) as e:
+                b.run()
+            assert e.value.status == zk.ERR_TIMEOUT
+        else:
+            b.run()
+        b.close()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    zk.ntt_device(curve, m, x, got)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("curve", Z.CURVES)
 def test_server_results_same_alone_and_in_the_mix(zk, curve):
     import torch
     nb = 1 << 13

@@ -1797,7 +1797,7 @@ struct zkg_batch {
   // persistent mode: the accumulation and every NTT pass in one launch (k_batch_work)
   bool persistent = false;
   uint32_t wait_limit = 1u << 24;   // polls of a pass-dependency wait (~2 s) before ZKG_ERR_TIMEOUT
-  bool inject_stall = false;        // testing: one pass waits for a tile that never comes
+  bool inject_stall = false;        // testing: one pass waits for a tile that never comes (graph form: see enqueue)
   bool persistent_wanted = true;    // build the persistent form (ZKB_BATCH_PERSISTENT / zkg_batch_set_mode)
   size_t err_pin_off = 0;           // error word's copy inside pin
   int work_grid = 0;
@@ -2076,9 +2076,11 @@ static zkg_status batch_build(zkg_batch* b, const host::Field<NL>& F) {
     for (int i = 0; i < nstreams; i++) ZKB_CUDA(cudaStreamWaitEvent(b->s_ntt[i], b->ev_fork[nstreams], 0));
     for (size_t i = 0; i < b->ntts.size(); i++) {
       const int si = (int)(i % nstreams);
+      NttRun run;
+      if (b->inject_stall && i == 0) run.wait_limit = 0;   // testing: every wait inside its passes runs out
       ZKB_TRY(ntt_plan_execute(*b->plans[i], reinterpret_cast<const uint32_t*>(b->ntts[i].d_src),
                                reinterpret_cast<uint32_t*>(b->ntts[i].d_tgt),
-                               reinterpret_cast<uint32_t*>(ws + b->ntt_scratch_off[si]), b->s_ntt[si]));
+                               reinterpret_cast<uint32_t*>(ws + b->ntt_scratch_off[si]), b->s_ntt[si], run));
     }
     if (!b->mp.reqs.empty()) {
       if (b->conv_off) {

@@ -382,7 +382,7 @@ static zkg_status build_plan(Context& cx, const host::Field<4>& F, int curve, in
 // Runs the plan d_src -> d_tgt; scratch (N elements) needed when there are >= 2 passes.
 template <class P>
 static zkg_status ntt_run(Context& cx, const NttPlan& pl, const uint32_t* d_src, uint32_t* d_tgt, uint32_t* scratch,
-                          cudaStream_t st) {
+                          cudaStream_t st, const NttRun& run = {}) {
   const int np = (int)pl.passes.size();
   const size_t N = (size_t)1 << pl.m;
   if (np == 0) {   // m = 0: copy (bn128_poly_mont.c:420-423)
@@ -394,7 +394,7 @@ static zkg_status ntt_run(Context& cx, const NttPlan& pl, const uint32_t* d_src,
     // the i-th executed pass writes tgt when (np-1-i) is even, scratch otherwise
     uint32_t* out = ((np - 1 - i) % 2 == 0) ? d_tgt : scratch;
     const NttPass& q = pl.inverse ? pl.passes[np - 1 - i] : pl.passes[i];
-    if (pl.mat) ZKB_TRY(ntt_mat_launch_pass<P>(pl, i, in, out, cx.sm_count, st));
+    if (pl.mat) ZKB_TRY(ntt_mat_launch_pass<P>(pl, i, in, out, cx.sm_count, run, st));
     else if (pl.dpf) ZKB_TRY(ntt_launch_pass<typename DpfOf<P>::type>(pl, q, in, out, pl.inverse && i == np - 1, st));
     else ZKB_TRY(ntt_launch_pass<P>(pl, q, in, out, pl.inverse && i == np - 1, st));
     in = out;
@@ -599,11 +599,11 @@ zkg_status ntt_plan_fault(const NttPlan& pl) {
 }
 
 zkg_status ntt_plan_execute(const NttPlan& pl, const uint32_t* d_src, uint32_t* d_tgt, uint32_t* scratch,
-                            cudaStream_t st) {
+                            cudaStream_t st, const NttRun& run) {
   Context* cx = nullptr;
   ZKB_TRY(get_context(&cx));
-  if (pl.curve == ZKG_BN254) return ntt_run<BnFr>(*cx, pl, d_src, d_tgt, scratch, st);
-  return ntt_run<BlsFr>(*cx, pl, d_src, d_tgt, scratch, st);
+  if (pl.curve == ZKG_BN254) return ntt_run<BnFr>(*cx, pl, d_src, d_tgt, scratch, st, run);
+  return ntt_run<BlsFr>(*cx, pl, d_src, d_tgt, scratch, st, run);
 }
 
 }  // namespace zkb

@@ -30,6 +30,13 @@ struct NttMatPass {
   int tw, tw_S;            // group twiddles applied to the outputs (-1: none); bits before that group
 };
 
+// How one execution of a plan runs. wait_limit: polls of a barrier inside a matrix pass (2^24: a third of
+// a second at the least) before the pass gives up.
+static constexpr uint32_t NTT_WAIT_LIMIT = 1u << 24;
+struct NttRun {
+  uint32_t wait_limit = NTT_WAIT_LIMIT;
+};
+
 struct NttPlan {
   int curve = -1, m = -1, inverse = 0, kmax = 0;
   bool dpf = false;                  // tables in radix R' = 2^260: passes multiply on the FP64 pipe
@@ -67,7 +74,7 @@ zkg_status ntt_launch_table(uint32_t* T, const uint32_t* A, const uint32_t* Bt, 
 // its network matrix and the powers of its fold base; a group boundary's twiddles in FP64 radix.
 template <class P>
 zkg_status ntt_mat_launch_pass(const NttPlan& pl, int exec, const uint32_t* in, uint32_t* out, int sms,
-                               cudaStream_t st);
+                               const NttRun& run, cudaStream_t st);
 template <class P>
 zkg_status ntt_mat_build(const uint32_t* net, const uint32_t* pw, int k, int u, int inverse, int nout, uint8_t* dst,
                          cudaStream_t st);
@@ -85,6 +92,6 @@ zkg_status ntt_plan_new(int curve, int m, const uint64_t* gen, int inverse, int 
 zkg_status ntt_plan_fault(const NttPlan& pl);
 // Runs a plan d_src -> d_tgt on stream st; scratch (2^m elements) is needed with >= 2 passes.
 zkg_status ntt_plan_execute(const NttPlan& pl, const uint32_t* d_src, uint32_t* d_tgt, uint32_t* scratch,
-                            cudaStream_t st);
+                            cudaStream_t st, const NttRun& run = {});
 
 }  // namespace zkb

@@ -54,7 +54,6 @@ template <bool TW> constexpr int nm_threads() { return 128 + 32 * nm_epi<TW>(); 
 static constexpr uint32_t NM_ROWS = 4096;            // one element of 128 columns of A
 static constexpr int NM_TS = 4;                      // elements per ring slot
 static constexpr uint32_t NM_SLOT = NM_TS * NM_ROWS;
-static constexpr uint32_t NM_WAIT_LIMIT = 1u << 24;  // polls of one barrier before the kernel gives up
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -77,15 +76,20 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Waits for the phase of the given parity, at most NM_WAIT_LIMIT polls; false when the limit or
-// another warp's failure (*stop) ended the wait.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* stop) {
-  for (uint32_t i = 0; i < NM_WAIT_LIMIT; i++) {
+// Waits for the phase of the given parity, at most `limit` polls; false when the limit or another
+// warp's failure (*stop) ended the wait.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* stop, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; i++) {
     if (mbar_try(bar, parity)) return true;
     if (*stop) return false;
   }
   *stop = 1;
   return false;
+}
+// Waits for copies or MMAs of this thread's own that are in flight, before the block may leave: bounded
+// like the others, but neither by the caller's limit nor by another warp's failure.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+  for (uint32_t i = 0; i < NTT_WAIT_LIMIT && !mbar_try(bar, parity); i++) {}
 }
 
 // Shared-memory matrix descriptor, K-major rows of 32 bytes with the 32-byte swizzle: 8-row groups
@@ -110,6 +114,7 @@ struct NttMatArgs {
   uint32_t* out;
   const uint32_t* tw;      // group twiddles in position order (FP64 radix), or null
   uint32_t* fault;         // host-visible word, set when a wait ran out
+  uint32_t wait_limit;     // polls of one barrier before the kernel gives up
   const uint8_t* in;
   int m, k, s, Mp, S, u;
   int inverse;             // load and store sides exchanged
@@ -228,7 +233,7 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
     for (uint32_t item = first; item < last && ok; item++) {
       const uint32_t key = key_of(item);
       if (key != cur) {
-        if (nkey) ok = mbar_wait(bfree, (nkey - 1) & 1, &s_stop);
+        if (nkey) ok = mbar_wait(bfree, (nkey - 1) & 1, &s_stop, g.wait_limit);
         if (!ok) break;
         mbar_expect(bfull, Sh::BBYTES);
         const uint8_t* src = g.mat + (size_t)key * Sh::BBYTES;
@@ -246,7 +251,7 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
       const uint32_t c0 = (item % g.ntiles) * 128u;
       for (int t = 0; t < R; t += NM_TS, it++) {
         const uint32_t slot = it % NS, round = it / NS;
-        ok = mbar_wait(empty + 8 * slot, (round & 1) ^ 1, &s_stop);
+        ok = mbar_wait(empty + 8 * slot, (round & 1) ^ 1, &s_stop, g.wait_limit);
         if (!ok) break;
         mbar_expect(full + 8 * slot, NM_TS * (g.first ? NM_ROWS : rows));
 #pragma unroll
@@ -264,32 +269,31 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
         }
       }
     }
-    if (!ok) {   // given up: wait (bounded) for the copies that are still in flight before leaving
-      volatile uint32_t never = 0;
-      if (nkey) mbar_wait(bfull, (nkey - 1) & 1, &never);
-      for (uint32_t j = it > (uint32_t)NS ? it - NS : 0; j < it; j++)
-        mbar_wait(full + 8 * (j % NS), (j / NS) & 1, &never);
-    }
+    // No copy may be in flight when the block ends. The consumers have waited for all of them unless some
+    // warp gave up, perhaps after this one's last copy.
+    if (nkey) mbar_drain(bfull, (nkey - 1) & 1);
+    for (uint32_t j = it > (uint32_t)NS ? it - NS : 0; j < it; j++) mbar_drain(full + 8 * (j % NS), (j / NS) & 1);
   } else if (warp == 1 && lane == 0) {   // ---- MMA issue
     constexpr uint32_t idesc = (2u << 4) | ((32u * NOUT / 8) << 17) | ((128u / 16) << 24);   // u8 x u8 -> s32
     uint32_t cur = 0xffffffffu, nkey = 0, it = 0, n = 0;
     bool ok = true;
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the limited waits start when the pass before is done
     for (uint32_t item = first; item < last && ok; item++, n++) {
       const uint32_t key = key_of(item);
       if (key != cur) {
-        ok = mbar_wait(bfull, nkey & 1, &s_stop);
+        ok = mbar_wait(bfull, nkey & 1, &s_stop, g.wait_limit);
         if (!ok) break;
         cur = key;
         nkey++;
       }
       const uint32_t buf = n & 1;
-      ok = mbar_wait(tempty + 8 * buf, ((n >> 1) & 1) ^ 1, &s_stop);
+      ok = mbar_wait(tempty + 8 * buf, ((n >> 1) & 1) ^ 1, &s_stop, g.wait_limit);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d = tmem + buf * (32 * NOUT);
       for (int t = 0; t < R; t += NM_TS, it++) {
         const uint32_t slot = it % NS;
-        ok = mbar_wait(full + 8 * slot, (it / NS) & 1, &s_stop);
+        ok = mbar_wait(full + 8 * slot, (it / NS) & 1, &s_stop, g.wait_limit);
         if (!ok) break;
 #pragma unroll
         for (int j = 0; j < NM_TS; j++)
@@ -305,11 +309,9 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
       if (item + 1 < last && key_of(item + 1) != key)
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bfree) : "memory");
     }
-    if (!ok) {   // given up: wait (bounded) for the MMAs that are still running
-      volatile uint32_t never = 0;
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain) : "memory");
-      mbar_wait(drain, 0, &never);
-    }
+    // Nor an MMA, when tensor memory is freed: the epilogue has waited for the last one unless it gave up.
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain) : "memory");
+    mbar_drain(drain, 0);
   } else if (warp >= 4) {   // ---- epilogue
     // jobs: output j of a tile's quarter (32 rows), taken in turn by the quarter's warps
     constexpr uint32_t STEP = nm_epi<TW>() / 4;
@@ -332,7 +334,7 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
       }
       Fe<PL> w;
       if (TW) w = fe_load_nc<PL>(g.tw + (size_t)(((kap >> g.tw_S) << (g.inverse ? g.Mp + K : g.Mp)) | rem) * 8);
-      const bool ok = mbar_wait(tfull + 8 * buf, (n >> 1) & 1, &s_stop);
+      const bool ok = mbar_wait(tfull + 8 * buf, (n >> 1) & 1, &s_stop, g.wait_limit);
       if (!__all_sync(0xffffffffu, ok)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       uint32_t sums[32];
@@ -441,7 +443,7 @@ static zkg_status nm_dispatch(const CUtensorMap& map, const NttMatArgs& g, int n
 
 template <class P>
 zkg_status ntt_mat_launch_pass(const NttPlan& pl, int exec, const uint32_t* in, uint32_t* out, int sms,
-                               cudaStream_t st) {
+                               const NttRun& run, cudaStream_t st) {
   const NttMatPass& q = pl.mpasses[exec];
   static const PFN_cuTensorMapEncodeTiled encode = [] {
     void* f = nullptr;
@@ -464,6 +466,7 @@ zkg_status ntt_mat_launch_pass(const NttPlan& pl, int exec, const uint32_t* in, 
   g.out = out;
   g.tw = q.tw >= 0 ? pl.d_gtw[q.tw] : nullptr;
   g.fault = pl.h_fault;
+  g.wait_limit = run.wait_limit;
   g.m = pl.m;
   g.k = q.k;
   g.Mp = q.Mp;
