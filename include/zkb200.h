@@ -539,7 +539,8 @@ zkg_status zkg_batch_destroy(zkg_batch *b);
  * zkg_server_wait_for waits at most timeout_ms (< 0: no limit) and returns ZKG_ERR_TIMEOUT if the
  * request is still pending (the ticket stays valid). zkg_server_inject_failure makes the
  * admission `admission` places from now fail on the host as a launch error would (testing of the
- * failure path; < 0 disarms it). */
+ * failure path; < 0 disarms it); zkg_server_inject_stall makes that admission's NTT passes give up at
+ * their first bounded wait (sizes from 2^9 on), which fails that request with ZKG_ERR_TIMEOUT. */
 typedef struct zkg_server zkg_server;
 zkg_status zkg_server_create(zkg_curve curve, const uint64_t *d_bases, int n_bases, int k_min, int k_max,
                              size_t hbm_budget, int slots, zkg_server **out);
@@ -549,6 +550,7 @@ zkg_status zkg_server_submit(zkg_server *s, int k, const uint64_t *values, uint6
 zkg_status zkg_server_wait(zkg_server *s, uint64_t ticket, double *latency_ms);
 zkg_status zkg_server_wait_for(zkg_server *s, uint64_t ticket, double timeout_ms, double *latency_ms);
 zkg_status zkg_server_inject_failure(zkg_server *s, long admission);
+zkg_status zkg_server_inject_stall(zkg_server *s, long admission);
 zkg_status zkg_server_stats(zkg_server *s, uint64_t *completed, int *max_inflight, size_t *peak_bytes);
 zkg_status zkg_server_destroy(zkg_server *s);
 

@@ -123,6 +123,32 @@ def test_server_injected_failure_completes_every_ticket(zk):
     srv.close()
 
 
+def test_server_stalled_transform_fails_its_own_request(zk):
+    """requests of one size share an NTT plan: the one whose transform gives up fails, and no other"""
+    import torch
+    curve, k = Z.BN254, 14
+    d_b = _bases(zk, curve, 1 << k, 62500)
+    for stalled in (0, 1, 2):
+        srv = zk.Server(curve, d_b, 1 << k, k, k, 1 << 30, 4)
+        vals = [torch.from_numpy(Z.rand_fr(curve, 1 << k, 62600 + i).view(np.int64)).pin_memory() for i in range(4)]
+        want = [srv.wait(srv.submit(k, v))[0] for v in vals]
+        srv.inject_stall(stalled)
+        tickets = []
+        for v in vals:
+            try:
+                tickets.append(srv.submit(k, v))
+            except zk.ZkgError:   # refused after the failure
+                break
+        assert len(tickets) > stalled
+        for i, t in enumerate(tickets):
+            try:
+                out, _ = srv.wait(t, timeout_ms=60000)
+                assert i != stalled and np.array_equal(out, want[i]), (stalled, i)
+            except zk.ZkgError as e:
+                assert i >= stalled and e.status == zk.ERR_TIMEOUT, (stalled, i)
+        srv.close()
+
+
 def test_server_deadline_and_large_request_admission(zk):
     import torch
     curve = Z.BN254

@@ -111,6 +111,8 @@ def lib():
     L.zkg_server_wait_for.restype = i
     L.zkg_server_inject_failure.argtypes = [vp, ctypes.c_long]
     L.zkg_server_inject_failure.restype = i
+    L.zkg_server_inject_stall.argtypes = [vp, ctypes.c_long]
+    L.zkg_server_inject_stall.restype = i
     L.zkg_server_stats.argtypes = [vp, ctypes.POINTER(ctypes.c_uint64), ctypes.POINTER(i), ctypes.POINTER(ctypes.c_size_t)]
     L.zkg_server_destroy.argtypes = [vp]
     L.zkg_autotune_msm.argtypes = [i, vp, i, i, i, vp]
@@ -523,6 +525,10 @@ class Server:
     def inject_failure(self, admission):
         """make the admission `admission` places from now fail on the host (failure-path tests)"""
         _check(lib().zkg_server_inject_failure(self._h, admission))
+
+    def inject_stall(self, admission):
+        """make the NTT of the admission `admission` places from now give up (failure-path tests)"""
+        _check(lib().zkg_server_inject_stall(self._h, admission))
 
     def stats(self):
         c, mi, pb = ctypes.c_uint64(), ctypes.c_int(), ctypes.c_size_t()

@@ -1784,6 +1784,7 @@ struct zkg_batch {
   void* ws = nullptr;           // device workspace (MSM pipeline + NTT scratch)
   size_t conv_off = 0;          // bases in the FP64 pipeline's radix (inside ws), 0 = integer pipeline
   uint32_t conv_n = 0;          // bases converted per run (largest request)
+  uint32_t* fault = nullptr;    // of the graph form's NTTs, behind the staging
   void* pin = nullptr;          // pinned copy of U
   size_t ubytes = 0;
   std::vector<size_t> ntt_scratch_off;
@@ -2062,7 +2063,9 @@ static zkg_status batch_build(zkg_batch* b, const host::Field<NL>& F) {
   if (!b->mp.reqs.empty())
     ZKB_CUDA(cudaMemcpy(ws + b->mp.o_reqs, b->mp.reqs.data(), b->mp.reqs.size() * sizeof(MReq), cudaMemcpyHostToDevice));
   b->ubytes = (size_t)b->mp.nwins * 4 * NL * 8;
-  ZKB_CUDA(cudaMallocHost(&b->pin, std::max<size_t>(b->ubytes, 64)));
+  ZKB_CUDA(cudaMallocHost(&b->pin, b->ubytes + 64));
+  b->fault = reinterpret_cast<uint32_t*>(static_cast<char*>(b->pin) + b->ubytes);
+  *b->fault = 0;
   ZKB_CUDA(cudaEventCreate(&b->ev0));
   ZKB_CUDA(cudaEventCreate(&b->ev1));
   for (int i = 0; i <= nstreams; i++) {
@@ -2077,6 +2080,7 @@ static zkg_status batch_build(zkg_batch* b, const host::Field<NL>& F) {
     for (size_t i = 0; i < b->ntts.size(); i++) {
       const int si = (int)(i % nstreams);
       NttRun run;
+      run.fault = b->fault;
       if (b->inject_stall && i == 0) run.wait_limit = 0;   // testing: every wait inside its passes runs out
       ZKB_TRY(ntt_plan_execute(*b->plans[i], reinterpret_cast<const uint32_t*>(b->ntts[i].d_src),
                                reinterpret_cast<uint32_t*>(b->ntts[i].d_tgt),
@@ -2139,7 +2143,7 @@ static zkg_status batch_run(zkg_batch* b, const host::Field<NL>& F) {
     std::memcpy(&err, static_cast<const char*>(b->pin) + b->err_pin_off, 4);
     if (err) return set_status(ZKG_ERR_TIMEOUT, "zkg_batch_run", "an NTT pass waited too long for its input");
   }
-  for (NttPlan* pl : b->own_plans) ZKB_TRY(ntt_plan_fault(*pl));
+  ZKB_TRY(ntt_fault_report(b->fault));
   std::vector<uint64_t*> outs;
   std::vector<int> kinds;
   for (auto& m : b->msms) { outs.push_back(m.out); kinds.push_back(m.kind); }
@@ -2187,6 +2191,7 @@ struct SrvSlot {
   cudaEvent_t done = nullptr;
   void* pin = nullptr;
   size_t pin_cap = 0;
+  uint32_t* fault = nullptr;   // of the slot's inverse NTT, behind the staging
   SrvReq req;
   MsmPlan P;
   size_t off = 0, bytes = 0;
@@ -2211,6 +2216,7 @@ struct Srv {
   std::vector<size_t> req_bytes;   // device bytes of one request, by k
   std::vector<MsmPlan> req_plan;   // its MSM plan, by k
   long inject_fail_at = -1;        // host-side failure injection: admission number that fails
+  long inject_stall_at = -1;       // testing: admission whose NTT passes give up at their first wait
   long admissions = 0;
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
@@ -2272,7 +2278,10 @@ static zkg_status srv_launch(Srv& S, SrvSlot& sl) {
   uint32_t* d_scr = reinterpret_cast<uint32_t*>(base + 2 * vb);
   char* ws = base + 3 * vb;
   ZKB_CUDA(cudaMemcpyAsync(d_vals, sl.req.values, N * 32, cudaMemcpyHostToDevice, sl.st));
-  ZKB_TRY(ntt_plan_execute(*S.plans[k], d_vals, d_coef, d_scr, sl.st));
+  NttRun run;
+  run.fault = sl.fault;
+  if (S.inject_stall_at >= 0 && S.admissions == S.inject_stall_at) run.wait_limit = 0;
+  ZKB_TRY(ntt_plan_execute(*S.plans[k], d_vals, d_coef, d_scr, sl.st, run));
   PartSet parts;
   parts.n = 1;
   parts.bsum[0] = reinterpret_cast<const uint32_t*>(ws + sl.P.o_bsum);
@@ -2317,7 +2326,7 @@ static void srv_loop(Srv* S, const host::Field<NL>* F) {
       if (!sl.busy || sl.finishing) continue;
       const cudaError_t q = cudaEventQuery(sl.done);
       if (q == cudaErrorNotReady) continue;
-      const zkg_status nf = q == cudaSuccess ? ntt_plan_fault(*S->plans[sl.req.k]) : ZKG_OK;
+      const zkg_status nf = q == cudaSuccess ? ntt_fault_report(sl.fault) : ZKG_OK;
       if (q != cudaSuccess || nf != ZKG_OK) {   // the device reported an error for this request's work
         (void)cudaGetLastError();
         if (S->error == ZKG_OK) S->error = nf != ZKG_OK ? nf : set_status(ZKG_ERR_CUDA, "server", cudaGetErrorString(q));
@@ -2455,8 +2464,10 @@ static zkg_status srv_start(Srv* S, const host::Field<NL>* F, const host::Field<
   for (auto& sl : S->slots) {   // page-locked staging of each slot's window sums, sized once
     ZKB_CUDA(cudaStreamCreateWithFlags(&sl.st, cudaStreamNonBlocking));
     ZKB_CUDA(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
-    ZKB_CUDA(cudaMallocHost(&sl.pin, ubytes_max));
+    ZKB_CUDA(cudaMallocHost(&sl.pin, ubytes_max + 64));
     sl.pin_cap = ubytes_max;
+    sl.fault = reinterpret_cast<uint32_t*>(static_cast<char*>(sl.pin) + ubytes_max);
+    *sl.fault = 0;
   }
   S->worker = std::thread(srv_loop<C, NL>, S, F);
   return ZKG_OK;
@@ -2863,6 +2874,13 @@ zkg_status zkg_server_inject_failure(zkg_server* srv, long admission) {
   if (!srv) return zkb::set_status(ZKG_ERR_ARG, "zkg_server_inject_failure", "null server");
   std::lock_guard<std::mutex> lk(srv->S.mu);
   srv->S.inject_fail_at = admission < 0 ? -1 : srv->S.admissions + admission;
+  return ZKG_OK;
+}
+
+zkg_status zkg_server_inject_stall(zkg_server* srv, long admission) {
+  if (!srv) return zkb::set_status(ZKG_ERR_ARG, "zkg_server_inject_stall", "null server");
+  std::lock_guard<std::mutex> lk(srv->S.mu);
+  srv->S.inject_stall_at = admission < 0 ? -1 : srv->S.admissions + admission;
   return ZKG_OK;
 }
 

@@ -172,8 +172,6 @@ static zkg_status build_mat(const host::Field<4>& F, NttPlan* pl, const host::El
   const std::vector<int> groups = ntt_mat_groups(m);
   const int sms = device_sm_count();
   pl->mat = true;
-  ZKB_CUDA(cudaHostAlloc(&pl->h_fault, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable));
-  *pl->h_fault = 0;
   std::vector<host::El<4>> hv;   // what the build kernels read
   auto powers = [&](size_t n, const host::El<4>& x0, const host::El<4>& g) {
     const size_t at = hv.size();
@@ -379,10 +377,18 @@ static zkg_status build_plan(Context& cx, const host::Field<4>& F, int curve, in
   return ZKG_OK;
 }
 
+// The calls on the context's stream, one at a time: its own fault word, cleared.
+static zkg_status ntt_context_run(Context& cx, NttRun& run) {
+  if (!cx.ntt_fault) ZKB_CUDA(cudaMallocHost(&cx.ntt_fault, sizeof(uint32_t)));
+  *cx.ntt_fault = 0;
+  run.fault = cx.ntt_fault;
+  return ZKG_OK;
+}
+
 // Runs the plan d_src -> d_tgt; scratch (N elements) needed when there are >= 2 passes.
 template <class P>
 static zkg_status ntt_run(Context& cx, const NttPlan& pl, const uint32_t* d_src, uint32_t* d_tgt, uint32_t* scratch,
-                          cudaStream_t st, const NttRun& run = {}) {
+                          cudaStream_t st, const NttRun& run) {
   const int np = (int)pl.passes.size();
   const size_t N = (size_t)1 << pl.m;
   if (np == 0) {   // m = 0: copy (bn128_poly_mont.c:420-423)
@@ -415,6 +421,8 @@ static zkg_status ntt_entry(const host::Field<4>& F, int curve, int m, const uin
   std::lock_guard<std::mutex> lk(cx.mu);
   NttPlan* pl = nullptr;
   ZKB_TRY(build_plan<P>(cx, F, curve, m, gen, inverse, &pl));
+  NttRun run;
+  ZKB_TRY(ntt_context_run(cx, run));
   const size_t N = (size_t)1 << m, bytes = N * 32, rb = (bytes + 255) & ~size_t(255);
   const bool need_scratch = pl->passes.size() >= 2;
   if (device_ptrs) {
@@ -425,7 +433,7 @@ static zkg_status ntt_entry(const host::Field<4>& F, int curve, int m, const uin
     if (!cx.user_stream) ZKB_CUDA(cudaDeviceSynchronize());   // inputs may come from any stream
     ZKB_CUDA(cudaEventRecord(cx.ev_a, st));
     ZKB_TRY(ntt_run<P>(cx, *pl, reinterpret_cast<const uint32_t*>(src), reinterpret_cast<uint32_t*>(tgt), scratch,
-                       st));
+                       st, run));
     ZKB_CUDA(cudaEventRecord(cx.ev_b, st));
     ZKB_CUDA(cudaStreamSynchronize(st));
   } else {
@@ -437,12 +445,12 @@ static zkg_status ntt_entry(const host::Field<4>& F, int curve, int m, const uin
     const cudaStream_t st = cx.compute();
     ZKB_TRY(copy_h2d(cx, d_src, src, bytes, st));
     ZKB_CUDA(cudaEventRecord(cx.ev_a, st));
-    ZKB_TRY(ntt_run<P>(cx, *pl, d_src, d_tgt, scratch, st));
+    ZKB_TRY(ntt_run<P>(cx, *pl, d_src, d_tgt, scratch, st, run));
     ZKB_CUDA(cudaEventRecord(cx.ev_b, st));
     ZKB_TRY(copy_d2h(cx, tgt, d_tgt, bytes, st));
   }
   ZKB_CUDA(cudaEventElapsedTime(&cx.last_kernel_ms, cx.ev_a, cx.ev_b));
-  ZKB_TRY(ntt_plan_fault(*pl));
+  ZKB_TRY(ntt_fault_report(cx.ntt_fault));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
 
@@ -491,6 +499,8 @@ static zkg_status ntt_shifted_entry(const host::Field<4>& F, int curve, const ui
   std::lock_guard<std::mutex> lk(cx.mu);
   NttPlan* pl = nullptr;
   ZKB_TRY(build_plan<P>(cx, F, curve, m, gen, inverse, &pl));
+  NttRun run;
+  ZKB_TRY(ntt_context_run(cx, run));
   const size_t N = (size_t)1 << m, bytes = N * 32, rb = (bytes + 255) & ~size_t(255);
   const int a = (m + 1) / 2;
   std::vector<host::El<4>> A, Bt;
@@ -515,16 +525,16 @@ static zkg_status ntt_shifted_entry(const host::Field<4>& F, int curve, const ui
   if (!inverse) {
     ZKB_TRY(launch("ntt_scale_pow", k_ntt_scale_pow<P>, g, dim3(256), 0, st, (const uint32_t*)d_a, d_b, (uint32_t)N,
                    (const uint32_t*)dA, (const uint32_t*)dB, a));
-    ZKB_TRY(ntt_run<P>(cx, *pl, d_b, d_c, scratch, st));
+    ZKB_TRY(ntt_run<P>(cx, *pl, d_b, d_c, scratch, st, run));
   } else {
-    ZKB_TRY(ntt_run<P>(cx, *pl, d_a, d_b, scratch, st));
+    ZKB_TRY(ntt_run<P>(cx, *pl, d_a, d_b, scratch, st, run));
     ZKB_TRY(launch("ntt_scale_pow", k_ntt_scale_pow<P>, g, dim3(256), 0, st, (const uint32_t*)d_b, d_c, (uint32_t)N,
                    (const uint32_t*)dA, (const uint32_t*)dB, a));
   }
   ZKB_CUDA(cudaEventRecord(cx.ev_b, st));
   ZKB_TRY(copy_d2h(cx, tgt, d_c, bytes, st));
   ZKB_CUDA(cudaEventElapsedTime(&cx.last_kernel_ms, cx.ev_a, cx.ev_b));
-  ZKB_TRY(ntt_plan_fault(*pl));
+  ZKB_TRY(ntt_fault_report(cx.ntt_fault));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
 
@@ -542,6 +552,8 @@ static zkg_status ntt_asym_entry(const host::Field<4>& F, int curve, int m_src, 
   std::lock_guard<std::mutex> lk(cx.mu);
   NttPlan* pl = nullptr;
   ZKB_TRY(build_plan<P>(cx, F, curve, m_src, gen_src, 0, &pl));
+  NttRun run;
+  ZKB_TRY(ntt_context_run(cx, run));
   const size_t Ns = (size_t)1 << m_src, K = (size_t)1 << (m_tgt - m_src), bs = Ns * 32;
   const size_t rbs = (bs + 255) & ~size_t(255), bt = Ns * K * 32, rbt = (bt + 255) & ~size_t(255);
   const int a = (m_src + 1) / 2;
@@ -569,7 +581,7 @@ static zkg_status ntt_asym_entry(const host::Field<4>& F, int curve, int m_src, 
     ZKB_CUDA(cudaMemcpyAsync(dB, Bt.data(), Bt.size() * 32, cudaMemcpyHostToDevice, st));
     ZKB_TRY(launch("ntt_scale_pow", k_ntt_scale_pow<P>, g, dim3(256), 0, st, (const uint32_t*)d_src, d_sh,
                    (uint32_t)Ns, (const uint32_t*)dA, (const uint32_t*)dB, a));
-    ZKB_TRY(ntt_run<P>(cx, *pl, d_sh, d_out, scratch, st));
+    ZKB_TRY(ntt_run<P>(cx, *pl, d_sh, d_out, scratch, st, run));
     ZKB_TRY(launch("ntt_interleave", k_ntt_interleave, g, dim3(256), 0, st, (const uint4*)d_out, (uint4*)d_tgt,
                    (uint32_t)Ns, (uint32_t)K, (uint32_t)k));
     ZKB_CUDA(cudaStreamSynchronize(st));   // the host-side tables are rewritten for the next k
@@ -577,7 +589,7 @@ static zkg_status ntt_asym_entry(const host::Field<4>& F, int curve, int m_src, 
   ZKB_CUDA(cudaEventRecord(cx.ev_b, st));
   ZKB_TRY(copy_d2h(cx, tgt, d_tgt, bt, st));
   ZKB_CUDA(cudaEventElapsedTime(&cx.last_kernel_ms, cx.ev_a, cx.ev_b));
-  ZKB_TRY(ntt_plan_fault(*pl));
+  ZKB_TRY(ntt_fault_report(cx.ntt_fault));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
 
@@ -591,8 +603,8 @@ zkg_status ntt_plan_new(int curve, int m, const uint64_t* gen, int inverse, int 
   return set_status(ZKG_ERR_ARG, "ntt", "unknown curve");
 }
 
-zkg_status ntt_plan_fault(const NttPlan& pl) {
-  volatile uint32_t* w = pl.h_fault;
+zkg_status ntt_fault_report(uint32_t* word) {
+  volatile uint32_t* w = word;
   if (!w || !*w) return ZKG_OK;
   *w = 0;
   return set_status(ZKG_ERR_TIMEOUT, "ntt", "a bounded wait inside a pass ran out");

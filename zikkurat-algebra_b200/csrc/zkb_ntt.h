@@ -30,10 +30,12 @@ struct NttMatPass {
   int tw, tw_S;            // group twiddles applied to the outputs (-1: none); bits before that group
 };
 
-// How one execution of a plan runs. wait_limit: polls of a barrier inside a matrix pass (2^24: a third of
+// How one execution of a plan runs. fault: page-locked host word that a pass sets whose bounded wait ran
+// out; it belongs to the execution (a plan may run on several streams at once). wait_limit: polls of a barrier inside a matrix pass (2^24: a third of
 // a second at the least) before the pass gives up.
 static constexpr uint32_t NTT_WAIT_LIMIT = 1u << 24;
 struct NttRun {
+  uint32_t* fault = nullptr;
   uint32_t wait_limit = NTT_WAIT_LIMIT;
 };
 
@@ -50,11 +52,9 @@ struct NttPlan {
   std::vector<NttMatPass> mpasses;
   uint32_t* d_gtw[4] = {nullptr};    // twiddles between the groups, in position order
   void* d_mblk = nullptr;            // the device block both lie in
-  uint32_t* h_fault = nullptr;       // host-mapped word, set by a pass whose bounded wait ran out
   size_t bytes = 0;
   ~NttPlan() {
     if (d_mblk) cudaFree(d_mblk);
-    if (h_fault) cudaFreeHost(h_fault);
     if (d_tw) cudaFree(d_tw);
     if (d_tw_last) cudaFree(d_tw_last);
     for (auto p : d_om) if (p) cudaFree(p);
@@ -87,9 +87,9 @@ zkg_status ntt_mat_twiddles(uint32_t* T, const uint32_t* A, const uint32_t* B, i
 // whatever the size (the batch's persistent kernel runs its tiles).
 zkg_status ntt_plan_new(int curve, int m, const uint64_t* gen, int inverse, int kmax, cudaStream_t st,
                         NttPlan** out, bool tiles = false);
-// ZKG_ERR_TIMEOUT (and the plan's word cleared) when a bounded wait inside one of its passes ran
-// out; to be called once the plan's work has finished.
-zkg_status ntt_plan_fault(const NttPlan& pl);
+// ZKG_ERR_TIMEOUT (and the word cleared) when a bounded wait inside a pass ran out; to be called once the
+// execution has finished.
+zkg_status ntt_fault_report(uint32_t* word);
 // Runs a plan d_src -> d_tgt on stream st; scratch (2^m elements) is needed with >= 2 passes.
 zkg_status ntt_plan_execute(const NttPlan& pl, const uint32_t* d_src, uint32_t* d_tgt, uint32_t* scratch,
                             cudaStream_t st, const NttRun& run = {});

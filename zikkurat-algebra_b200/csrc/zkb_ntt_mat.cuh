@@ -113,7 +113,7 @@ struct NttMatArgs {
   const uint8_t* mat;      // this pass's matrices (2^u images of (32 2^k)^2 bytes)
   uint32_t* out;
   const uint32_t* tw;      // group twiddles in position order (FP64 radix), or null
-  uint32_t* fault;         // host-visible word, set when a wait ran out
+  uint32_t* fault;         // the execution's host-visible word, set when a wait ran out
   uint32_t wait_limit;     // polls of one barrier before the kernel gives up
   const uint8_t* in;
   int m, k, s, Mp, S, u;
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(nm_threads<TW>(), 1) k_ntt_mat(const __grid_co
   __syncthreads();
   if (warp == 2)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TCOLS) : "memory");
-  if (threadIdx.x == 0 && s_stop) *(volatile uint32_t*)g.fault = 1u;
+  if (threadIdx.x == 0 && s_stop && g.fault) *(volatile uint32_t*)g.fault = 1u;
 }
 
 // The matrices of a pass, in the layout k_ntt_mat copies: image [kappa][output group][input element]
@@ -465,7 +465,7 @@ zkg_status ntt_mat_launch_pass(const NttPlan& pl, int exec, const uint32_t* in, 
   g.mat = q.d_mat;
   g.out = out;
   g.tw = q.tw >= 0 ? pl.d_gtw[q.tw] : nullptr;
-  g.fault = pl.h_fault;
+  g.fault = run.fault;
   g.wait_limit = run.wait_limit;
   g.m = pl.m;
   g.k = q.k;

@@ -80,6 +80,7 @@ struct Context {
   void* pinned = nullptr;           // small pinned staging for results
   size_t pinned_cap = 0;
   std::mutex mu;
+  uint32_t* ntt_fault = nullptr;    // page-locked word of the call's transforms (NttRun, zkb_ntt.h)
   std::vector<NttPlan*> ntt_plans;  // LRU-less cache, bounded by count
   float last_kernel_ms = 0.f;       // device time of the last hot-kernel region (for the bench)
   cudaEvent_t ev_phase[8] = {nullptr};
