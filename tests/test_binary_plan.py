@@ -33,3 +33,14 @@ def test_every_launch_fits_its_workspace_over_the_range(zk):
         npts = int(2 ** rng.uniform(10, 21.5))
         given, needed, _ = plan(zk, curve, host, nrows, npts)
         assert needed <= given, (curve, host, nrows, npts)
+
+
+@pytest.mark.parametrize("host,nrows,npts", [(0, 16384, 1 << 21), (0, 28000, 1 << 19), (1, 32768, 1 << 20),
+                                             (1, 1 << 20, 4096), (0, 1 << 17, 1 << 16), (1, 2048, 1 << 20)])
+@pytest.mark.parametrize("curve", Z.CURVES)
+def test_many_rows_are_planned_in_bounded_memory(zk, curve, host, nrows, npts):
+    """no size is refused, and the workspace is one point a row and one launch: at most 2^26 entries of 12
+    bytes, their chunks' partial sums and the buckets, below 2 GiB; not a point a row and column chunk"""
+    given, needed, total = plan(zk, curve, host, nrows, npts)
+    assert needed <= given <= 2 << 30
+    assert total <= given + nrows * 4 * Z.NLP[curve] * 8 + 512

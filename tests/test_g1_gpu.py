@@ -296,6 +296,48 @@ def test_binary_msm_ragged_last_chunk(zk, curve, nrows, npts):
     _binary_large(zk, curve, nrows, npts, 9950 + nrows, [0])
 
 
+@pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("nrows,npts", [(299, 70), (600, 300), (3001, 61), (2500, 700)])
+def test_binary_msm_many_rows(zk, curve, nrows, npts):
+    """rows summed by 128 threads, 64 and one warp; groups counted by several blocks a column"""
+    bases = Z.gen_bases_cpu(curve, Z.rand_fr(curve, npts, 9960 + npts))
+    co = (Z.splitmix64(9961 + nrows, nrows * npts) & np.uint64(1)).astype(np.uint8).reshape(nrows, npts)
+    got = zk.binary_multi_msm(curve, co, bases, affine=True)
+    rows = np.r_[0:nrows:max(1, nrows // 40), nrows - 1]
+    assert np.array_equal(got[rows], affine_rows(curve, "proj", Z.oracle_msm_binary(curve, co[rows], bases)))
+
+
+@pytest.mark.parametrize("curve", Z.CURVES)
+def test_binary_msm_row_batches(zk, curve):
+    """more rows than a launch takes, from host arrays (batches of 700 rows) and on the device, where a row is
+    also the MSM of 0/1 scalars"""
+    import torch
+    nl = Z.NLP[curve]
+    rng = np.random.default_rng(12)
+    nrows, npts = 2099, 40003
+    bases = torch.empty((1 << 20, 2 * nl), dtype=torch.int64, device="cuda")
+    zk.g1_gen_mul_device(curve, 1 << 20, torch.from_numpy(Z.rand_fr(curve, 1 << 20, 9970).view(np.int64)).cuda(), bases)
+    torch.cuda.synchronize()
+    def msm(bits):
+        s = torch.zeros((bits.shape[0], 4), dtype=torch.int64, device="cuda")
+        s[:, 0] = bits
+        return zk.msm_device(curve, bits.shape[0], s, bases, mont=False)
+    co = rng.integers(0, 2, (nrows, npts)).astype(np.uint8)
+    host = zk.binary_multi_msm(curve, co, bases[:npts].cpu().numpy().view(np.uint64), affine=True)
+    for r in (0, 699, 700, 1399, 1400, 2098):
+        assert np.array_equal(host[r], msm(torch.from_numpy(co[r]).cuda())), r
+    g = torch.Generator(device="cuda")
+    g.manual_seed(13)
+    nrows, npts = 1500, 1 << 20   # two batches
+    d_co = torch.randint(0, 2, (nrows, npts), dtype=torch.uint8, device="cuda", generator=g)
+    out = torch.empty((nrows, 2 * nl), dtype=torch.int64, device="cuda")
+    zk.msm_binary_device(curve, nrows, npts, d_co, npts, bases, out, kind=zk.OUT_AFFINE)
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().view(np.uint64)
+    for r in (0, 749, 750, 1499):
+        assert np.array_equal(got[r], msm(d_co[r])), r
+
+
 def test_binary_msm_rejects_bad_arguments(zk):
     L = zk.lib()
     b = np.zeros(16, np.uint64)

@@ -27,7 +27,7 @@
 // rows are grouped instead and the columns go to buckets by their bits in a group (zkb_msm_bits.h):
 // 64 rows of 2^18 columns are 17 M field products against 60 M by subset sums. Columns are processed
 // in chunks (host coefficient rows and bases are gathered into pinned staging and copied while the
-// previous chunk computes); every chunk leaves one partial sum a row, added up at the end. The order
+// previous chunk computes), many rows in batches; the chunks' sums add up in the rows' points. The order
 // of additions differs; every result is the same group element, written in the drop-in's encoding.
 #include <algorithm>
 #include <cstdlib>
@@ -393,31 +393,6 @@ __global__ void k_g1fft_store(int m, int bitrev, const uint32_t* __restrict__ a,
 }
 
 // ------------------------------------------------------------------------ binary MSM kernels
-// Sums of segments: block (seg b of row r) reduces in[r][b*256 .. min(L, b*256+256)) into
-// out[r][b]; 128 threads, shared-memory tree.
-template <class C>
-__global__ void __launch_bounds__(128) k_xyzz_reduce(int L, int B, const uint32_t* __restrict__ in,
-                                                     uint32_t* __restrict__ out) {
-  using F = typename C::Fp;
-  constexpr int XW = 4 * F::N;
-  __shared__ __align__(16) uint32_t sh[128 * XW];
-  const int r = blockIdx.y, b = blockIdx.x, t = threadIdx.x;
-  const int lo = b * 256;
-  Xyzz<F> acc = xyzz_inf<F>();
-  for (int e = lo + t; e < L && e < lo + 256; e += 128) acc = xyzz_sum(acc, xyzz_load<F>(in + ((size_t)r * L + e) * XW));
-  xyzz_store<F>(sh + t * XW, acc);
-  __syncthreads();
-  for (int w = 64; w >= 1; w >>= 1) {
-    if (t < w) {
-      Xyzz<F> x = xyzz_load<F>(sh + t * XW);
-      x = xyzz_sum(x, xyzz_load<F>(sh + (t + w) * XW));
-      xyzz_store<F>(sh + t * XW, x);
-    }
-    __syncthreads();
-  }
-  if (t == 0) xyzz_store<F>(out + ((size_t)r * B + b) * XW, xyzz_load<F>(sh));
-}
-
 template <class C>
 __global__ void k_xyzz_write(int n, int kind, const uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
   using F = typename C::Fp;
@@ -694,79 +669,79 @@ static zkg_status g1_fft_dev(int jac, int m, const uint64_t* gen, const uint64_t
 struct BinPlan {
   int rho = 1;            // rows a group
   int batch = 0;          // rows a launch
-  int cw = 0;             // columns a chunk
-  int G = 1;              // chunks = partial sums a row
+  int cw = 0;             // columns a launch
+  int nbatch = 0, nchunk = 0;
   size_t bits_bytes = 0;  // workspace of the launches: the largest any of them needs
+  int rows(int r, int nrows) const { return std::min(batch, nrows - r * batch); }
+  int cols(int q, int npoints) const { return std::min(cw, npoints - q * cw); }
 };
-static constexpr int BIN_ROWS = 32768;   // rows a launch (grid dimensions) and a reduction, at most
+static constexpr int BIN_ROWS_MIN = 1024, BIN_ROWS = 32768;   // rows a launch (grid dimensions)
+static constexpr size_t BIN_ENTRIES = (size_t)1 << 26;        // entries a launch: a column has one a group of rows
+static constexpr size_t BIN_STAGE = (size_t)32 << 20;         // staged coefficients, and bases, a launch
 
-// Chunks of up to 64 M entries (a column has one a group of rows); from host buffers also 32 MiB of
-// coefficients and of bases.
+// A launch costs about 10 field products an entry and 8 2^rho a row, however few columns it has, so what
+// is asked for is many columns first: rows go in batches such that a batch can have all the columns, if
+// that leaves 1024 rows. (All rows at once left host calls 8192 columns a launch at 4096 rows, at a rho
+// chosen for 2^20 of them: 5 times the products.) rho is chosen for the columns that a launch has.
 static zkg_status bin_plan(int nrows, int npoints, int nl, bool host, BinPlan& P) {
-  P.batch = std::min(nrows, BIN_ROWS);
-  P.rho = msm_bits_group(P.batch, npoints);
-  const int ngroups = (P.batch + P.rho - 1) / P.rho;
-  size_t cw = std::min<size_t>((size_t)npoints, ((size_t)1 << 26) / ngroups);
-  if (host) {
-    cw = std::min<size_t>(cw, ((size_t)32 << 20) / std::max(1, nrows));
-    cw = std::min<size_t>(cw, ((size_t)32 << 20) / (2 * (size_t)nl * 8));
+  const zkg_curve curve = nl == 4 ? ZKG_BN254 : ZKG_BLS12_381;
+  P.rho = msm_bits_group(nrows, npoints);
+  size_t rows = BIN_ENTRIES * P.rho / npoints;
+  if (host) rows = std::min(rows, BIN_STAGE / npoints);
+  rows = std::min<size_t>(nrows, std::min<size_t>(std::max<size_t>(rows, BIN_ROWS_MIN), BIN_ROWS));
+  P.nbatch = (int)((nrows + rows - 1) / rows);
+  P.batch = (nrows + P.nbatch - 1) / P.nbatch;
+  for (int round = 0; round < 4; round++) {
+    size_t cw = std::min<size_t>(npoints, BIN_ENTRIES / ((P.batch + P.rho - 1) / P.rho));
+    if (host) cw = std::min(cw, std::min(BIN_STAGE / P.batch, BIN_STAGE / (2 * (size_t)nl * 8)));
+    P.nchunk = (int)((npoints + cw - 1) / cw);
+    P.cw = (npoints + P.nchunk - 1) / P.nchunk;
+    const int rho = msm_bits_group(P.batch, P.cw);
+    if (rho == P.rho) break;
+    P.rho = rho;
   }
-  P.cw = (int)std::max<size_t>(cw, 1);
-  P.G = (npoints + P.cw - 1) / P.cw;
+  P.nbatch = (nrows + P.batch - 1) / P.batch;   // rounding up may have made the last ones empty
+  P.nchunk = (npoints + P.cw - 1) / P.cw;
   // A launch's workspace does not grow steadily with its size (a little fewer entries can make shorter and
   // so more chunks), so the last rows and the last columns are asked for as well.
   P.bits_bytes = 0;
-  for (const int rows : {P.batch, nrows % P.batch})
-    for (const int cols : {P.cw, npoints % P.cw}) {
+  for (const int r : {0, P.nbatch - 1})
+    for (const int q : {0, P.nchunk - 1}) {
       size_t b = 0;
-      if (rows && cols) ZKB_TRY(msm_bits_bytes(nl == 4 ? ZKG_BN254 : ZKG_BLS12_381, rows, cols, P.rho, &b));
+      ZKB_TRY(msm_bits_bytes(curve, P.rows(r, nrows), P.cols(q, npoints), P.rho, &b));
       P.bits_bytes = std::max(P.bits_bytes, b);
     }
   return ZKG_OK;
 }
 
-// Runs the chunk loop. get_chunk(q, col0, cw, &coeffs, &ld, &bases) makes chunk q's coefficient
-// rows (ld bytes apart) and bases available to the compute stream.
-template <class C, int NL, class Get>
+// Runs the launches: for each batch of rows the column chunks, whose sums add up in the rows' points.
+// get_tile(t, row0, rows, col0, cols, &coeffs, &ld, &bases) makes launch t's coefficient rows (ld bytes
+// apart) and bases available to the compute stream; done_tile(t) follows its kernels.
+template <class C, int NL, class Get, class Done>
 static zkg_status bin_run(Context& cx, const BinPlan& P, int nrows, int npoints, char* ws, cudaStream_t st,
-                          Get get_chunk, int kind, uint32_t* d_out) {
+                          Get get_tile, Done done_tile, int kind, uint32_t* d_out) {
   constexpr size_t XW = 4 * C::Fp::N;
-  uint32_t* partial = reinterpret_cast<uint32_t*>(ws);
-  char* work = ws + rup256((size_t)nrows * P.G * XW * 4);
-  const dim3 blk(128);
-  for (int q = 0; q < P.G; q++) {
-    const int col0 = q * P.cw;
-    const int cw = std::min(P.cw, npoints - col0);
-    const uint8_t* coeffs = nullptr;
-    size_t ld = 0;
-    const uint32_t* bases = nullptr;
-    ZKB_TRY(get_chunk(q, col0, cw, &coeffs, &ld, &bases));
-    for (int r = 0; r < nrows; r += P.batch)
-      ZKB_TRY(msm_bits_launch(cx, C::ID == 0 ? ZKG_BN254 : ZKG_BLS12_381, std::min(P.batch, nrows - r), cw, P.rho,
-                              coeffs + (size_t)r * ld, ld, bases, work, P.bits_bytes, partial + ((size_t)r * P.G + q) * XW,
-                              (size_t)P.G * XW, st));
-    ZKB_TRY(get_chunk(-1 - q, 0, 0, nullptr, nullptr, nullptr));   // chunk q's inputs are consumed
-  }
-  // reduce G partials per row: 256 per block per pass
-  int L = P.G;
-  uint32_t* in = partial;
-  uint32_t* tmp = reinterpret_cast<uint32_t*>(work);   // the launches' workspace is free again
-  while (L > 1) {
-    const int B = (L + 255) / 256;
-    for (int r = 0; r < nrows; r += BIN_ROWS)
-      ZKB_TRY(launch("xyzz_reduce", k_xyzz_reduce<C>, dim3((unsigned)B, (unsigned)std::min(BIN_ROWS, nrows - r)), blk, 0,
-                     st, L, B, (const uint32_t*)in + (size_t)r * L * XW, tmp + (size_t)r * B * XW));
-    std::swap(in, tmp);
-    L = B;
-  }
+  uint32_t* sums = reinterpret_cast<uint32_t*>(ws);
+  char* work = ws + rup256((size_t)nrows * XW * 4);
+  int t = 0;
+  for (int r = 0; r < P.nbatch; r++)
+    for (int q = 0; q < P.nchunk; q++, t++) {
+      const int rows = P.rows(r, nrows), cols = P.cols(q, npoints), row0 = r * P.batch;
+      const uint8_t* coeffs = nullptr;
+      size_t ld = 0;
+      const uint32_t* bases = nullptr;
+      ZKB_TRY(get_tile(t, row0, rows, q * P.cw, cols, &coeffs, &ld, &bases));
+      ZKB_TRY(msm_bits_launch(cx, C::ID == 0 ? ZKG_BN254 : ZKG_BLS12_381, rows, cols, P.rho, coeffs, ld, bases, work,
+                              P.bits_bytes, sums + row0 * XW, q > 0, st));
+      ZKB_TRY(done_tile(t));
+    }
   return launch("xyzz_write", k_xyzz_write<C>, dim3((unsigned)((nrows + 31) / 32)), dim3(32), 0, st, nrows, kind,
-                (const uint32_t*)in, d_out);
+                (const uint32_t*)sums, d_out);
 }
 
 template <int NL>
 static size_t bin_ws_bytes(const BinPlan& P, int nrows) {
-  const size_t part = rup256((size_t)nrows * P.G * 4 * NL * 8);
-  return part + std::max(rup256(P.bits_bytes), P.G > 1 ? part : 0);   // the reduction's second buffer
+  return rup256((size_t)nrows * 4 * NL * 8) + rup256(P.bits_bytes);
 }
 
 static zkg_status bin_check(zkg_curve curve, int kind, int nrows, int npoints, const void* rows, const void* bases,
@@ -797,7 +772,7 @@ static zkg_status bin_host(const host::Field<NL>& Fp, int kind, int nrows, int n
   BinPlan P;
   ZKB_TRY(bin_plan(nrows, npoints, NL, true, P));
   const size_t bb = 2 * NL * 8;
-  const size_t coef_chunk = rup256((size_t)nrows * P.cw), base_chunk = rup256((size_t)P.cw * bb);
+  const size_t coef_chunk = rup256((size_t)P.batch * P.cw), base_chunk = rup256((size_t)P.cw * bb);
   const size_t out_bytes = rup256((size_t)nrows * ow * 8);
   const size_t stage = coef_chunk + base_chunk;   // one pinned / device staging slot
   const size_t bytes = 2 * stage + out_bytes + bin_ws_bytes<NL>(P, nrows);
@@ -819,21 +794,16 @@ static zkg_status bin_host(const host::Field<NL>& Fp, int kind, int nrows, int n
   ZKB_CUDA(cudaEventRecord(ev_used[0], st));
   ZKB_CUDA(cudaEventRecord(ev_used[1], st));
   bool pending[2] = {false, false};
-  auto get_chunk = [&](int q, int col0, int cw, const uint8_t** coeffs, size_t* ld,
-                       const uint32_t** bases) -> zkg_status {
-    if (q < 0) {   // chunk -1 - q consumed by the kernels just queued
-      const int b = (-1 - q) & 1;
-      ZKB_CUDA(cudaEventRecord(ev_used[b], st));
-      return ZKG_OK;
-    }
-    const int b = q & 1;
+  auto get_tile = [&](int t, int row0, int rws, int col0, int cols, const uint8_t** coeffs, size_t* ld,
+                      const uint32_t** bases) -> zkg_status {
+    const int b = t & 1;
     char* hp = pin + b * stage;
     char* dp = dstage + b * stage;
     if (pending[b]) ZKB_CUDA(cudaEventSynchronize(ev_copied[b]));   // pinned slot b is free again
-    for (int r = 0; r < nrows; r++) std::memcpy(hp + (size_t)r * P.cw, rows[r] + col0, (size_t)cw);
-    std::memcpy(hp + coef_chunk, grps + (size_t)col0 * 2 * NL, (size_t)cw * bb);
+    for (int r = 0; r < rws; r++) std::memcpy(hp + (size_t)r * P.cw, rows[row0 + r] + col0, (size_t)cols);
+    std::memcpy(hp + coef_chunk, grps + (size_t)col0 * 2 * NL, (size_t)cols * bb);
     ZKB_CUDA(cudaStreamWaitEvent(cx.copy_stream, ev_used[b], 0));
-    ZKB_CUDA(cudaMemcpyAsync(dp, hp, coef_chunk + (size_t)cw * bb, cudaMemcpyHostToDevice, cx.copy_stream));
+    ZKB_CUDA(cudaMemcpyAsync(dp, hp, coef_chunk + (size_t)cols * bb, cudaMemcpyHostToDevice, cx.copy_stream));
     ZKB_CUDA(cudaEventRecord(ev_copied[b], cx.copy_stream));
     pending[b] = true;
     ZKB_CUDA(cudaStreamWaitEvent(st, ev_copied[b], 0));
@@ -842,7 +812,11 @@ static zkg_status bin_host(const host::Field<NL>& Fp, int kind, int nrows, int n
     *bases = reinterpret_cast<const uint32_t*>(dp + coef_chunk);
     return ZKG_OK;
   };
-  zkg_status rc = bin_run<C, NL>(cx, P, nrows, npoints, ws, st, get_chunk, kind, d_out);
+  auto done_tile = [&](int t) -> zkg_status {   // launch t's inputs are consumed by the kernels just queued
+    ZKB_CUDA(cudaEventRecord(ev_used[t & 1], st));
+    return ZKG_OK;
+  };
+  zkg_status rc = bin_run<C, NL>(cx, P, nrows, npoints, ws, st, get_tile, done_tile, kind, d_out);
   if (rc == ZKG_OK) {
     // the pinned slots may still feed a copy; wait for all of them before reusing pinned memory
     if (cudaStreamSynchronize(cx.copy_stream) != cudaSuccess) rc = set_status(ZKG_ERR_CUDA, "msm_binary", "copy sync");
@@ -896,16 +870,15 @@ static zkg_status bin_dev(int kind, int nrows, int npoints, const uint8_t* d_coe
   cx.arena.reset();
   char* ws = static_cast<char*>(cx.arena.take(bytes));
   if (!ws) return set_status(ZKG_ERR_NOMEM, "msm_binary_device", "arena");
-  auto get_chunk = [&](int q, int col0, int cw, const uint8_t** coeffs, size_t* pld,
-                       const uint32_t** bases) -> zkg_status {
-    if (q < 0) return ZKG_OK;
-    (void)cw;
-    *coeffs = d_coeffs + col0;
+  auto get_tile = [&](int, int row0, int, int col0, int, const uint8_t** coeffs, size_t* pld,
+                      const uint32_t** bases) -> zkg_status {
+    *coeffs = d_coeffs + (size_t)row0 * ld + col0;
     *pld = ld;
     *bases = reinterpret_cast<const uint32_t*>(d_bases + (size_t)col0 * 2 * NL);
     return ZKG_OK;
   };
-  ZKB_TRY((bin_run<C, NL>(cx, P, nrows, npoints, ws, st, get_chunk, kind, reinterpret_cast<uint32_t*>(d_out))));
+  auto done_tile = [](int) -> zkg_status { return ZKG_OK; };
+  ZKB_TRY((bin_run<C, NL>(cx, P, nrows, npoints, ws, st, get_tile, done_tile, kind, reinterpret_cast<uint32_t*>(d_out))));
   ZKB_CUDA(cudaStreamSynchronize(st));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
@@ -936,10 +909,10 @@ extern "C" zkg_status zkg_msm_binary_plan(zkg_curve curve, int from_host, int nr
   ZKB_TRY(bin_plan(nrows, npoints, nl, from_host != 0, P));
   info[0] = P.bits_bytes;
   info[1] = 0;
-  for (int r = 0; r < nrows; r += P.batch)   // the launches of bin_run
-    for (int q = 0; q < P.G; q++) {
+  for (int r = 0; r < P.nbatch; r++)   // the launches of bin_run
+    for (int q = 0; q < P.nchunk; q++) {
       size_t b = 0;
-      ZKB_TRY(msm_bits_bytes(curve, std::min(P.batch, nrows - r), std::min(P.cw, npoints - q * P.cw), P.rho, &b));
+      ZKB_TRY(msm_bits_bytes(curve, P.rows(r, nrows), P.cols(q, npoints), P.rho, &b));
       info[1] = std::max(info[1], b);
     }
   info[2] = nl == 4 ? bin_ws_bytes<4>(P, nrows) : bin_ws_bytes<6>(P, nrows);

@@ -273,6 +273,7 @@ static bool make_carry_table(int nwin, int nw, WinShape ws, CarryTable& T) {
 // --------------------------------------------------------------------------------- scan
 // Exclusive prefix sum of n u32 counts in three launches (blocks of 4096 elements).
 static constexpr int SCAN_T = 1024, SCAN_E = 4;
+static constexpr uint32_t SCAN_MAX = SCAN_T * SCAN_E * SCAN_T * SCAN_E;   // counts one scan takes
 
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* sm_warp, uint32_t& total) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1394,6 +1395,7 @@ int msm_bits_group(int nrows, double ncols) {
   double best = 1e300;
   int br = 1;
   for (int rho = 1; rho <= std::min(nrows, 14); rho++) {
+    if ((uint64_t)bits_groups(nrows, rho) << rho > SCAN_MAX) break;
     const double cost = bits_groups(nrows, rho) * 10.0 * (1.0 - std::ldexp(1.0, -rho)) * ncols +
                         (double)nrows * std::ldexp(16.0, rho - 1);
     if (cost < best) { best = cost; br = rho; }
@@ -1401,13 +1403,14 @@ int msm_bits_group(int nrows, double ncols) {
   return br;
 }
 
-// dig, rank as in hist_windows; thread i takes column i (neighbouring threads read neighbouring bytes).
+// dig, rank as in hist_windows; thread i takes column i (neighbouring threads read neighbouring bytes) and
+// every gridDim.y-th group.
 // Few rows, or rows that are mostly ones, send many columns to one bucket, so the lanes of a warp with
 // the same pattern count it once.
 __global__ void k_bits_hist(int n, const uint8_t* __restrict__ coeffs, size_t ld, WinShape ws, int ngroups,
                             uint32_t* __restrict__ cnt, uint32_t* __restrict__ dig, uint32_t* __restrict__ rank) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-  for (int w = 0; w < ngroups; w++) {
+  for (int w = blockIdx.y; w < ngroups; w += gridDim.y) {
     const int rows = ws.width(w) - 1, r0 = ws.start(w) - w;   // the shape's windows are one bit wider
     uint32_t v = 0;
     if (i < n)
@@ -1424,11 +1427,12 @@ __global__ void k_bits_hist(int n, const uint8_t* __restrict__ coeffs, size_t ld
   }
 }
 
-// Block r: the sum of its group's buckets with row r's bit set, canonical.
+// Block r: the sum of its group's buckets with row r's bit set (and, with `add`, of the point at out),
+// canonical.
 template <class C>
 __global__ void __launch_bounds__(256) k_bits_rows(WinShape ws, const uint32_t* __restrict__ off,
                                                    const uint32_t* __restrict__ bsum, uint32_t* __restrict__ out,
-                                                   size_t stride) {
+                                                   bool add) {
   using F = typename C::Fp;
   constexpr int XW = 4 * F::N;
   __shared__ __align__(16) uint32_t sm[8 * XW];
@@ -1436,24 +1440,36 @@ __global__ void __launch_bounds__(256) k_bits_rows(WinShape ws, const uint32_t* 
   const uint32_t few = (uint32_t)ws.base - 1, wide = (uint32_t)ws.extra * (few + 1);   // rows of a narrow group, of the wide ones
   const int w = (int)(r < wide ? r / (few + 1) : ws.extra + (r - wide) / few);
   const uint32_t k = r - (uint32_t)(ws.start(w) - w), cnt = ws.buckets(w) >> 1, quad = threadIdx.x >> 2;
+  const uint32_t quads = blockDim.x >> 2;
   const uint32_t s0 = ws.seg(w);
   auto item = [&](uint32_t j) {
     const uint32_t s = s0 + (((j >> k) << (k + 1)) | (1u << k) | (j & ((1u << k) - 1)));
     return j < cnt && __ldg(off + s) != __ldg(off + s + 1) ? quad_load<F>(bsum + (size_t)s * XW) : fe_zero<F>();
   };
-  Fe<F> a = fe_zero<F>(), nx = item(quad);
+  Fe<F> a = add && quad == 0 ? quad_load<F>(out + (size_t)r * XW) : fe_zero<F>(), nx = item(quad);
 #pragma unroll 1
-  for (uint32_t j0 = 0; j0 < cnt; j0 += 64) {
+  for (uint32_t j0 = 0; j0 < cnt; j0 += quads) {
     const Fe<F> x = nx;
-    nx = item(j0 + 64 + quad);
+    nx = item(j0 + quads + quad);
     a = quad_add(a, x);
   }
   a = quad_warp_sum(a);
-  if ((threadIdx.x & 31) < 4) quad_store(sm + (threadIdx.x >> 5) * XW, a);
-  __syncthreads();
-  if (threadIdx.x >= 32) return;
-  a = quad_warp_sum(quad_load<F>(sm + quad * XW));
-  if (threadIdx.x < 4) quad_store(out + (size_t)r * stride, fe_canon(a));
+  if (quads > 8) {
+    if ((threadIdx.x & 31) < 4) quad_store(sm + (threadIdx.x >> 5) * XW, a);
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    a = quad_warp_sum(quad < quads >> 3 ? quad_load<F>(sm + quad * XW) : fe_zero<F>());
+  }
+  if (threadIdx.x < 4) quad_store(out + (size_t)r * XW, fe_canon(a));
+}
+
+// Threads a row: eight warps for the shortest chain while the rows leave the GPU idle, fewer with many rows,
+// where the quads' own sums cost a warp three additions (25000 rows of 32 items: 2.05 ms with eight warps a
+// row, 0.44 with one).
+static unsigned bits_rows_threads(int nrows) {
+  unsigned t = 256;
+  while (t > 32 && (uint64_t)nrows * t > 512ull * (uint64_t)std::max(1, device_sm_count())) t >>= 1;
+  return t;
 }
 
 struct BitsPlan {
@@ -1477,7 +1493,7 @@ static zkg_status bits_plan(int nrows, int ncols, int rho, BitsPlan& P) {
   P.nch = std::max<uint32_t>(1, (uint32_t)((P.total + P.L1 - 1) / P.L1));
   P.pcap = P.nch / 8 + 2;
   const uint32_t nb = (P.nseg + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E);
-  if (nb > (uint32_t)SCAN_T * SCAN_E) return set_status(ZKG_ERR_ARG, "msm_binary", "too many buckets");
+  if (P.nseg > SCAN_MAX) return set_status(ZKG_ERR_ARG, "msm_binary", "too many buckets");
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t r = o; o = (o + bytes + 255) & ~size_t(255); return r; };
   P.o_cnt = take((size_t)P.nseg * 4 + 4);   // then: pieces
@@ -1499,15 +1515,17 @@ static zkg_status bits_plan(int nrows, int ncols, int rho, BitsPlan& P) {
 
 template <class C>
 static zkg_status bits_launch(int nrows, int ncols, int rho, const uint8_t* coeffs, size_t ld, const uint32_t* bases,
-                              char* ws, size_t ws_bytes, uint32_t* out, size_t stride, uint32_t* chk,
-                              cudaStream_t st) {
+                              char* ws, size_t ws_bytes, uint32_t* out, bool add, uint32_t* chk, cudaStream_t st) {
   BitsPlan P;
   ZKB_TRY(bits_plan<C>(nrows, ncols, rho, P));
   if (P.bytes > ws_bytes) return set_status(ZKG_ERR_NOMEM, "msm_binary", "workspace smaller than the launch needs");
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
   ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)P.nseg * 4 + 4, st));
   const dim3 gc((ncols + 255) / 256);
-  ZKB_TRY(launch("bits_hist", k_bits_hist, gc, dim3(256), 0, st, ncols, coeffs, ld, P.win, P.ngroups, U32(P.o_cnt),
+  // few columns: the groups in parallel too, up to eight blocks an SM
+  const uint32_t blocks = 8 * (uint32_t)std::max(1, device_sm_count());
+  const dim3 gh(gc.x, std::min<uint32_t>((uint32_t)P.ngroups, (blocks + gc.x - 1) / gc.x));
+  ZKB_TRY(launch("bits_hist", k_bits_hist, gh, dim3(256), 0, st, ncols, coeffs, ld, P.win, P.ngroups, U32(P.o_cnt),
                  U32(P.o_dig), U32(P.o_rank)));
   ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st));
   ZKB_TRY(launch("msm_scatter_d", k_msm_scatter_d, dim3(gc.x, P.ngroups), dim3(256), 0, st, ncols,
@@ -1523,8 +1541,8 @@ static zkg_status bits_launch(int nrows, int ncols, int rho, const uint8_t* coef
   const PieceList pl = {U32(P.o_cnt) + P.nseg, P.pcap, reinterpret_cast<Piece*>(ws + P.o_prec), U32(P.o_pdone),
                         U32(P.o_ppt)};
   ZKB_TRY(msm_launch_merge<C>(pl, off, chk, P.nch, P.L1, U32(P.o_key), U32(P.o_pt), U32(P.o_bsum), P.nseg, st));
-  return launch("bits_rows", k_bits_rows<C>, dim3(nrows), dim3(256), 0, st, P.win, off,
-                (const uint32_t*)U32(P.o_bsum), out, stride);
+  return launch("bits_rows", k_bits_rows<C>, dim3(nrows), dim3(bits_rows_threads(nrows)), 0, st, P.win, off,
+                (const uint32_t*)U32(P.o_bsum), out, add);
 }
 
 zkg_status msm_bits_bytes(int curve, int nrows, int ncols, int rho, size_t* bytes) {
@@ -1535,12 +1553,12 @@ zkg_status msm_bits_bytes(int curve, int nrows, int ncols, int rho, size_t* byte
 }
 
 zkg_status msm_bits_launch(Context& cx, int curve, int nrows, int ncols, int rho, const uint8_t* coeffs, size_t ld,
-                           const uint32_t* bases, char* ws, size_t ws_bytes, uint32_t* out, size_t stride,
+                           const uint32_t* bases, char* ws, size_t ws_bytes, uint32_t* out, bool add,
                            cudaStream_t st) {
   uint32_t* chk = dev_check_word(cx);
   if (curve == ZKG_BN254)
-    return bits_launch<BN254E>(nrows, ncols, rho, coeffs, ld, bases, ws, ws_bytes, out, stride, chk, st);
-  return bits_launch<BLS12_381E>(nrows, ncols, rho, coeffs, ld, bases, ws, ws_bytes, out, stride, chk, st);
+    return bits_launch<BN254E>(nrows, ncols, rho, coeffs, ld, bases, ws, ws_bytes, out, add, chk, st);
+  return bits_launch<BLS12_381E>(nrows, ncols, rho, coeffs, ld, bases, ws, ws_bytes, out, add, chk, st);
 }
 
 // =================================================================== batched MSMs (many sizes)
