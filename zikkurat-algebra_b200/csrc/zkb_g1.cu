@@ -513,7 +513,6 @@ static zkg_status launch_stage_quad(int inverse, int m, int s, const uint32_t* t
   constexpr size_t smem = 8 * CP::Fp::N * (QUAD_T + QUAD_T / 4) * 4;
   const size_t quads = ((size_t)1 << (m - 1)) * HALVES;
   auto k = inverse ? k_g1fft_stage_quad<CP, true, HALVES> : k_g1fft_stage_quad<CP, false, HALVES>;
-  ZKB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   return launch("g1fft_stage", k, dim3((unsigned)((quads * 4 + QUAD_T - 1) / QUAD_T)), dim3(QUAD_T), smem, st, m, s, tw,
                 top, beta, a);
 }

@@ -727,7 +727,6 @@ static uint64_t accum_wave() {
     else if constexpr (C::Fp::N == 8) {
       blocks = shape == 2 ? accum_w_occupancy<C, 384>() : shape == 3 ? accum_w_occupancy<C, 320>()
              : shape == 4 ? accum_w_occupancy<C, 448>() : accum_w_occupancy<C, 512>();
-      accum_w_occupancy<C, 384, 3>();   // the three-stage form's shared-memory limit
     }
     if (e != cudaSuccess || blocks < 1) blocks = 1;
     return (uint64_t)sms * (uint64_t)blocks * (uint64_t)accum_threads(shape);
@@ -743,7 +742,6 @@ static zkg_status launch_accum(uint32_t nch, cudaStream_t st, const uint32_t* en
   const dim3 g((nch + 255) / 256);
   if constexpr (C::Fp::N == 8) {   // three stages of 96-byte BLS12-381 bases exceed 48 KB of shared memory
     if (pf >= 3 && accum_shape<C>() == 2) {
-      accum_wave<C>();
       return launch("msm_accum", k_msm_accum_w<C, 384, 3>, dim3((nch + 383) / 384), dim3(384),
                     (size_t)3 * (C::Fp::N / 2) * 384 * 16, st, ent, off, nseg, nch, L, bases, bsum, key, pt, chk,
                     npts);
@@ -757,7 +755,6 @@ static zkg_status launch_accum(uint32_t nch, cudaStream_t st, const uint32_t* en
                     key, pt, chk, npts);
     if constexpr (C::Fp::N == 8) {
       if (shape >= 2) {
-        accum_wave<C>();   // sets the kernels' shared-memory limit
         const int nt = accum_threads(shape);
         const size_t smem = (size_t)2 * (C::Fp::N / 2) * nt * 16;
         const dim3 gw((nch + nt - 1) / nt);
@@ -918,17 +915,6 @@ static zkg_status msm_u_to_radix(const MsmPlan& P, char* ws, cudaStream_t st) {
   return ZKG_OK;
 }
 
-// Dynamic shared memory above the default 48 KB needs the kernel's attribute set, once per kernel
-// (the statics are per instantiation: FWD, C, L0, NT and PF name the tree kernel).
-template <bool FWD, class C, bool L0, int NT, int PF, class K>
-static zkg_status tree_smem_limit(K kernel, size_t bytes) {
-  static const cudaError_t e = bytes > 48 * 1024
-                                   ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-                                   : cudaSuccess;
-  if (e != cudaSuccess) return set_status(ZKG_ERR_CUDA, "msm", cudaGetErrorString(e));
-  return ZKG_OK;
-}
-
 // prefetch stages of the tree's backward pass (ZKB_MSM_TREE_PF = 2 or 3); the forward pass has 3
 static int g_tree_pf = env_int("ZKB_MSM_TREE_PF", 2);
 
@@ -938,7 +924,6 @@ static zkg_status launch_tree_bwd(const MsmPlan& P, int level, uint32_t nthr, cu
                                   const uint32_t* tinv, uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
   constexpr int NT = tree_nt<C>();
   const size_t smem = (size_t)PF * tree_bwd_pieces<typename C::Fp>() * NT * 16;
-  ZKB_TRY((tree_smem_limit<false, C, L0, NT, PF>(k_tree_bwd<C, L0, NT, PF>, smem)));
   return launch("msm_tree_bwd", k_tree_bwd<C, L0, NT, PF>, dim3(nthr / NT), dim3(NT), smem, st, ent, in_pts, total,
                 level, tree_wave<C>(), P.tB, pre, tinv, out_pts, level == P.tree - 1 ? 1 : 0, chk, npts);
 }
@@ -951,7 +936,6 @@ static zkg_status launch_tree_level(const MsmPlan& P, int level, cudaStream_t st
   constexpr int NT = tree_nt<C>(), PFF = 3;
   const uint32_t nthr = tree_threads<C>(P, level);
   const size_t smf = (size_t)PFF * tree_fwd_pieces<F>() * NT * 16;
-  ZKB_TRY((tree_smem_limit<true, C, L0, NT, PFF>(k_tree_fwd<C, L0, NT, PFF>, smf)));
   ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, L0, NT, PFF>, dim3(nthr / NT), dim3(NT), smf, st, ent, in_pts, total,
                  level, tree_wave<C>(), P.tB, pre, tt, chk, npts));
   // simultaneous inversion of the thread products: about 4 per thread
