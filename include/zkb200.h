@@ -583,6 +583,10 @@ int zkg_set_msm_parts(int parts);
  * to the automatic choice, >= 4 otherwise). Returns the previous level setting. Results do not
  * depend on either. */
 int zkg_set_msm_tree(int levels, int slots_per_thread);
+/* Device workspace of an MSM of Montgomery scalars on device buffers, planned on the host: info[0] bytes
+ * with the affine tree levels that the rules pick, info[1] without them (what a call takes when the
+ * device has less than info[0] free). */
+zkg_status zkg_msm_workspace(zkg_curve curve, int npoints, size_t info[2]);
 /* Window width the automatic rule picks for a curve and size. */
 int zkg_msm_window_for(zkg_curve curve, int npoints);
 /* Largest NTT pass (log2 of the per-pass network size, 1..11; default 8; 0 = back to the

@@ -792,6 +792,13 @@ static uint32_t quad_chunk_len(uint64_t total) {
   return (uint32_t)std::max<uint64_t>(4, (total + quads - 1) / quads);
 }
 
+// Entries the affine tree works on at a time: its lists and running products take about 64 bytes an entry
+// for BN254, 96 for BLS12-381 (four times the rest of an MSM's workspace), so beyond this many the windows
+// go in slabs: 2^24 points of BN254 take 10.3 GiB instead of 17.5, 2^26 19 instead of 64. Every slab has its
+// own last waves, so smaller ones cost time: 2^23 points 25.9 ms in one slab, 27.3 in two of 2^26 entries,
+// 28.9 in four; 2^24 53.4 in one, 55.7 in two, 56.3 in four.
+static const uint64_t g_tree_slab = (uint64_t)std::max(1, env_int("ZKB_MSM_TREE_SLAB", 1 << 27));
+
 struct MsmPlan {
   int n = 0, c = 0, nwin = 0, nw = 0;
   uint32_t B = 0, nseg = 0;
@@ -808,7 +815,10 @@ struct MsmPlan {
   int tree = 0;             // affine tree levels before the chunk accumulation (zkb_msm_tree.cuh)
   uint32_t tB = 32;         // slots per tree thread
   uint64_t total_pad = 0;   // entries with the padding the tree needs, at most
-  uint64_t acc_total = 0;   // entries of the chunk accumulation (a bound when tree > 0)
+  int slabs = 1, wslab = 0; // the tree and the accumulation after it run over slabs of wslab windows
+  uint32_t sseg = 0;        // segments and padded entries of a slab, at most
+  uint64_t spad = 0;
+  uint64_t acc_total = 0;   // entries of the chunk accumulation of a slab (a bound when tree > 0)
   // byte offsets into one arena block
   size_t o_std, o_cnt, o_off, o_cur, o_bs, o_ent, o_keyA, o_ptA, o_bsum, o_T, o_R, o_U, o_V, bytes;
   size_t o_prec, o_pdone, o_ppt;   // pieces of long segments (their count follows the histogram's counts)
@@ -824,11 +834,11 @@ static uint32_t tree_wave() { return (uint32_t)std::max(1, device_sm_count()) * 
 template <class C>
 static uint32_t tree_threads(const MsmPlan& P, int level) {
   const uint32_t wave = tree_wave<C>();
-  return wave * tree_waves(P.total_pad >> (level + 1), wave, P.tB);
+  return wave * tree_waves(P.spad >> (level + 1), wave, P.tB);
 }
 
 template <class C>
-static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force = 0) {
+static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force = 0, int tree_max = MAX_TREE) {
   using F = typename C::Fp;
   constexpr size_t XB = 16 * F::N;   // bytes of one XYZZ point
   P.n = n;
@@ -843,15 +853,23 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   P.total_max = (uint64_t)P.nwin * (uint64_t)n;
   if (P.total_max >= (1ull << 31)) return set_status(ZKG_ERR_ARG, "msm", "too many (window, point) entries for one launch");
   const MsmTune& T = msm_tune(C::ID, round_log2((uint64_t)n));
-  P.tree = pick_tree<C>(P.total_max, P.nseg, T.tree);
+  P.tree = std::min(tree_max, pick_tree<C>(P.total_max, P.nseg, T.tree));
   P.acc_total = P.total_max;
+  P.slabs = 1;
+  P.wslab = P.nwin;
   if (P.tree > 0) {   // segments padded to multiples of 2^tree
     P.tB = pick_tree_slots(P.total_max);
     P.total_pad = P.total_max + (uint64_t)P.nseg * ((1u << P.tree) - 1);
-    P.acc_total = P.total_pad >> P.tree;
+    P.wslab = (int)std::min<uint64_t>(P.nwin, std::max<uint64_t>(1, g_tree_slab / n));
+    P.slabs = (P.nwin + P.wslab - 1) / P.wslab;
+    P.wslab = (P.nwin + P.slabs - 1) / P.slabs;
+    P.slabs = (P.nwin + P.wslab - 1) / P.wslab;
+    P.spad = (uint64_t)P.wslab * n + (uint64_t)P.win.seg(P.wslab) * ((1u << P.tree) - 1);   // wide windows come first
+    P.acc_total = P.spad >> P.tree;
   } else {
-    P.total_pad = P.total_max;
+    P.total_pad = P.spad = P.total_max;
   }
+  P.sseg = P.win.seg(P.wslab);
   P.L1 = (int)chunk_len(P.acc_total, accum_wave<C>(), T.L1);
   P.pf = g_msm_pf_env || T.pf < 0 ? g_msm_pf : T.pf;
   P.quad = P.tree == 0 && P.total_max <= QUAD_TOTAL;
@@ -890,8 +908,8 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   P.o_toff = P.o_tpts[0] = P.o_tpts[1] = P.o_tpre = P.o_ttt = P.o_tscr = 0;
   if (P.tree > 0) {
     constexpr size_t AB = 8 * F::N, FB = 4 * F::N;   // bytes of an affine point, of a field element
-    const uint64_t q0 = P.total_pad / 2 + 1, thr = tree_threads<C>(P, 0);
-    P.o_toff = take((size_t)P.nseg * 4 + 4);
+    const uint64_t q0 = P.spad / 2 + 1, thr = tree_threads<C>(P, 0);
+    P.o_toff = take((size_t)P.sseg * 4 + 4);
     P.o_tpts[0] = take(q0 * AB);
     P.o_tpts[1] = take(P.tree > 1 ? (q0 / 2 + 1) * AB : 0);
     P.o_tpre = take(q0 * FB);
@@ -918,48 +936,54 @@ static zkg_status msm_u_to_radix(const MsmPlan& P, char* ws, cudaStream_t st) {
 // prefetch stages of the tree's backward pass (ZKB_MSM_TREE_PF = 2 or 3); the forward pass has 3
 static int g_tree_pf = env_int("ZKB_MSM_TREE_PF", 2);
 
+// One slab of windows: its segments' offsets (off[0 .. nseg]) among the padded entries.
+struct TreeSlab {
+  const uint32_t* off;
+  uint32_t nseg;
+};
+
 template <class C, bool L0, int PF>
 static zkg_status launch_tree_bwd(const MsmPlan& P, int level, uint32_t nthr, cudaStream_t st, const uint32_t* ent,
-                                  const uint32_t* in_pts, const uint32_t* total, const uint32_t* pre,
-                                  const uint32_t* tinv, uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
+                                  const uint32_t* in_pts, TreeSlab sl, const uint32_t* pre, const uint32_t* tinv,
+                                  uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
   constexpr int NT = tree_nt<C>();
   const size_t smem = (size_t)PF * tree_bwd_pieces<typename C::Fp>() * NT * 16;
-  return launch("msm_tree_bwd", k_tree_bwd<C, L0, NT, PF>, dim3(nthr / NT), dim3(NT), smem, st, ent, in_pts, total,
-                level, tree_wave<C>(), P.tB, pre, tinv, out_pts, level == P.tree - 1 ? 1 : 0, chk, npts);
+  return launch("msm_tree_bwd", k_tree_bwd<C, L0, NT, PF>, dim3(nthr / NT), dim3(NT), smem, st, ent, in_pts, sl.off,
+                sl.nseg, level, tree_wave<C>(), P.tB, pre, tinv, out_pts, level == P.tree - 1 ? 1 : 0, chk, npts);
 }
 
 template <class C, bool L0>
 static zkg_status launch_tree_level(const MsmPlan& P, int level, cudaStream_t st, const uint32_t* ent,
-                                    const uint32_t* in_pts, const uint32_t* total, uint32_t* pre, uint32_t* tt,
-                                    uint32_t* scr, uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
+                                    const uint32_t* in_pts, TreeSlab sl, uint32_t* pre, uint32_t* tt, uint32_t* scr,
+                                    uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
   using F = typename C::Fp;
   constexpr int NT = tree_nt<C>(), PFF = 3;
   const uint32_t nthr = tree_threads<C>(P, level);
   const size_t smf = (size_t)PFF * tree_fwd_pieces<F>() * NT * 16;
-  ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, L0, NT, PFF>, dim3(nthr / NT), dim3(NT), smf, st, ent, in_pts, total,
-                 level, tree_wave<C>(), P.tB, pre, tt, chk, npts));
+  ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, L0, NT, PFF>, dim3(nthr / NT), dim3(NT), smf, st, ent, in_pts, sl.off,
+                 sl.nseg, level, tree_wave<C>(), P.tB, pre, tt, chk, npts));
   // simultaneous inversion of the thread products: about 4 per thread
   const size_t T = std::min<size_t>(((size_t)nthr + 255) & ~size_t(255), std::max<size_t>(2048, (size_t)nthr / 4));
   ZKB_TRY(launch("msm_tree_inv", k_tree_inv<F>, dim3((unsigned)((T + 255) / 256)), dim3(256), 0, st, nthr, tt, scr));
   if (g_tree_pf >= 3)
-    return launch_tree_bwd<C, L0, 3>(P, level, nthr, st, ent, in_pts, total, pre, tt, out_pts, chk, npts);
-  return launch_tree_bwd<C, L0, 2>(P, level, nthr, st, ent, in_pts, total, pre, tt, out_pts, chk, npts);
+    return launch_tree_bwd<C, L0, 3>(P, level, nthr, st, ent, in_pts, sl, pre, tt, out_pts, chk, npts);
+  return launch_tree_bwd<C, L0, 2>(P, level, nthr, st, ent, in_pts, sl, pre, tt, out_pts, chk, npts);
 }
 
-// The affine tree levels of one point range (zkb_msm_tree.cuh), after the sort has placed the entries of
-// the padded segments: level l reads the entries and bases (l = 0) or level l - 1's list and writes its
-// points to o_tpts[l & 1]; the last list's offsets go to o_toff.
+// The affine tree levels of one slab of windows of one point range (zkb_msm_tree.cuh), after the sort has
+// placed the entries of the padded segments (ent: all of them; cnt, sl: the slab's). Level l reads the
+// entries and bases (l = 0) or level l - 1's list and writes its points to o_tpts[l & 1]; the last list's
+// offsets go to o_toff.
 template <class C>
-static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, uint32_t* ent, const uint32_t* off,
+static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, uint32_t* ent, const uint32_t* cnt, TreeSlab sl,
                                   const uint32_t* bases, cudaStream_t st, uint32_t* chk) {
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
-  ZKB_TRY(launch("msm_tree_pad", k_tree_pad, dim3(P.nseg / 256 + 1), dim3(256), 0, st, (const uint32_t*)U32(P.o_cnt), off,
-                 P.nseg, P.tree, ent, U32(P.o_toff), U32(P.o_cnt) + P.nseg + 1));
-  const uint32_t* total = off + P.nseg;
-  ZKB_TRY((launch_tree_level<C, true>(P, 0, st, ent, bases, total, U32(P.o_tpre), U32(P.o_ttt), U32(P.o_tscr),
+  ZKB_TRY(launch("msm_tree_pad", k_tree_pad, dim3(sl.nseg / 256 + 1), dim3(256), 0, st, cnt, sl.off, sl.nseg, P.tree,
+                 ent, U32(P.o_toff), U32(P.o_cnt) + P.nseg + 1));
+  ZKB_TRY((launch_tree_level<C, true>(P, 0, st, ent, bases, sl, U32(P.o_tpre), U32(P.o_ttt), U32(P.o_tscr),
                                       U32(P.o_tpts[0]), chk, (uint32_t)P.n)));
   for (int l = 1; l < P.tree; l++)
-    ZKB_TRY((launch_tree_level<C, false>(P, l, st, nullptr, U32(P.o_tpts[(l - 1) & 1]), total, U32(P.o_tpre),
+    ZKB_TRY((launch_tree_level<C, false>(P, l, st, nullptr, U32(P.o_tpts[(l - 1) & 1]), sl, U32(P.o_tpre),
                                          U32(P.o_ttt), U32(P.o_tscr), U32(P.o_tpts[l & 1]), nullptr, 0)));
   return ZKG_OK;
 }
@@ -1055,38 +1079,46 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
   }
   nvtx_sort.end();
   NvtxRange nvtx_acc("zkb.msm.accumulate_fold");
-  uint32_t acc_npts = (uint32_t)P.n;
-  if constexpr (!radix_conv_v<typename C::Fp>) {
-    if (P.tree > 0) {   // affine tree levels; the chunk accumulation takes the last level's list
-      NvtxRange nvtx_tree("zkb.msm.affine_tree");
-      ZKB_TRY(msm_tree_launch<C>(P, ws, U32(P.o_ent), off, bases, st, chk));
-      const int lt = (P.tree - 1) & 1;
-      ent = nullptr;
-      off = U32(P.o_toff);
-      bases = U32(P.o_tpts[lt]);
-      acc_npts = (uint32_t)P.acc_total;
-    }
-  }
   const PieceList pl = {U32(P.o_cnt) + P.nseg, P.pcap, reinterpret_cast<Piece*>(ws + P.o_prec), U32(P.o_pdone),
                         U32(P.o_ppt)};
-  if (P.quad)
-    ZKB_TRY(launch("msm_quad_accum", k_quad_accum<C>, dim3((P.nch + 31) / 32), dim3(128), 0, st, ent, off, P.nseg, P.nch,
-                   (uint32_t)P.L1, bases, U32(P.o_bsum), U32(P.o_keyA), U32(P.o_ptA), chk, acc_npts));
-  else
-    ZKB_TRY(launch_accum<C>(P.nch, st, ent, off, P.nseg, (uint32_t)P.L1, bases, U32(P.o_bsum), U32(P.o_keyA),
-                            U32(P.o_ptA), P.pf, chk, acc_npts));
-  if (last) ZKB_CUDA(cudaEventRecord(cx.ev_phase[2], st));
-  // fold_part >= 0: the merge of cut segments runs on the side stream (it is latency-bound, so the
-  // next part's sort and accumulation fill the rest); ev_fold[fold_part] marks it done
-  const cudaStream_t fst = fold_part >= 0 ? cx.side_stream : st;
-  if (fold_part >= 0) {
-    ZKB_CUDA(cudaEventRecord(cx.ev_acc[fold_part], st));
-    ZKB_CUDA(cudaStreamWaitEvent(fst, cx.ev_acc[fold_part], 0));
+  constexpr int XW = 4 * C::Fp::N;
+  for (int sl = 0; sl < P.slabs; sl++) {   // one slab without the tree
+    const int w0 = sl * P.wslab, w1 = std::min(P.nwin, w0 + P.wslab);
+    const uint32_t seg0 = P.win.seg(w0), nseg = P.win.seg(w1) - seg0;
+    uint32_t* bsum = U32(P.o_bsum) + (size_t)seg0 * XW;
+    const uint32_t *a_ent = ent, *a_off = off + seg0, *a_bases = bases;
+    uint32_t acc_npts = (uint32_t)P.n;
+    if (sl > 0) ZKB_CUDA(cudaMemsetAsync(pl.count, 0, 4, st));   // the slab before has used its pieces
+    if constexpr (!radix_conv_v<typename C::Fp>) {
+      if (P.tree > 0) {   // affine tree levels; the chunk accumulation takes the last level's list
+        NvtxRange nvtx_tree("zkb.msm.affine_tree");
+        ZKB_TRY(msm_tree_launch<C>(P, ws, U32(P.o_ent), U32(P.o_cnt) + seg0, {a_off, nseg}, bases, st, chk));
+        a_ent = nullptr;
+        a_off = U32(P.o_toff);
+        a_bases = U32(P.o_tpts[(P.tree - 1) & 1]);
+        acc_npts = (uint32_t)P.acc_total;
+      }
+    }
+    if (P.quad)
+      ZKB_TRY(launch("msm_quad_accum", k_quad_accum<C>, dim3((P.nch + 31) / 32), dim3(128), 0, st, a_ent, a_off, nseg,
+                     P.nch, (uint32_t)P.L1, a_bases, bsum, U32(P.o_keyA), U32(P.o_ptA), chk, acc_npts));
+    else
+      ZKB_TRY(launch_accum<C>(P.nch, st, a_ent, a_off, nseg, (uint32_t)P.L1, a_bases, bsum, U32(P.o_keyA),
+                              U32(P.o_ptA), P.pf, chk, acc_npts));
+    const bool end = sl + 1 == P.slabs;
+    if (last && end) ZKB_CUDA(cudaEventRecord(cx.ev_phase[2], st));
+    // fold_part >= 0: the merge of cut segments runs on the side stream (it is latency-bound, so the
+    // next part's sort and accumulation fill the rest), unless the next slab needs the slots;
+    // ev_fold[fold_part] marks it done
+    const cudaStream_t fst = fold_part >= 0 && P.slabs == 1 ? cx.side_stream : st;
+    if (fst != st) {
+      ZKB_CUDA(cudaEventRecord(cx.ev_acc[fold_part], st));
+      ZKB_CUDA(cudaStreamWaitEvent(fst, cx.ev_acc[fold_part], 0));
+    }
+    ZKB_TRY(msm_launch_merge<C>(pl, a_off, chk, P.nch, (uint32_t)P.L1, U32(P.o_keyA), U32(P.o_ptA), bsum, nseg, fst));
+    if (last && end) ZKB_CUDA(cudaEventRecord(cx.ev_phase[3], fst));
+    if (fold_part >= 0 && end) ZKB_CUDA(cudaEventRecord(cx.ev_fold[fold_part], fst));
   }
-  ZKB_TRY(msm_launch_merge<C>(pl, off, chk, P.nch, (uint32_t)P.L1, U32(P.o_keyA), U32(P.o_ptA), U32(P.o_bsum), P.nseg,
-                              fst));
-  if (last) ZKB_CUDA(cudaEventRecord(cx.ev_phase[3], fst));
-  if (fold_part >= 0) ZKB_CUDA(cudaEventRecord(cx.ev_fold[fold_part], fst));
   return ZKG_OK;
 }
 
@@ -1230,19 +1262,27 @@ static zkg_status msm_host_run(const host::Field<NL>& F, int n, const uint64_t* 
   MsmPlan P[4];
   size_t total = 0, off_s[4], off_b[4], off_w[4], off_c[4];
   auto rup = [](size_t x) { return (x + 255) & ~size_t(255); };
-  for (int q = 0; q < nparts; q++) {
-    const int nq = pstart[q + 1] - pstart[q];
-    ZKB_TRY(make_plan<CP>(nq, nlimbs, mont, P[q], c));
-    off_s[q] = total;
-    total += rup((size_t)nq * nlimbs * 8);
-    off_b[q] = total;
-    total += rup((size_t)nq * 2 * NL * 8);
-    off_c[q] = total;   // bases in the FP64 pipeline's radix
-    if (dpf) total += rup((size_t)nq * 2 * NL * 8);
-    off_w[q] = total;
-    total += rup(P[q].bytes);
+  zkg_status rs = ZKG_OK;
+  for (const int tree_max : {MAX_TREE, 0}) {   // without the tree where its lists do not fit
+    bool tree = false;
+    total = 0;
+    for (int q = 0; q < nparts; q++) {
+      const int nq = pstart[q + 1] - pstart[q];
+      ZKB_TRY(make_plan<CP>(nq, nlimbs, mont, P[q], c, tree_max));
+      tree |= P[q].tree > 0;
+      off_s[q] = total;
+      total += rup((size_t)nq * nlimbs * 8);
+      off_b[q] = total;
+      total += rup((size_t)nq * 2 * NL * 8);
+      off_c[q] = total;   // bases in the FP64 pipeline's radix
+      if (dpf) total += rup((size_t)nq * 2 * NL * 8);
+      off_w[q] = total;
+      total += rup(P[q].bytes);
+    }
+    rs = cx.arena.reserve(total);
+    if (rs != ZKG_ERR_NOMEM || !tree) break;
   }
-  ZKB_TRY(cx.arena.reserve(total));
+  ZKB_TRY(rs);
   cx.arena.reset();
   char* base = static_cast<char*>(cx.arena.take(total));
   if (!base) return set_status(ZKG_ERR_NOMEM, "msm", "arena");
@@ -1328,11 +1368,16 @@ static zkg_status msm_dev_run(const host::Field<NL>& F, int n, const uint64_t* d
   }
   if (!cx.user_stream) ZKB_CUDA(cudaDeviceSynchronize());   // inputs may come from any stream
   MsmPlan P;
-  ZKB_TRY(make_plan<CP>(n, nlimbs, mont, P));
   const bool convert = dpf && !pre_converted;
   const size_t cb = convert ? (((size_t)n * 2 * NL * 8 + 255) & ~size_t(255)) : 0;   // converted bases
   const size_t sb = h_expos ? (((size_t)n * nlimbs * 8 + 255) & ~size_t(255)) : 0;   // copied scalars
-  ZKB_TRY(cx.arena.reserve(P.bytes + cb + sb + 512));
+  zkg_status rs = ZKG_OK;
+  for (const int tree_max : {MAX_TREE, 0}) {   // without the tree where its lists do not fit
+    ZKB_TRY(make_plan<CP>(n, nlimbs, mont, P, 0, tree_max));
+    rs = cx.arena.reserve(P.bytes + cb + sb + 512);
+    if (rs != ZKG_ERR_NOMEM || P.tree == 0) break;
+  }
+  ZKB_TRY(rs);
   cx.arena.reset();
   char* ws = static_cast<char*>(cx.arena.take(P.bytes));
   char* conv = convert ? static_cast<char*>(cx.arena.take(cb)) : nullptr;
@@ -2260,9 +2305,15 @@ static void srv_free(Srv& S, size_t off, size_t bytes) {
 static inline size_t rup256(size_t x) { return (x + 255) & ~size_t(255); }
 
 template <class C>
-static size_t srv_bytes(int k, MsmPlan& P) {
-  if (make_plan<C>(1 << k, 4, 1, P) != ZKG_OK) return (size_t)-1;
-  return 3 * rup256(((size_t)32) << k) + rup256(P.bytes);
+static size_t srv_bytes(int k, size_t budget, int nslots, MsmPlan& P) {
+  for (const int tree_max : {MAX_TREE, 0}) {
+    if (make_plan<C>(1 << k, 4, 1, P, 0, tree_max) != ZKG_OK) return (size_t)-1;
+    const size_t b = 3 * rup256(((size_t)32) << k) + rup256(P.bytes);
+    // the tree's lists only where every slot may have them: they are four times the rest, and requests
+    // beside each other gain more than one alone
+    if (P.tree == 0 || b <= budget / nslots) return b;
+  }
+  return (size_t)-1;
 }
 
 template <class C, int NL>
@@ -2453,7 +2504,8 @@ static zkg_status srv_start(Srv* S, const host::Field<NL>* F, const host::Field<
   using CP = typename MsmCurve<C>::type;
   for (int k = kmin; k <= kmax; k++) {
     MsmPlan P;
-    const size_t b = g_msm_dpf ? srv_bytes<CP>(k, P) : srv_bytes<C>(k, P);
+    const size_t b = g_msm_dpf ? srv_bytes<CP>(k, S->budget, nslots, P)
+                               : srv_bytes<C>(k, S->budget, nslots, P);
     if (b == (size_t)-1 || b > S->budget)
       return set_status(ZKG_ERR_ARG, "zkg_server_create", "HBM budget smaller than one request of the largest size");
     S->req_bytes[k] = b;
@@ -2969,6 +3021,20 @@ int zkg_set_msm_window(int c) {
   const int prev = zkb::g_window_override;
   zkb::g_window_override = c < 0 ? 0 : c;
   return prev;
+}
+
+zkg_status zkg_msm_workspace(zkg_curve curve, int npoints, size_t info[2]) {
+  if ((curve != ZKG_BN254 && curve != ZKG_BLS12_381) || npoints < 1 || !info)
+    return zkb::set_status(ZKG_ERR_ARG, "zkg_msm_workspace", "bad argument");
+  for (int i = 0; i < 2; i++) {
+    zkb::MsmPlan P;
+    const int t = i == 0 ? zkb::MAX_TREE : 0;
+    ZKB_TRY(curve == ZKG_BN254
+                ? zkb::make_plan<zkb::MsmCurve<zkb::BN254>::type>(npoints, 4, 1, P, 0, t)
+                : zkb::make_plan<zkb::MsmCurve<zkb::BLS12_381>::type>(npoints, 4, 1, P, 0, t));
+    info[i] = P.bytes;
+  }
+  return zkb::set_status(ZKG_OK, nullptr, nullptr);
 }
 
 int zkg_msm_window_for(zkg_curve curve, int npoints) {

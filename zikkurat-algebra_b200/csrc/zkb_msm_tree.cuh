@@ -43,8 +43,9 @@ __device__ __forceinline__ uint32_t tree_kind(const Fe<F>& x0, const Fe<F>& y0, 
   return fe_eq(y0, y1) ? TREE_DBL : TREE_INF;
 }
 
-// Pads every segment of cnt[s] entries at off[s] with null entries up to its multiple of 2^T, writes the
-// last list's offsets and adds the real entries up (*total, zeroed with the counts).
+// For the nseg segments of a slab: pads every segment of cnt[s] entries at off[s] with null entries up to its
+// multiple of 2^T, writes the last list's offsets and adds the real entries up (*total, zeroed with the
+// counts).
 __global__ void __launch_bounds__(256) k_tree_pad(const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ off,
                                                   uint32_t nseg, int T, uint32_t* __restrict__ entries,
                                                   uint32_t* __restrict__ last_off, uint32_t* __restrict__ total) {
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(256) k_tree_pad(const uint32_t* __restrict__ c
   uint32_t c = 0;
   if (s <= nseg) {
     const uint32_t lo = off[s];
-    last_off[s] = lo >> T;
+    last_off[s] = (lo - off[0]) >> T;
     if (s < nseg) {
       c = cnt[s];
       const uint32_t m = (1u << T) - 1, end = (c + m) & ~m;
@@ -145,19 +146,26 @@ __host__ __device__ inline uint32_t tree_slots(uint32_t Q, uint32_t wave, uint32
   return (uint32_t)((Q + t - 1) / t);
 }
 
+// The levels run over the entries [off[0], off[nseg]) of one slab of windows: level l has half of them >> l
+// slots, numbered from 0.
+__device__ __forceinline__ uint32_t tree_level_slots(const uint32_t* __restrict__ off, uint32_t nseg, int level) {
+  return (__ldg(off + nseg) - __ldg(off)) >> (level + 1);
+}
+
 // Forward pass: thread i of block b has slots b NT B + k NT + i, k < B (B = tree_slots). pre[q] = product of the
 // denominators of the thread's addition slots before q (stored for addition slots with k > 0);
 // tt[thread] = product of all of them (1 when none). The inputs' x coordinates arrive through PF
 // cp.async stages, PF - 1 slots ahead, their entries one slot earlier still.
 template <class C, bool L0, int NT, int PF>
 __global__ void __launch_bounds__(NT) k_tree_fwd(const uint32_t* __restrict__ ent, const uint32_t* __restrict__ pts,
-                                                 const uint32_t* __restrict__ total, int level, uint32_t wave, uint32_t tB,
-                                                 uint32_t* __restrict__ pre, uint32_t* __restrict__ tt, uint32_t* chk,
-                                                 uint32_t npts) {
+                                                 const uint32_t* __restrict__ off, uint32_t nseg, int level, uint32_t wave,
+                                                 uint32_t tB, uint32_t* __restrict__ pre, uint32_t* __restrict__ tt,
+                                                 uint32_t* chk, uint32_t npts) {
   using F = typename C::Fp;
   constexpr int FW = F::N, QF = F::N / 4, QS = tree_fwd_pieces<F>();
   extern __shared__ uint4 tsm[];
-  const uint32_t Q = __ldg(total) >> (level + 1), B = tree_slots(Q, wave, tB);
+  const uint32_t Q = tree_level_slots(off, nseg, level), B = tree_slots(Q, wave, tB);
+  if constexpr (L0) ent += __ldg(off);
   const uint32_t base = blockIdx.x * NT * B + threadIdx.x;
   const uint32_t n = base < Q ? min(B, (Q - base + NT - 1) / NT) : 0;   // slots of this thread
   Fe<F> acc = fe_one<F>();
@@ -239,13 +247,15 @@ __global__ void __launch_bounds__(256) k_tree_inv(uint32_t n, uint32_t* __restri
 // arrive through PF cp.async stages, PF - 1 slots ahead.
 template <class C, bool L0, int NT, int PF>
 __global__ void __launch_bounds__(NT, 1) k_tree_bwd(const uint32_t* __restrict__ ent, const uint32_t* __restrict__ pts,
-                                                    const uint32_t* __restrict__ total, int level, uint32_t wave, uint32_t tB,
-                                                    const uint32_t* __restrict__ pre, const uint32_t* __restrict__ tinv,
-                                                    uint32_t* __restrict__ out, int last, uint32_t* chk, uint32_t npts) {
+                                                    const uint32_t* __restrict__ off, uint32_t nseg, int level, uint32_t wave,
+                                                    uint32_t tB, const uint32_t* __restrict__ pre,
+                                                    const uint32_t* __restrict__ tinv, uint32_t* __restrict__ out, int last,
+                                                    uint32_t* chk, uint32_t npts) {
   using F = typename C::Fp;
   constexpr int FW = F::N, AW = 2 * F::N, QF = F::N / 4, QA = 2 * QF, QS = tree_bwd_pieces<F>();
   extern __shared__ uint4 tsm[];
-  const uint32_t Q = __ldg(total) >> (level + 1), B = tree_slots(Q, wave, tB);
+  const uint32_t Q = tree_level_slots(off, nseg, level), B = tree_slots(Q, wave, tB);
+  if constexpr (L0) ent += __ldg(off);
   const uint32_t base = blockIdx.x * NT * B + threadIdx.x;
   if (base >= Q) return;
   const int n = (int)min(B, (Q - base + NT - 1) / NT);

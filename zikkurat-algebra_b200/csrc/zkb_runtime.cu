@@ -27,6 +27,9 @@ zkg_status set_status(zkg_status s, const char* where, const char* detail) {
 
 zkg_status Arena::reserve(size_t bytes) {
   if (bytes <= cap) return ZKG_OK;
+  size_t free_bytes = 0, all = 0;   // what cannot fit is refused with the present buffer kept
+  if (cudaMemGetInfo(&free_bytes, &all) == cudaSuccess && bytes > cap + free_bytes)
+    return set_status(ZKG_ERR_NOMEM, "arena reserve", "more than the device has free");
   if (base) {
     cudaFree(base);
     base = nullptr;
