@@ -133,6 +133,38 @@ def test_msm_degenerate_cases_affine_tree(zk, curve, levels, slots):
 
 
 @pytest.mark.parametrize("curve", Z.CURVES)
+@pytest.mark.parametrize("n", [3000, 1 << 17, 1 << 20])
+def test_msm_of_few_entries(zk, curve, n):
+    """chunks shortened to the entries there are: mostly zero scalars equal the MSM of the others, and scalars
+    of a few bits the sum over their values"""
+    import torch
+    nl = Z.NLP[curve]
+    ks = Z.rand_fr(curve, n, 16100 + curve)
+    bases = torch.empty((n, 2 * nl), dtype=torch.int64, device="cuda")
+    zk.g1_gen_mul_device(curve, n, torch.from_numpy(ks.view(np.int64)).cuda(), bases)
+    s = torch.from_numpy(Z.rand_fr(curve, n, 16200 + curve).view(np.int64)).cuda()
+    rng = np.random.default_rng(161)
+    for count in (1, 8, 100, 2999, n // 40):
+        at = torch.from_numpy(np.sort(rng.choice(n, count, replace=False))).cuda()
+        t = torch.zeros_like(s)
+        t[at] = s[at]
+        got = zk.msm_device(curve, n, t, bases, mont=False)
+        want = zk.msm_device(curve, count, s[at].contiguous(), bases[at].contiguous(), mont=False)
+        assert np.array_equal(got, want), count
+    k_int = [Z.from_limbs(v) for v in ks]
+    for bits in (1, 16):   # the bases are ks[i] G: one scalar multiple of G
+        v = rng.integers(0, 1 << bits, n)
+        t = torch.zeros_like(s)
+        t[:, 0] = torch.from_numpy(v).cuda()
+        got = zk.msm_device(curve, n, t, bases, mont=False)
+        e = sum(int(a) * b for a, b in zip(v, k_int)) % zk.R_MOD[curve]
+        one = torch.empty((1, 2 * nl), dtype=torch.int64, device="cuda")
+        zk.g1_gen_mul_device(curve, 1, torch.from_numpy(np.asarray(Z.to_limbs(e, 4)).view(np.int64)).cuda(), one)
+        torch.cuda.synchronize()
+        assert np.array_equal(got, one.cpu().numpy().view(np.uint64)[0]), bits
+
+
+@pytest.mark.parametrize("curve", Z.CURVES)
 def test_msm_affine_tree_levels_match_oracle(zk, curve):
     """random MSMs with 0..8 affine tree levels and several thread batch sizes equal the oracle"""
     L = zk.lib()

@@ -172,7 +172,9 @@ __global__ void __launch_bounds__(128) k_quad_accum(const uint32_t* __restrict__
   using F = typename C::Fp;
   constexpr int XW = 4 * F::N;
   const uint32_t t = (blockIdx.x * 128 + threadIdx.x) >> 2;
-  const uint32_t total = __ldg(off + nseg), start = t * L;
+  const uint32_t total = __ldg(off + nseg);
+  L = counted_len(total, nchunks, L);
+  const uint32_t start = t * L;
   uint32_t end = start, s = 0, seg_lo = 0, seg_hi = 0;
   if (t < nchunks && start < total) {
     end = min(start + L, total);
@@ -238,6 +240,7 @@ __global__ void __launch_bounds__(128) k_cut_merge(const uint32_t* __restrict__ 
   constexpr int XW = 4 * F::N;
   const uint32_t t = (blockIdx.x * 128 + threadIdx.x) >> 2;
   uint32_t s = INVALID, more = 0;   // partial sums after the first
+  L = counted_len(__ldg(off + nseg), nchunks, L);
   if (t + 1 < nchunks) {
     s = __ldg(skey + 2 * (size_t)t + 1);
     if (chk && s != INVALID && s >= nseg) { atomicOr(chk, CHK_SEGMENT); s = INVALID; }
