@@ -28,6 +28,22 @@ def test_tree_in_slabs_of_windows_changes_no_result(zk, slab, levels, tmp_path):
         assert np.array_equal(got[k], v), k
 
 
+def test_device_checks_on_the_small_sort_and_binary_rows(zk):
+    """with the bounds checks on, valid inputs set no bit and give the same points"""
+    code = ("import sys; sys.path.insert(0, %r); import numpy as np, zkutil as Z; zk = Z.load_package()\n"
+            "for c in Z.CURVES:\n"
+            "    b = Z.gen_bases_cpu(c, Z.rand_fr(c, 900, 1)); s = Z.rand_fr(c, 900, 2)\n"
+            "    co = (Z.splitmix64(3, 30 * 900) & np.uint64(1)).astype(np.uint8).reshape(30, 900)\n"
+            "    for mont in (True, False):\n"
+            "        assert np.array_equal(zk.msm_affine(c, s, b, mont=mont), Z.oracle_msm_affine(c, s, 4, mont, b))\n"
+            "    r = zk.binary_multi_msm(c, co, b, affine=True)\n"
+            "    z = np.zeros((900, 4), np.uint64); z[:, 0] = co[29]\n"
+            "    assert np.array_equal(r[29], Z.oracle_msm_affine(c, z, 4, False, b))\n" % K.HERE)
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, ZKB_DEVICE_CHECKS="1"), capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def _bases(zk, curve, n):
     import torch
     b = torch.empty((n, 2 * Z.NLP[curve]), dtype=torch.int64, device="cuda")

@@ -823,6 +823,7 @@ static zkg_status bin_host(const host::Field<NL>& Fp, int kind, int nrows, int n
   if (rc == ZKG_OK && cudaMemcpyAsync(pin, d_out, (size_t)nrows * ow * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess)
     rc = set_status(ZKG_ERR_CUDA, "msm_binary", "output copy");
   if (rc == ZKG_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = set_status(ZKG_ERR_CUDA, "msm_binary", "sync");
+  if (rc == ZKG_OK) rc = dev_check_report(cx, "msm_binary");
   if (rc == ZKG_OK) std::memcpy(tgt, pin, (size_t)nrows * ow * 8);
   if (rc != ZKG_OK) {
     cudaStreamSynchronize(cx.copy_stream);
@@ -879,6 +880,7 @@ static zkg_status bin_dev(int kind, int nrows, int npoints, const uint8_t* d_coe
   auto done_tile = [](int) -> zkg_status { return ZKG_OK; };
   ZKB_TRY((bin_run<C, NL>(cx, P, nrows, npoints, ws, st, get_tile, done_tile, kind, reinterpret_cast<uint32_t*>(d_out))));
   ZKB_CUDA(cudaStreamSynchronize(st));
+  ZKB_TRY(dev_check_report(cx, "msm_binary"));
   return set_status(ZKG_OK, nullptr, nullptr);
 }
 

@@ -406,7 +406,8 @@ static Bias digit_bias(const WinShape& ws, int nwin) {
 template <class C, bool MONT>
 __global__ void __launch_bounds__(SMALL_T) k_sort_small(int n, const uint32_t* __restrict__ scal, int nw, WinShape ws,
                                                         const Bias bias, uint32_t nseg, uint32_t* __restrict__ off,
-                                                        uint32_t* __restrict__ entries, uint32_t* __restrict__ nonzero) {
+                                                        uint32_t* __restrict__ entries, uint32_t* __restrict__ nonzero,
+                                                        uint32_t* chk) {
   using Fr = typename C::Fr;
   static_assert(SMALL_N == SMALL_T, "one point a thread");
   __shared__ uint32_t cnt[SMALL_B + 1], smw[32];
@@ -437,6 +438,7 @@ __global__ void __launch_bounds__(SMALL_T) k_sort_small(int n, const uint32_t* _
       uint32_t carry = 0;
       for (int w = 0; w <= win; w++) d = next_digit(scal + (size_t)nw * i, nw, ws.start(w), ws.width(w), carry, neg);
     }
+    if (chk && d > B) { atomicOr(chk, CHK_BUCKET); d = 0; }
     if (d) b = d - 1;
     rank = atomicAdd(cnt + b, 1u);
   }
@@ -458,6 +460,7 @@ __global__ void __launch_bounds__(SMALL_T) k_sort_small(int n, const uint32_t* _
     if (win == (int)gridDim.x - 1) off[nseg] = gridDim.x * (uint32_t)n;
   }
   __syncthreads();
+  if (chk && i < n && cnt[b] + rank >= (uint32_t)n) { atomicOr(chk, CHK_ENTRY); return; }
   if (i < n) entries[(size_t)win * n + cnt[b] + rank] = b == B ? NULL_ENTRY : (uint32_t)i | (neg << 31);
 }
 
@@ -979,7 +982,7 @@ static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, uint32_t* ent, con
                                   const uint32_t* bases, cudaStream_t st, uint32_t* chk) {
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
   ZKB_TRY(launch("msm_tree_pad", k_tree_pad, dim3(sl.nseg / 256 + 1), dim3(256), 0, st, cnt, sl.off, sl.nseg, P.tree,
-                 ent, U32(P.o_toff), U32(P.o_cnt) + P.nseg + 1));
+                 ent, U32(P.o_toff), U32(P.o_cnt) + P.nseg + 1, chk, (uint32_t)P.total_pad));
   ZKB_TRY((launch_tree_level<C, true>(P, 0, st, ent, bases, sl, U32(P.o_tpre), U32(P.o_ttt), U32(P.o_tscr),
                                       U32(P.o_tpts[0]), chk, (uint32_t)P.n)));
   for (int l = 1; l < P.tree; l++)
@@ -1027,7 +1030,7 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
     ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt) + P.nseg, 0, (size_t)(2 + P.nwin) * 4, st));
     auto small = mont ? k_sort_small<C, true> : k_sort_small<C, false>;
     ZKB_TRY(launch("msm_sort_small", small, dim3(P.nwin), dim3(SMALL_T), 0, st, n, scal, P.nw, P.win,
-                   digit_bias(P.win, P.nwin), P.nseg, U32(P.o_off), U32(P.o_ent), U32(P.o_cnt) + P.nseg + 1));
+                   digit_bias(P.win, P.nwin), P.nseg, U32(P.o_off), U32(P.o_ent), U32(P.o_cnt) + P.nseg + 1, chk));
   } else {
     if (mont && !hist_mont) {
       ZKB_TRY(launch("msm_scalar_from_mont", k_msm_scalar_from_mont<C>, dim3((n + 255) / 256), dim3(256), 0, st,
@@ -1437,13 +1440,15 @@ int msm_bits_group(int nrows, double ncols) {
 // Few rows, or rows that are mostly ones, send many columns to one bucket, so the lanes of a warp with
 // the same pattern count it once.
 __global__ void k_bits_hist(int n, const uint8_t* __restrict__ coeffs, size_t ld, WinShape ws, int ngroups,
-                            uint32_t* __restrict__ cnt, uint32_t* __restrict__ dig, uint32_t* __restrict__ rank) {
+                            uint32_t* __restrict__ cnt, uint32_t* __restrict__ dig, uint32_t* __restrict__ rank,
+                            uint32_t* chk) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   for (int w = blockIdx.y; w < ngroups; w += gridDim.y) {
     const int rows = ws.width(w) - 1, r0 = ws.start(w) - w;   // the shape's windows are one bit wider
     uint32_t v = 0;
     if (i < n)
       for (int j = 0; j < rows; j++) v |= (__ldg(coeffs + (size_t)(r0 + j) * ld + i) ? 1u : 0u) << j;
+    if (chk && v >= ws.buckets(w)) { atomicOr(chk, CHK_BUCKET); v = 0; }
     const uint32_t same = __match_any_sync(0xffffffffu, v);
     const int leader = __ffs((int)same) - 1;
     uint32_t at = 0;
@@ -1555,7 +1560,7 @@ static zkg_status bits_launch(int nrows, int ncols, int rho, const uint8_t* coef
   const uint32_t blocks = 8 * (uint32_t)std::max(1, device_sm_count());
   const dim3 gh(gc.x, std::min<uint32_t>((uint32_t)P.ngroups, (blocks + gc.x - 1) / gc.x));
   ZKB_TRY(launch("bits_hist", k_bits_hist, gh, dim3(256), 0, st, ncols, coeffs, ld, P.win, P.ngroups, U32(P.o_cnt),
-                 U32(P.o_dig), U32(P.o_rank)));
+                 U32(P.o_dig), U32(P.o_rank), chk));
   ZKB_TRY(scan_counts(U32(P.o_cnt), U32(P.o_off), U32(P.o_cur), U32(P.o_bs), P.nseg, st));
   ZKB_TRY(launch("msm_scatter_d", k_msm_scatter_d, dim3(gc.x, P.ngroups), dim3(256), 0, st, ncols,
                  (const uint32_t*)U32(P.o_dig), (const uint32_t*)U32(P.o_rank), P.win, (const uint32_t*)U32(P.o_off),

@@ -45,10 +45,11 @@ __device__ __forceinline__ uint32_t tree_kind(const Fe<F>& x0, const Fe<F>& y0, 
 
 // For the nseg segments of a slab: pads every segment of cnt[s] entries at off[s] with null entries up to its
 // multiple of 2^T, writes the last list's offsets and adds the real entries up (*total, zeroed with the
-// counts).
+// counts). cap: entries there is room for (device checks).
 __global__ void __launch_bounds__(256) k_tree_pad(const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ off,
                                                   uint32_t nseg, int T, uint32_t* __restrict__ entries,
-                                                  uint32_t* __restrict__ last_off, uint32_t* __restrict__ total) {
+                                                  uint32_t* __restrict__ last_off, uint32_t* __restrict__ total,
+                                                  uint32_t* chk, uint32_t cap) {
   __shared__ uint32_t sum;
   if (threadIdx.x == 0) sum = 0;
   __syncthreads();
@@ -60,7 +61,10 @@ __global__ void __launch_bounds__(256) k_tree_pad(const uint32_t* __restrict__ c
     if (s < nseg) {
       c = cnt[s];
       const uint32_t m = (1u << T) - 1, end = (c + m) & ~m;
-      for (uint32_t i = c; i < end; i++) entries[lo + i] = NULL_ENTRY;
+      for (uint32_t i = c; i < end; i++) {
+        if (chk && lo + i >= cap) { atomicOr(chk, CHK_ENTRY); break; }
+        entries[lo + i] = NULL_ENTRY;
+      }
     }
   }
   c = __reduce_add_sync(0xffffffffu, c);
