@@ -160,14 +160,9 @@ template <int NL>
 inline void mul_adx(const Field<NL>&, const uint64_t*, const uint64_t*, uint64_t*) {}
 #endif
 
+// Out of line: inlined beside the form above it costs the host tail 2% (the smallest MSMs' 2 us).
 template <int NL>
-inline El<NL> mul(const Field<NL>& F, const El<NL>& a, const El<NL>& b) {
-  if (has_mulx_adx()) {
-    El<NL> r;
-    mul_adx(F, a.v, b.v, r.v);
-    reduce_once<NL>(F, r.v, 0);
-    return r;
-  }
+__attribute__((noinline)) El<NL> mul_portable(const Field<NL>& F, const El<NL>& a, const El<NL>& b) {
   uint64_t t[NL + 2] = {0};
   for (int i = 0; i < NL; i++) {
     u128 c = 0;
@@ -195,6 +190,16 @@ inline El<NL> mul(const Field<NL>& F, const El<NL>& a, const El<NL>& b) {
   std::memcpy(r.v, t, sizeof(r.v));
   reduce_once<NL>(F, r.v, t[NL]);
   return r;
+}
+template <int NL>
+inline El<NL> mul(const Field<NL>& F, const El<NL>& a, const El<NL>& b) {
+  if (has_mulx_adx()) {
+    El<NL> r;
+    mul_adx(F, a.v, b.v, r.v);
+    reduce_once<NL>(F, r.v, 0);
+    return r;
+  }
+  return mul_portable(F, a, b);
 }
 template <int NL>
 inline El<NL> one(const Field<NL>& F) {

@@ -945,17 +945,17 @@ struct TreeSlab {
   uint32_t nseg;
 };
 
-template <class C, bool L0, int PF>
+template <class C, TreeSrc SRC, int PF>
 static zkg_status launch_tree_bwd(const MsmPlan& P, int level, uint32_t nthr, cudaStream_t st, const uint32_t* ent,
                                   const uint32_t* in_pts, TreeSlab sl, const uint32_t* pre, const uint32_t* tinv,
                                   uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
   constexpr int NT = tree_nt<C>();
   const size_t smem = (size_t)PF * tree_bwd_pieces<typename C::Fp>() * NT * 16;
-  return launch("msm_tree_bwd", k_tree_bwd<C, L0, NT, PF>, dim3(nthr / NT), dim3(NT), smem, st, ent, in_pts, sl.off,
+  return launch("msm_tree_bwd", k_tree_bwd<C, SRC, NT, PF>, dim3(nthr / NT), dim3(NT), smem, st, ent, in_pts, sl.off,
                 sl.nseg, level, tree_wave<C>(), P.tB, pre, tinv, out_pts, level == P.tree - 1 ? 1 : 0, chk, npts);
 }
 
-template <class C, bool L0>
+template <class C, TreeSrc SRC>
 static zkg_status launch_tree_level(const MsmPlan& P, int level, cudaStream_t st, const uint32_t* ent,
                                     const uint32_t* in_pts, TreeSlab sl, uint32_t* pre, uint32_t* tt, uint32_t* scr,
                                     uint32_t* out_pts, uint32_t* chk, uint32_t npts) {
@@ -963,14 +963,14 @@ static zkg_status launch_tree_level(const MsmPlan& P, int level, cudaStream_t st
   constexpr int NT = tree_nt<C>(), PFF = 3;
   const uint32_t nthr = tree_threads<C>(P, level);
   const size_t smf = (size_t)PFF * tree_fwd_pieces<F>() * NT * 16;
-  ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, L0, NT, PFF>, dim3(nthr / NT), dim3(NT), smf, st, ent, in_pts, sl.off,
+  ZKB_TRY(launch("msm_tree_fwd", k_tree_fwd<C, SRC, NT, PFF>, dim3(nthr / NT), dim3(NT), smf, st, ent, in_pts, sl.off,
                  sl.nseg, level, tree_wave<C>(), P.tB, pre, tt, chk, npts));
   // simultaneous inversion of the thread products: about 4 per thread
   const size_t T = std::min<size_t>(((size_t)nthr + 255) & ~size_t(255), std::max<size_t>(2048, (size_t)nthr / 4));
   ZKB_TRY(launch("msm_tree_inv", k_tree_inv<F>, dim3((unsigned)((T + 255) / 256)), dim3(256), 0, st, nthr, tt, scr));
-  if (g_tree_pf >= 3)
-    return launch_tree_bwd<C, L0, 3>(P, level, nthr, st, ent, in_pts, sl, pre, tt, out_pts, chk, npts);
-  return launch_tree_bwd<C, L0, 2>(P, level, nthr, st, ent, in_pts, sl, pre, tt, out_pts, chk, npts);
+  if (g_tree_pf >= 3 && SRC != SRC_SLAB)
+    return launch_tree_bwd<C, SRC == SRC_SLAB ? SRC_ENTRIES : SRC, 3>(P, level, nthr, st, ent, in_pts, sl, pre, tt, out_pts, chk, npts);
+  return launch_tree_bwd<C, SRC, 2>(P, level, nthr, st, ent, in_pts, sl, pre, tt, out_pts, chk, npts);
 }
 
 // The affine tree levels of one slab of windows of one point range (zkb_msm_tree.cuh), after the sort has
@@ -983,10 +983,11 @@ static zkg_status msm_tree_launch(const MsmPlan& P, char* ws, uint32_t* ent, con
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
   ZKB_TRY(launch("msm_tree_pad", k_tree_pad, dim3(sl.nseg / 256 + 1), dim3(256), 0, st, cnt, sl.off, sl.nseg, P.tree,
                  ent, U32(P.o_toff), U32(P.o_cnt) + P.nseg + 1, chk, (uint32_t)P.total_pad));
-  ZKB_TRY((launch_tree_level<C, true>(P, 0, st, ent, bases, sl, U32(P.o_tpre), U32(P.o_ttt), U32(P.o_tscr),
-                                      U32(P.o_tpts[0]), chk, (uint32_t)P.n)));
+  const auto level0 = P.slabs > 1 ? launch_tree_level<C, SRC_SLAB> : launch_tree_level<C, SRC_ENTRIES>;
+  ZKB_TRY(level0(P, 0, st, ent, bases, sl, U32(P.o_tpre), U32(P.o_ttt), U32(P.o_tscr), U32(P.o_tpts[0]), chk,
+                 (uint32_t)P.n));
   for (int l = 1; l < P.tree; l++)
-    ZKB_TRY((launch_tree_level<C, false>(P, l, st, nullptr, U32(P.o_tpts[(l - 1) & 1]), sl, U32(P.o_tpre),
+    ZKB_TRY((launch_tree_level<C, SRC_LIST>(P, l, st, nullptr, U32(P.o_tpts[(l - 1) & 1]), sl, U32(P.o_tpre),
                                          U32(P.o_ttt), U32(P.o_tscr), U32(P.o_tpts[l & 1]), nullptr, 0)));
   return ZKG_OK;
 }
@@ -1480,7 +1481,7 @@ __global__ void __launch_bounds__(256) k_bits_rows(WinShape ws, const uint32_t* 
     const uint32_t s = s0 + (((j >> k) << (k + 1)) | (1u << k) | (j & ((1u << k) - 1)));
     return j < cnt && __ldg(off + s) != __ldg(off + s + 1) ? quad_load<F>(bsum + (size_t)s * XW) : fe_zero<F>();
   };
-  Fe<F> a = add && quad == 0 ? quad_load<F>(out + (size_t)r * XW) : fe_zero<F>(), nx = item(quad);
+  Fe<F> a = fe_zero<F>(), nx = item(quad);
 #pragma unroll 1
   for (uint32_t j0 = 0; j0 < cnt; j0 += quads) {
     const Fe<F> x = nx;
@@ -1494,6 +1495,7 @@ __global__ void __launch_bounds__(256) k_bits_rows(WinShape ws, const uint32_t* 
     if (threadIdx.x >= 32) return;
     a = quad_warp_sum(quad < quads >> 3 ? quad_load<F>(sm + quad * XW) : fe_zero<F>());
   }
+  if (add) a = quad_add(a, quad_load<F>(out + (size_t)r * XW));
   if (threadIdx.x < 4) quad_store(out + (size_t)r * XW, fe_canon(a));
 }
 
@@ -1556,8 +1558,8 @@ static zkg_status bits_launch(int nrows, int ncols, int rho, const uint8_t* coef
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
   ZKB_CUDA(cudaMemsetAsync(U32(P.o_cnt), 0, (size_t)P.nseg * 4 + 4, st));
   const dim3 gc((ncols + 255) / 256);
-  // few columns: the groups in parallel too, up to eight blocks an SM
-  const uint32_t blocks = 8 * (uint32_t)std::max(1, device_sm_count());
+  // few columns: the groups in parallel too, up to four blocks an SM
+  const uint32_t blocks = 4 * (uint32_t)std::max(1, device_sm_count());
   const dim3 gh(gc.x, std::min<uint32_t>((uint32_t)P.ngroups, (blocks + gc.x - 1) / gc.x));
   ZKB_TRY(launch("bits_hist", k_bits_hist, gh, dim3(256), 0, st, ncols, coeffs, ld, P.win, P.ngroups, U32(P.o_cnt),
                  U32(P.o_dig), U32(P.o_rank), chk));

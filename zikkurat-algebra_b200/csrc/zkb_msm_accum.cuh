@@ -22,24 +22,22 @@ __device__ __forceinline__ uint32_t find_seg(const uint32_t* __restrict__ off, u
 }
 
 // Chunk length for the entries that were counted, in a launch of nchunks chunks planned with length L for
-// the most there can be: the same chunks, shorter, down to 8 entries. With small or mostly zero scalars a
-// few percent of the entries exist, and chunks of the planned 120 left most threads without one (2^22
-// points of BN254 with 16-bit scalars: 3.04 -> 1.84 ms). Every kernel that works on the chunks takes its length
-// from here.
+// the most there can be: with less than three quarters of them the same chunks, shorter, down to 8 entries.
+// With small or mostly zero scalars a few percent of the entries exist, and chunks of the planned 120 left
+// most threads without one (2^22 points of BN254 with 16-bit scalars: 3.04 -> 1.84 ms). Every kernel that
+// works on the chunks takes its length from here.
 __device__ __forceinline__ uint32_t counted_len(uint32_t total, uint32_t nchunks, uint32_t L) {
+  if (L <= 8 || (uint64_t)total * 4 >= (uint64_t)nchunks * L * 3) return L;
   return min(L, max(8u, (total + nchunks - 1) / nchunks));
 }
 
-// Route a finished run of segment s inside chunk [start, start+L): the whole segment goes to
-// the bucket array, a cut one to this chunk's slot A (segment began before the chunk) or
-// slot B (segment continues after it).
+// Route a finished run of segment s inside a chunk: the whole segment goes to the bucket array, a cut
+// one to this chunk's slot A (segment began before the chunk) or slot B (segment continues after it).
 template <class F>
-__device__ __forceinline__ void route_run(uint32_t s, const Xyzz<F>& acc, uint64_t seg_lo, uint64_t seg_hi,
-                                          uint64_t start, uint64_t L, uint32_t t, uint32_t* __restrict__ bsum,
+__device__ __forceinline__ void route_run(uint32_t s, const Xyzz<F>& acc, bool before, bool after, uint32_t t,
+                                          uint32_t* __restrict__ bsum,
                                           uint32_t* __restrict__ spt, uint32_t& keyA, uint32_t& keyB) {
   constexpr int XW = 4 * F::N;
-  const bool before = seg_lo < start;
-  const bool after = seg_hi > start + L;
   if (!before && !after) {
     xyzz_store<F>(bsum + (size_t)s * XW, acc);
   } else if (before) {
@@ -72,8 +70,6 @@ __device__ __forceinline__ void accum_block(uint32_t blk, const uint32_t* __rest
   const uint32_t t = blk * NT + threadIdx.x;
   if (t >= nchunks) return;
   const uint32_t total = __ldg(off + nseg);
-  L = counted_len(total, nchunks, L);
-  const uint32_t start = t * L;
   uint32_t keyA = INVALID, keyB = INVALID;
   auto ent_at = [&](uint32_t pos) -> uint32_t { return entries ? __ldg(entries + pos) : pos; };
   // point index of an entry; with device checks on, an index outside the base set is recorded and
@@ -92,10 +88,14 @@ __device__ __forceinline__ void accum_block(uint32_t blk, const uint32_t* __rest
     for (int q = 0; q < Q; q++) cp_async16(&pf[(stage * Q + q) * NT + threadIdx.x], src + q);
     cp_async_commit();
   };
+  // The planned length's segment is searched while the total is on its way.
+  uint32_t s = find_seg(off, nseg, t * L);
+  const uint32_t len = counted_len(total, nchunks, L), start = t * len;
+  if (len != L) s = find_seg(off, nseg, start);
   if (start < total) {
-    const uint32_t end = min(start + L, total);
-    uint32_t s = find_seg(off, nseg, start);
-    uint32_t seg_lo = __ldg(off + s), seg_hi = __ldg(off + s + 1);
+    const uint32_t end = min(start + len, total);
+    uint32_t seg_hi = __ldg(off + s + 1);
+    bool cut = __ldg(off + s) < start;   // the run's segment began before the chunk
     Xyzz<F> acc = xyzz_inf<F>();
     bool have = false;
     uint32_t e = ent_at(start);
@@ -103,33 +103,32 @@ __device__ __forceinline__ void accum_block(uint32_t blk, const uint32_t* __rest
     if constexpr (PF > 0) {
 #pragma unroll
       for (int k = 0; k < PF - 1; k++)
-        if (start + k < end) issue(ent_at(start + k), k);
+        if (start + k < end) issue(ent_at(start + k), (start + k) % PF);
     } else {
       nxt = affine_load<F>(bases + (size_t)pidx(e) * AW);
     }
     for (uint32_t pos = start; pos < end; pos++) {
       while (pos >= seg_hi) {
-        if (have) route_run<F>(s, acc, seg_lo, seg_hi, start, L, t, bsum, spt, keyA, keyB);
+        if (have) route_run<F>(s, acc, cut, seg_hi > end, t, bsum, spt, keyA, keyB);
         have = false;
         acc = xyzz_inf<F>();
         s++;
-        seg_lo = seg_hi;
+        cut = false;
         seg_hi = __ldg(off + s + 1);
       }
       Affine<F> a;
       uint32_t neg;
       if constexpr (PF > 0) {
-        const uint32_t i = pos - start;
-        if (i > 0) e = ent_at(pos);
+        e = ent_at(pos);
         neg = e >> 31;
         // start the copy PF - 1 bases ahead, then wait for this base's copy (groups issued after
         // it may stay in flight)
-        if (pos + PF - 1 < end) issue(ent_at(pos + PF - 1), (i + PF - 1) % PF);
+        if (pos + PF - 1 < end) issue(ent_at(pos + PF - 1), (pos + PF - 1) % PF);
         const uint32_t later = min((uint32_t)(PF - 1), end - 1 - pos);
         if (PF > 2 && later >= 2) cp_async_wait<(PF > 2 ? 2 : 0)>();
         else if (later >= 1) cp_async_wait<1>();
         else cp_async_wait<0>();
-        const uint32_t stage = i % PF;
+        const uint32_t stage = pos % PF;
         uint32_t w[AW];
 #pragma unroll
         for (int q = 0; q < Q; q++) {
@@ -154,7 +153,7 @@ __device__ __forceinline__ void accum_block(uint32_t blk, const uint32_t* __rest
       }
       have = true;
     }
-    if (have) route_run<F>(s, acc, seg_lo, seg_hi, start, L, t, bsum, spt, keyA, keyB);
+    if (have) route_run<F>(s, acc, cut, seg_hi > end, t, bsum, spt, keyA, keyB);
   }
   skey[2 * t] = keyA;
   skey[2 * t + 1] = keyB;

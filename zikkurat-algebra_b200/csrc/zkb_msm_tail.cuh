@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(128) k_quad_accum(const uint32_t* __restrict__
   Fe<F> a = fe_zero<F>(), q = point(start);
   // the finished run of segment s: the whole segment to its bucket, a cut one to this chunk's slots
   auto flush = [&] {
-    const bool before = seg_lo < start, after = seg_hi > start + L;
+    const bool before = seg_lo < start, after = seg_hi > end;
     if (before) keyA = s; else if (after) keyB = s;
     quad_store(!before && !after ? bsum + (size_t)s * XW : spt + (size_t)(2 * t + (before ? 0 : 1)) * XW, a);
   };
@@ -240,9 +240,10 @@ __global__ void __launch_bounds__(128) k_cut_merge(const uint32_t* __restrict__ 
   constexpr int XW = 4 * F::N;
   const uint32_t t = (blockIdx.x * 128 + threadIdx.x) >> 2;
   uint32_t s = INVALID, more = 0;   // partial sums after the first
-  L = counted_len(__ldg(off + nseg), nchunks, L);
   if (t + 1 < nchunks) {
+    const uint32_t total = __ldg(off + nseg);
     s = __ldg(skey + 2 * (size_t)t + 1);
+    L = counted_len(total, nchunks, L);
     if (chk && s != INVALID && s >= nseg) { atomicOr(chk, CHK_SEGMENT); s = INVALID; }
     if (s != INVALID) {
       more = (__ldg(off + s + 1) - 1) / L - t;

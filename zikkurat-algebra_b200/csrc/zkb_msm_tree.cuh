@@ -150,6 +150,10 @@ __host__ __device__ inline uint32_t tree_slots(uint32_t Q, uint32_t wave, uint32
   return (uint32_t)((Q + t - 1) / t);
 }
 
+// What a level reads: the list of the level before, or the entries from the first one on, or those of a slab
+// of windows further on, from off[0] (a form of its own: a pointer that is not a kernel argument cost
+// BLS12-381's backward pass spills and 5%).
+enum TreeSrc : int { SRC_LIST = 0, SRC_ENTRIES = 1, SRC_SLAB = 2 };
 // The levels run over the entries [off[0], off[nseg]) of one slab of windows: level l has half of them >> l
 // slots, numbered from 0.
 __device__ __forceinline__ uint32_t tree_level_slots(const uint32_t* __restrict__ off, uint32_t nseg, int level) {
@@ -160,16 +164,17 @@ __device__ __forceinline__ uint32_t tree_level_slots(const uint32_t* __restrict_
 // denominators of the thread's addition slots before q (stored for addition slots with k > 0);
 // tt[thread] = product of all of them (1 when none). The inputs' x coordinates arrive through PF
 // cp.async stages, PF - 1 slots ahead, their entries one slot earlier still.
-template <class C, bool L0, int NT, int PF>
+template <class C, TreeSrc SRC, int NT, int PF>
 __global__ void __launch_bounds__(NT) k_tree_fwd(const uint32_t* __restrict__ ent, const uint32_t* __restrict__ pts,
                                                  const uint32_t* __restrict__ off, uint32_t nseg, int level, uint32_t wave,
                                                  uint32_t tB, uint32_t* __restrict__ pre, uint32_t* __restrict__ tt,
                                                  uint32_t* chk, uint32_t npts) {
   using F = typename C::Fp;
+  constexpr bool L0 = SRC != SRC_LIST;
   constexpr int FW = F::N, QF = F::N / 4, QS = tree_fwd_pieces<F>();
   extern __shared__ uint4 tsm[];
   const uint32_t Q = tree_level_slots(off, nseg, level), B = tree_slots(Q, wave, tB);
-  if constexpr (L0) ent += __ldg(off);
+  if constexpr (SRC == SRC_SLAB) ent += __ldg(off);
   const uint32_t base = blockIdx.x * NT * B + threadIdx.x;
   const uint32_t n = base < Q ? min(B, (Q - base + NT - 1) / NT) : 0;   // slots of this thread
   Fe<F> acc = fe_one<F>();
@@ -249,17 +254,18 @@ __global__ void __launch_bounds__(256) k_tree_inv(uint32_t n, uint32_t* __restri
 // denominators not yet peeled off, so a slot's inverse is acc * pre[q] and the next acc is
 // acc * den. Every slot's sum is written, canonical, to out. A slot's inputs and running product
 // arrive through PF cp.async stages, PF - 1 slots ahead.
-template <class C, bool L0, int NT, int PF>
+template <class C, TreeSrc SRC, int NT, int PF>
 __global__ void __launch_bounds__(NT, 1) k_tree_bwd(const uint32_t* __restrict__ ent, const uint32_t* __restrict__ pts,
                                                     const uint32_t* __restrict__ off, uint32_t nseg, int level, uint32_t wave,
                                                     uint32_t tB, const uint32_t* __restrict__ pre,
                                                     const uint32_t* __restrict__ tinv, uint32_t* __restrict__ out, int last,
                                                     uint32_t* chk, uint32_t npts) {
   using F = typename C::Fp;
+  constexpr bool L0 = SRC != SRC_LIST;
   constexpr int FW = F::N, AW = 2 * F::N, QF = F::N / 4, QA = 2 * QF, QS = tree_bwd_pieces<F>();
   extern __shared__ uint4 tsm[];
   const uint32_t Q = tree_level_slots(off, nseg, level), B = tree_slots(Q, wave, tB);
-  if constexpr (L0) ent += __ldg(off);
+  if constexpr (SRC == SRC_SLAB) ent += __ldg(off);
   const uint32_t base = blockIdx.x * NT * B + threadIdx.x;
   if (base >= Q) return;
   const int n = (int)min(B, (Q - base + NT - 1) / NT);
