@@ -2267,8 +2267,9 @@ struct Srv {
   uint64_t next_ticket = 1, completed = 0;
   int inflight = 0, max_inflight = 0;
   zkg_status error = ZKG_OK;
-  std::vector<size_t> req_bytes;   // device bytes of one request, by k
-  std::vector<MsmPlan> req_plan;   // its MSM plan, by k
+  std::vector<size_t> req_bytes, tree_bytes;     // device bytes of one request by k, without and with the affine
+  std::vector<MsmPlan> req_plan, tree_plan;      // tree (0: the rules pick none), and its MSM plans
+  size_t max_bytes = 0;                          // of req_bytes
   long inject_fail_at = -1;        // host-side failure injection: admission number that fails
   long inject_stall_at = -1;       // testing: admission whose NTT passes give up at their first wait
   long admissions = 0;
@@ -2311,16 +2312,32 @@ static void srv_free(Srv& S, size_t off, size_t bytes) {
 
 static inline size_t rup256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// A request's MSM plan with at most tree_max affine tree levels, and its device bytes.
 template <class C>
-static size_t srv_bytes(int k, size_t budget, int nslots, MsmPlan& P) {
-  for (const int tree_max : {MAX_TREE, 0}) {
-    if (make_plan<C>(1 << k, 4, 1, P, 0, tree_max) != ZKG_OK) return (size_t)-1;
-    const size_t b = 3 * rup256(((size_t)32) << k) + rup256(P.bytes);
-    // the tree's lists only where every slot may have them: they are four times the rest, and requests
-    // beside each other gain more than one alone
-    if (P.tree == 0 || b <= budget / nslots) return b;
+static zkg_status srv_plan(int k, int tree_max, MsmPlan& P, size_t& bytes) {
+  ZKB_TRY(make_plan<C>(1 << k, 4, 1, P, 0, tree_max));
+  bytes = 3 * rup256(((size_t)32) << k) + rup256(P.bytes);
+  return ZKG_OK;
+}
+
+// Pool memory for a request of size 2^k and the plan that it runs by; (size_t)-1 if there is none. The
+// tree's lists are four times the rest of a workspace, so they are taken only while every other free slot
+// could still run a request of any size without them: no request waits for another one's tree.
+static size_t srv_admit(Srv& S, int k, const MsmPlan*& P, size_t& bytes) {
+  size_t others = 0;
+  for (auto& sl : S.slots) others += sl.busy ? 0 : 1;
+  const size_t with_tree = S.tree_bytes[k];
+  if (with_tree && S.budget - S.used >= with_tree + (others - 1) * S.max_bytes) {
+    const size_t off = srv_alloc(S, with_tree);
+    if (off != (size_t)-1) {
+      P = &S.tree_plan[k];
+      bytes = with_tree;
+      return off;
+    }
   }
-  return (size_t)-1;
+  P = &S.req_plan[k];
+  bytes = S.req_bytes[k];
+  return srv_alloc(S, bytes);
 }
 
 template <class C, int NL>
@@ -2427,9 +2444,10 @@ static void srv_loop(Srv* S, const host::Field<NL>* F) {
         if (!sl.busy) { free_slot = &sl; break; }
       if (!free_slot) break;
       const bool head_only = S->pending.front().overtaken >= SRV_MAX_OVERTAKE;
-      size_t pick = (size_t)-1, off = (size_t)-1;
+      size_t pick = (size_t)-1, off = (size_t)-1, bytes = 0;
+      const MsmPlan* plan = nullptr;
       for (size_t q = 0; q < S->pending.size() && (q == 0 || !head_only); q++) {
-        off = srv_alloc(*S, S->req_bytes[S->pending[q].k]);
+        off = srv_admit(*S, S->pending[q].k, plan, bytes);
         if (off != (size_t)-1) { pick = q; break; }
       }
       if (pick == (size_t)-1) break;
@@ -2437,9 +2455,9 @@ static void srv_loop(Srv* S, const host::Field<NL>* F) {
       const int k = S->pending[pick].k;
       free_slot->req = S->pending[pick];
       S->pending.erase(S->pending.begin() + (long)pick);
-      free_slot->P = S->req_plan[k];
+      free_slot->P = *plan;
       free_slot->off = off;
-      free_slot->bytes = S->req_bytes[k];
+      free_slot->bytes = bytes;
       free_slot->busy = true;
       S->inflight++;
       S->max_inflight = std::max(S->max_inflight, S->inflight);
@@ -2506,18 +2524,20 @@ static zkg_status srv_start(Srv* S, const host::Field<NL>* F, const host::Field<
   // plans and device bytes of every request size, once; every admissible request must fit in
   // the budget on its own
   S->req_bytes.assign(kmax + 1, (size_t)-1);
+  S->tree_bytes.assign(kmax + 1, 0);
   S->req_plan.assign(kmax + 1, MsmPlan());
+  S->tree_plan.assign(kmax + 1, MsmPlan());
   size_t ubytes_max = 64;
   using CP = typename MsmCurve<C>::type;
+  const auto plan = g_msm_dpf ? srv_plan<CP> : srv_plan<C>;
   for (int k = kmin; k <= kmax; k++) {
-    MsmPlan P;
-    const size_t b = g_msm_dpf ? srv_bytes<CP>(k, S->budget, nslots, P)
-                               : srv_bytes<C>(k, S->budget, nslots, P);
-    if (b == (size_t)-1 || b > S->budget)
+    const zkg_status st = plan(k, 0, S->req_plan[k], S->req_bytes[k]);
+    if (st != ZKG_OK || S->req_bytes[k] > S->budget)
       return set_status(ZKG_ERR_ARG, "zkg_server_create", "HBM budget smaller than one request of the largest size");
-    S->req_bytes[k] = b;
-    S->req_plan[k] = P;
-    ubytes_max = std::max(ubytes_max, (size_t)P.nwin * 4 * NL * 8);
+    ZKB_TRY(plan(k, MAX_TREE, S->tree_plan[k], S->tree_bytes[k]));
+    if (S->tree_plan[k].tree == 0) S->tree_bytes[k] = 0;
+    S->max_bytes = std::max(S->max_bytes, S->req_bytes[k]);
+    ubytes_max = std::max(ubytes_max, (size_t)S->req_plan[k].nwin * 4 * NL * 8);
   }
   ZKB_CUDA(cudaMalloc(&S->pool, S->budget));
   S->free_list[0] = S->budget;
