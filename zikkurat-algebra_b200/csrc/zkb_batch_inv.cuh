@@ -6,7 +6,8 @@
 
 namespace zkb {
 
-// The inverse of every thread's v (none zero) with one inversion per block of NW warps: products up a
+// The inverse of every thread's v with one inversion per block of NW warps (one zero among them makes every
+// result of the block zero, as the inverse of zero is; the Fr operations' flag covers the other blocks): products up a
 // binary tree (butterfly shuffles in the warp, then the warps' products in warp 0), the inversion of the
 // total by warp 0's lanes alike, and down again, a child's inverse being its parent's times its
 // sibling's product: 2 (5 + log2 NW) products in a row. (Two exclusive scans took 30.) sw: 2 NW elements;

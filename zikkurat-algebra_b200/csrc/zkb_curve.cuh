@@ -145,14 +145,6 @@ __device__ __forceinline__ void xyzz_add(Xyzz<F>& acc, const Xyzz<F>& q) {
   acc.Y = Y3;
 }
 
-// canonical coordinates (values in [0, p)) of a point whose field keeps a redundant range
-template <class F>
-__device__ __forceinline__ Xyzz<F> xyzz_canon(const Xyzz<F>& p) {
-  Xyzz<F> r;
-  r.X = fe_canon(p.X); r.Y = fe_canon(p.Y); r.ZZ = fe_canon(p.ZZ); r.ZZZ = fe_canon(p.ZZZ);
-  return r;
-}
-
 // acc += q with the independent products in pairs (one call computes two, interleaving their
 // reduction chains): the MSM's bucket merge and reduction kernels, whose short sequential chains
 // of additions run at low occupancy, where the halved dependency depth pays

@@ -344,8 +344,10 @@ __device__ __forceinline__ Fe<P> fe_pow(const Fe<P>& a, const uint32_t (&e)[EW])
 
 // Inverse of the integer a (0 < a < 2p, prime to p) modulo p, in words, for one thread that others wait
 // for: Bernstein and Yang's division steps ("Fast constant-time gcd computation and modular inversion",
-// 2019) in variable time, 30 at a time. The steps of one batch see only the low words of f and g and
-// give a matrix (u v; q r) with entries up to 2^30; then
+// 2019), 30 at a time, in the variable-time form that libsecp256k1 gave them (modinv: trailing zeros of g
+// counted at once, eta for -delta, and up to six low bits of g cancelled together by way of f (2 - f f), the
+// inverse of f modulo 2^6; the update of d and e is this file's own). The steps of one batch see only the
+// low words of f and g and give a matrix (u v; q r) with entries up to 2^30; then
 //     f, g <- (u f + v g) / 2^30, (q f + r g) / 2^30            exactly, two's complement
 //     d, e <- (u d + v e) / 2^30, (q d + r e) / 2^30   mod p    in [0, p), by a Montgomery step
 // keep d a = f and e a = g (mod p) from f = p, g = a, d = 0, e = 1 until g = 0, f = +-1. At most

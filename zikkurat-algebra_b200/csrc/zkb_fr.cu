@@ -10,8 +10,8 @@
 //   - mul_by_powers: the reference loop starts at i = 1 with x = A, so tgt[0] is left unwritten
 //     and tgt[i] = src[i] * A * B^(i-1) for i >= 1 (bn128_arr_mont.c:203-211); kept as is;
 //   - batch inversion: Montgomery's trick over the strided subset i = t, t + T, ... of each
-//     thread, the thread products combined across the block by two scans, one inversion (division
-//     steps) per block. The reference multiplies all n elements into one
+//     thread, the thread products combined across the block by a binary tree, one inversion
+//     (division steps) per block. The reference multiplies all n elements into one
 //     product and inverts it, so one zero element makes every output zero; a device flag
 //     reproduces that;
 //   - dot product: block partial sums, then one block sums the partials (modular sums are exact

@@ -37,14 +37,6 @@ inline bool is_zero(const El<NL>& a) {
   return x == 0;
 }
 template <int NL>
-inline bool ge_p(const Field<NL>& F, const uint64_t* a) {
-  for (int i = NL - 1; i >= 0; i--) {
-    if (a[i] > F.p[i]) return true;
-    if (a[i] < F.p[i]) return false;
-  }
-  return true;
-}
-template <int NL>
 inline uint64_t sub_raw(const uint64_t* a, const uint64_t* b, uint64_t* o) {
   uint64_t br = 0;
   for (int i = 0; i < NL; i++) {

@@ -21,8 +21,8 @@
 //                    (zkb_dpf.cuh). Complete segments go straight to the bucket array;
 //                    segments cut by a chunk boundary leave partial sums in slots.
 //   6. merge         a segment cut by chunk boundaries is summed from its slots (zkb_msm_tail.cuh);
-//                    a long one (any digit distribution) in pieces, a block a piece. MSMs of few
-//                    entries skip chunks altogether: four lanes sum one segment
+//                    a long one (any digit distribution) in pieces, a block a piece. In MSMs of
+//                    few entries four lanes take a chunk
 //   7. bucket reduce (the point-range parts of a host-buffer MSM summed first, in one parallel
 //                    pass) per (window, group of K buckets) running sums (T_g, R_g), then per
 //                    window sum_b b*S_b = sum R_g + K * sum_k 2^k sum_{g: bit k of g} T_g
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(NT, 1) k_msm_accum_w(const uint32_t* __restric
 // With BN254D / BLS12_381D (the curves over BnFpD / BlsFpD of zkb_dpf.cuh) the bucket pipeline
 // (accumulation, folds, bucket reduction) runs unchanged but with FP64-pipe products, on values
 // in the radix R' = 2^(52 L). Bases enter that radix once per MSM (x R -> mont'(x R, R'^2 / R)
-// = x R'); the per-window sums U leave it once (x R' -> mont'(x R', R) = x R), so the host tail
+// = x R'); the window values V leave it once (x R' -> mont'(x R', R) = x R), so the host tail
 // and the output encodings are unchanged. Both conversions are exact field products.
 // affine points, radix R -> R' (the identity (0, 0) stays (0, 0))
 template <class CD>
@@ -549,7 +549,7 @@ __global__ void k_msm_merge_parts(PartSet parts, uint32_t nseg, uint32_t* __rest
 // ---------------------------------------------------------------------------- planning
 
 static int g_window_override = 0;
-// tuning knobs (ZKB_MSM_L1: level-1 chunk length, entries per accumulation thread; ZKB_MSM_K1: buckets per
+// tuning knobs (ZKB_MSM_L1: chunk length, entries per accumulation thread; ZKB_MSM_K1: buckets per
 // running-sum group, a power of two); read once from the environment
 static int env_int(const char* name, int dflt) {
   const char* v = std::getenv(name);
@@ -571,7 +571,7 @@ static int g_msm_digits = env_int("ZKB_MSM_DIGITS", 1);
 static const bool g_msm_pf_env = std::getenv("ZKB_MSM_PF") != nullptr;
 
 // Tuned settings per curve and round(log2 n), from zkg_autotune_msm or the persisted tuning
-// cache: window width, level-1 chunk length, running-sum group size, prefetch stages (0 / -1 =
+// cache: window width, chunk length, running-sum group size, prefetch stages (0 / -1 =
 // the default rule). An environment knob, when set, wins over a tuned value.
 struct MsmTune {
   int c = 0, L1 = 0, K1 = 0, pf = -1;
@@ -619,8 +619,11 @@ static int ilog2_floor(uint64_t x) {
 // running-sum additions weigh more where the bucket kernels are latency-bound (n from 2^17 on) and
 // more again once the affine tree makes an entry cheaper (from 2^19 on). Best measured c / picked,
 // BN254: 2^16 12 or 13 / 13, 2^17 13 / 13, 2^18 13 / 13, 2^19 14 / 14, 2^20 15 / 15, 2^21 15 / 15,
-// 2^22 15 or 16 / 16; BLS12-381: 2^17 13 / 13, 2^18 13 / 13, 2^19 15 / 15, 1000003 14 / 14, 2^21
-// 15 / 15, 2^22 16 / 16 (2^22 with the weight of small n: c = 18, 31.6 ms against 27.0).
+// 2^22 15 or 16 / 16; BLS12-381: 2^17 13 / 13, 2^18 13 / 13, 2^19 15 / 15, 2^21 15 / 15, 2^22 16 / 16
+// (2^22 with the weight of small n: c = 18, 31.6 ms against 27.0). Between, BLS12-381 in us with c = 13 /
+// 14 / 15: 600000 4654 / 4630 / 4880 (picked 15), 700000 5321 / 5261 / 5394 (15), 800000 5811 / 5848 /
+// 5949 (14), 900000 6434 / 6446 / 6527 (14), 1000003 6999 / 7062 / 7061 (14), 2^20 7315 / 7342 / 7327
+// (15), 1.2 M 8321 / 8342 / 8257 (15): within 1% of the best from 800,000 on, 2 to 5% off below.
 static double bucket_weight(int curve, int n) {
   const bool bls = curve == ZKG_BLS12_381;
   if (n < (1 << 17)) return bls ? 3.5 : 2.8;
@@ -1023,7 +1026,7 @@ static zkg_status msm_launch_part(Context& cx, const MsmPlan& P, char* ws, const
   uint32_t* chk = dev_check_word(cx);
   const int n = P.n;
   auto U32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
-  // phase events: 0 start, 1 sorted, 2 level-1 accumulated, 3 levels folded, 4 reduced
+  // phase events: 0 start, 1 sorted, 2 accumulated, 3 cut segments merged, 4 reduced
   if (first) ZKB_CUDA(cudaEventRecord(cx.ev_phase[0], st));
   const uint32_t* scal = reinterpret_cast<const uint32_t*>(d_scal);
   const bool hist_mont = mont && P.use_dig;   // conversion inside the histogram
@@ -1304,8 +1307,10 @@ static zkg_status msm_host_run(const host::Field<NL>& F, int n, const uint64_t* 
   for (int k = 0; k < ntev; k++) ZKB_CUDA(cudaEventCreate(&tev[k]));
   if (ntev) ZKB_CUDA(cudaEventRecord(tev[0], st));
   // per part: scalars, then bases, then the part's launches; a part's sort waits only for its
-  // scalars, its accumulation for its bases, so the sort runs while the bases are still in
-  // flight, and staging the next part's pageable host data overlaps this part's compute
+  // scalars, its accumulation for its bases, so from page-locked arrays the sort runs while the bases are
+  // still in flight. Pageable arrays are staged before the part's launches, each up to 32 MB as a whole, so
+  // there only the next part's staging overlaps this part's compute, and one part (below 2^19 points) runs
+  // copy, sort and accumulation one after another.
   for (int q = 0; q < nparts; q++) {
     const size_t first = (size_t)pstart[q], nq = P[q].n;
     ZKB_TRY(copy_h2d(cx, base + off_s[q], expos + first * nlimbs, nq * nlimbs * 8, cx.copy_stream));
@@ -2049,7 +2054,7 @@ static zkg_status batch_build_persistent(zkg_batch* b, const host::Field<NL>& F)
                        reinterpret_cast<uint32_t*>(ws + b->conv_off)));
       ZKB_TRY(multi_msm_launch<CD>(b->mp, ws, msm_bases, st, 1));
     }
-    // level-1 slot keys start as "unused": if a run stops early (a wait ran out), the merge and
+    // the chunks' slot keys start as "unused": if a run stops early (a wait ran out), the merge and
     // fold kernels after it then find no slot of an accumulation block that never ran
     if (!b->mp.reqs.empty()) ZKB_CUDA(cudaMemsetAsync(W.key, 0xff, (size_t)2 * W.nch * 4, st));
     if (b->work_tasks)
@@ -2578,7 +2583,7 @@ __global__ void k_rand_scalars(uint64_t* out, uint32_t n, uint64_t seed) {
 
 // Tunes the MSM for n = 2^L, L in [lmin, lmax], on device-resident bases and random scalars:
 // window width first (around the cost model's choice, other settings at their defaults), then
-// with that width the level-1 chunk length, the running-sum group size and the prefetch stages,
+// with that width the chunk length, the running-sum group size and the prefetch stages,
 // one at a time (coordinate search). Each setting is timed as the best of two calls after a
 // warm-up call. The winners become that size's settings (and are persisted when ZKG_TUNE_CACHE
 // is set). Results never depend on them: only the order of exact operations changes.

@@ -268,7 +268,8 @@ __global__ void __launch_bounds__(128) k_cut_merge(const uint32_t* __restrict__ 
 // Group (w, g): buckets j = gK .. gK + K - 1 of window w (bucket number j + 1): T = sum S_j,
 // R = sum (j - gK + 1) S_j, by running sums from the top. Two quads a group: one adds the buckets up
 // (T), the other, one step behind, adds the T's up (R), so a step of both is one addition's latency.
-// off == null: every bucket present.
+// off == null: every bucket present. A narrow window has half the buckets; its missing groups are stored as
+// the identity.
 template <class C>
 __global__ void __launch_bounds__(128) k_bucket_rs(const MReqs Q, uint32_t ngroups, const uint32_t* __restrict__ bsum,
                                                    const uint32_t* __restrict__ off, uint32_t* __restrict__ Tout,
@@ -305,7 +306,6 @@ __global__ void __launch_bounds__(128) k_bucket_rs(const MReqs Q, uint32_t ngrou
   if (live) quad_store((upper ? Rout : Tout) + (size_t)t * XW, a);
 }
 
-// A narrow window's missing groups are stored as the identity above.
 // Block (w, k): k < gbits: 2^k K times the sum of the T_g with bit k of g set; k == gbits: sum R_g.
 // The window's last block to finish adds its gbits + 1 terms up: the window's value, canonical. done:
 // finished blocks a window (zeroed with the histogram). Block size: four rounds of its quads, up to

@@ -4,8 +4,8 @@
 // add nothing), so a level is one list of pairs: slot q of level l + 1 is the sum of elements 2q and
 // 2q + 1 of level l, and a segment's range is its first one shifted right by l. No slot needs to know
 // its segment (walking segment boundaries with two cursors a thread, each step waiting for offsets,
-// left the product pipes half idle: 6.1 ms for the first level at 2^22 points of BN254, now 5.6: forward
-// 1.37 at 5.7 TB/s of DRAM, inversions 0.16, backward 4.08 bound by the products' issue), and threads take slots a block's width apart, so entries, running products and sums are read and
+// left the product pipes half idle: 6.1 ms for the first level at 2^22 points of BN254, now 5.0: forward
+// 1.32 at 5.7 TB/s of DRAM, inversions 0.08, backward 3.63 bound by the products' issue), and threads take slots a block's width apart, so entries, running products and sums are read and
 // written in full lines. An affine sum P0 + P1 needs one field inversion
 // (lambda = (y1 - y0) / (x1 - x0), or 3 x0^2 / (2 y0) when P0 = P1); a whole level shares its
 // inversions by Montgomery's simultaneous-inversion trick, so one addition costs six field

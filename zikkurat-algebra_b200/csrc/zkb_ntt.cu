@@ -1,4 +1,4 @@
-// NTT planning and entry points (kernels: zkb_ntt_kernels.cuh).
+// NTT planning and entry points (kernels: zkb_ntt_mat.cuh, zkb_ntt_kernels.cuh).
 //
 // Reference: lib/cbits/curves/poly/mont/bn128_poly_mont.c:418-473 (forward: recursive radix-2
 // decimation in time, twiddles g^j, natural order in and out) and :565-622 (inverse: recursive
@@ -20,8 +20,9 @@
 //     forward reads  x[in(c,t)],  in(c,t)  = (c mod 2^M') + ((c >> M') << (M'+k)) + (t << M')
 //     forward writes y[out(c,k1)], out(c,k1) = c + (k1 << (m-k)), times g^(((c mod 2^M')*k1) << s)
 // A CTA owns a tile of consecutive columns, so every global access is a run of consecutive
-// 32-byte elements. The tile lives in shared memory; each thread runs 3 butterfly stages at a
-// time on 8 elements held in registers.
+// 32-byte elements. From 2^9 elements on a pass is a matrix product on the tensor cores
+// (zkb_ntt_mat.cuh); below, and in a batch's persistent kernel, its tile lives in shared memory and each
+// thread runs 2 butterfly stages at a time on 4 elements held in registers.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -31,7 +31,7 @@
 //
 // Measured (B200, BN254, kernel time, against the tile form's product-bound passes): 2^12 67 -> 21 us,
 // 2^14 75 -> 23 us, 2^18 105 -> 50 us, 2^20 341 -> 141 us, 2^22 1.21 -> 0.48 ms, 2^24 5.03 -> 2.03 ms
-// forward, 5.07 -> 2.06 ms inverse. At 2^24 a pass without twiddles takes 275 us: 1.6 GB through L2 (A is
+// forward, 5.07 -> 2.05 ms inverse (2.05 to 2.37 over seven runs). At 2^24 a pass without twiddles takes 275 us: 1.6 GB through L2 (A is
 // read by two CTAs) at 5.8 TB/s, the tensor pipe half busy, HBM's floor 164 us; the pass with the twiddle
 // product 650 us, bound by its ~620 instructions an element at 96 registers and 16 warps. Ring slots of
 // four elements (16 KB): one barrier an element took 0.69 ms at 2^22. Forward stores: keeping kappa in
