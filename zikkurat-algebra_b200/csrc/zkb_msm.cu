@@ -624,12 +624,19 @@ static int ilog2_floor(uint64_t x) {
 // 14 / 15: 600000 4654 / 4630 / 4880 (picked 15), 700000 5321 / 5261 / 5394 (15), 800000 5811 / 5848 /
 // 5949 (14), 900000 6434 / 6446 / 6527 (14), 1000003 6999 / 7062 / 7061 (14), 2^20 7315 / 7342 / 7327
 // (15), 1.2 M 8321 / 8342 / 8257 (15): within 1% of the best from 800,000 on, 2 to 5% off below.
+// From 2^22 on the weight grows with n, so that the segments get longer instead of the windows wider: the
+// tree's gain rests on long segments (ms at 2^24 of BN254: c = 16 with the tree 46.5, c = 19 56 with it and
+// 48 without, c = 20 without 47.4; 2^25 of BLS12-381: 183, 191, 211, 201). Beyond 20 M points of BN254 the
+// tree's gathers of 1.3 GB of bases cost what it saves (20 M c = 16 with the tree 55, c = 20 without 56;
+// 25 M 70 and 69; 2^25 93 and 90), and without it wide windows are the cheaper ones.
+static constexpr int TREE_MAX_BN254 = 20000000;
 static double bucket_weight(int curve, int n) {
   const bool bls = curve == ZKG_BLS12_381;
+  if (!bls && n > TREE_MAX_BN254) return 2.8;
   if (n < (1 << 17)) return bls ? 3.5 : 2.8;
   if (n < (1 << 18)) return 5.0;
   if (n < (bls ? 800000 : 1 << 21)) return 8.0;
-  return bls ? 16.0 : 12.0;
+  return (bls ? 16.0 : 12.0) * std::max(1.0, n / 4194304.0);
 }
 static int auto_window(int n, int scalar_bits, double w) {
   if (n <= 1) return 2;
@@ -637,6 +644,7 @@ static int auto_window(int n, int scalar_bits, double w) {
   int bestc = 2;
   for (int c = 2; c <= 20; c++) {
     const int nwin = (scalar_bits + 1 + c - 1) / c;
+    if (c < 20 && (uint64_t)nwin * (uint64_t)n >= (1ull << 31)) continue;   // more entries than a launch has
     const double cost = (double)nwin * ((double)n + 4000.0) + w * (double)win_shape(scalar_bits + 1, nwin).seg(nwin);
     if (cost < best) { best = cost; bestc = c; }
   }
@@ -670,14 +678,14 @@ static int g_tree_env = env_int("ZKB_MSM_TREE", -1);
 static uint32_t g_tree_B = (uint32_t)std::max(0, env_int("ZKB_MSM_TREE_B", 0));   // 0: by e
 
 template <class C>
-static int pick_tree(uint64_t total, uint32_t nseg, int tuned) {
+static int pick_tree(int n, uint64_t total, uint32_t nseg, int tuned) {
   if constexpr (radix_conv_v<typename C::Fp>) {
     return 0;   // the tree's inversion works in the reference's radix
   } else {
     int k = g_tree_env >= 0 ? g_tree_env : tuned - 1;
     if (k < 0) {
       const uint64_t e = total / std::max<uint32_t>(1, nseg);
-      if (total < 8000000) return 0;
+      if (total < 8000000 || (C::Fp::N == 8 && n > TREE_MAX_BN254)) return 0;
       if (C::Fp::N == 8) k = e < 40 ? 0 : e < 92 ? 1 : e < 200 ? 2 : 3;
       else k = e < 28 ? 0 : e < 60 ? 1 : e < 200 ? 2 : 3;
     }
@@ -800,9 +808,10 @@ static uint32_t quad_chunk_len(uint64_t total) {
 
 // Entries the affine tree works on at a time: its lists and running products take about 64 bytes an entry
 // for BN254, 96 for BLS12-381 (four times the rest of an MSM's workspace), so beyond this many the windows
-// go in slabs: 2^24 points of BN254 take 10.3 GiB instead of 17.5, 2^26 19 instead of 64. Every slab has its
-// own last waves, so smaller ones cost time: 2^23 points 25.9 ms in one slab, 27.3 in two of 2^26 entries,
-// 28.9 in four; 2^24 53.4 in one, 55.7 in two, 56.3 in four.
+// go in slabs: 2^24 points of BN254 take 11.3 GiB in two, 18 in one, 2^26 of BLS12-381 24 instead of 96.
+// Every slab has its own last waves, so smaller ones cost time: 2^23 points of BN254 23.0 ms in one slab, 23.3
+// in two of 2^26 entries, 23.9 in four; 2^24 45.5 in one, 45.2 in two, 46.0 in four; BLS12-381 2^23 45.6,
+// 47.2, 48.7.
 static const uint64_t g_tree_slab = (uint64_t)std::max(1, env_int("ZKB_MSM_TREE_SLAB", 1 << 27));
 
 struct MsmPlan {
@@ -859,7 +868,7 @@ static zkg_status make_plan(int n, int nlimbs, int mont, MsmPlan& P, int c_force
   P.total_max = (uint64_t)P.nwin * (uint64_t)n;
   if (P.total_max >= (1ull << 31)) return set_status(ZKG_ERR_ARG, "msm", "too many (window, point) entries for one launch");
   const MsmTune& T = msm_tune(C::ID, round_log2((uint64_t)n));
-  P.tree = std::min(tree_max, pick_tree<C>(P.total_max, P.nseg, T.tree));
+  P.tree = std::min(tree_max, pick_tree<C>(n, P.total_max, P.nseg, T.tree));
   P.acc_total = P.total_max;
   P.slabs = 1;
   P.wslab = P.nwin;
