@@ -152,9 +152,8 @@ template <int NL>
 inline void mul_adx(const Field<NL>&, const uint64_t*, const uint64_t*, uint64_t*) {}
 #endif
 
-// Out of line: inlined beside the form above it costs the host tail 2% (the smallest MSMs' 2 us).
 template <int NL>
-__attribute__((noinline)) El<NL> mul_portable(const Field<NL>& F, const El<NL>& a, const El<NL>& b) {
+inline El<NL> mul_rows(const Field<NL>& F, const El<NL>& a, const El<NL>& b) {
   uint64_t t[NL + 2] = {0};
   for (int i = 0; i < NL; i++) {
     u128 c = 0;
@@ -183,6 +182,12 @@ __attribute__((noinline)) El<NL> mul_portable(const Field<NL>& F, const El<NL>& 
   reduce_once<NL>(F, r.v, t[NL]);
   return r;
 }
+// For four words the form without mulx stays out of line: inlined beside the other, it made the compiler's
+// choices for the host tail 2% slower or faster with every change of its callers.
+__attribute__((noinline)) inline El<4> mul_portable(const Field<4>& F, const El<4>& a, const El<4>& b) {
+  return mul_rows<4>(F, a, b);
+}
+inline El<6> mul_portable(const Field<6>& F, const El<6>& a, const El<6>& b) { return mul_rows<6>(F, a, b); }
 template <int NL>
 inline El<NL> mul(const Field<NL>& F, const El<NL>& a, const El<NL>& b) {
   if (has_mulx_adx()) {

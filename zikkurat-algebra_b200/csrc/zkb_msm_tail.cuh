@@ -174,42 +174,41 @@ __global__ void __launch_bounds__(128) k_quad_accum(const uint32_t* __restrict__
   const uint32_t t = (blockIdx.x * 128 + threadIdx.x) >> 2;
   const uint32_t total = __ldg(off + nseg);
   L = counted_len(total, nchunks, L);
-  const uint32_t start = t * L;
-  uint32_t end = start, s = 0, seg_lo = 0, seg_hi = 0;
-  if (t < nchunks && start < total) {
-    end = min(start + L, total);
-    s = find_seg(off, nseg, start);
-    seg_lo = __ldg(off + s);
+  uint32_t pos = t * L, end = pos, s = 0, seg_hi = 0;
+  bool cut = false;   // the run's segment began before the chunk
+  if (t < nchunks && pos < total) {
+    end = min(pos + L, total);
+    s = find_seg(off, nseg, pos);
+    cut = __ldg(off + s) < pos;
     seg_hi = __ldg(off + s + 1);
   }
   uint32_t keyA = INVALID, keyB = INVALID;
   // the next entry and its point are fetched while an addition runs
-  auto point = [&](uint32_t pos) {
-    const uint32_t e = pos < end ? __ldg(entries + pos) : NULL_ENTRY;
+  auto point = [&](uint32_t at) {
+    const uint32_t e = at < end ? __ldg(entries + at) : NULL_ENTRY;
     uint32_t i = e & 0x7fffffffu;
     const bool null = i == NULL_ENTRY;
     if (null) i = 0;
     if (chk && i >= npts) { atomicOr(chk, CHK_POINT); i = 0; }
     return fe_sel(null, fe_zero<F>(), quad_from_affine<F>(bases + (size_t)i * 2 * F::N, e >> 31));
   };
-  Fe<F> a = fe_zero<F>(), q = point(start);
+  Fe<F> a = fe_zero<F>(), q = point(pos);
   // the finished run of segment s: the whole segment to its bucket, a cut one to this chunk's slots
   auto flush = [&] {
-    const bool before = seg_lo < start, after = seg_hi > end;
-    if (before) keyA = s; else if (after) keyB = s;
-    quad_store(!before && !after ? bsum + (size_t)s * XW : spt + (size_t)(2 * t + (before ? 0 : 1)) * XW, a);
+    const bool after = seg_hi > end;
+    if (cut) keyA = s; else if (after) keyB = s;
+    quad_store(!cut && !after ? bsum + (size_t)s * XW : spt + (size_t)(2 * t + (cut ? 0 : 1)) * XW, a);
   };
   bool have = false;
 #pragma unroll 1
-  for (uint32_t i = 0; __any_sync(FULL, start + i < end); i++) {
-    const uint32_t pos = start + i;
+  for (; __any_sync(FULL, pos < end); pos++) {
     const Fe<F> nx = point(pos + 1);
     if (pos < end) {
       while (pos >= seg_hi) {
         if (have) { flush(); a = fe_zero<F>(); }
         have = false;
         s++;
-        seg_lo = seg_hi;
+        cut = false;
         seg_hi = __ldg(off + s + 1);
       }
       have = true;

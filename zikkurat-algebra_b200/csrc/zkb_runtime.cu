@@ -25,6 +25,11 @@ zkg_status set_status(zkg_status s, const char* where, const char* detail) {
   return s;
 }
 
+zkg_status allow_smem(const void* kernel, size_t bytes) {
+  ZKB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return ZKG_OK;
+}
+
 zkg_status Arena::reserve(size_t bytes) {
   if (bytes <= cap) return ZKG_OK;
   size_t free_bytes = 0, all = 0;   // what cannot fit is refused with the present buffer kept

@@ -150,12 +150,13 @@ int device_sm_count();
 // have is asked for on each launch: the limit belongs to the kernel on the current device, so a call
 // remembered once for the process leaves the second device's launches failing.
 static constexpr size_t SMEM_DEFAULT = 48 * 1024;
+zkg_status allow_smem(const void* kernel, size_t bytes);
 extern std::atomic<uint64_t> g_launches;
 template <typename... KArgs, typename... Args>
 inline zkg_status launch(const char* name, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
                          cudaStream_t st, Args... args) {
   if (grid.x == 0 || grid.y == 0 || grid.z == 0) return ZKG_OK;
-  if (smem > SMEM_DEFAULT) ZKB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > SMEM_DEFAULT) ZKB_TRY(allow_smem((const void*)kern, smem));
   kern<<<grid, block, smem, st>>>(args...);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   cudaError_t e = cudaGetLastError();
