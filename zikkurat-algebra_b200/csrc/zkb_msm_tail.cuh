@@ -242,10 +242,10 @@ __global__ void __launch_bounds__(128) k_cut_merge(const uint32_t* __restrict__ 
   if (t + 1 < nchunks) {
     const uint32_t total = __ldg(off + nseg);
     s = __ldg(skey + 2 * (size_t)t + 1);
-    L = counted_len(total, nchunks, L);
     if (chk && s != INVALID && s >= nseg) { atomicOr(chk, CHK_SEGMENT); s = INVALID; }
     if (s != INVALID) {
-      more = (__ldg(off + s + 1) - 1) / L - t;
+      const uint32_t last = __ldg(off + s + 1) - 1;   // on its way while the total is looked at
+      more = last / counted_len(total, nchunks, L) - t;
       if (more > RUN_MAX) {
         if (quad_lane() == 0) piece_push(P, s, t, more + 1);
         s = INVALID;
